@@ -277,6 +277,34 @@ __device__ __forceinline__ float warp_max(float v) {
     return v;
 }
 
+// Sums each of v[0 .. V - 1] over the lanes of a warp (V a power of two, up to 64).  Half of the values change sides at
+// every step, so the whole takes about V shuffles.  Lane l ends with max(1, V / 32) totals, v[0], ..., which are those of the
+// values base, base + 1, ...; `base` is returned.  With V < 32 several lanes hold the same one.
+template <int V>
+__device__ __forceinline__ int lane_totals(float (&v)[V], int lane) {
+    int base = 0;
+    int n = V;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        if (n > 1) {
+            const int half = n >> 1;
+            const bool up = (lane & off) != 0;
+#pragma unroll
+            for (int i = 0; i < V / 2; ++i) {
+                if (i < half) {
+                    const float send = up ? v[i] : v[i + half], keep = up ? v[i + half] : v[i];
+                    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+                }
+            }
+            base += up ? half : 0;
+            n = half;
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
+        }
+    }
+    return base;
+}
+
 // Sum over a block of up to 1024 threads; every thread gets the result.
 // `scratch` holds 33 floats.  The order of additions is fixed, so the result
 // does not depend on anything but the inputs.

@@ -3,7 +3,7 @@
 Each ``csrc/<name>.cu`` becomes ``csrc/_build/lib<name>.so``: compiled with
 nvcc for sm_100a the first time something needs it (or when its source
 changed), then loaded with ctypes.  A model only builds what it uses: the
-float32 path needs ``generic`` alone.  There is no fallback: if a library
+float32 path needs ``generic``, ``linear_f32`` and ``attention_f32``.  There is no fallback: if a library
 cannot be built or loaded the call raises ``ExtensionError``.
 """
 from __future__ import annotations
@@ -25,7 +25,8 @@ from ..errors import ExtensionError
 CSRC = Path(__file__).resolve().parent.parent / "csrc"
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
               "-Xcompiler", "-fPIC", "-shared"]
-LIBRARIES = ("generic", "gemm_sm100", "linear_skinny", "attention_mma", "attention_tc", "recurrent", "state_space")
+LIBRARIES = ("generic", "gemm_sm100", "linear_skinny", "attention_mma", "attention_tc", "recurrent", "state_space",
+             "linear_f32", "attention_f32")
 
 _loaded: Dict[str, ctypes.CDLL] = {}
 _lock = threading.Lock()

@@ -42,6 +42,11 @@ def _ptr(t: Optional[torch.Tensor]):
     raise InvalidArgument("kernels take contiguous tensors")
 
 
+def _aligned(t) -> bool:
+    """Whether a tensor starts on a 16-byte boundary (a shape-only one counts as if it did)."""
+    return t.is_meta or t.data_ptr() % 16 == 0
+
+
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
@@ -110,7 +115,7 @@ def launch_overlap(on: bool) -> None:
     tensor-core products (their set-up; up to 64 tokens also their first weight tiles), prefill attention (its
     set-up) and the norms between them.
     On by default; off, every kernel waits for the one before it to be over, and the results are the same bits."""
-    for name in ("linear_skinny", "gemm_sm100", "generic", "attention_tc"):
+    for name in ("linear_skinny", "gemm_sm100", "generic", "attention_tc", "linear_f32"):
         getattr(library.load(name), f"nncpu_launch_overlap_{name}")(ctypes.c_int(1 if on else 0))
 
 
@@ -268,6 +273,28 @@ def linear_simt(x, w, bias, out, accumulate: bool = False) -> None:
     assert w.shape[1] == k and out.shape == (m, n)
     _call("generic", "nncpu_linear_simt", _ptr(x), _i(_code(x)), _ptr(w), _i(_code(w)), _ptr(bias),
           _i(_code(bias)), _ptr(out), _i(_code(out)), _i(m), _i(n), _i(k), _i(k), _i(n), _i(accumulate), _stream())
+
+
+LINEAR_F32_MAX_TOKENS = 16
+# From how many weights on a product of float32 runs goes to ``linear_f32``.  Below, ``linear_simt`` adds every element over
+# ascending k for any number of rows, so a small model gives the same bits for portions and for whole prompts; what that costs
+# there is mostly launches (see ``linear_f32.cu`` for both kernels' times at this line).
+LINEAR_F32_MIN_WEIGHTS = 1 << 20
+
+
+def linear_f32_supported(x, w) -> bool:
+    """Whether ``linear_f32`` takes this product: few rows of float32, of whole 16-byte pieces, on both sides."""
+    return (x.dtype == torch.float32 and w.dtype == torch.float32 and 0 < x.shape[0] <= LINEAR_F32_MAX_TOKENS
+            and x.shape[1] % 4 == 0 and _aligned(x) and _aligned(w))
+
+
+def linear_f32(x, w, bias, out, accumulate: bool = False) -> None:
+    """out (+)= x . w^T + bias for at most 16 rows, in true 32-bit: a stream over the weights on CUDA cores."""
+    m, k = x.shape
+    n = w.shape[0]
+    assert w.shape[1] == k and out.shape == (m, n) and x.dtype == w.dtype == torch.float32
+    _call("linear_f32", "nncpu_linear_f32", _ptr(x), _ptr(w), _ptr(bias), _i(_code(bias)), _ptr(out), _i(_code(out)),
+          _i(m), _i(n), _i(k), _i(k), _i(n), _i(accumulate), _stream())
 
 
 def linear_tc_supported(m: int, n: int, k: int) -> bool:
@@ -591,6 +618,49 @@ def attention(q, k_pages, v_pages, block_table, tok_seq, tok_pos, out, n_heads: 
           _ptr(block_table), _i(block_table.shape[1]), _ptr(tok_seq), _ptr(tok_pos), _ptr(out), _i(_code(out)),
           _i(n), _i(n_heads), _i(n_kv), _i(head_dim), _i(v_head_dim), _i(v_lanes), _f(scale), _i(window), _i(keep),
           _f(slope_base), _ptr(sinks), _f(cap), *_head_gate(head_gate, n, n_heads), _stream())
+
+
+ATTENTION_F32_STRETCH = 128         # keys of a stretch: one round of a block of the token-by-token kernel
+
+
+def attention_f32_supported(q, k_pages, v_pages, out, n_heads: int, n_kv: int, head_dim: int, v_head_dim: int, v_lanes: int) -> bool:
+    """The 32-bit attention kernels for heads of at most 128 lanes (rows of whole 16-byte pieces, float32 throughout)."""
+    return (all(t.dtype == torch.float32 and _aligned(t) for t in (q, k_pages, v_pages, out)) and n_kv > 0
+            and n_heads % n_kv == 0 and n_heads // n_kv <= 32
+            and all(0 < d <= 128 and d % 4 == 0 for d in (head_dim, v_head_dim, v_lanes)) and v_lanes <= v_head_dim)
+
+
+def attention_f32_plan(n_tokens: int, is_decode: bool, longest: int):
+    """(keys of a stretch, stretches of the longest sequence) for the token-by-token kernel, or (0, 0) for the kernel of
+    whole prompts.  Token by token where the step is a decode step, and for a prompt of up to 16 tokens: as one
+    tile of query rows it would walk through its keys on a handful of SMs.  A sequence of up to 4 096 keys (1 024 in a step of
+    more than 64 tokens, which has blocks enough) is cut every 128 keys whatever else the step holds; beyond, the
+    stretches grow, so that there are at most 32 (8) to keep room for and to add up."""
+    if not is_decode and n_tokens > LINEAR_F32_MAX_TOKENS:
+        return 0, 0
+    chunk = ATTENTION_F32_STRETCH
+    while longest > chunk * (32 if n_tokens <= 64 else 8):
+        chunk *= 2
+    return chunk, max(1, (longest + chunk - 1) // chunk)
+
+
+def attention_f32(q, k_pages, v_pages, block_table, tok_seq, tok_pos, out, scratch, n_heads: int, n_kv: int, head_dim: int,
+                  scale: float, plan, sm_count: int, window: int = 0, v_head_dim: int = 0, slope_base: float = 0.0, sinks=None,
+                  keep: int = 0, v_lanes: int = 0, cap: float = 0.0, head_gate=None) -> None:
+    """``attention`` for float32 heads of at most 128 lanes.  ``plan`` is ``attention_f32_plan``'s; with more than one
+    stretch ``scratch`` holds n * n_heads * stretches * (v_head_dim + 2) floats."""
+    n = q.shape[0]
+    v_head_dim = v_head_dim or head_dim
+    v_lanes = v_lanes or v_head_dim
+    chunk, n_chunks = plan
+    assert q.shape == (n, n_heads * head_dim) and out.shape == (n, n_heads * v_lanes)
+    assert (keep == 0 or window > 0) and block_table.dtype == torch.int32
+    assert n_chunks <= 1 or scratch.numel() >= n * n_heads * n_chunks * (v_head_dim + 2)
+    assert sinks is None or (sinks.dtype == torch.float32 and sinks.numel() == n_heads)
+    _call("attention_f32", "nncpu_attention_f32", _ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(block_table),
+          _i(block_table.shape[1]), _ptr(tok_seq), _ptr(tok_pos), _ptr(out), _ptr(scratch), _i(n), _i(n_heads), _i(n_kv),
+          _i(head_dim), _i(v_head_dim), _i(v_lanes), _f(scale), _i(window), _i(keep), _f(slope_base), _ptr(sinks), _f(cap),
+          *_head_gate(head_gate, n, n_heads), _i(chunk), _i(n_chunks), _i(sm_count), _stream())
 
 
 def attention_mma_supported(n_heads: int, n_kv: int, head_dim: int, *tensors) -> bool:

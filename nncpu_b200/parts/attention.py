@@ -312,10 +312,19 @@ class Attention(Mixer):
     def _attend(self, ctx, q, cache, attn, head_gate=None):
         """bfloat16 with a head size the tensor-core kernels take: split-key
         decode, tcgen05 prefill for prompts, mma.sync prefill for a few tokens
-        per sequence; everything else: the 32-bit kernel."""
+        per sequence; float32 heads of at most 128 lanes: the 32-bit kernels made for them; everything else: the general one."""
         s, extra = self.spec, {"keep": self.spec.keep_first, "v_lanes": self.v_dim, "cap": self.spec.score_cap,
                                "head_gate": head_gate}
         if not (self._tensor_core_rows() and ops.attention_mma_supported(s.n_heads, s.n_kv_heads, self.k_row, q, cache.k_pages, attn)):
+            if ops.attention_f32_supported(q, cache.k_pages, cache.v_pages, attn, s.n_heads, s.n_kv_heads, self.k_row, self.v_row,
+                                           self.v_dim):
+                plan = ops.attention_f32_plan(ctx.n_tokens, ctx.is_decode, ctx.max_kv_len)
+                scratch = (self.rt.empty(ctx.n_tokens * s.n_heads * plan[1] * (self.v_row + 2), dtype=torch.float32)
+                           if plan[1] > 1 else None)
+                ops.attention_f32(q, cache.k_pages, cache.v_pages, cache.block_table, ctx.tok_seq, ctx.tok_pos, attn, scratch,
+                                  s.n_heads, s.n_kv_heads, self.k_row, s.scale, plan, self.rt.sm_count, self.span, self.v_row,
+                                  s.slope_base, self.sinks, **extra)
+                return
             ops.attention(q, cache.k_pages, cache.v_pages, cache.block_table, ctx.tok_seq, ctx.tok_pos, attn,
                           s.n_heads, s.n_kv_heads, self.k_row, s.scale, self.span, self.v_row, s.slope_base, self.sinks,
                           **extra)

@@ -196,7 +196,9 @@ class Runtime:
                 then_norm.result = made
         else:
             assert epilogue == "plain" and activation is None, "fused epilogues exist on the tensor-core path only"
-            ops.linear_simt(x, w, bias, out, accumulate)
+            # small layers stay with the kernel whose sums have one order for every number of rows: see the constant
+            fast = w.numel() >= ops.LINEAR_F32_MIN_WEIGHTS and ops.linear_f32_supported(x, w)
+            (ops.linear_f32 if fast else ops.linear_simt)(x, w, bias, out, accumulate)
 
     def fuses_norms(self, n_tokens: int, n_out: int) -> bool:
         """Whether the bfloat16 products of a step of ``n_tokens`` rows (``n_out`` output features) may carry the norms

@@ -1,0 +1,116 @@
+"""The kernels of true float32 runs: the product of a few tokens, and attention over float32 pages, against 64-bit sums and
+against the general kernels."""
+from __future__ import annotations
+
+import math
+
+import pytest
+import torch
+
+from gpu_util import DEV, check, scatter_pages
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from nncpu_b200.kernels import ops
+    return ops
+
+
+def bound(x, w, extra=4):
+    """Largest error that a 32-bit sum of k products in any order may have: (k + extra) roundings of 2^-24 of the sum of the
+    products' magnitudes."""
+    return (x.shape[1] + extra) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 8, 9, 16])
+@pytest.mark.parametrize("n,k", [(1, 4), (7, 124), (64, 128), (37, 132), (130, 516), (96, 2048), (33, 6144)])
+def test_few_token_product(ops, m, n, k):
+    g = torch.Generator(device=DEV).manual_seed(m * n + k)
+    x, w, b = (torch.randn(s, generator=g, device=DEV) for s in ((m, k), (n, k), (n,)))
+    assert ops.linear_f32_supported(x, w)
+    want, tol = x.double() @ w.double().T, bound(x, w) + 1e-6
+    out = torch.full((m, n), 7.0, device=DEV)
+    ops.linear_f32(x, w, b, out)
+    assert ((out - (want + b)).abs() <= tol + b.abs() * 2.0 ** -23).all()
+    ops.linear_f32(x, w, None, out, accumulate=True)
+    assert ((out - (2 * want + b)).abs() <= 3 * tol + b.abs() * 2.0 ** -22).all()
+    half = torch.empty(m, n, dtype=torch.bfloat16, device=DEV)
+    ops.linear_f32(x, w, b.bfloat16(), half)
+    assert ((half - (want + b.bfloat16())).abs() <= tol + 2.0 ** -8 * (want + b.bfloat16()).abs()).all()
+    # a row's result does not depend on the rows beside it
+    one = torch.empty(1, n, device=DEV)
+    many = torch.empty(16, n, device=DEV)
+    ops.linear_f32(x[m - 1:].contiguous(), w, None, one)
+    ops.linear_f32(x[m - 1:].expand(16, k).contiguous(), w, None, many)
+    assert torch.equal(one.expand(16, n), many)
+
+
+def test_few_token_product_of_other_forms_stays_general(ops):
+    x, w = torch.randn(4, 128, device=DEV), torch.randn(8, 128, device=DEV)
+    assert not ops.linear_f32_supported(x.bfloat16(), w) and not ops.linear_f32_supported(x, w.bfloat16())
+    assert not ops.linear_f32_supported(x[:, :126].contiguous(), w[:, :126].contiguous())
+    shifted = torch.randn(8 * 128 + 1, device=DEV)[1:].view(8, 128)
+    assert not ops.linear_f32_supported(x, shifted)
+
+
+def run_attention(ops, q, kp, vp, table, tok_seq, tok_pos, nh, nkv, hd, vd, vo, plan, **how):
+    out = torch.full((q.shape[0], nh * vo), 9.0, device=DEV)
+    scratch = torch.full((q.shape[0] * nh * plan[1] * (vd + 2),), float("nan"), device=DEV) if plan[1] > 1 else None
+    ops.attention_f32(q, kp, vp, table, tok_seq, tok_pos, out, scratch, nh, nkv, hd, 1 / math.sqrt(hd), plan, 148,
+                      v_head_dim=vd, v_lanes=vo, **how)
+    return out
+
+
+@pytest.mark.parametrize("nh,nkv,hd,vd,vo", [(4, 4, 128, 128, 128), (2, 1, 64, 64, 64), (6, 2, 16, 36, 20), (4, 1, 128, 64, 64),
+                                             (16, 2, 4, 4, 4), (9, 1, 100, 128, 100), (32, 1, 48, 48, 48)])
+@pytest.mark.parametrize("how", [dict(), dict(window=50), dict(window=70, keep=5), dict(window=-64), dict(slope_base=8.0),
+                                 dict(cap=5.0), dict(sinks=True), dict(head_gate=True)], ids=str)
+def test_attention_against_the_general_kernel(ops, nh, nkv, hd, vd, vo, how):
+    """Token by token, in every cut of the keys, and in tiles of query rows: lengths at the edges of pages and stretches,
+    portions behind a past, a padding row.  Both kernels' softmax weights and sums are 32-bit; 700 keys leave 2e-5 at most."""
+    seqs = [700, 1, 64, 65, 128, 129, 300]
+    kp, _, table, _, _ = scatter_pages(32, nkv, hd, seqs, torch.float32, seed=hd)
+    vp, _, _, _, _ = scatter_pages(32, nkv, vd, seqs, torch.float32, seed=hd)
+    g = torch.Generator().manual_seed(nh)
+    # the last tokens of every sequence, in order; a padding row between two of them
+    tok = [(0, p) for p in range(663, 700)] + [(1, 0)] + [(2, p) for p in range(64)] + [(3, 64), (-1, 3)] + \
+        [(4, p) for p in range(120, 128)] + [(5, 127), (5, 128)] + [(6, p) for p in range(300)]
+    tok_seq = torch.tensor([t[0] for t in tok], dtype=torch.int32, device=DEV)
+    tok_pos = torch.tensor([t[1] for t in tok], dtype=torch.int32, device=DEV)
+    q = torch.randn(len(tok), nh * hd, generator=g).to(DEV)
+    how = dict(how)
+    if how.get("sinks"):
+        how["sinks"] = torch.randn(nh, generator=g).to(DEV)
+    if how.get("head_gate"):
+        how["head_gate"] = (torch.randn(len(tok), nh + 3, generator=g).to(DEV), 2)
+    want = torch.empty(len(tok), nh * vo, device=DEV)
+    ops.attention(q, kp, vp, table, tok_seq, tok_pos, want, nh, nkv, hd, 1 / math.sqrt(hd), v_head_dim=vd, v_lanes=vo, **how)
+    assert ops.attention_f32_supported(q, kp, vp, want, nh, nkv, hd, vd, vo)
+    for plan in ((0, 0), (128, 6), (256, 3), (1024, 1)):
+        got = run_attention(ops, q, kp, vp, table, tok_seq, tok_pos, nh, nkv, hd, vd, vo, plan, **how)
+        check(got, want, 2e-5, f"plan {plan}")
+        assert float(got[tok_seq < 0].abs().sum()) == 0.0
+
+
+def test_attention_keeps_to_what_a_query_sees(ops):
+    """Infinities in the values of keys that a query does not see, in its own tile and page, stay out of its output; a row's bits
+    do not depend on the rows beside it."""
+    nh, nkv, hd, n = 4, 1, 128, 90
+    kp, vp, table, _, _ = scatter_pages(4, nkv, hd, [n], torch.float32, seed=1)
+    q = torch.randn(n, nh * hd, generator=torch.Generator().manual_seed(2)).to(DEV)
+    seq, pos = torch.zeros(n, dtype=torch.int32, device=DEV), torch.arange(n, dtype=torch.int32, device=DEV)
+    args = (nh, nkv, hd, hd, hd)
+    clean = {plan: run_attention(ops, q, kp, vp, table, seq, pos, *args, plan) for plan in ((0, 0), (128, 1))}
+    for at in (5, 70):
+        page = int(table[0, at // 64])
+        dirty = vp.clone()
+        dirty[page, 0, at % 64, 3] = math.inf
+        for plan, want in clean.items():
+            got = run_attention(ops, q, kp, dirty, table, seq, pos, *args, plan)
+            assert torch.equal(got[:at], want[:at]) and torch.isinf(got[at:].view(-1, nh, hd)[:, :, 3]).all()
+    for plan, want in clean.items():
+        for t in (0, 63, 64, 89):
+            one = run_attention(ops, q[t:t + 1], kp, vp, table, seq[t:t + 1].clone(), pos[t:t + 1].clone(), *args, plan)
+            assert torch.equal(one[0], want[t])
