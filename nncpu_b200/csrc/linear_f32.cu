@@ -11,6 +11,13 @@
 // An element is summed over k in an order that K alone decides (per lane ascending, then the lanes' tree, then the
 // four warps), so a row's result does not depend on how many tokens the step has, up to the 16.
 //
+// More tokens: the tensor cores, on numbers cut in two.  x = h + l with h the nearest tf32 number (11 bits); the rest l is at most
+// 2^11 of x's last places, so it is a tf32 number too and nothing is lost.  w . x = h h' + h l' + l h' (l l' is below 2^-24 of
+// the product), all three accumulated in 32-bit by tcgen05.mma kind::tf32.  The tensor core does not round its running
+// sum to nearest, so it only sums 64 columns at a time; these sums are added in registers, with float additions.  Against
+// 64-bit sums the result is as near as the CUDA cores' chain of fmaf or nearer (figures at f32_many_kernel).
+// Weights are the 128-row operand and tokens the other one (BN of them), K may be cut into slices that a second kernel adds.
+//
 // The reference computes these products with its float row kernels (crates/nncpu/src/kernels/mod.rs:337-360).
 
 #include <math.h>
@@ -18,6 +25,7 @@
 #define NN_LIB linear_f32
 #define NN_LAUNCH_OVERLAP
 #include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace {
 
@@ -113,6 +121,384 @@ cudaError_t launch_few(const float* X, const float* W, const void* bias, int bia
     return cudaLaunchKernelEx(&cfg, f32_few_kernel<MT, WR>, X, W, bias, bias_dt, C, c_dt, M, N, K, lda, ldc, accumulate);
 }
 
+// ---------------------------------------------------------------------------
+// More tokens.
+//
+// A block's warps: 0 copies tiles of 32 columns to shared memory by TMA, 1 issues the matrix instructions, 2-7 cut what arrived into h (in its place) and l (behind it), 8-15 add the sums of 64 columns that
+// tensor memory holds in turn to their registers (two warps per quarter of the lanes, half of the tokens each) and store.
+// The adders take registers over from the others: 2 x 72 + 2 x 184 a warpgroup's thread, the 4 x 128 of the launch.
+//
+// Bound by shared memory: per k-block a block moves its (128 + BN) x 128 bytes seven times through it (in by TMA, out and
+// twice in by the cutters, three times out to the tensor core), 128 bytes a cycle, which takes longer than the matrix
+// instructions themselves up to BN 256; so BN is as large as the tokens and the two accumulators of tensor memory allow.
+// Measured (weights from memory): N 12288, K 2048, 300 tokens 143 us, 2 048 tokens 644 us (160 TFLOP/s of true 32-bit results,
+// where the CUDA cores' peak is 72); N 2048, K 6144, 300 tokens 63 us.  A layer of 300 tokens (hidden
+// 2048): 279 us for its four products, 3 130 us in the general kernel.
+// Error against 64-bit sums (2-norm, N(0, 1) times N(0, 0.02)), here / the general kernel's chain of fmaf: K 2048 4.7e-7 / 8.1e-7,
+// K 6144 4.8e-7 / 1.4e-6.  Cutting with six warps and integer rounding instead of four and cvt.rna, and asking the
+// weights into L2 eight k-blocks ahead, took 12 % off.
+// ---------------------------------------------------------------------------
+constexpr int kManyThreads = 16 * 32;
+constexpr int kCutters = 6;            // warps 2 to 7
+constexpr int kManyRegsFew = 72, kManyRegsMany = 184;
+static_assert(2 * kManyRegsFew + 2 * kManyRegsMany <= 4 * 128, "no more registers than the launch has");
+constexpr int kManyK = 32;             // columns of a k-block: 128 bytes, one swizzle row
+constexpr int kManyFlush = 2;          // k-blocks that the tensor core sums by itself
+constexpr int kManyAhead = 8;          // k-blocks of weights that are asked into L2 ahead of their copies
+
+struct ManyParams {
+    const float* x;       // for results that are not finite: see below
+    const float* w;
+    const void* bias;
+    int bias_dt;
+    void* out;
+    int out_dt;
+    float* part;          // slices > 1: [slices, M, N]
+    int M, N, K, lda, ldc, accumulate;
+    int tiles_a, tiles_b, slices, kb_total;
+    int* status;
+};
+
+__device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n"
+        "}\n" ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+// The nearest number of 11 bits (halves away from zero), in two integer instructions at full rate.  The sum may carry into the
+// exponent, as it should, up to infinity; of a NaN it may make a number, and x minus that is the NaN again.
+__device__ __forceinline__ float nearest_tf32(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u); }
+
+// Asks for a tile to come to L2.
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"((uint64_t)map), "r"(x), "r"(y) : "memory");
+}
+
+// One result in plain float arithmetic over its slice of K: what a sum that is not finite is replaced by, because the cut
+// of an infinity, or of a number next to the largest, is not a number (inf - inf) where the product itself may be one.
+__device__ __noinline__ float plain_dot(const float* x, const float* w, int n) {
+    float a = 0.0f;
+    for (int k = 0; k < n; ++k) a = fmaf(x[k], w[k], a);
+    return a;
+}
+
+template <int BN>
+constexpr int kManyStages = BN > 160 ? 2 : (BN > 96 ? 3 : 4);     // as many as shared memory holds
+template <int BN>
+constexpr size_t kManySmem = 1024 + (size_t)kManyStages<BN> * 2 * (128 + BN) * 128 + 256;
+
+template <int BN>
+__global__ void __launch_bounds__(kManyThreads, 1)
+f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const ManyParams p) {
+    constexpr int kStages = kManyStages<BN>;
+    constexpr int kHalfBytes = (128 + BN) * 128;      // the h (or l) parts of a k-block: 128 rows of weights, BN of tokens
+    constexpr int kStageBytes = 2 * kHalfBytes;
+    constexpr int kTmemCols = BN <= 32 ? 64 : (BN <= 64 ? 128 : (BN <= 128 ? 256 : 512));     // two accumulators
+    constexpr int kCols = BN / 2;                     // columns of an adding thread
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint64_t* full = (uint64_t*)(smem + kStages * kStageBytes);
+    uint64_t* cut = full + kStages;
+    uint64_t* empty = cut + kStages;
+    uint64_t* acc_full = empty + kStages;   // [2]
+    uint64_t* acc_empty = acc_full + 2;     // [2]
+    uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    let_next_kernel_start();
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kStages; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&cut[s], kCutters);
+            mbar_init(&empty[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&acc_full[b], 1);
+            mbar_init(&acc_empty[b], 8);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kTmemCols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = *tmem_slot;
+    wait_for_previous_kernels();
+
+    const int tiles = p.tiles_a * p.tiles_b, n_items = tiles * p.slices;
+    // item i: the tiles of tokens of one tile of weights stand together, so that its weights are read from memory once
+    auto first_kb = [&](int slice) { return (int)((long)slice * p.kb_total / p.slices); };
+
+    if (warp < 8) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kManyRegsFew));
+        if (warp == 0 && lane == 0) {
+            int run = 0;
+            bool ok = true;
+            for (int i = blockIdx.x; i < n_items && ok; i += gridDim.x) {
+                const int n0 = (i % p.tiles_b) * BN, m0 = (i / p.tiles_b % p.tiles_a) * 128, slice = i / tiles;
+                for (int kb = first_kb(slice); kb < first_kb(slice + 1); ++kb, ++run) {
+                    const int s = run % kStages;
+                    if (!mbar_wait(&empty[s], ((run / kStages) & 1) ^ 1)) {
+                        atomicExch(p.status, 201);
+                        ok = false;
+                        break;
+                    }
+                    mbar_expect_tx(&full[s], kHalfBytes);     // (rows past the end are filled with zeros and counted)
+                    if (kb + kManyAhead < first_kb(slice + 1)) tma_prefetch_2d(&map_w, (kb + kManyAhead) * kManyK, m0);
+                    tma_load_2d(smem + s * kStageBytes, &map_w, &full[s], kb * kManyK, m0);
+                    tma_load_2d(smem + s * kStageBytes + 128 * 128, &map_x, &full[s], kb * kManyK, n0);
+                }
+            }
+            // let the copies in flight land before the block gives up its shared memory
+            if (!ok)
+                for (int r = max(0, run - kStages); r < run; ++r) mbar_wait(&full[r % kStages], (r / kStages) & 1);
+        }
+        if (warp == 1 && lane == 0) {
+            // 32-bit accumulator, tf32 operands, both K-major
+            constexpr uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+            int run = 0, sum = 0;
+            bool ok = true;
+            for (int i = blockIdx.x; i < n_items && ok; i += gridDim.x) {
+                const int slice = i / tiles, kb0 = first_kb(slice), kb1 = first_kb(slice + 1);
+                for (int kb = kb0; kb < kb1; ++kb, ++run) {
+                    const int s = run % kStages, nth = (kb - kb0) % kManyFlush;
+                    if (nth == 0 && !mbar_wait(&acc_empty[sum & 1], ((sum >> 1) & 1) ^ 1)) {
+                        atomicExch(p.status, 202);
+                        ok = false;
+                        break;
+                    }
+                    if (!mbar_wait(&cut[s], (run / kStages) & 1)) {
+                        atomicExch(p.status, 203);
+                        ok = false;
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t d = tmem_base + (uint32_t)((sum & 1) * BN);
+                    const uint32_t wh = smem_u32(smem + s * kStageBytes), xh = wh + 128 * 128;
+                    const uint32_t wl = wh + kHalfBytes, xl = xh + kHalfBytes;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {             // 8 columns an instruction
+                        umma_tf32(d, smem_desc_sw128(wl + k * 32), smem_desc_sw128(xh + k * 32), idesc, (nth > 0 || k > 0) ? 1u : 0u);
+                        umma_tf32(d, smem_desc_sw128(wh + k * 32), smem_desc_sw128(xl + k * 32), idesc, 1u);
+                        umma_tf32(d, smem_desc_sw128(wh + k * 32), smem_desc_sw128(xh + k * 32), idesc, 1u);
+                    }
+                    umma_commit(&empty[s]);
+                    if (nth == kManyFlush - 1 || kb + 1 == kb1) {
+                        umma_commit(&acc_full[sum & 1]);
+                        ++sum;
+                    }
+                }
+            }
+        }
+        if (warp >= 2) {
+            const int tid = threadIdx.x - 64;
+            int run = 0;
+            bool ok = true;
+            for (int i = blockIdx.x; i < n_items && ok; i += gridDim.x) {
+                const int slice = i / tiles, n_kb = first_kb(slice + 1) - first_kb(slice);
+                for (int kb = 0; kb < n_kb; ++kb, ++run) {
+                    const int s = run % kStages;
+                    if (!mbar_wait(&full[s], (run / kStages) & 1)) {
+                        if (lane == 0) atomicExch(p.status, 204);
+                        ok = false;
+                        break;
+                    }
+                    float4* h = reinterpret_cast<float4*>(smem + s * kStageBytes);
+                    float4* l = reinterpret_cast<float4*>(smem + s * kStageBytes + kHalfBytes);
+#pragma unroll 4
+                    for (int e = tid; e < kHalfBytes / 16; e += kCutters * 32) {
+                        const float4 v = h[e];
+                        float4 hi, lo;
+                        hi.x = nearest_tf32(v.x); hi.y = nearest_tf32(v.y); hi.z = nearest_tf32(v.z); hi.w = nearest_tf32(v.w);
+                        lo.x = v.x - hi.x; lo.y = v.y - hi.y; lo.z = v.z - hi.z; lo.w = v.w - hi.w;
+                        h[e] = hi;
+                        l[e] = lo;
+                    }
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&cut[s]);
+                }
+            }
+        }
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kManyRegsMany));
+        const int quarter = warp & 3, half = (warp - 8) >> 2;     // the lanes and the columns that this warp adds up
+        const int row_in_tile = quarter * 32 + lane;
+        int sum = 0;
+        bool ok = true;
+        for (int i = blockIdx.x; i < n_items && ok; i += gridDim.x) {
+            const int n0 = (i % p.tiles_b) * BN + half * kCols, m0 = (i / p.tiles_b % p.tiles_a) * 128, slice = i / tiles;
+            const int kb0 = first_kb(slice), kb1 = first_kb(slice + 1);
+            float acc[kCols];
+#pragma unroll
+            for (int c = 0; c < kCols; ++c) acc[c] = 0.0f;
+            for (int kb = kb0; kb < kb1; kb += kManyFlush, ++sum) {
+                if (!mbar_wait(&acc_full[sum & 1], (sum >> 1) & 1)) {
+                    if (lane == 0) atomicExch(p.status, 205);
+                    ok = false;
+                    break;
+                }
+                __syncwarp();
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((sum & 1) * BN + half * kCols);
+#pragma unroll
+                for (int c = 0; c < kCols; c += 16) {
+                    float v[16];
+                    tmem_ld16(taddr + (uint32_t)c, v);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) acc[c + j] += v[j];
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&acc_empty[sum & 1]);
+            }
+            const int row = m0 + row_in_tile;
+            if (!ok || row >= p.N) continue;
+            const float b = p.slices == 1 && p.bias ? ld_f(p.bias, row, p.bias_dt) : 0.0f;
+            // the lanes of a warp write neighbouring features of a token
+#pragma unroll
+            for (int c0 = 0; c0 < kCols; c0 += 16) {
+                float old[16];
+#pragma unroll
+                for (int c = 0; c < 16; ++c) {       // all loads before the first store
+                    const int t = n0 + c0 + c;
+                    old[c] = p.slices == 1 && p.accumulate && t < p.M ? ld_f(p.out, (size_t)t * p.ldc + row, p.out_dt) : 0.0f;
+                }
+#pragma unroll
+                for (int c = 0; c < 16; ++c) {
+                    const int t = n0 + c0 + c;
+                    if (t >= p.M) break;
+                    float v = acc[c0 + c];
+                    if (!(fabsf(v) < INFINITY)) {
+                        const int k0 = kb0 * kManyK;
+                        v = plain_dot(p.x + (size_t)t * p.lda + k0, p.w + (size_t)row * p.K + k0, min(kb1 * kManyK, p.K) - k0);
+                    }
+                    if (p.slices == 1) st_f(p.out, (size_t)t * p.ldc + row, p.out_dt, (v + b) + old[c]);
+                    else p.part[((size_t)slice * p.M + t) * p.N + row] = v;
+                }
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
+    }
+}
+
+// Adds the slices' sums in their order, then bias and what is already there.
+__global__ void __launch_bounds__(256)
+f32_slices_kernel(const ManyParams p) {
+    let_next_kernel_start();
+    wait_for_previous_kernels();
+    const long total = (long)p.M * p.N;
+    const long e = ((long)blockIdx.x * 256 + threadIdx.x);
+    if (e >= total) return;
+    const int t = (int)(e / p.N), row = (int)(e % p.N);
+    float v = 0.0f;
+    for (int s = 0; s < p.slices; ++s) v += p.part[(size_t)s * total + e];
+    if (p.bias) v += ld_f(p.bias, row, p.bias_dt);
+    const size_t o = (size_t)t * p.ldc + row;
+    if (p.accumulate) v += ld_f(p.out, o, p.out_dt);
+    st_f(p.out, o, p.out_dt, v);
+}
+
+int sm_count() {
+    static int counts[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    if (counts[dev] == 0 && cudaDeviceGetAttribute(&counts[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        counts[dev] = 148;
+    return counts[dev];
+}
+
+// How a product is cut: tokens in equal tiles of at most 256 (a multiple of 32), K in slices.
+struct ManyPlan {
+    int bn, tiles_b, slices;
+};
+
+// The slices with the smallest sum of rounds of the SMs times k-blocks of a slice (six more for filling and draining a
+// block's pipeline), and the passes of the slices' sums through memory, in k-blocks too: one takes (128 + BN) x 7
+// cycles of shared memory; the sums pass at some 2 KB a cycle, and a launch costs 4 000 cycles.
+ManyPlan many_plan(int M, int N, int K) {
+    ManyPlan plan;
+    plan.tiles_b = (M + 255) / 256;
+    plan.bn = ((M + plan.tiles_b - 1) / plan.tiles_b + 31) / 32 * 32;
+    const int kb = (K + kManyK - 1) / kManyK, sms = sm_count();
+    const long tiles = (long)((N + 127) / 128) * plan.tiles_b;
+    const double per_kb = (128.0 + plan.bn) * 7.0;
+    plan.slices = 1;
+    double best = 0.0;
+    for (int s = 1; s <= 8 && (s == 1 || kb / s >= 8); ++s) {
+        const double rounds = (double)((tiles * s + sms - 1) / sms);
+        double cost = rounds * ((kb + s - 1) / s + 6);
+        if (s > 1) cost += (4000.0 + (double)s * M * N * 8.0 / 2048.0) / per_kb;
+        if (s == 1 || cost < best) {
+            best = cost;
+            plan.slices = s;
+        }
+    }
+    return plan;
+}
+
+// A [rows, K] float matrix with rows of `ld` floats, in boxes of box_rows x 32.
+int make_map_f32(CUtensorMap* map, const void* base, int rows, int K, long ld, int box_rows) {
+    EncodeTiledFn fn = encode_tiled();
+    NN_CHECK(fn != nullptr, "linear (32-bit): the driver does not offer cuTensorMapEncodeTiled");
+    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
+    const cuuint32_t box[2] = {(cuuint32_t)kManyK, (cuuint32_t)box_rows};
+    const cuuint32_t elem[2] = {1, 1};
+    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, elem,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    NN_CHECK(r == CUDA_SUCCESS, "linear (32-bit): cuTensorMapEncodeTiled failed with code %d (rows %d, K %d, ld %ld, box %d)", (int)r,
+             rows, K, ld, box_rows);
+    return 0;
+}
+
+template <int BN>
+int launch_many(const ManyParams& p, cudaStream_t stream) {
+    CUtensorMap mw, mx;
+    if (int e = make_map_f32(&mw, p.w, p.N, p.K, p.K, 128)) return e;
+    if (int e = make_map_f32(&mx, p.x, p.M, p.K, p.lda, BN)) return e;
+    constexpr size_t smem = kManySmem<BN>;
+    static_assert(smem <= 227 * 1024, "the stages fit shared memory");
+    static bool configured[64] = {};
+    if (first_use_on_this_device(configured)) {
+        const cudaError_t e = cudaFuncSetAttribute(f32_many_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        NN_CHECK(e == cudaSuccess, "linear (32-bit): cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
+    }
+    const long items = (long)p.tiles_a * p.tiles_b * p.slices;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(items < sm_count() ? items : sm_count()));
+    cfg.blockDim = dim3(kManyThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    cfg.numAttrs = overlap_attribute(attr);
+    cfg.attrs = attr;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, f32_many_kernel<BN>, mw, mx, p);
+    NN_CHECK(e == cudaSuccess, "linear (32-bit): launch failed: %s", cudaGetErrorString(e));
+    if (p.slices > 1) {
+        cfg.gridDim = dim3((unsigned)(((long)p.M * p.N + 255) / 256));
+        cfg.blockDim = dim3(256);
+        cfg.dynamicSmemBytes = 0;
+        e = cudaLaunchKernelEx(&cfg, f32_slices_kernel, p);
+        NN_CHECK(e == cudaSuccess, "linear (32-bit, adding slices): launch failed: %s", cudaGetErrorString(e));
+    }
+    return 0;
+}
+
 }  // namespace
 
 // What the products here take: rows of whole 16-byte pieces.
@@ -136,4 +522,36 @@ extern "C" int nncpu_linear_f32(const void* X, const void* W, const void* bias, 
                  : launch_few<16, 2>(x, w, bias, bias_dt, C, c_dt, M, N, K, lda, ldc, accumulate, st);
     NN_CHECK(e == cudaSuccess, "linear (32-bit): launch failed: %s", cudaGetErrorString(e));
     return 0;
+}
+
+// Floats of scratch that nncpu_linear_f32_many needs at these sizes (0: none).
+extern "C" long nncpu_linear_f32_many_scratch(int M, int N, int K) {
+    if (M <= 0 || N <= 0 || K <= 0) return 0;
+    const ManyPlan plan = many_plan(M, N, K);
+    return plan.slices > 1 ? (long)plan.slices * M * N : 0;
+}
+
+// The same product for any number of tokens, on the tensor cores.  `scratch`: see above.  `status` is set when a bounded wait
+// runs out.
+extern "C" int nncpu_linear_f32_many(const void* X, const void* W, const void* bias, int bias_dt, void* C, int c_dt, int M, int N,
+                                     int K, int lda, int ldc, int accumulate, void* scratch, int* status, void* stream_) {
+    cudaStream_t st = (cudaStream_t)stream_;
+    NN_CHECK(M > 0 && N > 0 && K > 0 && K % 4 == 0 && lda % 4 == 0 && lda >= K && ldc >= N,
+             "linear (32-bit): M %d, N %d, K %d, lda %d, ldc %d", M, N, K, lda, ldc);
+    NN_CHECK((uintptr_t)X % 16 == 0 && (uintptr_t)W % 16 == 0, "linear (32-bit): operands must be 16-byte aligned");
+    const ManyPlan plan = many_plan(M, N, K);
+    NN_CHECK(plan.slices == 1 || scratch != nullptr, "linear (32-bit): %d slices of K need scratch memory", plan.slices);
+    ManyParams p{(const float*)X, (const float*)W, bias, bias_dt, C, c_dt, (float*)scratch, M, N, K, lda, ldc, accumulate,
+                 (N + 127) / 128, plan.tiles_b, plan.slices, (K + kManyK - 1) / kManyK, status};
+    NN_CHECK((long)p.tiles_a * p.tiles_b * p.slices < (1L << 31), "linear (32-bit): %d tokens of %d features", M, N);
+    switch (plan.bn) {
+        case 32: return launch_many<32>(p, st);
+        case 64: return launch_many<64>(p, st);
+        case 96: return launch_many<96>(p, st);
+        case 128: return launch_many<128>(p, st);
+        case 160: return launch_many<160>(p, st);
+        case 192: return launch_many<192>(p, st);
+        case 224: return launch_many<224>(p, st);
+        default: return launch_many<256>(p, st);
+    }
 }

@@ -283,9 +283,9 @@ LINEAR_F32_MIN_WEIGHTS = 1 << 20
 
 
 def linear_f32_supported(x, w) -> bool:
-    """Whether ``linear_f32`` takes this product: few rows of float32, of whole 16-byte pieces, on both sides."""
-    return (x.dtype == torch.float32 and w.dtype == torch.float32 and 0 < x.shape[0] <= LINEAR_F32_MAX_TOKENS
-            and x.shape[1] % 4 == 0 and _aligned(x) and _aligned(w))
+    """Whether ``linear_f32`` and ``linear_f32_many`` take this product: float32 rows of whole 16-byte pieces on both sides."""
+    return (x.dtype == torch.float32 and w.dtype == torch.float32 and x.shape[0] > 0 and x.shape[1] % 4 == 0
+            and _aligned(x) and _aligned(w))
 
 
 def linear_f32(x, w, bias, out, accumulate: bool = False) -> None:
@@ -295,6 +295,24 @@ def linear_f32(x, w, bias, out, accumulate: bool = False) -> None:
     assert w.shape[1] == k and out.shape == (m, n) and x.dtype == w.dtype == torch.float32
     _call("linear_f32", "nncpu_linear_f32", _ptr(x), _ptr(w), _ptr(bias), _i(_code(bias)), _ptr(out), _i(_code(out)),
           _i(m), _i(n), _i(k), _i(k), _i(n), _i(accumulate), _stream())
+
+
+def linear_f32_many_scratch_floats(m: int, n: int, k: int) -> int:
+    """Floats of scratch that ``linear_f32_many`` needs at these sizes."""
+    lib = library.load("linear_f32")
+    lib.nncpu_linear_f32_many_scratch.restype = ctypes.c_long
+    return lib.nncpu_linear_f32_many_scratch(_i(m), _i(n), _i(k))
+
+
+def linear_f32_many(x, w, bias, out, scratch, workspace: "GemmWorkspace", accumulate: bool = False) -> None:
+    """out (+)= x . w^T + bias for any number of rows: the tensor cores on numbers cut in two, with the error of a
+    32-bit sum.  ``scratch`` holds ``linear_f32_many_scratch_floats`` floats (None where that is 0)."""
+    m, k = x.shape
+    n = w.shape[0]
+    assert w.shape[1] == k and out.shape == (m, n) and x.dtype == w.dtype == torch.float32
+    assert scratch is None or scratch.dtype == torch.float32
+    _call("linear_f32", "nncpu_linear_f32_many", _ptr(x), _ptr(w), _ptr(bias), _i(_code(bias)), _ptr(out), _i(_code(out)),
+          _i(m), _i(n), _i(k), _i(k), _i(n), _i(accumulate), _ptr(scratch), _ptr(workspace.status), _stream())
 
 
 def linear_tc_supported(m: int, n: int, k: int) -> bool:
@@ -309,10 +327,15 @@ class GemmWorkspace:
     stream)."""
 
     def __init__(self, device):
+        self.device = device
+        self.status = torch.zeros(1, dtype=torch.int32, device=device)
+
+    @functools.cached_property
+    def scratch(self) -> torch.Tensor:
+        """Made with the first bfloat16 product: a float32 run needs the status word alone."""
         lib = library.load("gemm_sm100")
         lib.nncpu_linear_tc_scratch_floats.restype = ctypes.c_long
-        self.scratch = torch.empty(lib.nncpu_linear_tc_scratch_floats(), dtype=torch.float32, device=device)
-        self.status = torch.zeros(1, dtype=torch.int32, device=device)
+        return torch.empty(lib.nncpu_linear_tc_scratch_floats(), dtype=torch.float32, device=self.device)
 
 
 # Which kernel a tensor-core product runs with, where a measurement or a test wants another than its sizes would get.

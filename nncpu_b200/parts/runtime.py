@@ -140,7 +140,7 @@ class Runtime:
 
     @property
     def workspace(self) -> ops.GemmWorkspace:
-        """Made when the first tensor-core product needs it (a float32 run never does)."""
+        """Made when the first tensor-core product needs it."""
         if self._workspace is None:
             self._workspace = ops.GemmWorkspace(self.device)
         return self._workspace
@@ -197,8 +197,15 @@ class Runtime:
         else:
             assert epilogue == "plain" and activation is None, "fused epilogues exist on the tensor-core path only"
             # small layers stay with the kernel whose sums have one order for every number of rows: see the constant
-            fast = w.numel() >= ops.LINEAR_F32_MIN_WEIGHTS and ops.linear_f32_supported(x, w)
-            (ops.linear_f32 if fast else ops.linear_simt)(x, w, bias, out, accumulate)
+            if w.numel() < ops.LINEAR_F32_MIN_WEIGHTS or not ops.linear_f32_supported(x, w):
+                ops.linear_simt(x, w, bias, out, accumulate)
+            elif x.shape[0] <= ops.LINEAR_F32_MAX_TOKENS:
+                ops.linear_f32(x, w, bias, out, accumulate)
+            else:
+                with self.scope():
+                    floats = ops.linear_f32_many_scratch_floats(x.shape[0], w.shape[0], x.shape[1])
+                    scratch = self.empty(floats, dtype=torch.float32) if floats else None
+                    ops.linear_f32_many(x, w, bias, out, scratch, self.workspace, accumulate)
 
     def fuses_norms(self, n_tokens: int, n_out: int) -> bool:
         """Whether the bfloat16 products of a step of ``n_tokens`` rows (``n_out`` output features) may carry the norms

@@ -1,4 +1,4 @@
-"""The kernels of true float32 runs: the product of a few tokens, and attention over float32 pages, against 64-bit sums and
+"""The kernels of true float32 runs: the products of few and of many tokens, and attention over float32 pages, against 64-bit sums and
 against the general kernels."""
 from __future__ import annotations
 
@@ -45,6 +45,56 @@ def test_few_token_product(ops, m, n, k):
     ops.linear_f32(x[m - 1:].contiguous(), w, None, one)
     ops.linear_f32(x[m - 1:].expand(16, k).contiguous(), w, None, many)
     assert torch.equal(one.expand(16, n), many)
+
+
+@pytest.mark.parametrize("m", [1, 17, 32, 33, 64, 90, 128, 160, 190, 224, 256, 257, 300, 520])
+@pytest.mark.parametrize("n,k", [(5, 4), (128, 32), (129, 36), (200, 100), (300, 1000), (1536, 2048), (256, 6144)])
+def test_many_token_product(ops, m, n, k):
+    """On the tensor cores with numbers cut in two: the bound of a 32-bit sum holds, and over longer sums the error is no
+    larger than that of the general kernel, which adds k products one after the other."""
+    g = torch.Generator(device=DEV).manual_seed(m * n + k)
+    x, w, b = (torch.randn(s, generator=g, device=DEV) for s in ((m, k), (n, k), (n,)))
+    want, tol = x.double() @ w.double().T, bound(x, w) + 1e-6
+    floats = ops.linear_f32_many_scratch_floats(m, n, k)
+    scratch = torch.full((floats,), float("nan"), device=DEV) if floats else None
+    work = ops.GemmWorkspace(DEV)
+    out = torch.full((m, n), 7.0, device=DEV)
+    ops.linear_f32_many(x, w, b, out, scratch, work)
+    assert ((out - (want + b)).abs() <= tol + b.abs() * 2.0 ** -23).all()
+    ops.linear_f32_many(x, w, None, out, scratch, work, accumulate=True)
+    assert ((out - (2 * want + b)).abs() <= 3 * tol + b.abs() * 2.0 ** -22).all()
+    ops.linear_f32_many(x, w, None, out, scratch, work)
+    again, general = torch.empty_like(out), torch.empty_like(out)
+    ops.linear_f32_many(x, w, None, again, scratch, work)
+    ops.linear_simt(x, w, None, general)
+    assert torch.equal(out, again) and int(work.status.item()) == 0
+    if k >= 1000 and m >= 17:
+        assert (out - want).norm() <= (general - want).norm()
+    half = torch.empty(m, n, dtype=torch.bfloat16, device=DEV)
+    ops.linear_f32_many(x, w, b.bfloat16(), half, scratch, work)
+    assert ((half - (want + b.bfloat16())).abs() <= tol + 2.0 ** -8 * (want + b.bfloat16()).abs()).all()
+
+
+def test_many_token_product_of_numbers_at_the_edges(ops):
+    """Infinities, numbers next to the largest and NaN give what float arithmetic gives; tiny and huge scales keep their bits."""
+    m, n, k = 40, 1100, 1024
+    g = torch.Generator(device=DEV).manual_seed(4)
+    x, w = torch.randn(m, k, generator=g, device=DEV), torch.randn(n, k, generator=g, device=DEV)
+    for scale_x, scale_w in ((1e18, 1e18), (1e-12, 1e-12), (1e30, 1e-30)):
+        a, b = x * scale_x, w * scale_w
+        floats = ops.linear_f32_many_scratch_floats(m, n, k)
+        scratch = torch.empty(floats, device=DEV) if floats else None
+        out = torch.empty(m, n, device=DEV)
+        ops.linear_f32_many(a, b, None, out, scratch, ops.GemmWorkspace(DEV))
+        assert ((out - a.double() @ b.double().T).abs() <= bound(a, b)).all()
+    x[3, 700], w[5, 9], w[6, 10], x[8, 20], w[11, 20] = math.inf, -math.inf, math.nan, 3.4028234e38, 1.0
+    w[:, 700] = w[:, 700].abs()
+    got, want = torch.empty(m, n, device=DEV), torch.empty(m, n, device=DEV)
+    ops.linear_f32_many(x, w, None, got, scratch, ops.GemmWorkspace(DEV))
+    ops.linear_simt(x, w, None, want)
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    assert torch.equal(got[got.isinf()], want[want.isinf()])
+    assert want.isinf().any() and want.isnan().any()
 
 
 def test_few_token_product_of_other_forms_stays_general(ops):
