@@ -24,7 +24,14 @@
 //     row's largest score is found, the reference moves up to it, the row's O
 //     (between two O updates, never under one) and sum are rescaled and the
 //     step's weights computed again.
-// The output row is O / sum.  The reference computes the same attention row by
+// The output row is O / sum.
+//
+// A few rows over a long past make few blocks: a message of 24 tokens behind 700 others, 16 heads over 4, is 8 of them,
+// each walking six steps one after the other while 140 SMs idle.  There a cluster of 2, 4 or 8 blocks shares a tile: each walks
+// its part of the steps, leaves reference maximum, sum and O (32-bit) in its shared memory, and adds up its share of the columns
+// over the cluster's blocks, in their order, through distributed shared memory.
+//
+// The reference computes the same attention row by
 // row (crates/nncpu/src/model/forward.rs:141-160,383-426); softmax runs in 32-bit here
 // as there.
 //
@@ -46,6 +53,7 @@ namespace {
 constexpr int kQRows = 128;   // query rows per block = tensor-core M
 constexpr int kKeys = 2 * kPage;  // keys per step: two cache pages
 constexpr int kStages = 2;    // steps of K and of V in flight
+constexpr int kMaxSplits = 8; // blocks of a cluster that shares a tile
 constexpr int kStreamCols = 256;  // tensor-memory columns per head: S (P over its second half) | O
 constexpr int kPOffset = 64;      // P lies over the second half of S
 constexpr float kSumLimit = 256.0f;  // a step's weights of a row may add up to this before the row's reference maximum is moved
@@ -72,6 +80,7 @@ struct AttnParams {
     // two scores an instruction.  Elsewhere u = 1 - 2 / (1 + 2^(cap_in * unscaled score)): two more special-function
     // results a score, which is what the softmax has least of.
     float cap_in, cap_x, cap_small, score_mul;
+    int splits;               // blocks of the cluster that shares a tile's steps (1: none)
     const float* head_gate;   // or null: row t (at t * gate_ld) holds a logit a head, whose sigmoid multiplies the head's output
     long gate_ld;
     int* status;
@@ -146,6 +155,19 @@ __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, u
         : "memory");
 }
 
+__device__ __forceinline__ void cluster_barrier() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ float ld_cluster_f32(uint32_t local_addr, uint32_t rank) {
+    uint32_t remote;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local_addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
+    return v;
+}
+
 // Threads: warp 0 producer, warp 1 tensor-core issue and tensor memory, then one warpgroup per head.
 template <int HD, int VD, int kStreams, bool kCap>
 __global__ void __launch_bounds__(64 + 128 * kStreams, 1)
@@ -205,13 +227,16 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     const int key_lo = first_visible_key(pos0, p.window);
     const PageWalk walk(key_lo, key_hi, p.keep);     // the pages that hold keys these rows see
     const int n_pages = walk.n;
-    const int n_steps = (n_pages + 1) / 2;           // two pages a step; the last step may hold one
+    // two pages a step, of which the last may hold one; this block walks the steps s0 .. s0 + n_steps - 1 of them
+    const int all_steps = (n_pages + 1) / 2, split = (int)blockIdx.x % p.splits;
+    const int s0 = split * all_steps / p.splits, n_steps = (split + 1) * all_steps / p.splits - s0;
     // the heads of a key/value head are dealt out two to a block; an odd group's last block has one
     const int group = p.n_heads / p.n_kv;
     const int per_kv = (group + kStreams - 1) / kStreams;
-    const int kvh = blockIdx.x / per_kv;
-    const int head0 = kvh * group + (blockIdx.x % per_kv) * kStreams;
-    const int n_streams = min(kStreams, group - (blockIdx.x % per_kv) * kStreams);
+    const int head_block = (int)blockIdx.x / p.splits;
+    const int kvh = head_block / per_kv;
+    const int head0 = kvh * group + (head_block % per_kv) * kStreams;
+    const int n_streams = min(kStreams, group - (head_block % per_kv) * kStreams);
 
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
@@ -240,9 +265,10 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
     wait_for_previous_kernels();
+    float m_ref = -INFINITY, l = 0.0f;     // a softmax thread's row: the reference maximum, the sum of its weights
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (lane == 0 && n_steps > 0) {
             const int* table = p.block_table + (size_t)seq * p.bt_stride;
             mbar_expect_tx(q_full, n_streams * kQBytes);
             for (int t = 0; t < n_streams; ++t)
@@ -257,23 +283,23 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                 bool moved = false;
                 if (jk < n_steps && mbar_test_wait(&k_empty[jk % kStages], ((jk / kStages) & 1) ^ 1)) {
                     const int st = jk % kStages;
-                    const int pages = min(2, n_pages - 2 * jk);
+                    const int pages = min(2, n_pages - 2 * (s0 + jk));
                     mbar_expect_tx(&k_full[st], pages * kPageBytes);
                     for (int pg = 0; pg < pages; ++pg)
                         for (int s = 0; s < kSlabs; ++s)
                             tma_load_4d(smem_k + st * kKBytes + s * kKvSlab + pg * (kPage * 128), &map_k, &k_full[st],
-                                        64 * s, 0, kvh, table[walk.page(2 * jk + pg)]);
+                                        64 * s, 0, kvh, table[walk.page(2 * (s0 + jk) + pg)]);
                     ++jk;
                     moved = true;
                 }
                 if (jv < jk && mbar_test_wait(&v_empty[jv % kStages], ((jv / kStages) & 1) ^ 1)) {
                     const int st = jv % kStages;
-                    const int pages = min(2, n_pages - 2 * jv);
+                    const int pages = min(2, n_pages - 2 * (s0 + jv));
                     mbar_expect_tx(&v_full[st], pages * kVPageBytes);
                     for (int pg = 0; pg < pages; ++pg)
                         for (int s = 0; s < kVSlabs; ++s)
                             tma_load_4d(smem_v + st * kVBytes + s * kKvSlab + pg * (kPage * 128), &map_v, &v_full[st],
-                                        64 * s, 0, kvh, table[walk.page(2 * jv + pg)]);
+                                        64 * s, 0, kvh, table[walk.page(2 * (s0 + jv) + pg)]);
                     ++jv;
                     moved = true;
                 }
@@ -293,14 +319,14 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (lane == 0 && n_steps > 0) {
             constexpr uint32_t idesc_s128 = instr_desc_bf16(kQRows, 128), idesc_s64 = instr_desc_bf16(kQRows, 64);
             constexpr uint32_t idesc_o = instr_desc_bf16(kQRows, VD) | (1u << 16);   // B (V) is MN-major
             bool ok = mbar_wait(q_full, 0);
             if (!ok) atomicExch(p.status, kTimeoutQ);
             // S_t(i) = Q_t . K(i)^T into the head's S columns; K(i) has landed
             auto issue_scores = [&](int t, int i) {
-                const int keys = min(2, n_pages - 2 * i) * kPage;
+                const int keys = min(2, n_pages - 2 * (s0 + i)) * kPage;
                 const uint32_t k_addr = smem_u32(smem_k + (i % kStages) * kKBytes);
                 const uint32_t q_addr = smem_u32(smem_q + t * kQBytes);
                 const uint32_t tmem_s = tmem_base + (uint32_t)(t * kStreamCols);
@@ -327,7 +353,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             // head's matrices are being multiplied the other head's warpgroup does its exponentials.
             for (int i = 0; i < n_steps && ok; ++i) {
                 const int st = i % kStages;
-                const int ksteps = min(2, n_pages - 2 * i) * (kPage / 16);
+                const int ksteps = min(2, n_pages - 2 * (s0 + i)) * (kPage / 16);
                 const bool more = i + 1 < n_steps;
                 for (int t = 0; t < n_streams && ok; ++t) {
                     if (!mbar_wait(&p_full[t], i & 1)) {
@@ -375,23 +401,29 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         const int quarter = warp & 3;             // the tensor-memory lanes this warp may touch
         const int row = quarter * 32 + lane;
         const int h = head0 + t;
-        const int lim_hi = row < n_rows ? pos0 + row : -1;
+        // a lane without a row sees what the tile's last row sees (a limit of its own would make its warp mask every page:
+        // 24 rows behind 1 500 keys took 45 us, 32 rows 29); nothing else is done for it and its result is not stored
+        const bool valid = row < n_rows;
+        const int lim_hi = valid ? pos0 + row : key_hi;
         const int lim_lo = first_visible_key(lim_hi, p.window);
         const uint32_t tmem_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(t * kStreamCols);
         // the distance bias in the unit of the unscaled scores (the scale is applied with the reference maximum)
         const float bias_per_key = p.slope_base != 0.0f
             ? exp2f(-p.slope_base * (float)(h + 1) / (float)p.n_heads) * 1.4426950408889634f / p.scale2 : 0.0f;
-        float m_ref = -INFINITY, l = 0.0f;
-        bool ok = t < n_streams;   // the second warpgroup of a block with one head has nothing to do
+        bool ok = t < n_streams && n_steps > 0;   // the second warpgroup of a block with one head has nothing to do
         for (int i = 0; ok && i < n_steps; ++i) {
             ok = __all_sync(0xffffffffu, mbar_wait(&s_full[t], i & 1));
             if (!ok) {
                 if (lane == 0) atomicExch(p.status, kTimeoutS);
                 break;
             }
+            if (quarter * 32 >= n_rows) {      // a warp without rows: what the tensor core makes of its lanes is not read
+                mbar_arrive(&p_full[t]);
+                continue;
+            }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int halves = min(2, n_pages - 2 * i);
-            const int k_base[2] = {walk.page(2 * i) * kPage, walk.page(2 * i + 1) * kPage};
+            const int halves = min(2, n_pages - 2 * (s0 + i));
+            const int k_base[2] = {walk.page(2 * (s0 + i)) * kPage, walk.page(2 * (s0 + i) + 1) * kPage};
             // A step costs one pass over the row's scores: weights against the reference maximum as it stands (as
             // bfloat16 pairs) and their sum.  The largest score is not looked for: a sum of at most 2^8 proves that
             // no weight is above 2^8.  Only when a row's sum says otherwise (or the row has seen no key yet) is the
@@ -463,9 +495,9 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                 }
                 sum = (sm[0] + sm[1]) + (sm[2] + sm[3]);
             };
-            const bool unseen = __any_sync(0xffffffffu, m_ref == -INFINITY && lim_hi >= 0);
+            const bool unseen = __any_sync(0xffffffffu, m_ref == -INFINITY && valid);
             if (!unseen) weights();
-            if (unseen || __any_sync(0xffffffffu, !(sum <= kSumLimit))) {
+            if (unseen || __any_sync(0xffffffffu, valid && !(sum <= kSumLimit))) {
                 float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
                 for (int hf = 0; hf < 2; ++hf) {
@@ -506,7 +538,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             ok = __all_sync(0xffffffffu, mbar_wait(&o_done[t], 0));
             if (!ok && lane == 0) atomicExch(p.status, kTimeoutPv);
         }
-        if (ok) {
+        if (ok && p.splits == 1) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             // the sink's term, in the unit of the row's sums: powers of two relative to the reference maximum
             if (p.sinks != nullptr && l > 0.0f) l += exp2f(p.sinks[h] * 1.4426950408889634f - m_ref);
@@ -539,6 +571,91 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (p.splits > 1) {
+        // The copies have landed and the matrix instructions have retired, so the tiles' memory is free: it takes this block's
+        // part, [kStreams][VD columns][128 rows] of O, then the rows' reference maxima and sums.  (A block whose wait ran
+        // out comes here, too: what it leaves is not valid, and the status word says so.)
+        float* part_o = reinterpret_cast<float*>(smem);
+        float* part_m = part_o + kStreams * VD * kQRows;     // [kStreams][128]
+        float* part_l = part_m + kStreams * kQRows;
+        const int t = (warp - 2) >> 2, quarter = warp & 3, row = quarter * 32 + lane;
+        const bool mine = warp >= 2 && t < n_streams && quarter * 32 < n_rows;      // this warp has rows
+        if (mine) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t tmem_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(t * kStreamCols);
+            if (n_steps > 0) {
+#pragma unroll 1
+                for (int c0 = 0; c0 < VD; c0 += 32) {
+                    uint32_t o[32];
+                    tmem_ld32(tmem_row + (uint32_t)(kKeys + c0), o);
+#pragma unroll
+                    for (int c = 0; c < 32; ++c) part_o[(t * VD + c0 + c) * kQRows + row] = __uint_as_float(o[c]);
+                }
+            }
+            part_m[t * kQRows + row] = m_ref;
+            part_l[t * kQRows + row] = l;
+        }
+        cluster_barrier();
+        if (mine) {
+            const uint32_t o_at = smem_u32(part_o + t * VD * kQRows + row), m_at = smem_u32(part_m + t * kQRows + row);
+            const uint32_t l_at = smem_u32(part_l + t * kQRows + row);
+            const int h = head0 + t;
+            float ms[kMaxSplits], ls[kMaxSplits], top = -INFINITY;
+#pragma unroll
+            for (int c = 0; c < kMaxSplits; ++c) {
+                ms[c] = -INFINITY;
+                ls[c] = 0.0f;
+                if (c < p.splits) {
+                    ms[c] = ld_cluster_f32(m_at, (uint32_t)c);
+                    ls[c] = ld_cluster_f32(l_at, (uint32_t)c);
+                }
+                top = fmaxf(top, ms[c]);
+            }
+            float sum = 0.0f;
+#pragma unroll
+            for (int c = 0; c < kMaxSplits; ++c) {
+                // a block in which the row saw no key counts for nothing, whatever its memory holds
+                const bool none = ls[c] == 0.0f && ms[c] == -INFINITY;
+                ms[c] = none ? -1.0f : exp2f(ms[c] - top);     // from here on: the block's factor, or below zero
+                if (!none) sum = fmaf(ms[c], ls[c], sum);
+            }
+            if (p.sinks != nullptr && sum > 0.0f) sum += exp2f(p.sinks[h] * 1.4426950408889634f - top);
+            float inv = sum > 0.0f ? 1.0f / sum : 0.0f;
+            if (p.head_gate != nullptr && row < n_rows)
+                inv *= 1.0f / (1.0f + expf(-p.head_gate[(size_t)(q0 + row) * p.gate_ld + h]));
+            __nv_bfloat16* dst = p.out + ((size_t)(q0 + row) * p.n_heads + h) * p.vo;
+            const int cols = VD / p.splits;        // 8 at least
+#pragma unroll 1
+            for (int c0 = split * cols; c0 < (split + 1) * cols; c0 += 8) {
+                float acc[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[j] = 0.0f;
+#pragma unroll
+                for (int c = 0; c < kMaxSplits; ++c) {
+                    if (c < p.splits) {
+                        float v[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) v[j] = ld_cluster_f32(o_at + (uint32_t)((c0 + j) * kQRows * 4), (uint32_t)c);
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) acc[j] = ms[c] < 0.0f ? acc[j] : fmaf(ms[c], v[j], acc[j]);
+                    }
+                }
+                if (row < n_rows && (p.vo & 7) != 0) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if (c0 + j < p.vo) dst[c0 + j] = __float2bfloat16_rn(acc[j] * inv);
+                } else if (row < n_rows && c0 < p.vo) {
+                    uint4 w;
+                    w.x = pack_bf16(acc[0] * inv, acc[1] * inv);
+                    w.y = pack_bf16(acc[2] * inv, acc[3] * inv);
+                    w.z = pack_bf16(acc[4] * inv, acc[5] * inv);
+                    w.w = pack_bf16(acc[6] * inv, acc[7] * inv);
+                    *reinterpret_cast<uint4*>(dst + c0) = w;
+                }
+            }
+        }
+        cluster_barrier();      // a block's memory is read until every block is done
+    }
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols)
@@ -597,8 +714,11 @@ struct MapCache {
 MapCache g_maps;
 
 template <int HD, int VD, int kStreams, bool kCap>
-int launch_one(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AttnParams& p, int n_tok,
-           cudaStream_t stream) {
+int launch_one(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, AttnParams p, int n_tok, int longest,
+               cudaStream_t stream) {
+    static_assert((kStreams * VD + 2 * kStreams) * kQRows * 4 <= kStreams * kQRows * HD * 2 + kStages * kKeys * (HD + VD) * 2,
+                  "a split tile's part fits the memory of its operands");
+    static_assert(VD / kMaxSplits >= 8, "a block of a cluster adds up eight columns at least");
     constexpr int smem = kStreams * kQRows * HD * 2 + kStages * kKeys * (HD + VD) * 2 + 256 + 1024;
     static bool configured[64] = {};
     if (first_use_on_this_device(configured)) {
@@ -609,25 +729,55 @@ int launch_one(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& 
     }
     // tiles: an upper bound, since the sequence boundaries live on the device; spare blocks leave at once
     const int group = p.n_heads / p.n_kv;
-    const dim3 grid(p.n_kv * ((group + kStreams - 1) / kStreams), (n_tok + kQRows - 1) / kQRows + p.n_seqs);
+    const int head_blocks = p.n_kv * ((group + kStreams - 1) / kStreams);
+    // (a sequence of n tokens has ceil(n / 128) tiles; all together at most these)
+    const int tiles = n_tok < p.n_seqs ? n_tok : (n_tok - p.n_seqs) / kQRows + p.n_seqs;
+    const int tiles_y = (n_tok + kQRows - 1) / kQRows + p.n_seqs;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
     cfg.blockDim = dim3(64 + 128 * kStreams);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    cfg.attrs = attr;
-    cfg.numAttrs = overlap_attribute(attr);
+    cudaLaunchAttribute attr[2];
+    auto with_splits = [&](int n) {
+        cfg.gridDim = dim3((unsigned)(head_blocks * n), (unsigned)tiles_y);
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)n;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = n > 1 ? attr : attr + 1;
+        cfg.numAttrs = n > 1 ? 1 : 0;
+    };
+    // A tile's steps are shared by as many blocks as leave each a step of the longest walk, as long as all clusters run at
+    // once (a second round costs more than the split gains: 16 tiles of 4 000 keys took 52 us as 16 clusters of 8, of
+    // which 14 fit, and 34 us as clusters of 4).  How many fit is the device's to say: clusters lie within a GPC.
+    static int fit[64][4] = {};      // per device, for clusters of 2, 4 and 8 (0: not asked yet)
+    int dev = 0;
+    p.splits = 1;
+    if (longest > kKeys && cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64) {
+        for (int n = 2, i = 1; n <= kMaxSplits && (n - 1) * kKeys < longest; n *= 2, ++i) {
+            if (fit[dev][i] == 0) {
+                with_splits(n);
+                int clusters = 0;
+                if (cudaOccupancyMaxActiveClusters(&clusters, prefill_tc_kernel<HD, VD, kStreams, kCap>, &cfg) != cudaSuccess) {
+                    cudaGetLastError();
+                    clusters = 0;
+                }
+                fit[dev][i] = clusters > 0 ? clusters : -1;
+            }
+            if ((long)head_blocks * tiles <= fit[dev][i]) p.splits = n;
+        }
+    }
+    with_splits(p.splits);
+    cfg.numAttrs += overlap_attribute(attr + 1);
     const cudaError_t e = cudaLaunchKernelEx(&cfg, prefill_tc_kernel<HD, VD, kStreams, kCap>, mq, mk, mv, p);
     NN_CHECK(e == cudaSuccess, "attention prefill (tensor cores): launch failed: %s", cudaGetErrorString(e));
     return 0;
 }
 
 template <int HD, int VD, int kStreams>
-int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AttnParams& p, int n_tok,
+int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AttnParams& p, int n_tok, int longest,
            cudaStream_t stream) {
-    return p.cap_in != 0.0f ? launch_one<HD, VD, kStreams, true>(mq, mk, mv, p, n_tok, stream)
-                            : launch_one<HD, VD, kStreams, false>(mq, mk, mv, p, n_tok, stream);
+    return p.cap_in != 0.0f ? launch_one<HD, VD, kStreams, true>(mq, mk, mv, p, n_tok, longest, stream)
+                            : launch_one<HD, VD, kStreams, false>(mq, mk, mv, p, n_tok, longest, stream);
 }
 
 }  // namespace
@@ -641,13 +791,14 @@ extern "C" int nncpu_attention_prefill_tc_supported(int n_heads, int n_kv, int h
 // window, the sequence's first keys that stay visible; cu_seqlens [n_seqs + 1] row ranges of the sequences;
 // tok_pos [n_tok] positions (consecutive within a sequence); cap > 0: a scaled score z becomes cap tanh(z / cap) (not
 // together with a distance bias); head_gate (or null): token t's n_heads logits at t * gate_ld, whose sigmoids multiply the
-// heads' outputs.  *status receives a code if a wait runs out.
+// heads' outputs; longest: at least as many keys as any row sees (a tile may be split over its steps, see the head of this
+// file; 0: it is not).  *status receives a code if a wait runs out.
 extern "C" int nncpu_attention_prefill_tc(const void* q, const void* k_pages, const void* v_pages, int n_pages,
                                           const int* block_table, int bt_stride, const int* cu_seqlens,
                                           const int* tok_pos, void* out, int n_tok, int n_seqs, int n_heads, int n_kv,
                                           int head_dim, int vp, int vo, float scale, int window, int keep,
                                           float slope_base, const float* sinks, float cap, const float* head_gate,
-                                          int gate_ld, int* status, void* stream_) {
+                                          int gate_ld, int longest, int* status, void* stream_) {
     NN_CHECK(nncpu_attention_prefill_tc_supported(n_heads, n_kv, head_dim),
              "attention (tensor cores): head size %d with %d heads over %d key/value heads is not supported "
              "(head size 64 or 128, heads a multiple of key/value heads)", head_dim, n_heads, n_kv);
@@ -691,7 +842,7 @@ extern "C" int nncpu_attention_prefill_tc(const void* q, const void* k_pages, co
     cudaStream_t stream = (cudaStream_t)stream_;
     // two heads to a block where a key/value head has two to give; one head per block otherwise
     const bool one = n_heads == n_kv;
-    if (head_dim == 64) return one ? launch<64, 64, 1>(mq, mk, mv, p, n_tok, stream) : launch<64, 64, 2>(mq, mk, mv, p, n_tok, stream);
-    if (vp == 64) return one ? launch<128, 64, 1>(mq, mk, mv, p, n_tok, stream) : launch<128, 64, 2>(mq, mk, mv, p, n_tok, stream);
-    return one ? launch<128, 128, 1>(mq, mk, mv, p, n_tok, stream) : launch<128, 128, 2>(mq, mk, mv, p, n_tok, stream);
+    if (head_dim == 64) return one ? launch<64, 64, 1>(mq, mk, mv, p, n_tok, longest, stream) : launch<64, 64, 2>(mq, mk, mv, p, n_tok, longest, stream);
+    if (vp == 64) return one ? launch<128, 64, 1>(mq, mk, mv, p, n_tok, longest, stream) : launch<128, 64, 2>(mq, mk, mv, p, n_tok, longest, stream);
+    return one ? launch<128, 128, 1>(mq, mk, mv, p, n_tok, longest, stream) : launch<128, 128, 2>(mq, mk, mv, p, n_tok, longest, stream);
 }

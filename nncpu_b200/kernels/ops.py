@@ -711,6 +711,13 @@ DECODE_MIN_KEYS_PER_SPLIT = 256
 DECODE_CLUSTER_MAX_SPLITS = 8      # up to here the splits merge inside a thread-block cluster, without scratch
 
 
+# A short portion of one sequence goes through the decode kernel, token by token, while its tokens times key/value heads times
+# keys are at most this; beyond, as tiles of 128 rows (``attention_prefill_tc``).  Measured at the line (us, token by token /
+# tiles): 16 heads over 4, 64 tokens behind 700 15.3 / 16.0; 32 over 8, 16 behind 1 500 17 / 20; far below it (24 tokens of
+# 16 heads over 4 behind 700) 11.9 / 18.3; above it (32 over 8, 64 behind 1 500) 50 / 20.
+FEW_TOKENS_MAX_KEYS = 200_000
+
+
 def attention_decode_splits(n_tokens: int, n_kv: int, longest: int, sm_count: int) -> int:
     """As many splits as keep every block of the grid running at once (never a second wave), each with at
     least ``DECODE_MIN_KEYS_PER_SPLIT`` keys of the longest sequence.  Up to twice what a cluster merges is cut
@@ -820,10 +827,13 @@ def attention_prefill_tc_supported(n_heads: int, n_kv: int, head_dim: int, *tens
 
 def attention_prefill_tc(q, k_pages, v_pages, block_table, cu_seqlens, tok_pos, out, status, n_seqs: int,
                          n_heads: int, n_kv: int, head_dim: int, scale: float, window: int, slope_base: float = 0.0,
-                         sinks=None, keep: int = 0, v_lanes: int = 0, cap: float = 0.0, head_gate=None) -> None:
+                         sinks=None, keep: int = 0, v_lanes: int = 0, cap: float = 0.0, head_gate=None,
+                         longest: int = 0) -> None:
     """Prefill attention on the tcgen05 tensor cores: any number of new tokens per sequence, at consecutive
     positions; ``status`` is an int32 word on the device that receives a code if a bounded wait runs out.
-    ``slope_base``, ``sinks`` and ``keep`` as in ``attention``, ``v_lanes`` as in ``attention_decode_mma``."""
+    ``slope_base``, ``sinks`` and ``keep`` as in ``attention``, ``v_lanes`` as in ``attention_decode_mma``.  ``longest``:
+    at least as many keys as any token sees; where there are few tiles of tokens their keys are then shared by several blocks
+    (0: never)."""
     assert sinks is None or (sinks.dtype == torch.float32 and sinks.numel() == n_heads)
     n = q.shape[0]
     v_lanes = v_lanes or head_dim
@@ -834,7 +844,7 @@ def attention_prefill_tc(q, k_pages, v_pages, block_table, cu_seqlens, tok_pos, 
     _call("attention_tc", "nncpu_attention_prefill_tc", _ptr(q), _ptr(k_pages), _ptr(v_pages), _i(k_pages.shape[0]),
           _ptr(block_table), _i(block_table.shape[1]), _ptr(cu_seqlens), _ptr(tok_pos), _ptr(out), _i(n), _i(n_seqs),
           _i(n_heads), _i(n_kv), _i(head_dim), _i(v_pages.shape[-1]), _i(v_lanes), _f(scale), _i(window), _i(keep),
-          _f(slope_base), _ptr(sinks), _f(cap), *_head_gate(head_gate, n, n_heads), _ptr(status), _stream())
+          _f(slope_base), _ptr(sinks), _f(cap), *_head_gate(head_gate, n, n_heads), _i(longest), _ptr(status), _stream())
 
 
 GATED_ACTS = {"silu": 0, "gelu_tanh": 1, "swish_clamp": 2}

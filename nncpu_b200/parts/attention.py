@@ -293,12 +293,22 @@ class Attention(Mixer):
         """Splits of every token's keys in a decode step, and the scratch their merge needs (None: they merge
         inside a thread-block cluster)."""
         s = self.spec
-        limit = s.window + s.keep_first if s.window else s.chunk
-        longest = min(ctx.max_kv_len, limit) if limit > 0 else ctx.max_kv_len
+        longest = self._longest_span(ctx)
         n_splits = ops.attention_decode_splits(ctx.n_tokens, s.n_kv_heads, longest, self.rt.sm_count)
         floats = 0 if n_splits <= ops.DECODE_CLUSTER_MAX_SPLITS else ops.attention_decode_scratch_floats(
             ctx.n_tokens, s.n_heads, s.n_kv_heads, self.v_row, n_splits)
         return n_splits, (self.rt.empty(floats, dtype=torch.float32) if floats else None)
+
+    def _few_over_short(self, ctx) -> bool:
+        """Whether a short portion of one sequence attends faster token by token, every token with keys of its own, than
+        as one tile of 128 rows: while the keys that all tokens read together are few."""
+        return (ctx.n_seqs == 1 and ctx.n_tokens <= 64
+                and ctx.n_tokens * self.spec.n_kv_heads * self._longest_span(ctx) <= ops.FEW_TOKENS_MAX_KEYS)
+
+    def _longest_span(self, ctx) -> int:
+        s = self.spec
+        limit = s.window + s.keep_first if s.window else s.chunk
+        return min(ctx.max_kv_len, limit) if limit > 0 else ctx.max_kv_len
 
     def _fused_qkv(self, x, cache) -> bool:
         s = self.spec
@@ -328,17 +338,19 @@ class Attention(Mixer):
             ops.attention(q, cache.k_pages, cache.v_pages, cache.block_table, ctx.tok_seq, ctx.tok_pos, attn,
                           s.n_heads, s.n_kv_heads, self.k_row, s.scale, self.span, self.v_row, s.slope_base, self.sinks,
                           **extra)
-        elif ctx.is_decode:
+        elif ctx.is_decode or self._few_over_short(ctx):
             n_splits, scratch = self._decode_splits(ctx)
             ops.attention_decode_mma(q, cache.k_pages, cache.v_pages, cache.block_table, ctx.tok_seq, ctx.tok_pos,
                                      attn, scratch, s.n_heads, s.n_kv_heads, self.k_row, s.scale, self.span, n_splits,
                                      s.slope_base, self.sinks, **extra)
-        elif ctx.n_tokens >= 32 * ctx.n_seqs and ops.attention_prefill_tc_supported(
+        elif (ctx.n_tokens >= 32 * ctx.n_seqs or ctx.n_seqs == 1) and ops.attention_prefill_tc_supported(
                 s.n_heads, s.n_kv_heads, self.k_row, q, cache.k_pages, attn):
-            # prompts: 128-row tiles on the tcgen05 tensor cores
+            # prompts: 128-row tiles on the tcgen05 tensor cores, the keys of few tiles shared by several blocks
+            span = s.window + s.keep_first if s.window else s.chunk
+            longest = min(ctx.max_kv_len, span + 128) if span else ctx.max_kv_len
             ops.attention_prefill_tc(q, cache.k_pages, cache.v_pages, cache.block_table, ctx.cu_seqlens, ctx.tok_pos,
                                      attn, self.rt.workspace.status, ctx.n_seqs, s.n_heads, s.n_kv_heads, self.k_row,
-                                     s.scale, self.span, s.slope_base, self.sinks, **extra)
+                                     s.scale, self.span, s.slope_base, self.sinks, longest=longest, **extra)
         else:
             # a few new tokens per sequence: 64-row tiles
             ops.attention_prefill_mma(q, cache.k_pages, cache.v_pages, cache.block_table, ctx.cu_seqlens, ctx.tok_pos,

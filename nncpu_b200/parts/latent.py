@@ -211,7 +211,7 @@ class LatentAttention(Mixer):
                                      s.scale, 0, n_splits, 0.0, self.sinks)
         elif ctx.n_tokens >= 32 * ctx.n_seqs and ops.attention_prefill_tc_supported(H, 1, r, q, pages, out):
             ops.attention_prefill_tc(q, pages, pages, cache.block_table, ctx.cu_seqlens, ctx.tok_pos, out,
-                                     rt.workspace.status, ctx.n_seqs, H, 1, r, s.scale, 0, 0.0, self.sinks)
+                                     rt.workspace.status, ctx.n_seqs, H, 1, r, s.scale, 0, 0.0, self.sinks, longest=ctx.max_kv_len)
         else:
             ops.attention_prefill_mma(q, pages, pages, cache.block_table, ctx.cu_seqlens, ctx.tok_pos, out, ctx.n_seqs,
                                       H, 1, r, s.scale, 0, 0.0, self.sinks)
