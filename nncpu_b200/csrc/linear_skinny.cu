@@ -71,12 +71,30 @@ __device__ __forceinline__ uint4 ldg16_stream(const __nv_bfloat16* p) {
 }
 
 
+// The few-token products of routed experts (kGrouped): blockIdx.y names a group of rows that share a matrix, by the plan that
+// sorts a step's rows (tile t: matrix tile_group[t], rows tile_row0[t] .. tile_row_end[t] - 1, at most 16 of them).
+struct SkinnyGroups {
+    const int* n_tiles;
+    const int* tile_group;
+    const int* tile_row0;
+    const int* tile_row_end;
+};
+
 // NT = number of 8-token tiles (1: up to 8 tokens, 2: up to 16); kW = warps of the block (8 or 4).
-template <int NT, int kEpi, int kW>
+template <int NT, int kEpi, int kW, bool kGrouped>
 __global__ void __launch_bounds__(kW * 32, 16 / kW)
 skinny_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restrict__ W, const void* __restrict__ bias,
               int bias_dt, void* __restrict__ out, int out_dt, int M, int N, int K, int lda, int ldc, int accumulate,
-              const NormFusion nf) {
+              const NormFusion nf, const SkinnyGroups groups) {
+    if constexpr (kGrouped) {
+        const int tile = blockIdx.y;
+        if (tile >= *groups.n_tiles) return;       // the grid is an upper bound
+        const int row = groups.tile_row0[tile];
+        M = min(groups.tile_row_end[tile] - row, NT * 8);
+        X += (size_t)row * lda;
+        W += (size_t)groups.tile_group[tile] * N * K;
+        out = out_dt == DT_F32 ? (void*)((float*)out + (size_t)row * ldc) : (void*)((__nv_bfloat16*)out + (size_t)row * ldc);
+    }
     constexpr int kU = NT == 1 ? kUnroll : 6;
     constexpr int kThreadsHere = kW * 32;
     constexpr int kPasses = kRows * 16 / kThreadsHere;   // output elements per thread: (token, row) pairs of 16 x 16
@@ -303,12 +321,25 @@ int launch(const void* X, const void* W, const void* bias, int bias_dt, void* C,
     cfg.numAttrs = overlap ? overlap_attribute(attr) : 0;
     cfg.attrs = attr;
     const cudaError_t e =
-        small ? cudaLaunchKernelEx(&cfg, skinny_kernel<NT, kEpi, 4>, (const __nv_bfloat16*)X, (const __nv_bfloat16*)W, bias,
-                                   bias_dt, C, c_dt, M, N, K, lda, ldc, accumulate, nf)
-              : cudaLaunchKernelEx(&cfg, skinny_kernel<NT, kEpi, 8>, (const __nv_bfloat16*)X, (const __nv_bfloat16*)W, bias,
-                                   bias_dt, C, c_dt, M, N, K, lda, ldc, accumulate, nf);
+        small ? cudaLaunchKernelEx(&cfg, skinny_kernel<NT, kEpi, 4, false>, (const __nv_bfloat16*)X, (const __nv_bfloat16*)W, bias,
+                                   bias_dt, C, c_dt, M, N, K, lda, ldc, accumulate, nf, SkinnyGroups{})
+              : cudaLaunchKernelEx(&cfg, skinny_kernel<NT, kEpi, 8, false>, (const __nv_bfloat16*)X, (const __nv_bfloat16*)W, bias,
+                                   bias_dt, C, c_dt, M, N, K, lda, ldc, accumulate, nf, SkinnyGroups{});
     NN_CHECK(e == cudaSuccess, "linear (few tokens): launch failed: %s", cudaGetErrorString(e));
     return 0;
+}
+
+template <int NT, int kEpi>
+void launch_grouped(const void* X, const void* W, void* C, int c_dt, int N, int K, int lda, int ldc, int tiles,
+                    const NormFusion& nf, const SkinnyGroups& g, cudaStream_t stream) {
+    const int blocks = (N + kRows - 1) / kRows;
+    const dim3 grid((unsigned)blocks, (unsigned)tiles);
+    if (four_warps_pay(blocks * tiles, K, NT == 1 ? kUnroll : 6, sm_count()))
+        skinny_kernel<NT, kEpi, 4, true><<<grid, 128, 0, stream>>>((const __nv_bfloat16*)X, (const __nv_bfloat16*)W, nullptr, 0, C,
+                                                                   c_dt, 0, N, K, lda, ldc, 0, nf, g);
+    else
+        skinny_kernel<NT, kEpi, 8, true><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)X, (const __nv_bfloat16*)W, nullptr, 0, C,
+                                                                   c_dt, 0, N, K, lda, ldc, 0, nf, g);
 }
 
 }  // namespace
@@ -376,4 +407,37 @@ extern "C" int nncpu_linear_skinny(const void* X, const void* W, const void* bia
     }
     return M <= 8 ? launch<1, kPlain>(X, W, bias, bias_dt, C, c_dt, M, N, K, lda, ldc, accumulate, nf, after_skinny != 0, stream)
                   : launch<2, kPlain>(X, W, bias, bias_dt, C, c_dt, M, N, K, lda, ldc, accumulate, nf, after_skinny != 0, stream);
+}
+
+// C[r, :] = X[r, :] . W_e^T for the rows r of group e, of which no group has more than 16 (the routed experts of a step of up to
+// 16 tokens): as nncpu_linear_tc_grouped, whose plan and epilogues these are, with every weight of a group that has rows
+// read once.  The tensor-core kernel gives a group a tile of 128 rows whatever it has and a single SM 256 features of it:
+// 16 rows of 16 experts, gate/up of 3072 x 2048 each, took it 48 us and the down product 26 us.  most_rows: the most
+// rows a group can have; max_tiles: the most groups that can have rows.
+extern "C" int nncpu_linear_skinny_grouped(const void* X, const void* W, void* C, int c_dt, int S, int N, int K, int n_groups,
+                                           int lda, int ldc, int epilogue, int act, float act_a, const int* n_tiles,
+                                           const int* tile_group, const int* tile_row0, const int* tile_row_end, int max_tiles,
+                                           int most_rows, void* stream_) {
+    NN_CHECK(S > 0 && N > 0 && K > 0 && n_groups > 0 && max_tiles > 0 && max_tiles <= 65535 && most_rows > 0 && most_rows <= 16,
+             "linear (few tokens, grouped): %d rows in %d groups of %d x %d, at most %d rows a group", S, n_groups, N, K, most_rows);
+    NN_CHECK(K % 8 == 0 && lda % 8 == 0 && lda >= K && ((uintptr_t)X % 16) == 0 && ((uintptr_t)W % 16) == 0,
+             "linear (few tokens, grouped): K %d and lda %d must be multiples of 8, operands 16-byte aligned", K, lda);
+    NN_CHECK(epilogue == kPlain || epilogue == kSwiglu, "linear (few tokens, grouped): unknown epilogue %d", epilogue);
+    const int n_out = epilogue == kSwiglu ? N / 2 : N;
+    NN_CHECK(ldc >= n_out && (epilogue == kPlain || N % 16 == 0), "linear (few tokens, grouped): ldc %d, N %d", ldc, N);
+    NN_CHECK(epilogue == kSwiglu ? (act == kActNone || act == kActGateGelu || act == kActGateSwishClamp) : act == kActNone,
+             "linear (few tokens, grouped): activation %d with epilogue %d", act, epilogue);
+    NormFusion nf{};
+    nf.act = act; nf.act_a = act_a;
+    const SkinnyGroups g{n_tiles, tile_group, tile_row0, tile_row_end};
+    cudaStream_t st = (cudaStream_t)stream_;
+    if (epilogue == kSwiglu) {
+        if (most_rows <= 8) launch_grouped<1, kSwiglu>(X, W, C, c_dt, N, K, lda, ldc, max_tiles, nf, g, st);
+        else launch_grouped<2, kSwiglu>(X, W, C, c_dt, N, K, lda, ldc, max_tiles, nf, g, st);
+    } else {
+        if (most_rows <= 8) launch_grouped<1, kPlain>(X, W, C, c_dt, N, K, lda, ldc, max_tiles, nf, g, st);
+        else launch_grouped<2, kPlain>(X, W, C, c_dt, N, K, lda, ldc, max_tiles, nf, g, st);
+    }
+    NN_LAUNCH_OK("linear (few tokens, grouped)");
+    return 0;
 }

@@ -1154,6 +1154,22 @@ def linear_tc_grouped(xs, w, out, plan, n_experts: int, workspace: GemmWorkspace
           _ptr(workspace.status), _stream())
 
 
+
+def linear_skinny_grouped(xs, w, out, plan, n_experts: int, most_rows: int, epilogue: str = "plain", activation=None) -> None:
+    """``linear_tc_grouped`` where no expert has more than ``most_rows`` <= 16 rows: a stream over the weights of the experts
+    that have any."""
+    S, K = xs.shape
+    E, N, _ = w.shape
+    mt = moe_plan_tiles(S, n_experts)
+    assert E == n_experts and w.shape[2] == K and xs.dtype == w.dtype == torch.bfloat16 and w.is_contiguous()
+    assert out.shape == (S, N // 2 if epilogue == "swiglu" else N) and plan.numel() == 1 + 3 * mt
+    base, dry = (0 if plan.is_meta else plan.data_ptr()), plan.is_meta and _dry
+    at = lambda k: None if dry else _vp(base + 4 * k)
+    act, a, _b = _activation(activation)
+    _call("linear_skinny", "nncpu_linear_skinny_grouped", _ptr(xs), _ptr(w), _ptr(out), _i(_code(out)), _i(S), _i(N), _i(K),
+          _i(E), _i(K), _i(out.shape[1]), _i(EPILOGUES[epilogue]), act, a, at(0), at(1), at(1 + mt), at(1 + 2 * mt),
+          _i(min(S, n_experts)), _i(most_rows), _stream())
+
 def xielu(x, params, out) -> None:
     """out = xIELU(x) elementwise with the two learned numbers ``params`` = (p, q): for z > 0
     softplus(p) z^2 + z/2, else (1/2 + softplus(q)) (exp(z) - 1 - z) + z/2; computed in 32-bit."""

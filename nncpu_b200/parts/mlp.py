@@ -237,6 +237,7 @@ class RoutedExperts(FeedForward):
             # many tokens: sorted by expert, one grouped product each for gate/up (activation in its epilogue) and
             # down on the tensor cores, then the choices of a token added up in their order
             act = (s.activation, float(s.limit), 0.0) if s.activation != "silu" else None
+            few = n <= ops.SKINNY_MAX_TOKENS        # a token chooses an expert once: no expert has more rows than that
             with rt.phase("moe_sort", nbytes=4.0 * S * h):
                 rows, slots = rt.empty(S, dtype=torch.int32), rt.empty(S, dtype=torch.int32)
                 plan = rt.empty(1 + 3 * ops.moe_plan_tiles(S, s.n_experts), dtype=torch.int32)
@@ -245,10 +246,16 @@ class RoutedExperts(FeedForward):
                 ops.moe_gather(x, slots, s.top, xs, weights if on_input else None)
             mid = rt.empty(S, f, dtype=torch.bfloat16)
             with rt.phase("moe_gate_up", nbytes=experts_read * 2.0 * f * h * esize, flops=4.0 * S * f * h):
-                ops.linear_tc_grouped(xs, self.w_gate, mid, plan, s.n_experts, rt.workspace, "swiglu", act)
+                if few:
+                    ops.linear_skinny_grouped(xs, self.w_gate, mid, plan, s.n_experts, n, "swiglu", act)
+                else:
+                    ops.linear_tc_grouped(xs, self.w_gate, mid, plan, s.n_experts, rt.workspace, "swiglu", act)
             y = rt.empty(S, h, dtype=torch.float32)
             with rt.phase("moe_down", nbytes=experts_read * 1.0 * f * h * esize + 4.0 * S * h, flops=2.0 * S * f * h):
-                ops.linear_tc_grouped(mid, self.w_down, y, plan, s.n_experts, rt.workspace)
+                if few:
+                    ops.linear_skinny_grouped(mid, self.w_down, y, plan, s.n_experts, n)
+                else:
+                    ops.linear_tc_grouped(mid, self.w_down, y, plan, s.n_experts, rt.workspace)
             branch = closing = None
             if own:
                 # the shared part in a branch of its own; the sum over a token's experts takes it in, times the gate
