@@ -79,6 +79,16 @@ inline bool first_use_on_this_device(bool (&done)[64]) {
     return true;
 }
 
+// SMs of the current device.
+inline int sm_count() {
+    static int counts[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    if (counts[dev] == 0 && cudaDeviceGetAttribute(&counts[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        counts[dev] = 148;
+    return counts[dev];
+}
+
 // Programmatic dependent launch: a kernel launched with `overlap_attribute` may start while the kernel before it in
 // the stream still runs, once every block of that kernel has called let_next_kernel_start() (or has ended).  It
 // may do only what does not depend on earlier kernels (fetch weights) until wait_for_previous_kernels() returns:

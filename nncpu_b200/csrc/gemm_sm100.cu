@@ -1584,16 +1584,6 @@ struct MapCache {
 
 MapCache g_maps;
 
-int sm_count() {
-    static int n = [] {
-        int dev = 0, v = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-        return v > 0 ? v : 148;
-    }();
-    return n;
-}
-
 template <int BN, int kStages>
 constexpr size_t smem_bytes() {
     return 1024 + (size_t)kStages * (kBlockM * kBlockK * 2 + BN * kBlockK * 2) + (2 * kStages + 4) * sizeof(uint64_t) + 16;

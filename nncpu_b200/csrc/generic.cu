@@ -18,6 +18,22 @@
 #define NN_LAUNCH_OVERLAP
 #include "common.cuh"
 
+// Launches a kernel that calls let_next_kernel_start() and wait_for_previous_kernels() first: its launch then passes under the
+// end of the kernel before it, and the product that follows may ask for its first weights under this one.  For the
+// kernels between the products, which at a few tokens take little longer than a launch.
+template <typename... Params, typename... Args>
+void launch_overlapped(void (*kernel)(Params...), dim3 grid, unsigned block, size_t smem, cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    cfg.attrs = attr;
+    cfg.numAttrs = overlap_attribute(attr);
+    cudaLaunchKernelEx(&cfg, kernel, Params(args)...);      // (the caller looks at the last error)
+}
+
 // ---------------------------------------------------------------------------
 // Embedding rows: out[t, :] = table[ids[t], :] * scale, float32 out.
 // A negative id (a padded row) gives zeros.  With a table of learned position
@@ -183,6 +199,8 @@ __global__ void __launch_bounds__(256)
 rmsnorm_pair_kernel(const float* __restrict__ b, float* __restrict__ r, const void* __restrict__ g1, float off1,
                     const void* __restrict__ g2, float off2, int g_dt, void* __restrict__ y, int y_dt, int dim,
                     float eps1, float eps2) {
+    let_next_kernel_start();
+    wait_for_previous_kernels();
     __shared__ float scratch[33];
     const int row = blockIdx.x, n4 = dim >> 2;
     float4 v[kVec];
@@ -239,10 +257,10 @@ extern "C" int nncpu_rmsnorm_pair(const float* b, float* r, const void* g1, floa
              "rmsnorm_pair: rows must be 16-byte aligned and the branch must not be the stream");
     if (n_rows == 0) return 0;
     cudaStream_t st = (cudaStream_t)stream;
-    if (dim <= 256 * 4) rmsnorm_pair_kernel<1><<<n_rows, 256, 0, st>>>(b, r, g1, off1, g2, off2, g_dt, y, y_dt, dim, eps1, eps2);
-    else if (dim <= 256 * 4 * 2) rmsnorm_pair_kernel<2><<<n_rows, 256, 0, st>>>(b, r, g1, off1, g2, off2, g_dt, y, y_dt, dim, eps1, eps2);
-    else if (dim <= 256 * 4 * 4) rmsnorm_pair_kernel<4><<<n_rows, 256, 0, st>>>(b, r, g1, off1, g2, off2, g_dt, y, y_dt, dim, eps1, eps2);
-    else rmsnorm_pair_kernel<8><<<n_rows, 256, 0, st>>>(b, r, g1, off1, g2, off2, g_dt, y, y_dt, dim, eps1, eps2);
+    if (dim <= 256 * 4) launch_overlapped(rmsnorm_pair_kernel<1>, dim3(n_rows), 256, 0, st, b, r, g1, off1, g2, off2, g_dt, y, y_dt, dim, eps1, eps2);
+    else if (dim <= 256 * 4 * 2) launch_overlapped(rmsnorm_pair_kernel<2>, dim3(n_rows), 256, 0, st, b, r, g1, off1, g2, off2, g_dt, y, y_dt, dim, eps1, eps2);
+    else if (dim <= 256 * 4 * 4) launch_overlapped(rmsnorm_pair_kernel<4>, dim3(n_rows), 256, 0, st, b, r, g1, off1, g2, off2, g_dt, y, y_dt, dim, eps1, eps2);
+    else launch_overlapped(rmsnorm_pair_kernel<8>, dim3(n_rows), 256, 0, st, b, r, g1, off1, g2, off2, g_dt, y, y_dt, dim, eps1, eps2);
     NN_LAUNCH_OK("rmsnorm_pair");
     return 0;
 }
@@ -1228,6 +1246,8 @@ extern "C" int nncpu_xielu(const void* x, int in_dt, const void* params, int p_d
 // Soft cap in place: x <- cap * tanh(x / cap), float32.
 // ---------------------------------------------------------------------------
 __global__ void softcap_kernel(float* __restrict__ x, long n, float cap) {
+    let_next_kernel_start();
+    wait_for_previous_kernels();
     const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx < n) x[idx] = cap * tanhf(x[idx] / cap);
 }
@@ -1235,7 +1255,7 @@ __global__ void softcap_kernel(float* __restrict__ x, long n, float cap) {
 extern "C" int nncpu_softcap(float* x, long n, float cap, void* stream) {
     NN_CHECK(n >= 0 && cap > 0.0f, "softcap: %ld elements, cap %g", n, cap);
     if (n == 0) return 0;
-    softcap_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(x, n, cap);
+    launch_overlapped(softcap_kernel, dim3((unsigned)((n + 255) / 256)), 256, 0, (cudaStream_t)stream, x, n, cap);
     NN_LAUNCH_OK("softcap");
     return 0;
 }
@@ -2042,6 +2062,8 @@ extern "C" int nncpu_sample_temperature(const float* logits, const double* u, in
 // ---------------------------------------------------------------------------
 __global__ void stream_add_kernel(float* __restrict__ x, const float* __restrict__ rows, const void* __restrict__ vec,
                                   int vec_dt, long total, int dim) {
+    let_next_kernel_start();
+    wait_for_previous_kernels();
     const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= total) return;
     float v = x[idx];
@@ -2055,7 +2077,7 @@ extern "C" int nncpu_stream_add(float* x, const float* rows, const void* vec, in
     NN_CHECK(n_tok >= 0 && dim > 0, "stream add: %d rows of %d", n_tok, dim);
     if (n_tok == 0 || (rows == nullptr && vec == nullptr)) return 0;
     const long total = (long)n_tok * dim;
-    stream_add_kernel<<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(x, rows, vec, vec_dt, total, dim);
+    launch_overlapped(stream_add_kernel, dim3((unsigned)((total + 255) / 256)), 256, 0, (cudaStream_t)stream, x, rows, vec, vec_dt, total, dim);
     NN_LAUNCH_OK("stream add");
     return 0;
 }
@@ -2091,6 +2113,8 @@ template <int kVec>
 __global__ void __launch_bounds__(256)
 rmsnorm_dual_f32_kernel(const float* __restrict__ x, const void* __restrict__ g1, const void* __restrict__ g2, int g_dt,
                         float eps1, float eps2, void* __restrict__ y1, void* __restrict__ y2, int y_dt, int dim) {
+    let_next_kernel_start();
+    wait_for_previous_kernels();
     __shared__ float scratch[33];
     const int n4 = dim >> 2;
     const float4* src = reinterpret_cast<const float4*>(x + (size_t)blockIdx.x * dim);
@@ -2138,7 +2162,7 @@ extern "C" int nncpu_rmsnorm_dual(const float* x, const void* g1, const void* g2
         (uintptr_t)y2 % 16 == 0) {
         const auto kernel = dim <= 256 * 4 * 2 ? rmsnorm_dual_f32_kernel<2> : dim <= 256 * 4 * 4 ? rmsnorm_dual_f32_kernel<4>
                                                                                                     : rmsnorm_dual_f32_kernel<8>;
-        kernel<<<n_rows, 256, 0, (cudaStream_t)stream>>>(x, g1, g2, g_dt, eps1, eps2, y1, y2, y_dt, dim);
+        launch_overlapped(kernel, dim3(n_rows), 256, 0, (cudaStream_t)stream, x, g1, g2, g_dt, eps1, eps2, y1, y2, y_dt, dim);
         NN_LAUNCH_OK("rmsnorm (two outputs)");
         return 0;
     }
@@ -2656,6 +2680,8 @@ __global__ void __launch_bounds__(256)
 moe_router_kernel(const void* __restrict__ x, int x_dt, const void* __restrict__ w, int w_dt, const void* __restrict__ bias,
                   int b_dt, int n_tok, int per_block, int n_experts, int top, int width, int* __restrict__ ids,
                   float* __restrict__ weights, const RouteRule rule, float* __restrict__ gate) {
+    let_next_kernel_start();
+    wait_for_previous_kernels();
     extern __shared__ float smem[];          // a token's input, then its logits
     float* z = smem + width;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
@@ -2694,8 +2720,7 @@ extern "C" int nncpu_moe_router(const void* x, int x_dt, const void* w, int w_dt
     // One token a block: with several a block the router's rows did not stay in L1 and the grid got too small
     // (2 048 tokens of 4 096 lanes, 16 experts: 88 us a launch with one token a block, 124 us with eight).
     const int per_block = 1;
-    moe_router_kernel<<<(n_tok + per_block - 1) / per_block, 256, (size_t)(width + n_experts + rule.extra(n_experts)) * 4,
-                        (cudaStream_t)stream>>>(x, x_dt, w, w_dt, bias, b_dt, n_tok, per_block, n_experts, top, width, ids,
+    launch_overlapped(moe_router_kernel, dim3((n_tok + per_block - 1) / per_block), 256, (size_t)(width + n_experts + rule.extra(n_experts)) * 4, (cudaStream_t)stream, x, x_dt, w, w_dt, bias, b_dt, n_tok, per_block, n_experts, top, width, ids,
                                                 weights, rule, gate);
     NN_LAUNCH_OK("router");
     return 0;
@@ -2827,6 +2852,8 @@ __global__ void __launch_bounds__(1024)
 moe_plan_kernel(const int* __restrict__ ids, int n_slots, int n_experts, int* __restrict__ row_of_slot,
                 int* __restrict__ slot_of_row, int* __restrict__ n_tiles, int* __restrict__ tile_group,
                 int* __restrict__ tile_row0, int* __restrict__ tile_row_end, int max_tiles) {
+    let_next_kernel_start();
+    wait_for_previous_kernels();
     extern __shared__ int plan_smem[];
     int* count = plan_smem;
     int* offset = plan_smem + n_experts;
@@ -2870,7 +2897,7 @@ extern "C" int nncpu_moe_plan(const int* ids, int n_slots, int n_experts, int* r
                               void* stream) {
     NN_CHECK(n_slots > 0 && n_experts > 0 && n_experts <= kRouteMaxExperts && max_tiles >= (n_slots + 127) / 128 + n_experts,
              "experts (plan): %d slots, %d experts, room for %d tiles", n_slots, n_experts, max_tiles);
-    moe_plan_kernel<<<1, 1024, ((size_t)3 * n_experts + 1) * sizeof(int), (cudaStream_t)stream>>>(
+    launch_overlapped(moe_plan_kernel, dim3(1), 1024, ((size_t)3 * n_experts + 1) * sizeof(int), (cudaStream_t)stream, 
         ids, n_slots, n_experts, row_of_slot, slot_of_row, n_tiles, tile_group, tile_row0, tile_row_end, max_tiles);
     NN_LAUNCH_OK("experts (plan)");
     return 0;
@@ -2879,6 +2906,8 @@ extern "C" int nncpu_moe_plan(const int* ids, int n_slots, int n_experts, int* r
 __global__ void __launch_bounds__(256)
 moe_gather_kernel(const void* __restrict__ x, int x_dt, const int* __restrict__ slot_of_row, int top,
                   const float* __restrict__ weights, __nv_bfloat16* __restrict__ xs, int width) {
+    let_next_kernel_start();
+    wait_for_previous_kernels();
     const int row = blockIdx.x;
     if (slot_of_row[row] < 0) return;       // no slot came here: no product reads the row for a result
     const int t = slot_of_row[row] / top;
@@ -2916,7 +2945,7 @@ moe_gather_kernel(const void* __restrict__ x, int x_dt, const int* __restrict__ 
 extern "C" int nncpu_moe_gather(const void* x, int x_dt, const int* slot_of_row, int top, const float* weights, void* xs,
                                 int n_slots, int width, void* stream) {
     NN_CHECK(n_slots > 0 && top > 0 && width > 0, "experts (gather): %d slots of %d", n_slots, width);
-    moe_gather_kernel<<<n_slots, 256, 0, (cudaStream_t)stream>>>(x, x_dt, slot_of_row, top, weights, (__nv_bfloat16*)xs, width);
+    launch_overlapped(moe_gather_kernel, dim3(n_slots), 256, 0, (cudaStream_t)stream, x, x_dt, slot_of_row, top, weights, (__nv_bfloat16*)xs, width);
     NN_LAUNCH_OK("experts (gather)");
     return 0;
 }
@@ -2925,6 +2954,8 @@ __global__ void __launch_bounds__(256)
 moe_combine_kernel(const void* __restrict__ y, int y_dt, const int* __restrict__ row_of_slot,
                    const float* __restrict__ weights, float* __restrict__ out, int top, int width,
                    const void* __restrict__ x, int x_dt, int fresh) {
+    let_next_kernel_start();
+    wait_for_previous_kernels();
     const int t = blockIdx.x;
     if (y_dt == DT_F32 && (width & 3) == 0) {
         // 16 bytes a thread; the choices' rows are asked for one after the other and added in their order
@@ -2969,6 +3000,8 @@ moe_combine_close_kernel(const float* __restrict__ y, const int* __restrict__ ro
                          float* __restrict__ out, int top, int width, const float* __restrict__ branch,
                          const float* __restrict__ gate, const void* __restrict__ gamma, int g_dt, float gamma_offset,
                          float eps, void* __restrict__ norm_out, int norm_dt) {
+    let_next_kernel_start();
+    wait_for_previous_kernels();
     __shared__ float scratch[33];
     const int t = blockIdx.x, n4 = width >> 2;
     const float g = branch != nullptr ? (gate != nullptr ? gate[t] : 1.0f) : 0.0f;
@@ -3030,7 +3063,7 @@ extern "C" int nncpu_moe_combine(const void* y, int y_dt, const int* row_of_slot
     NN_CHECK(n_tok > 0 && top > 0 && width > 0, "experts (combine): %d tokens of %d", n_tok, width);
     NN_CHECK((uintptr_t)x % 16 == 0, "experts (combine): rows must be 16-byte aligned");
     if (branch == nullptr && norm_out == nullptr && weights != nullptr) {
-        moe_combine_kernel<<<n_tok, 256, 0, (cudaStream_t)stream>>>(y, y_dt, row_of_slot, weights, out, top, width, x, x_dt,
+        launch_overlapped(moe_combine_kernel, dim3(n_tok), 256, 0, (cudaStream_t)stream, y, y_dt, row_of_slot, weights, out, top, width, x, x_dt,
                                                                     fresh);
         NN_LAUNCH_OK("experts (combine)");
         return 0;
@@ -3040,7 +3073,7 @@ extern "C" int nncpu_moe_combine(const void* y, int y_dt, const int* row_of_slot
     NN_CHECK(((uintptr_t)y | (uintptr_t)out | (uintptr_t)branch | (uintptr_t)norm_out) % 16 == 0,
              "experts (combine): rows must be 16-byte aligned");
 #define NN_CLOSE(V)                                                                                                     \
-    moe_combine_close_kernel<V><<<n_tok, 256, 0, (cudaStream_t)stream>>>((const float*)y, row_of_slot, weights, out, top, \
+    launch_overlapped(moe_combine_close_kernel<V>, dim3(n_tok), 256, 0, (cudaStream_t)stream, (const float*)y, row_of_slot, weights, out, top, \
                                                                          width, branch, gate, gamma, g_dt, gamma_offset, eps, norm_out, norm_dt)
     if (width <= 256 * 4) NN_CLOSE(1);
     else if (width <= 256 * 4 * 2) NN_CLOSE(2);
@@ -3060,6 +3093,8 @@ moe_combine_pair_kernel(const float* __restrict__ y, const int* __restrict__ row
                         int top, int width, const void* __restrict__ x, int x_dt, float* __restrict__ r,
                         const void* __restrict__ g1, float off1, float eps1, const void* __restrict__ g2, float off2,
                         float eps2, int g_dt, void* __restrict__ y2, int y2_dt) {
+    let_next_kernel_start();
+    wait_for_previous_kernels();
     __shared__ float scratch[33];
     const int t = blockIdx.x, n4 = width >> 2;
     float4 v[kVec];
@@ -3126,7 +3161,7 @@ extern "C" int nncpu_moe_combine_pair(const float* y, const int* row_of_slot, co
     NN_CHECK(((uintptr_t)y | (uintptr_t)x | (uintptr_t)r | (uintptr_t)y2 | (uintptr_t)g1 | (uintptr_t)g2) % 16 == 0,
              "experts (combine): rows must be 16-byte aligned");
 #define NN_PAIR(V)                                                                                                       \
-    moe_combine_pair_kernel<V><<<n_tok, 256, 0, (cudaStream_t)stream>>>(y, row_of_slot, weights, top, width, x, x_dt, r, \
+    launch_overlapped(moe_combine_pair_kernel<V>, dim3(n_tok), 256, 0, (cudaStream_t)stream, y, row_of_slot, weights, top, width, x, x_dt, r, \
                                                                         g1, off1, eps1, g2, off2, eps2, g_dt, y2, y2_dt)
     if (width <= 256 * 4) NN_PAIR(1);
     else if (width <= 256 * 4 * 2) NN_PAIR(2);
@@ -3176,6 +3211,8 @@ template <int kVec>
 __global__ void __launch_bounds__(256)
 layernorm_f32_kernel(const float* __restrict__ x, const void* __restrict__ w, const void* __restrict__ b, int p_dt,
                      void* __restrict__ y, int y_dt, const int* __restrict__ rows, int dim, float eps) {
+    let_next_kernel_start();
+    wait_for_previous_kernels();
     __shared__ float scratch[33];
     const int r_out = blockIdx.x;
     const int r_in = rows ? rows[r_out] : r_out;
@@ -3226,10 +3263,10 @@ extern "C" int nncpu_layernorm(const float* x, const void* w, const void* b, int
     if (n_rows == 0) return 0;
     cudaStream_t st = (cudaStream_t)stream;
     if (dim % 4 == 0 && dim <= 256 * 4 * 8 && ((uintptr_t)x % 16) == 0 && ((uintptr_t)y % 16) == 0) {
-        if (dim <= 1024) layernorm_f32_kernel<1><<<n_rows, 256, 0, st>>>(x, w, b, p_dt, y, y_dt, rows, dim, eps);
-        else if (dim <= 2048) layernorm_f32_kernel<2><<<n_rows, 256, 0, st>>>(x, w, b, p_dt, y, y_dt, rows, dim, eps);
-        else if (dim <= 4096) layernorm_f32_kernel<4><<<n_rows, 256, 0, st>>>(x, w, b, p_dt, y, y_dt, rows, dim, eps);
-        else layernorm_f32_kernel<8><<<n_rows, 256, 0, st>>>(x, w, b, p_dt, y, y_dt, rows, dim, eps);
+        if (dim <= 1024) launch_overlapped(layernorm_f32_kernel<1>, dim3(n_rows), 256, 0, st, x, w, b, p_dt, y, y_dt, rows, dim, eps);
+        else if (dim <= 2048) launch_overlapped(layernorm_f32_kernel<2>, dim3(n_rows), 256, 0, st, x, w, b, p_dt, y, y_dt, rows, dim, eps);
+        else if (dim <= 4096) launch_overlapped(layernorm_f32_kernel<4>, dim3(n_rows), 256, 0, st, x, w, b, p_dt, y, y_dt, rows, dim, eps);
+        else launch_overlapped(layernorm_f32_kernel<8>, dim3(n_rows), 256, 0, st, x, w, b, p_dt, y, y_dt, rows, dim, eps);
         NN_LAUNCH_OK("layernorm");
         return 0;
     }

@@ -412,15 +412,6 @@ f32_slices_kernel(const ManyParams p) {
     st_f(p.out, o, p.out_dt, v);
 }
 
-int sm_count() {
-    static int counts[64] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-    if (counts[dev] == 0 && cudaDeviceGetAttribute(&counts[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        counts[dev] = 148;
-    return counts[dev];
-}
-
 // How a product is cut: tokens in equal tiles of at most 256 (a multiple of 32), K in slices.
 struct ManyPlan {
     int bn, tiles_b, slices;

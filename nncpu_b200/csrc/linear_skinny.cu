@@ -278,15 +278,6 @@ skinny_kernel(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restri
     }
 }
 
-int sm_count() {
-    static int counts[64] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-    if (counts[dev] == 0 && cudaDeviceGetAttribute(&counts[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        counts[dev] = 148;
-    return counts[dev];
-}
-
 // Blocks of 4 warps (four per SM) or of 8 (two per SM)?  What a product costs beyond its bytes are the round trips
 // to memory that follow one another: a warp makes one per round of `unroll` groups of its share of K, and a grid
 // makes one pass per filling of the SMs' places.  The smaller count of (passes x rounds) wins; on a tie the

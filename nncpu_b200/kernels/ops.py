@@ -91,6 +91,10 @@ def add_launches(n: int) -> None:
 _last_fn = ""      # the entry point that launched last (a hint for launches that can overlap with their like)
 
 
+# The kernels under whose end a few-token product may start: they use little shared memory (see linear_skinny.cu).
+_BEFORE_SKINNY = frozenset(("nncpu_linear_skinny", "nncpu_rmsnorm", "nncpu_rmsnorm_pair", "nncpu_rmsnorm_dual", "nncpu_layernorm",
+                            "nncpu_moe_combine", "nncpu_moe_combine_pair", "nncpu_stream_add", "nncpu_linear_skinny_grouped"))
+
 _entry_points = {}     # (library, function) -> (the function, its library): found once
 
 
@@ -478,7 +482,7 @@ def linear_skinny(x, w, bias, out, accumulate: bool = False, epilogue: str = "pl
         bins_in, eps = norm_in
         assert bins_in.dtype == torch.int64 and bins_in.numel() == NORM_WORDS
     # a product that follows another one may start while that one ends (see launch_overlap)
-    after_skinny = _last_fn == "nncpu_linear_skinny"
+    after_skinny = _last_fn in _BEFORE_SKINNY
     _call("linear_skinny", "nncpu_linear_skinny", _ptr(x), _ptr(w), _ptr(bias), _i(_code(bias)), _ptr(out),
           _i(_code(out)), _i(m), _i(n), _i(k), _i(k), _i(out.shape[1]), _i(accumulate), _i(EPILOGUES[epilogue]),
           _ptr(xg), _ptr(gamma), _i(_code(gamma)), _ptr(bins_out), _ptr(bins_clear), _ptr(bins_in), _f(eps),
