@@ -18,6 +18,7 @@
 #include <math.h>
 
 #define NN_LIB attention_f32
+#define NN_LAUNCH_OVERLAP
 #include "common.cuh"
 
 namespace {
@@ -75,6 +76,8 @@ decode_f32_kernel(const AttnF32 p) {
     __shared__ float sc[kDecodeKeys][GB];
     __shared__ float red[4][GB];
     __shared__ __align__(16) float part_o[4][GB][128];
+    let_next_kernel_start();
+    wait_for_previous_kernels();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int group = p.n_heads / p.n_kv, per_kv = (group + GB - 1) / GB;
     const int kvh = blockIdx.x / per_kv, g0 = (blockIdx.x % per_kv) * GB;
@@ -213,6 +216,8 @@ decode_f32_kernel(const AttnF32 p) {
 // Adds the stretches' parts in their order: a block per (head, token), a thread per lane of the values.
 __global__ void __launch_bounds__(128)
 merge_f32_kernel(const AttnF32 p) {
+    let_next_kernel_start();
+    wait_for_previous_kernels();
     const int h = blockIdx.x, t = blockIdx.y, d = threadIdx.x;
     const size_t out = ((size_t)t * p.n_heads + h) * p.vo + d;
     if (p.tok_seq[t] < 0) {
@@ -465,13 +470,22 @@ extern "C" int nncpu_attention_f32(const void* q, const void* k_pages, const voi
         long per = (8L * sm_count + pairs - 1) / pairs;
         if (per > n_chunks) per = n_chunks;
         const dim3 grid((unsigned)blocks_x, (unsigned)per, (unsigned)n_tok);
-        if (gb == 8) decode_f32_kernel<8><<<grid, 128, 0, st>>>(p);
-        else if (gb == 4) decode_f32_kernel<4><<<grid, 128, 0, st>>>(p);
-        else if (gb == 2) decode_f32_kernel<2><<<grid, 128, 0, st>>>(p);
-        else decode_f32_kernel<1><<<grid, 128, 0, st>>>(p);
-        NN_LAUNCH_OK("attention (32-bit)");
-        if (n_chunks > 1) merge_f32_kernel<<<dim3(n_heads, n_tok), 128, 0, st>>>(p);
-        NN_LAUNCH_OK("attention (32-bit, merge)");
+        // both launched to start while the kernel before them ends: their launches are as long as their work
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = grid;
+        cfg.blockDim = dim3(128);
+        cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        cfg.attrs = attr;
+        cfg.numAttrs = overlap_attribute(attr);
+        const auto kernel = gb == 8 ? decode_f32_kernel<8> : gb == 4 ? decode_f32_kernel<4> : gb == 2 ? decode_f32_kernel<2> : decode_f32_kernel<1>;
+        cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
+        NN_CHECK(e == cudaSuccess, "attention (32-bit): launch failed: %s", cudaGetErrorString(e));
+        if (n_chunks > 1) {
+            cfg.gridDim = dim3((unsigned)n_heads, (unsigned)n_tok);
+            e = cudaLaunchKernelEx(&cfg, merge_f32_kernel, p);
+            NN_CHECK(e == cudaSuccess, "attention (32-bit, merge): launch failed: %s", cudaGetErrorString(e));
+        }
         return 0;
     }
     const int per_block = kRowsQ / group;

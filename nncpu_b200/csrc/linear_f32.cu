@@ -395,12 +395,37 @@ f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     }
 }
 
-// Adds the slices' sums in their order, then bias and what is already there.
+// Adds the slices' sums in their order, then bias and what is already there.  Bound by the slices' passes through L2; kVec: four
+// features a thread (N and ldc multiples of 4, 32-bit output), else one.  A layer of 300 tokens (hidden 2048) spent 50 us
+// of 329 here one feature at a time.
+template <bool kVec>
 __global__ void __launch_bounds__(256)
 f32_slices_kernel(const ManyParams p) {
     let_next_kernel_start();
     wait_for_previous_kernels();
     const long total = (long)p.M * p.N;
+    if constexpr (kVec) {
+        const long e = ((long)blockIdx.x * 256 + threadIdx.x) * 4;
+        if (e >= total) return;
+        const int t = (int)(e / p.N), row = (int)(e % p.N);
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 4
+        for (int s = 0; s < p.slices; ++s) {
+            const float4 x = __ldcs(reinterpret_cast<const float4*>(p.part + (size_t)s * total + e));
+            v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+        }
+        if (p.bias) {
+            v.x += ld_f(p.bias, row, p.bias_dt); v.y += ld_f(p.bias, row + 1, p.bias_dt);
+            v.z += ld_f(p.bias, row + 2, p.bias_dt); v.w += ld_f(p.bias, row + 3, p.bias_dt);
+        }
+        float4* at = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + (size_t)t * p.ldc + row);
+        if (p.accumulate) {
+            const float4 x = *at;
+            v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+        }
+        *at = v;
+        return;
+    }
     const long e = ((long)blockIdx.x * 256 + threadIdx.x);
     if (e >= total) return;
     const int t = (int)(e / p.N), row = (int)(e % p.N);
@@ -481,10 +506,12 @@ int launch_many(const ManyParams& p, cudaStream_t stream) {
     cudaError_t e = cudaLaunchKernelEx(&cfg, f32_many_kernel<BN>, mw, mx, p);
     NN_CHECK(e == cudaSuccess, "linear (32-bit): launch failed: %s", cudaGetErrorString(e));
     if (p.slices > 1) {
-        cfg.gridDim = dim3((unsigned)(((long)p.M * p.N + 255) / 256));
+        const bool vec = p.N % 4 == 0 && p.ldc % 4 == 0 && p.out_dt == DT_F32 && (uintptr_t)p.out % 16 == 0 && (uintptr_t)p.part % 16 == 0;
+        const long per = vec ? 1024 : 256;
+        cfg.gridDim = dim3((unsigned)(((long)p.M * p.N + per - 1) / per));
         cfg.blockDim = dim3(256);
         cfg.dynamicSmemBytes = 0;
-        e = cudaLaunchKernelEx(&cfg, f32_slices_kernel, p);
+        e = vec ? cudaLaunchKernelEx(&cfg, f32_slices_kernel<true>, p) : cudaLaunchKernelEx(&cfg, f32_slices_kernel<false>, p);
         NN_CHECK(e == cudaSuccess, "linear (32-bit, adding slices): launch failed: %s", cudaGetErrorString(e));
     }
     return 0;

@@ -119,7 +119,7 @@ def launch_overlap(on: bool) -> None:
     tensor-core products (their set-up; up to 64 tokens also their first weight tiles), prefill attention (its
     set-up) and the norms between them.
     On by default; off, every kernel waits for the one before it to be over, and the results are the same bits."""
-    for name in ("linear_skinny", "gemm_sm100", "generic", "attention_tc", "linear_f32"):
+    for name in ("linear_skinny", "gemm_sm100", "generic", "attention_tc", "linear_f32", "attention_f32"):
         getattr(library.load(name), f"nncpu_launch_overlap_{name}")(ctypes.c_int(1 if on else 0))
 
 

@@ -48,7 +48,7 @@ def test_few_token_product(ops, m, n, k):
 
 
 @pytest.mark.parametrize("m", [1, 17, 32, 33, 64, 90, 128, 160, 190, 224, 256, 257, 300, 520])
-@pytest.mark.parametrize("n,k", [(5, 4), (128, 32), (129, 36), (200, 100), (300, 1000), (1536, 2048), (256, 6144)])
+@pytest.mark.parametrize("n,k", [(5, 4), (128, 32), (129, 36), (200, 100), (201, 1000), (300, 1000), (1536, 2048), (256, 6144)])
 def test_many_token_product(ops, m, n, k):
     """On the tensor cores with numbers cut in two: the bound of a 32-bit sum holds, and over longer sums the error is no
     larger than that of the general kernel, which adds k products one after the other."""
