@@ -1170,6 +1170,8 @@ extern "C" int nncpu_attention(const void* q, int q_dt, const void* k_pages, con
 // ---------------------------------------------------------------------------
 __global__ void gated_act_kernel(const void* __restrict__ gu, int in_dt, void* __restrict__ out, int out_dt,
                                  long n_tok, int inter, int kind, float limit) {
+    let_next_kernel_start();
+    wait_for_previous_kernels();
     const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= n_tok * inter) return;
     const long t = idx / inter;
@@ -1185,7 +1187,7 @@ extern "C" int nncpu_gated_act(const void* gu, int in_dt, void* out, int out_dt,
     NN_CHECK(kind >= kGateSilu && kind <= kGateSwishClamp, "gated activation: kind %d", kind);
     if (n_tok == 0) return 0;
     const long total = (long)n_tok * inter;
-    gated_act_kernel<<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(gu, in_dt, out, out_dt, n_tok,
+    launch_overlapped(gated_act_kernel, dim3((unsigned)((total + 255) / 256)), 256, 0, (cudaStream_t)stream, gu, in_dt, out, out_dt, n_tok,
                                                                                          inter, kind, limit);
     NN_LAUNCH_OK("gated activation");
     return 0;
@@ -2277,10 +2279,16 @@ latent_append_kernel(const float* __restrict__ proj, int ld, int col, const void
                      int qn_rank, void* __restrict__ cq_out, int cq_dt) {
     __shared__ float scratch[33];
     const int t = blockIdx.x;
-    if (q_out != nullptr)
-        for (int i = threadIdx.x; i < q_size; i += blockDim.x)
+    // With few tokens the three parts (the kept row; the query's norm; the query's lanes) are blocks of their own, else one
+    // block does all: the numbers are the same.
+    const int part = blockIdx.y, parts = gridDim.y;
+    if (q_out != nullptr && (parts == 1 || part >= 2)) {
+        const int copiers = parts == 1 ? 1 : parts - 2, me = parts == 1 ? 0 : part - 2;
+        for (int i = me * blockDim.x + threadIdx.x; i < q_size; i += copiers * blockDim.x)
             q_out[(size_t)t * q_size + i] = __float2bfloat16_rn(proj[(size_t)t * ld + i]);
-    if (qn_gamma != nullptr) {
+    }
+    if (part >= 2) return;
+    if (qn_gamma != nullptr && (parts == 1 || part == 1)) {
         const float* zq = proj + (size_t)t * ld + qn_col;
         float sq = 0.0f;
         for (int i = threadIdx.x; i < qn_rank; i += blockDim.x) sq = fmaf(zq[i], zq[i], sq);
@@ -2289,6 +2297,7 @@ latent_append_kernel(const float* __restrict__ proj, int ld, int col, const void
         for (int i = threadIdx.x; i < qn_rank; i += blockDim.x)
             st_f(cq_out, (size_t)t * qn_rank + i, cq_dt, (zq[i] * sc) * ld_f(qn_gamma, i, g_dt));
     }
+    if (part != 0) return;
     const int seq = tok_seq[t];
     if (seq < 0 || pages == nullptr) return;   // a padded row owns no place in the cache
     const float* z = proj + (size_t)t * ld + col;
@@ -2324,7 +2333,9 @@ extern "C" int nncpu_latent_append(const float* proj, int ld, int col, const voi
     NN_CHECK(qn_gamma == nullptr || (qn_rank > 0 && qn_col >= 0 && qn_col + qn_rank <= ld && cq_out != nullptr),
              "latent append: a query latent of %d lanes at column %d of %d", qn_rank, qn_col, ld);
     if (n_tok == 0) return 0;
-    latent_append_kernel<<<n_tok, 128, 0, (cudaStream_t)stream>>>(proj, ld, col, gamma, g_dt, eps, tok_seq, tok_pos,
+    // (one block a token walked through the parts one after the other: 9.6 us for four tokens with a query latent of 1 536)
+    const int parts = n_tok * 6 <= sm_count() * 4 ? (q_out != nullptr ? 6 : 2) : 1;
+    latent_append_kernel<<<dim3(n_tok, parts), 128, 0, (cudaStream_t)stream>>>(proj, ld, col, gamma, g_dt, eps, tok_seq, tok_pos,
                                                                   block_table, bt_stride, pages, kv_dt, rank,
                                                                   (__nv_bfloat16*)q_out, q_size, rot_dim,
                                                                   (const float2*)cs, rot_half, qn_gamma, qn_col, qn_rank,
@@ -2345,12 +2356,15 @@ latent_query_kernel(const float* __restrict__ q, int n_heads, int hd, int rot_di
                     int rot_half, void* __restrict__ q_lat, int lat_dt, int rank, __nv_bfloat16* __restrict__ q16) {
     const int t = blockIdx.x;
     const int per = hd + rot_dim;
-    const float* row = q + (size_t)t * n_heads * per;
+    const int heads = n_heads;
+    const float* row = q + (size_t)t * heads * per;
+    const size_t o = (size_t)t * heads * (rank + rot_dim);
+    // this block's heads (gridDim.y blocks share a token's)
+    const int first = (int)((long)blockIdx.y * heads / gridDim.y), last = (int)((long)(blockIdx.y + 1) * heads / gridDim.y);
     if (q16 != nullptr)
-        for (int i = threadIdx.x; i < n_heads * per; i += blockDim.x)
-            q16[(size_t)t * n_heads * per + i] = __float2bfloat16_rn(row[i]);
-    const size_t o = (size_t)t * n_heads * (rank + rot_dim);
-    for (int idx = threadIdx.x; idx < n_heads * rot_half; idx += blockDim.x) {
+        for (int i = first * per + threadIdx.x; i < last * per; i += blockDim.x)
+            q16[(size_t)t * heads * per + i] = __float2bfloat16_rn(row[i]);
+    for (int idx = first * rot_half + threadIdx.x; idx < last * rot_half; idx += blockDim.x) {
         const int a = idx / rot_half, i = idx % rot_half;
         const float2 c = cs[(size_t)t * rot_half + i];
         const float u = row[a * per + hd + 2 * i], v = row[a * per + hd + 2 * i + 1];
@@ -2358,7 +2372,7 @@ latent_query_kernel(const float* __restrict__ q, int n_heads, int hd, int rot_di
         st_f(q_lat, o + (size_t)a * (rank + rot_dim) + rank + 2 * i + 1, lat_dt, c.x * v + c.y * u);
     }
     const int rest = rot_dim - 2 * rot_half;
-    for (int idx = threadIdx.x; idx < n_heads * rest; idx += blockDim.x) {
+    for (int idx = first * rest + threadIdx.x; idx < last * rest; idx += blockDim.x) {
         const int a = idx / rest, i = 2 * rot_half + idx % rest;
         st_f(q_lat, o + (size_t)a * (rank + rot_dim) + rank + i, lat_dt, row[a * per + hd + i]);
     }
@@ -2370,7 +2384,10 @@ extern "C" int nncpu_latent_query(const float* q, int n_tok, int n_heads, int hd
     NN_CHECK(rot_half >= 0 && 2 * rot_half <= rot_dim && (rot_half == 0 || cs != nullptr) && (uintptr_t)cs % 8 == 0,
              "latent query: %d rotated pairs of %d lanes", rot_half, rot_dim);
     if (n_tok == 0) return 0;
-    latent_query_kernel<<<n_tok, 128, 0, (cudaStream_t)stream>>>(q, n_heads, hd, rot_dim, (const float2*)cs, rot_half,
+    // With few tokens several blocks share a token's heads (one block: 12 us for four tokens of 32 heads).
+    int share = sm_count() * 4 / n_tok;
+    share = share < 1 ? 1 : (share > n_heads ? n_heads : share);
+    latent_query_kernel<<<dim3(n_tok, share), 128, 0, (cudaStream_t)stream>>>(q, n_heads, hd, rot_dim, (const float2*)cs, rot_half,
                                                                  q_lat, lat_dt, rank, (__nv_bfloat16*)q16);
     NN_LAUNCH_OK("latent query");
     return 0;
