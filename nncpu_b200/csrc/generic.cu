@@ -2855,7 +2855,7 @@ extern "C" int nncpu_moe_experts(const void* x, int x_dt, const void* wg, const 
 // as one grouped product on the tensor cores (gemm_sm100.cu), and the choices of a token are added up afterwards.
 //   plan: counts the slots of every expert, gives every slot a row (its expert's rows follow one another; the order
 //     inside an expert is whatever the atomics give, which changes no result: a row's product does not depend on its
-//     place), and lists the 128-row tiles of the grouped product.  A slot whose id lies beyond the experts (an identity
+//     place), and lists the tiles of the grouped product, of at most `tile_rows` rows each.  A slot whose id lies beyond the experts (an identity
 //     expert) gets row kIdentityRow and takes no part in the products; the rows that are left over hold slot -1.  One block.
 //   gather: xs[row] = x[slot_of_row[row] / top] (times the slot's weight, where that multiplies the experts' input).
 //   combine: out[t] += sum_c weight[t, c] * y[row_of_slot[t * top + c]], choices in their order; with a shared
@@ -2868,7 +2868,7 @@ constexpr int kIdentityRow = -2;
 __global__ void __launch_bounds__(1024)
 moe_plan_kernel(const int* __restrict__ ids, int n_slots, int n_experts, int* __restrict__ row_of_slot,
                 int* __restrict__ slot_of_row, int* __restrict__ n_tiles, int* __restrict__ tile_group,
-                int* __restrict__ tile_row0, int* __restrict__ tile_row_end, int max_tiles) {
+                int* __restrict__ tile_row0, int* __restrict__ tile_row_end, int max_tiles, int tile_rows) {
     let_next_kernel_start();
     wait_for_previous_kernels();
     extern __shared__ int plan_smem[];
@@ -2886,7 +2886,7 @@ moe_plan_kernel(const int* __restrict__ ids, int n_slots, int n_experts, int* __
         int acc = 0, tiles = 0;
         for (int e = 0; e < n_experts; ++e) {
             offset[e] = acc;
-            for (int r = 0; r < count[e]; r += 128, ++tiles) {
+            for (int r = 0; r < count[e]; r += tile_rows, ++tiles) {
                 if (tiles < max_tiles) {
                     tile_group[tiles] = e;
                     tile_row0[tiles] = acc + r;
@@ -2911,11 +2911,12 @@ moe_plan_kernel(const int* __restrict__ ids, int n_slots, int n_experts, int* __
 
 extern "C" int nncpu_moe_plan(const int* ids, int n_slots, int n_experts, int* row_of_slot, int* slot_of_row,
                               int* n_tiles, int* tile_group, int* tile_row0, int* tile_row_end, int max_tiles,
-                              void* stream) {
-    NN_CHECK(n_slots > 0 && n_experts > 0 && n_experts <= kRouteMaxExperts && max_tiles >= (n_slots + 127) / 128 + n_experts,
-             "experts (plan): %d slots, %d experts, room for %d tiles", n_slots, n_experts, max_tiles);
+                              int tile_rows, void* stream) {
+    NN_CHECK(n_slots > 0 && n_experts > 0 && n_experts <= kRouteMaxExperts && tile_rows > 0 &&
+                 max_tiles >= (n_slots + tile_rows - 1) / tile_rows + n_experts,
+             "experts (plan): %d slots, %d experts, room for %d tiles of %d rows", n_slots, n_experts, max_tiles, tile_rows);
     launch_overlapped(moe_plan_kernel, dim3(1), 1024, ((size_t)3 * n_experts + 1) * sizeof(int), (cudaStream_t)stream, 
-        ids, n_slots, n_experts, row_of_slot, slot_of_row, n_tiles, tile_group, tile_row0, tile_row_end, max_tiles);
+        ids, n_slots, n_experts, row_of_slot, slot_of_row, n_tiles, tile_group, tile_row0, tile_row_end, max_tiles, tile_rows);
     NN_LAUNCH_OK("experts (plan)");
     return 0;
 }

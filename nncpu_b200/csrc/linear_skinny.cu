@@ -72,7 +72,8 @@ __device__ __forceinline__ uint4 ldg16_stream(const __nv_bfloat16* p) {
 
 
 // The few-token products of routed experts (kGrouped): blockIdx.y names a group of rows that share a matrix, by the plan that
-// sorts a step's rows (tile t: matrix tile_group[t], rows tile_row0[t] .. tile_row_end[t] - 1, at most 16 of them).
+// sorts a step's rows (tile t: matrix tile_group[t], rows from tile_row0[t] on, at most NT * 8 of them and none from
+// tile_row_end[t] on).
 struct SkinnyGroups {
     const int* n_tiles;
     const int* tile_group;
@@ -400,17 +401,17 @@ extern "C" int nncpu_linear_skinny(const void* X, const void* W, const void* bia
                   : launch<2, kPlain>(X, W, bias, bias_dt, C, c_dt, M, N, K, lda, ldc, accumulate, nf, after_skinny != 0, stream);
 }
 
-// C[r, :] = X[r, :] . W_e^T for the rows r of group e, of which no group has more than 16 (the routed experts of a step of up to
-// 16 tokens): as nncpu_linear_tc_grouped, whose plan and epilogues these are, with every weight of a group that has rows
-// read once.  The tensor-core kernel gives a group a tile of 128 rows whatever it has and a single SM 256 features of it:
-// 16 rows of 16 experts, gate/up of 3072 x 2048 each, took it 48 us and the down product 26 us.  most_rows: the most
-// rows a group can have; max_tiles: the most groups that can have rows.
+// C[r, :] = X[r, :] . W_e^T for the rows r of group e, in tiles of at most 8 or 16 rows (the routed experts of a step of up to
+// 16 tokens, where as good as every group with rows is one tile): as nncpu_linear_tc_grouped, whose epilogues these are, with
+// every weight of such a group read once.  The tensor-core kernel gives a group a tile of 128 rows whatever it has and a single SM 256 features of it:
+// 16 rows of 16 experts, gate/up of 3072 x 2048 each, took it 48 us and the down product 26 us.  most_rows: the step's
+// tokens (tiles of 8 rows up to 8 of them, else of 16); max_tiles: the most tiles the plan can have.
 extern "C" int nncpu_linear_skinny_grouped(const void* X, const void* W, void* C, int c_dt, int S, int N, int K, int n_groups,
                                            int lda, int ldc, int epilogue, int act, float act_a, const int* n_tiles,
                                            const int* tile_group, const int* tile_row0, const int* tile_row_end, int max_tiles,
                                            int most_rows, void* stream_) {
     NN_CHECK(S > 0 && N > 0 && K > 0 && n_groups > 0 && max_tiles > 0 && max_tiles <= 65535 && most_rows > 0 && most_rows <= 16,
-             "linear (few tokens, grouped): %d rows in %d groups of %d x %d, at most %d rows a group", S, n_groups, N, K, most_rows);
+             "linear (few tokens, grouped): %d rows in %d groups of %d x %d, tiles of at most %d rows", S, n_groups, N, K, most_rows);
     NN_CHECK(K % 8 == 0 && lda % 8 == 0 && lda >= K && ((uintptr_t)X % 16) == 0 && ((uintptr_t)W % 16) == 0,
              "linear (few tokens, grouped): K %d and lda %d must be multiples of 8, operands 16-byte aligned", K, lda);
     NN_CHECK(epilogue == kPlain || epilogue == kSwiglu, "linear (few tokens, grouped): unknown epilogue %d", epilogue);

@@ -1066,24 +1066,25 @@ def moe_experts(x, w_gate, w_up, w_down, ids, weights, act, out, kind: str, limi
           _i(identity), _i(fresh), _stream())
 
 
-def moe_plan_tiles(n_slots: int, n_experts: int) -> int:
-    """The most 128-row tiles a grouped product over ``n_slots`` rows in ``n_experts`` groups can have."""
-    return (n_slots + 127) // 128 + n_experts
+def moe_plan_tiles(n_slots: int, n_experts: int, tile_rows: int = 128) -> int:
+    """The most tiles of ``tile_rows`` rows that a grouped product over ``n_slots`` rows in ``n_experts`` groups can have."""
+    return (n_slots + tile_rows - 1) // tile_rows + n_experts
 
 
-def moe_plan(ids, n_experts: int, row_of_slot, slot_of_row, plan) -> None:
+def moe_plan(ids, n_experts: int, row_of_slot, slot_of_row, plan, tile_rows: int = 128) -> None:
     """Sorts the token slots (row-major ``ids`` [n, top]) by expert: ``row_of_slot`` / ``slot_of_row`` (int32 [n * top])
-    map slots to rows and back, and ``plan`` (int32 [1 + 3 * moe_plan_tiles]) receives the number of 128-row tiles and
-    per tile its expert, first row and its expert's last row + 1, for ``linear_tc_grouped``.  A slot whose id is n_experts or
-    more (an identity expert) gets row -2; the rows beyond the experts' slots get slot -1."""
+    map slots to rows and back, and ``plan`` (int32 [1 + 3 * moe_plan_tiles]) receives the number of tiles of at most ``tile_rows``
+    rows and per tile its expert, first row and its expert's last row + 1, for ``linear_tc_grouped`` (128 rows) and
+    ``linear_skinny_grouped`` (``skinny_grouped_rows``).  A slot whose id is n_experts or more (an identity expert) gets row -2;
+    the rows beyond the experts' slots get slot -1."""
     S = ids.numel()
-    mt = moe_plan_tiles(S, n_experts)
+    mt = moe_plan_tiles(S, n_experts, tile_rows)
     assert ids.dtype == row_of_slot.dtype == slot_of_row.dtype == plan.dtype == torch.int32
     assert row_of_slot.numel() == slot_of_row.numel() == S and plan.numel() == 1 + 3 * mt and plan.is_contiguous()
     base, dry = (0 if plan.is_meta else plan.data_ptr()), plan.is_meta and _dry
     at = lambda k: None if dry else _vp(base + 4 * k)
     _call("generic", "nncpu_moe_plan", _ptr(ids), _i(S), _i(n_experts), _ptr(row_of_slot), _ptr(slot_of_row), at(0), at(1),
-          at(1 + mt), at(1 + 2 * mt), _i(mt), _stream())
+          at(1 + mt), at(1 + 2 * mt), _i(mt), _i(tile_rows), _stream())
 
 
 def moe_gather(x, slot_of_row, top: int, xs, weights=None) -> None:
@@ -1159,20 +1160,28 @@ def linear_tc_grouped(xs, w, out, plan, n_experts: int, workspace: GemmWorkspace
 
 
 
+def skinny_grouped_rows(most_rows: int) -> int:
+    """Rows of a tile of ``linear_skinny_grouped``: 8 or 16, for steps of so many tokens."""
+    return 8 if most_rows <= 8 else 16
+
+
 def linear_skinny_grouped(xs, w, out, plan, n_experts: int, most_rows: int, epilogue: str = "plain", activation=None) -> None:
-    """``linear_tc_grouped`` where no expert has more than ``most_rows`` <= 16 rows: a stream over the weights of the experts
-    that have any."""
+    """``linear_tc_grouped`` for steps of ``most_rows`` <= 16 tokens: a stream over the weights of the experts that have any row.
+    ``plan`` is ``moe_plan``'s with tiles of ``skinny_grouped_rows(most_rows)`` rows: a token that is not a number may choose an
+    expert several times, so an expert's rows may be more than the tokens (with tiles of 128 rows they may not)."""
     S, K = xs.shape
     E, N, _ = w.shape
-    mt = moe_plan_tiles(S, n_experts)
+    mt = (plan.numel() - 1) // 3
     assert E == n_experts and w.shape[2] == K and xs.dtype == w.dtype == torch.bfloat16 and w.is_contiguous()
-    assert out.shape == (S, N // 2 if epilogue == "swiglu" else N) and plan.numel() == 1 + 3 * mt
+    assert out.shape == (S, N // 2 if epilogue == "swiglu" else N) and plan.numel() == 1 + 3 * mt >= 1 + 3 * moe_plan_tiles(S, E)
     base, dry = (0 if plan.is_meta else plan.data_ptr()), plan.is_meta and _dry
     at = lambda k: None if dry else _vp(base + 4 * k)
     act, a, _b = _activation(activation)
+    # (every tile but an expert's last is full)
     _call("linear_skinny", "nncpu_linear_skinny_grouped", _ptr(xs), _ptr(w), _ptr(out), _i(_code(out)), _i(S), _i(N), _i(K),
           _i(E), _i(K), _i(out.shape[1]), _i(EPILOGUES[epilogue]), act, a, at(0), at(1), at(1 + mt), at(1 + 2 * mt),
-          _i(min(S, n_experts)), _i(most_rows), _stream())
+          _i(min(S, n_experts + S // skinny_grouped_rows(most_rows))), _i(most_rows), _stream())
+
 
 def xielu(x, params, out) -> None:
     """out = xIELU(x) elementwise with the two learned numbers ``params`` = (p, q): for z > 0

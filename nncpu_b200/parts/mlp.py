@@ -237,11 +237,12 @@ class RoutedExperts(FeedForward):
             # many tokens: sorted by expert, one grouped product each for gate/up (activation in its epilogue) and
             # down on the tensor cores, then the choices of a token added up in their order
             act = (s.activation, float(s.limit), 0.0) if s.activation != "silu" else None
-            few = n <= ops.SKINNY_MAX_TOKENS        # a token chooses an expert once: no expert has more rows than that
+            few = n <= ops.SKINNY_MAX_TOKENS
+            tile_rows = ops.skinny_grouped_rows(n) if few else 128
             with rt.phase("moe_sort", nbytes=4.0 * S * h):
                 rows, slots = rt.empty(S, dtype=torch.int32), rt.empty(S, dtype=torch.int32)
-                plan = rt.empty(1 + 3 * ops.moe_plan_tiles(S, s.n_experts), dtype=torch.int32)
-                ops.moe_plan(ids, s.n_experts, rows, slots, plan)
+                plan = rt.empty(1 + 3 * ops.moe_plan_tiles(S, s.n_experts, tile_rows), dtype=torch.int32)
+                ops.moe_plan(ids, s.n_experts, rows, slots, plan, tile_rows)
                 xs = rt.empty(S, h, dtype=torch.bfloat16)
                 ops.moe_gather(x, slots, s.top, xs, weights if on_input else None)
             mid = rt.empty(S, f, dtype=torch.bfloat16)

@@ -35,3 +35,38 @@ def test_few_rows_grouped(n, experts, top, N, K, epilogue, activation):
         expert = ids.flatten()[slots.long()].long()
         want = torch.einsum("sk,snk->sn", xs.double(), w[expert].double())
         check(out, want.float(), 2e-5, "64-bit sums")
+
+
+@pytest.mark.parametrize("n,bad,top", [(4, 1, 4), (8, 4, 6), (9, 3, 2), (16, 10, 4)])
+def test_tokens_that_are_not_numbers_keep_to_themselves(n, bad, top):
+    """A token whose router logits are not numbers chooses expert 0 over and over, so that expert has more rows than the step has
+    tokens.  Every row is computed all the same: the other tokens, which choose it too, get the bits they get beside
+    healthy tokens, out of memory that held NaN before."""
+    from types import SimpleNamespace
+    from nncpu_b200.config.specs import RoutedExpertsSpec
+    from nncpu_b200.parts import Runtime, base
+    from nncpu_b200.parts.runtime import Arena
+    width, ff, E = 128, 64, 7
+    spec = RoutedExpertsSpec(kind="routed_experts", name="m", hidden_size=width, intermediate_size=ff, n_experts=E, top=top,
+                             activation="silu", limit=0.0, router_bias=True)
+    part, rt = base.build("feed_forward", spec), Runtime(DEV, torch.bfloat16)
+    g = torch.Generator(device=DEV).manual_seed(n)
+    tensors = {p.name: (torch.randn(p.shape, generator=g, device=DEV) * 0.1).bfloat16() for p in part.params()}
+    tensors["m.router.b"][0] = 50.0                  # everybody's first choice
+    part.bind(tensors, rt)
+    x = torch.randn(n, width, generator=g, device=DEV).bfloat16()
+    outs = []
+    for spoilt in (False, True):
+        arena = Arena(rt.device)
+        arena.reserve(1 << 20)
+        arena.buf.fill_(255)
+        arena.begin()
+        rows = x.clone()
+        if spoilt:
+            rows[:bad] = float("nan")
+        out = torch.zeros(n, width, device=DEV)
+        with rt.using(arena):
+            part.forward(SimpleNamespace(n_tokens=n), rows, out)
+        outs.append(out)
+    assert torch.isfinite(outs[0]).all() and not torch.isfinite(outs[1][:bad]).any()
+    assert torch.equal(outs[0][bad:], outs[1][bad:])
