@@ -29,7 +29,9 @@
 // A few rows over a long past make few blocks: a message of 24 tokens behind 700 others, 16 heads over 4, is 8 of them,
 // each walking six steps one after the other while 140 SMs idle.  There a cluster of 2, 4 or 8 blocks shares a tile: each walks
 // its part of the steps, leaves reference maximum, sum and O (32-bit) in its shared memory, and adds up its share of the columns
-// over the cluster's blocks, in their order, through distributed shared memory.
+// over the cluster's blocks, in their order, through distributed shared memory.  The launch knows only how many keys there may
+// be (a captured step: the cache's capacity), the device how many there are: a tile of up to kAloneSteps steps is walked by its
+// cluster's first block alone, the others leave.
 //
 // The reference computes the same attention row by
 // row (crates/nncpu/src/model/forward.rs:141-160,383-426); softmax runs in 32-bit here
@@ -54,6 +56,10 @@ constexpr int kQRows = 128;   // query rows per block = tensor-core M
 constexpr int kKeys = 2 * kPage;  // keys per step: two cache pages
 constexpr int kStages = 2;    // steps of K and of V in flight
 constexpr int kMaxSplits = 8; // blocks of a cluster that shares a tile
+// Up to so many steps a tile is not shared: a step costs 2 us, the parts' way through distributed shared memory and its two
+// barriers cost about 5.  24 rows of 16 heads over 4, as a cluster of eight / by one block: one step 11.8 / 6.8 us, three
+// 14.5 / 12.3, six 14.5 / 18.1.
+constexpr int kAloneSteps = 4;
 constexpr int kStreamCols = 256;  // tensor-memory columns per head: S (P over its second half) | O
 constexpr int kPOffset = 64;      // P lies over the second half of S
 constexpr float kSumLimit = 256.0f;  // a step's weights of a row may add up to this before the row's reference maximum is moved
@@ -229,7 +235,9 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     const int n_pages = walk.n;
     // two pages a step, of which the last may hold one; this block walks the steps s0 .. s0 + n_steps - 1 of them
     const int all_steps = (n_pages + 1) / 2, split = (int)blockIdx.x % p.splits;
-    const int s0 = split * all_steps / p.splits, n_steps = (split + 1) * all_steps / p.splits - s0;
+    const int splits = all_steps <= kAloneSteps ? 1 : p.splits;      // the same for all blocks of a cluster
+    if (split >= splits) return;                                     // (nobody of its cluster will wait for it)
+    const int s0 = split * all_steps / splits, n_steps = (split + 1) * all_steps / splits - s0;
     // the heads of a key/value head are dealt out two to a block; an odd group's last block has one
     const int group = p.n_heads / p.n_kv;
     const int per_kv = (group + kStreams - 1) / kStreams;
@@ -538,7 +546,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             ok = __all_sync(0xffffffffu, mbar_wait(&o_done[t], 0));
             if (!ok && lane == 0) atomicExch(p.status, kTimeoutPv);
         }
-        if (ok && p.splits == 1) {
+        if (ok && splits == 1) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             // the sink's term, in the unit of the row's sums: powers of two relative to the reference maximum
             if (p.sinks != nullptr && l > 0.0f) l += exp2f(p.sinks[h] * 1.4426950408889634f - m_ref);
@@ -571,7 +579,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (p.splits > 1) {
+    if (splits > 1) {
         // The copies have landed and the matrix instructions have retired, so the tiles' memory is free: it takes this block's
         // part, [kStreams][VD columns][128 rows] of O, then the rows' reference maxima and sums.  (A block whose wait ran
         // out comes here, too: what it leaves is not valid, and the status word says so.)
@@ -605,7 +613,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             for (int c = 0; c < kMaxSplits; ++c) {
                 ms[c] = -INFINITY;
                 ls[c] = 0.0f;
-                if (c < p.splits) {
+                if (c < splits) {
                     ms[c] = ld_cluster_f32(m_at, (uint32_t)c);
                     ls[c] = ld_cluster_f32(l_at, (uint32_t)c);
                 }
@@ -624,7 +632,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             if (p.head_gate != nullptr && row < n_rows)
                 inv *= 1.0f / (1.0f + expf(-p.head_gate[(size_t)(q0 + row) * p.gate_ld + h]));
             __nv_bfloat16* dst = p.out + ((size_t)(q0 + row) * p.n_heads + h) * p.vo;
-            const int cols = VD / p.splits;        // 8 at least
+            const int cols = VD / splits;        // 8 at least
 #pragma unroll 1
             for (int c0 = split * cols; c0 < (split + 1) * cols; c0 += 8) {
                 float acc[8];
@@ -632,7 +640,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                 for (int j = 0; j < 8; ++j) acc[j] = 0.0f;
 #pragma unroll
                 for (int c = 0; c < kMaxSplits; ++c) {
-                    if (c < p.splits) {
+                    if (c < splits) {
                         float v[8];
 #pragma unroll
                         for (int j = 0; j < 8; ++j) v[j] = ld_cluster_f32(o_at + (uint32_t)((c0 + j) * kQRows * 4), (uint32_t)c);
@@ -715,7 +723,8 @@ MapCache g_maps;
 
 template <int HD, int VD, int kStreams, bool kCap>
 int launch_one(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, AttnParams p, int n_tok, int longest,
-               cudaStream_t stream) {
+               int* splits_only, cudaStream_t stream) {
+    // (splits_only: receives the number of blocks that would share a tile, and nothing is launched)
     static_assert((kStreams * VD + 2 * kStreams) * kQRows * 4 <= kStreams * kQRows * HD * 2 + kStages * kKeys * (HD + VD) * 2,
                   "a split tile's part fits the memory of its operands");
     static_assert(VD / kMaxSplits >= 8, "a block of a cluster adds up eight columns at least");
@@ -752,7 +761,7 @@ int launch_one(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& 
     static int fit[64][4] = {};      // per device, for clusters of 2, 4 and 8 (0: not asked yet)
     int dev = 0;
     p.splits = 1;
-    if (longest > kKeys && cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64) {
+    if (longest > kAloneSteps * kKeys && cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64) {
         for (int n = 2, i = 1; n <= kMaxSplits && (n - 1) * kKeys < longest; n *= 2, ++i) {
             if (fit[dev][i] == 0) {
                 with_splits(n);
@@ -766,6 +775,10 @@ int launch_one(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& 
             if ((long)head_blocks * tiles <= fit[dev][i]) p.splits = n;
         }
     }
+    if (splits_only != nullptr) {
+        *splits_only = p.splits;
+        return 0;
+    }
     with_splits(p.splits);
     cfg.numAttrs += overlap_attribute(attr + 1);
     const cudaError_t e = cudaLaunchKernelEx(&cfg, prefill_tc_kernel<HD, VD, kStreams, kCap>, mq, mk, mv, p);
@@ -773,11 +786,23 @@ int launch_one(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& 
     return 0;
 }
 
-template <int HD, int VD, int kStreams>
+template <int HD, int VD>
 int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AttnParams& p, int n_tok, int longest,
-           cudaStream_t stream) {
-    return p.cap_in != 0.0f ? launch_one<HD, VD, kStreams, true>(mq, mk, mv, p, n_tok, longest, stream)
-                            : launch_one<HD, VD, kStreams, false>(mq, mk, mv, p, n_tok, longest, stream);
+           int* splits_only, cudaStream_t stream) {
+    // two heads to a block where a key/value head has two to give; one head per block otherwise
+    const bool cap = p.cap_in != 0.0f;
+    if (p.n_heads == p.n_kv)
+        return cap ? launch_one<HD, VD, 1, true>(mq, mk, mv, p, n_tok, longest, splits_only, stream)
+                   : launch_one<HD, VD, 1, false>(mq, mk, mv, p, n_tok, longest, splits_only, stream);
+    return cap ? launch_one<HD, VD, 2, true>(mq, mk, mv, p, n_tok, longest, splits_only, stream)
+               : launch_one<HD, VD, 2, false>(mq, mk, mv, p, n_tok, longest, splits_only, stream);
+}
+
+int launch_any(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AttnParams& p, int head_dim, int vp,
+               int n_tok, int longest, int* splits_only, cudaStream_t stream) {
+    if (head_dim == 64) return launch<64, 64>(mq, mk, mv, p, n_tok, longest, splits_only, stream);
+    if (vp == 64) return launch<128, 64>(mq, mk, mv, p, n_tok, longest, splits_only, stream);
+    return launch<128, 128>(mq, mk, mv, p, n_tok, longest, splits_only, stream);
 }
 
 }  // namespace
@@ -840,9 +865,20 @@ extern "C" int nncpu_attention_prefill_tc(const void* q, const void* k_pages, co
     p.gate_ld = gate_ld;
     p.status = status;
     cudaStream_t stream = (cudaStream_t)stream_;
-    // two heads to a block where a key/value head has two to give; one head per block otherwise
-    const bool one = n_heads == n_kv;
-    if (head_dim == 64) return one ? launch<64, 64, 1>(mq, mk, mv, p, n_tok, longest, stream) : launch<64, 64, 2>(mq, mk, mv, p, n_tok, longest, stream);
-    if (vp == 64) return one ? launch<128, 64, 1>(mq, mk, mv, p, n_tok, longest, stream) : launch<128, 64, 2>(mq, mk, mv, p, n_tok, longest, stream);
-    return one ? launch<128, 128, 1>(mq, mk, mv, p, n_tok, longest, stream) : launch<128, 128, 2>(mq, mk, mv, p, n_tok, longest, stream);
+    return launch_any(mq, mk, mv, p, head_dim, vp, n_tok, longest, nullptr, stream);
+}
+
+// For tests: how many blocks would share a tile of such a step (the tiles of up to kAloneSteps steps among them are walked by one
+// all the same); 0: not supported.
+extern "C" int nncpu_attention_prefill_tc_splits(int n_heads, int n_kv, int head_dim, int vp, int capped, int n_tok, int n_seqs,
+                                                 int longest) {
+    if (!nncpu_attention_prefill_tc_supported(n_heads, n_kv, head_dim) || n_tok <= 0 || n_seqs <= 0) return 0;
+    AttnParams p{};
+    p.n_heads = n_heads;
+    p.n_kv = n_kv;
+    p.n_seqs = n_seqs;
+    p.cap_in = capped ? 1.0f : 0.0f;
+    int splits = 0;
+    const CUtensorMap none{};
+    return launch_any(none, none, none, p, head_dim, vp, n_tok, longest, &splits, nullptr) == 0 ? splits : 0;
 }

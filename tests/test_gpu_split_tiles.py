@@ -58,3 +58,35 @@ def test_split_tiles(ops, nh, nkv, hd, vd, how):
     seq = torch.tensor(tok_seq, dtype=torch.int32).to(DEV)
     ops.attention(q.to(DEV), kp, vp, table, seq, tok_pos, want, nh, nkv, hd, 1 / math.sqrt(hd), window, v_head_dim=vd, **how)
     check(outs[1130], want, 1.5e-2, "the 32-bit kernel")
+
+
+@pytest.mark.parametrize("nh,nkv,new,longest,splits", [(4, 1, [24], 512, 1), (4, 1, [24], 700, 4), (4, 1, [24], 2000, 8),
+                                                       (32, 8, [40, 300], 2000, 2), (32, 8, [128] * 20, 2000, 1)])
+def test_how_many_blocks_share_a_tile(ops, nh, nkv, new, longest, splits):
+    """As many as have a step of the longest walk each while all clusters run at once; and a tile that has few steps is walked by one
+    block, with the bits of a step that shares nothing, whatever the step's longest walk may be."""
+    from nncpu_b200.kernels import library
+    lib = library.load("attention_tc")
+    assert lib.nncpu_attention_prefill_tc_splits(nh, nkv, 128, 128, 0, sum(new), len(new), longest) == splits
+    past = [0 if i % 2 else 1800 for i in range(len(new))]         # every other sequence starts: few steps
+    seqs = [p + m for p, m in zip(past, new)]
+    kp, vp, table, _, _ = scatter_pages(sum((s + 63) // 64 for s in seqs), nkv, 128, seqs, torch.bfloat16, seed=nh)
+    n = sum(new)
+    q = torch.randn(n, nh * 128, generator=torch.Generator().manual_seed(5)).bfloat16().to(DEV)
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(new)]).astype(np.int32)).to(DEV)
+    pos = torch.tensor([p + i for p, m in zip(past, new) for i in range(m)], dtype=torch.int32).to(DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+
+    def run(longest):
+        out = torch.full((n, nh * 128), 9.0, dtype=torch.bfloat16, device=DEV)
+        ops.attention_prefill_tc(q, kp, vp, table, cu, pos, out, status, len(new), nh, nkv, 128, 128 ** -0.5, 0, longest=longest)
+        return out
+    alone, shared = run(0), run(longest)
+    assert int(status.item()) == 0
+    check(shared, alone, 1.5e-2, "shared")
+    for i in range(len(new)):
+        rows = slice(int(cu[i]), int(cu[i + 1]))
+        if i % 2 or splits == 1:
+            assert torch.equal(shared[rows], alone[rows])
+        else:
+            assert not torch.equal(shared[rows], alone[rows])      # several references and orders of sums: other roundings
