@@ -716,10 +716,13 @@ DECODE_CLUSTER_MAX_SPLITS = 8      # up to here the splits merge inside a thread
 
 
 # A short portion of one sequence goes through the decode kernel, token by token, while its tokens times key/value heads times
-# keys are at most this; beyond, as tiles of 128 rows (``attention_prefill_tc``).  Measured at the line (us, token by token /
-# tiles): 16 heads over 4, 64 tokens behind 700 15.3 / 16.0; 32 over 8, 16 behind 1 500 17 / 20; far below it (24 tokens of
-# 16 heads over 4 behind 700) 11.9 / 18.3; above it (32 over 8, 64 behind 1 500) 50 / 20.
+# the keys that the step may hold are at most the first (a captured step may hold as many as the cache's sequences can grow to,
+# whatever its sequence holds), and its tokens times key/value heads, which are blocks of their own, at most the second; beyond,
+# as tiles of 128 rows (``attention_prefill_tc``).  Measured (us, token by token / tiles): at the first line, 16 heads over
+# 4, 64 tokens behind 700 14.5 / 15.3, 32 over 8, 16 behind 1 500 16.4 / 16.1; below it (32 tokens of 16 heads over 4 behind
+# 100) 4.9 / 8.1; above (32 over 8, 64 behind 1 500) 49 / 19; above the second (32 over 8, 64 tokens, no past) 8.1 / 7.0.
 FEW_TOKENS_MAX_KEYS = 200_000
+FEW_TOKENS_MAX_BLOCKS = 256
 
 
 def attention_decode_splits(n_tokens: int, n_kv: int, longest: int, sm_count: int) -> int:

@@ -301,9 +301,11 @@ class Attention(Mixer):
 
     def _few_over_short(self, ctx) -> bool:
         """Whether a short portion of one sequence attends faster token by token, every token with keys of its own, than
-        as one tile of 128 rows: while the keys that all tokens read together are few."""
-        return (ctx.n_seqs == 1 and ctx.n_tokens <= 64
-                and ctx.n_tokens * self.spec.n_kv_heads * self._longest_span(ctx) <= ops.FEW_TOKENS_MAX_KEYS)
+        as one tile of 128 rows: while its tokens are few, and the keys that they may read together.  (In a captured step
+        these are as many as the cache's sequences can grow to: the step is captured once for all lengths.)"""
+        blocks = ctx.n_tokens * self.spec.n_kv_heads
+        return (ctx.n_seqs == 1 and ctx.n_tokens <= 64 and blocks <= ops.FEW_TOKENS_MAX_BLOCKS
+                and blocks * self._longest_span(ctx) <= ops.FEW_TOKENS_MAX_KEYS)
 
     def _longest_span(self, ctx) -> int:
         s = self.spec

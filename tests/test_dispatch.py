@@ -1,0 +1,22 @@
+"""Rules that choose a kernel by sizes alone, without a GPU."""
+from __future__ import annotations
+
+from types import SimpleNamespace
+
+import pytest
+
+from nncpu_b200.kernels import ops
+from nncpu_b200.parts.attention import Attention
+
+
+@pytest.mark.parametrize("n_seqs,tokens,n_kv,window,longest,few", [
+    (1, 24, 4, 0, 724, True), (1, 24, 4, 0, 4096, False),      # by the keys there may be
+    (1, 16, 8, 0, 1500, True), (1, 16, 8, 0, 1600, False),
+    (1, 64, 4, 0, 300, True), (1, 64, 8, 0, 65, False),        # by the blocks
+    (1, 32, 8, 0, 100, True), (1, 33, 8, 0, 100, False),
+    (1, 24, 4, 512, 40960, True),                              # a window bounds the keys
+    (2, 24, 4, 0, 100, False), (1, 65, 1, 0, 100, False)])
+def test_short_portions_token_by_token(n_seqs, tokens, n_kv, window, longest, few):
+    part = Attention.__new__(Attention)
+    part.spec = SimpleNamespace(n_kv_heads=n_kv, window=window, keep_first=0, chunk=0)
+    assert part._few_over_short(SimpleNamespace(n_seqs=n_seqs, n_tokens=tokens, max_kv_len=longest)) is few
