@@ -80,8 +80,8 @@ decode_f32_kernel(const AttnF32 p) {
     wait_for_previous_kernels();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int group = p.n_heads / p.n_kv, per_kv = (group + GB - 1) / GB;
-    const int kvh = blockIdx.x / per_kv, g0 = (blockIdx.x % per_kv) * GB;
-    const int t = blockIdx.z;
+    const int kvh = blockIdx.y / per_kv, g0 = (blockIdx.y % per_kv) * GB;
+    const int t = blockIdx.x;                    // (the dimension of a grid that takes any number of tokens)
     const int seq = p.tok_seq[t];
     if (seq < 0) {          // padding: zeros (from the block of the first stretch when nothing is merged)
         if (p.n_chunks == 1)
@@ -102,7 +102,7 @@ decode_f32_kernel(const AttnF32 p) {
         q[g] = d4 < p.hd ? *reinterpret_cast<const float4*>(p.q + ((size_t)t * p.n_heads + h) * p.hd + d4) : zero;
         slope[g] = slope_of(p, h);
     }
-    for (int c = blockIdx.y; c < p.n_chunks; c += gridDim.y) {
+    for (int c = blockIdx.z; c < p.n_chunks; c += gridDim.z) {
         const int begin = c * p.chunk, end = min(begin + p.chunk, pos + 1);
         if (begin > pos) break;
         float m[GB], l[GB];
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(128)
 merge_f32_kernel(const AttnF32 p) {
     let_next_kernel_start();
     wait_for_previous_kernels();
-    const int h = blockIdx.x, t = blockIdx.y, d = threadIdx.x;
+    const int t = blockIdx.x, h = blockIdx.y, d = threadIdx.x;
     const size_t out = ((size_t)t * p.n_heads + h) * p.vo + d;
     if (p.tok_seq[t] < 0) {
         if (d < p.vo) p.out[out] = 0.0f;
@@ -261,8 +261,9 @@ prompt_f32_kernel(const AttnF32 p) {
     float* ps = vs + kPage * p.vd;                  // [64][36]
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const int group = p.n_heads / p.n_kv, per_block = kRowsQ / group;      // tokens of a block
-    const int kvh = blockIdx.x;
-    const int t0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * per_block;     // the longest walks first
+    // one dimension of blocks: key/value heads, then the tiles, the last tokens' first (their walks are the longest)
+    const int kvh = (int)(blockIdx.x % p.n_kv), n_tiles = (p.n_tok + per_block - 1) / per_block;
+    const int t0 = (n_tiles - 1 - (int)(blockIdx.x / p.n_kv)) * per_block;
     const int t1 = min(t0 + per_block, p.n_tok);
 
     for (int i = tid; i < kRowsQ * (p.hd / 4); i += 128) {
@@ -461,15 +462,15 @@ extern "C" int nncpu_attention_f32(const void* q, const void* k_pages, const voi
               (float*)out, (float*)part, n_tok, n_heads, n_kv, hd, vd, vo, scale, window, keep, slope_base, sinks, cap,
               head_gate, gate_ld, chunk, n_chunks};
     const int group = n_heads / n_kv;
+    NN_CHECK(n_heads <= 65535, "attention (32-bit): %d heads", n_heads);
     if (chunk > 0) {
         const int gb = group >= 8 ? 8 : (group > 2 ? 4 : group);
         const int blocks_x = n_kv * ((group + gb - 1) / gb);
-        NN_CHECK(n_tok <= 65535, "attention (32-bit): %d tokens one by one", n_tok);
         // as many blocks as eight per SM ask for; a block with several stretches takes them in turn
         const long pairs = (long)blocks_x * n_tok;
         long per = (8L * sm_count + pairs - 1) / pairs;
         if (per > n_chunks) per = n_chunks;
-        const dim3 grid((unsigned)blocks_x, (unsigned)per, (unsigned)n_tok);
+        const dim3 grid((unsigned)n_tok, (unsigned)blocks_x, (unsigned)per);
         // both launched to start while the kernel before them ends: their launches are as long as their work
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = grid;
@@ -482,7 +483,7 @@ extern "C" int nncpu_attention_f32(const void* q, const void* k_pages, const voi
         cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
         NN_CHECK(e == cudaSuccess, "attention (32-bit): launch failed: %s", cudaGetErrorString(e));
         if (n_chunks > 1) {
-            cfg.gridDim = dim3((unsigned)n_heads, (unsigned)n_tok);
+            cfg.gridDim = dim3((unsigned)n_tok, (unsigned)n_heads);
             e = cudaLaunchKernelEx(&cfg, merge_f32_kernel, p);
             NN_CHECK(e == cudaSuccess, "attention (32-bit, merge): launch failed: %s", cudaGetErrorString(e));
         }
@@ -490,14 +491,14 @@ extern "C" int nncpu_attention_f32(const void* q, const void* k_pages, const voi
     }
     const int per_block = kRowsQ / group;
     const long tiles = ((long)n_tok + per_block - 1) / per_block;
-    NN_CHECK(tiles <= 65535, "attention (32-bit): %d tokens in tiles of %d", n_tok, per_block);
+    NN_CHECK(tiles * n_kv < (1L << 31), "attention (32-bit): %d tokens in tiles of %d", n_tok, per_block);
     const size_t smem = sizeof(float) * ((size_t)kRowsQ * (hd + 4) + (size_t)kPage * (hd + 4) + (size_t)kPage * vd + (size_t)kPage * kPsLd);
     static bool done[64];
     if (first_use_on_this_device(done)) {
         const cudaError_t e = cudaFuncSetAttribute(prompt_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
         NN_CHECK(e == cudaSuccess, "attention (32-bit): shared memory: %s", cudaGetErrorString(e));
     }
-    prompt_f32_kernel<<<dim3(n_kv, (unsigned)tiles), 128, smem, st>>>(p);
+    prompt_f32_kernel<<<(unsigned)(tiles * n_kv), 128, smem, st>>>(p);
     NN_LAUNCH_OK("attention (32-bit)");
     return 0;
 }

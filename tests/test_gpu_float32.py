@@ -164,3 +164,25 @@ def test_attention_keeps_to_what_a_query_sees(ops):
         for t in (0, 63, 64, 89):
             one = run_attention(ops, q[t:t + 1], kp, vp, table, seq[t:t + 1].clone(), pos[t:t + 1].clone(), *args, plan)
             assert torch.equal(one[0], want[t])
+
+
+def test_attention_of_more_tokens_than_a_grid_is_high(ops):
+    """Beyond 65 535 decode rows, and beyond 65 535 tiles of query rows (32 query heads on one key/value head: a tile a token)."""
+    n = 66001
+    g = torch.Generator(device=DEV).manual_seed(3)
+    kp, vp = (torch.randn(n, 1, 64, 4, generator=g, device=DEV) for _ in range(2))
+    table = torch.randperm(n, generator=g, device=DEV).to(torch.int32).view(n, 1)
+    seq = torch.arange(n, dtype=torch.int32, device=DEV)
+    pos = torch.randint(0, 64, (n,), generator=g, device=DEV).to(torch.int32)
+    q = torch.randn(n, 2 * 4, generator=g, device=DEV)
+    want = torch.empty(n, 2 * 4, device=DEV)
+    ops.attention(q, kp, vp, table, seq, pos, want, 2, 1, 4, 0.5)
+    for plan in ((128, 1), (128, 3)):
+        check(run_attention(ops, q, kp, vp, table, seq, pos, 2, 1, 4, 4, 4, plan), want, 2e-5, f"decode rows, plan {plan}")
+    pages = (n + 63) // 64
+    table = torch.randperm(pages, generator=g, device=DEV).to(torch.int32).view(1, pages)
+    seq, pos = torch.zeros(n, dtype=torch.int32, device=DEV), torch.arange(n, dtype=torch.int32, device=DEV)
+    q = torch.randn(n, 32 * 4, generator=g, device=DEV)
+    want = torch.empty(n, 32 * 4, device=DEV)
+    ops.attention(q, kp, vp, table, seq, pos, want, 32, 1, 4, 0.5, 70)
+    check(run_attention(ops, q, kp, vp, table, seq, pos, 32, 1, 4, 4, 4, (0, 0), window=70), want, 2e-5, "prompt")
