@@ -6,8 +6,8 @@
 //     a warp reads whole rows (32 lanes x 16 bytes), eight of them in flight.  The stretches' parts meet in
 //     merge_f32_kernel.  Stretches have a length that the longest possible sequence decides, not the step, so a row's
 //     result does not depend on the batch.
-//   * prompt_f32_kernel: a block takes 32 query rows (a few neighbouring tokens times the query heads of one key/value
-//     head) and walks through the pages they see; scores and outputs are 32-bit products out of shared memory, four by four
+//   * prompt_f32_kernel: a block takes 32 query rows (a few neighbouring tokens of one sequence times the query heads of one
+//     key/value head) and walks through the pages they see; scores and outputs are 32-bit products out of shared memory, four by four
 //     and four by eight numbers per thread.
 // Measured, 16 heads over 4 of 128 lanes: two sequences of some 600 keys 14 us with the merge (172 in the general kernel),
 // a prompt of 300 tokens 57 us (414).  The first is bound by latency (a stretch is two rounds of loads), the second by
@@ -42,6 +42,7 @@ struct AttnF32 {
     const float* head_gate;
     int gate_ld;
     int chunk, n_chunks;       // keys of a stretch (a multiple of 128), stretches of the longest sequence
+    int runs;                  // prompts: blocks a tile of tokens has for the sequences in it
 };
 
 __device__ __forceinline__ float slope_of(const AttnF32& p, int h) {
@@ -261,10 +262,27 @@ prompt_f32_kernel(const AttnF32 p) {
     float* ps = vs + kPage * p.vd;                  // [64][36]
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const int group = p.n_heads / p.n_kv, per_block = kRowsQ / group;      // tokens of a block
-    // one dimension of blocks: key/value heads, then the tiles, the last tokens' first (their walks are the longest)
-    const int kvh = (int)(blockIdx.x % p.n_kv), n_tiles = (p.n_tok + per_block - 1) / per_block;
-    const int t0 = (n_tiles - 1 - (int)(blockIdx.x / p.n_kv)) * per_block;
-    const int t1 = min(t0 + per_block, p.n_tok);
+    // One dimension of blocks: key/value heads, then the runs of a tile (tokens of one sequence), then the tiles, the last
+    // tokens' first (their walks are the longest).
+    const int kvh = (int)(blockIdx.x % p.n_kv), nth = (int)(blockIdx.x / p.n_kv) % p.runs;
+    const int n_tiles = (p.n_tok + per_block - 1) / per_block;
+    int t0 = (n_tiles - 1 - (int)(blockIdx.x / p.n_kv) / p.runs) * per_block;
+    int t1 = min(t0 + per_block, p.n_tok);
+    if (p.runs > 1) {
+        // this block's run; the last block of a tile takes the runs that are left
+        int r = t0, run = 0;
+        for (; run < nth && r < t1; ++run) {
+            const int seq = p.tok_seq[r];
+            for (++r; r < t1 && p.tok_seq[r] == seq; ++r) {}
+        }
+        if (r >= t1) return;
+        t0 = r;
+        if (nth + 1 < p.runs) {
+            const int seq = p.tok_seq[r];
+            for (++r; r < t1 && p.tok_seq[r] == seq; ++r) {}
+            t1 = r;
+        }
+    }
 
     for (int i = tid; i < kRowsQ * (p.hd / 4); i += 128) {
         const int r = i / (p.hd / 4), d = (i % (p.hd / 4)) * 4;
@@ -289,7 +307,7 @@ prompt_f32_kernel(const AttnF32 p) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
     }
-    // a run of tokens of one sequence after the other (most blocks hold one)
+    // a run of tokens of one sequence after the other (a block that has the rest of a tile may hold several)
     for (int r0 = t0; r0 < t1;) {
         const int seq = p.tok_seq[r0];
         int r1 = r0 + 1;
@@ -441,13 +459,13 @@ extern "C" int nncpu_attention_f32_supported(int n_heads, int n_kv, int hd, int 
 }
 
 // chunk > 0: token by token, every token's keys in stretches of `chunk` (a multiple of 128), n_chunks for the longest sequence that
-// the step may hold (more than one: `part` holds n_tok * n_heads * n_chunks * (vd + 2) floats).  chunk 0: query rows in tiles;
-// tokens of one sequence stand together, in ascending order of position.
+// the step may hold (more than one: `part` holds n_tok * n_heads * n_chunks * (vd + 2) floats).  chunk 0: query rows in tiles; tokens of one sequence stand together, in ascending order of position;
+// n_seqs: sequences of the step, each of which gets blocks of its own in a tile (0: not known).
 extern "C" int nncpu_attention_f32(const void* q, const void* k_pages, const void* v_pages, const int* block_table,
                                    int bt_stride, const int* tok_seq, const int* tok_pos, void* out, void* part, int n_tok,
                                    int n_heads, int n_kv, int hd, int vd, int vo, float scale, int window, int keep,
                                    float slope_base, const float* sinks, float cap, const float* head_gate, int gate_ld,
-                                   int chunk, int n_chunks, int sm_count, void* stream) {
+                                   int chunk, int n_chunks, int n_seqs, int sm_count, void* stream) {
     NN_CHECK(n_tok >= 0 && nncpu_attention_f32_supported(n_heads, n_kv, hd, vd, vo),
              "attention (32-bit): %d heads over %d, %d lanes of keys, %d of values, %d of outputs", n_heads, n_kv, hd, vd, vo);
     NN_CHECK(cap >= 0.0f && keep >= 0 && (head_gate == nullptr || gate_ld >= n_heads), "attention (32-bit): cap %f, %d kept keys, gate rows of %d",
@@ -460,7 +478,7 @@ extern "C" int nncpu_attention_f32(const void* q, const void* k_pages, const voi
     cudaStream_t st = (cudaStream_t)stream;
     AttnF32 p{(const float*)q, (const float*)k_pages, (const float*)v_pages, block_table, bt_stride, tok_seq, tok_pos,
               (float*)out, (float*)part, n_tok, n_heads, n_kv, hd, vd, vo, scale, window, keep, slope_base, sinks, cap,
-              head_gate, gate_ld, chunk, n_chunks};
+              head_gate, gate_ld, chunk, n_chunks, 1};
     const int group = n_heads / n_kv;
     NN_CHECK(n_heads <= 65535, "attention (32-bit): %d heads", n_heads);
     if (chunk > 0) {
@@ -491,14 +509,15 @@ extern "C" int nncpu_attention_f32(const void* q, const void* k_pages, const voi
     }
     const int per_block = kRowsQ / group;
     const long tiles = ((long)n_tok + per_block - 1) / per_block;
-    NN_CHECK(tiles * n_kv < (1L << 31), "attention (32-bit): %d tokens in tiles of %d", n_tok, per_block);
+    p.runs = n_seqs > 0 && n_seqs < per_block ? n_seqs : per_block;
+    NN_CHECK(tiles * n_kv * p.runs < (1L << 31), "attention (32-bit): %d tokens in tiles of %d", n_tok, per_block);
     const size_t smem = sizeof(float) * ((size_t)kRowsQ * (hd + 4) + (size_t)kPage * (hd + 4) + (size_t)kPage * vd + (size_t)kPage * kPsLd);
     static bool done[64];
     if (first_use_on_this_device(done)) {
         const cudaError_t e = cudaFuncSetAttribute(prompt_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
         NN_CHECK(e == cudaSuccess, "attention (32-bit): shared memory: %s", cudaGetErrorString(e));
     }
-    prompt_f32_kernel<<<(unsigned)(tiles * n_kv), 128, smem, st>>>(p);
+    prompt_f32_kernel<<<(unsigned)(tiles * n_kv * p.runs), 128, smem, st>>>(p);
     NN_LAUNCH_OK("attention (32-bit)");
     return 0;
 }

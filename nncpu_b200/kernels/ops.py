@@ -657,25 +657,33 @@ def attention_f32_supported(q, k_pages, v_pages, out, n_heads: int, n_kv: int, h
             and all(0 < d <= 128 and d % 4 == 0 for d in (head_dim, v_head_dim, v_lanes)) and v_lanes <= v_head_dim)
 
 
-def attention_f32_plan(n_tokens: int, is_decode: bool, longest: int):
+# Up to so many tokens, or so many a sequence, a float32 step attends token by token.  Measured (us, token by token / tiles of
+# query rows / the general kernel): 64 tokens behind 1 000, 16 heads over 4 47 / 164 / 521, 16 over 16 84 / 167 / 509; 17
+# behind 200, 8 heads over 8 12 / 44 / 27; 63 decode rows of 1 000 keys beside a portion of 20, 16 over 16 176 / 831 / 610;
+# beyond the line, 256 tokens of 32 sequences of 1 000, 32 over 8 343 / 232 / 4 050.
+ATTENTION_F32_FEW_TOKENS = 64
+ATTENTION_F32_FEW_PER_SEQUENCE = 4
+
+
+def attention_f32_plan(n_tokens: int, is_decode: bool, longest: int, n_seqs: int = 1):
     """(keys of a stretch, stretches of the longest sequence) for the token-by-token kernel, or (0, 0) for the kernel of
-    whole prompts.  Token by token where the step is a decode step, and for a prompt of up to 16 tokens: as one
-    tile of query rows it would walk through its keys on a handful of SMs.  A sequence of up to 4 096 keys (1 024 in a step of
-    more than 64 tokens, which has blocks enough) is cut every 128 keys whatever else the step holds; beyond, the
+    whole prompts, one tile of whose query rows walks through its keys on a single SM.  A sequence of up to 4 096 keys (1 024 in
+    a step of more than 64 tokens, which has blocks enough) is cut every 128 keys whatever else the step holds; beyond, the
     stretches grow, so that there are at most 32 (8) to keep room for and to add up."""
-    if not is_decode and n_tokens > LINEAR_F32_MAX_TOKENS:
+    if not (is_decode or n_tokens <= ATTENTION_F32_FEW_TOKENS or n_tokens <= ATTENTION_F32_FEW_PER_SEQUENCE * n_seqs):
         return 0, 0
     chunk = ATTENTION_F32_STRETCH
-    while longest > chunk * (32 if n_tokens <= 64 else 8):
+    while longest > chunk * (32 if n_tokens <= ATTENTION_F32_FEW_TOKENS else 8):
         chunk *= 2
     return chunk, max(1, (longest + chunk - 1) // chunk)
 
 
 def attention_f32(q, k_pages, v_pages, block_table, tok_seq, tok_pos, out, scratch, n_heads: int, n_kv: int, head_dim: int,
                   scale: float, plan, sm_count: int, window: int = 0, v_head_dim: int = 0, slope_base: float = 0.0, sinks=None,
-                  keep: int = 0, v_lanes: int = 0, cap: float = 0.0, head_gate=None) -> None:
+                  keep: int = 0, v_lanes: int = 0, cap: float = 0.0, head_gate=None, n_seqs: int = 0) -> None:
     """``attention`` for float32 heads of at most 128 lanes.  ``plan`` is ``attention_f32_plan``'s; with more than one
-    stretch ``scratch`` holds n * n_heads * stretches * (v_head_dim + 2) floats."""
+    stretch ``scratch`` holds n * n_heads * stretches * (v_head_dim + 2) floats.  ``n_seqs``: the step's sequences (0: not
+    known, which costs blocks that find nothing to do)."""
     n = q.shape[0]
     v_head_dim = v_head_dim or head_dim
     v_lanes = v_lanes or v_head_dim
@@ -687,7 +695,7 @@ def attention_f32(q, k_pages, v_pages, block_table, tok_seq, tok_pos, out, scrat
     _call("attention_f32", "nncpu_attention_f32", _ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(block_table),
           _i(block_table.shape[1]), _ptr(tok_seq), _ptr(tok_pos), _ptr(out), _ptr(scratch), _i(n), _i(n_heads), _i(n_kv),
           _i(head_dim), _i(v_head_dim), _i(v_lanes), _f(scale), _i(window), _i(keep), _f(slope_base), _ptr(sinks), _f(cap),
-          *_head_gate(head_gate, n, n_heads), _i(chunk), _i(n_chunks), _i(sm_count), _stream())
+          *_head_gate(head_gate, n, n_heads), _i(chunk), _i(n_chunks), _i(n_seqs), _i(sm_count), _stream())
 
 
 def attention_mma_supported(n_heads: int, n_kv: int, head_dim: int, *tensors) -> bool:

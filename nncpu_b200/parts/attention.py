@@ -330,12 +330,12 @@ class Attention(Mixer):
         if not (self._tensor_core_rows() and ops.attention_mma_supported(s.n_heads, s.n_kv_heads, self.k_row, q, cache.k_pages, attn)):
             if ops.attention_f32_supported(q, cache.k_pages, cache.v_pages, attn, s.n_heads, s.n_kv_heads, self.k_row, self.v_row,
                                            self.v_dim):
-                plan = ops.attention_f32_plan(ctx.n_tokens, ctx.is_decode, ctx.max_kv_len)
+                plan = ops.attention_f32_plan(ctx.n_tokens, ctx.is_decode, ctx.max_kv_len, ctx.n_seqs)
                 scratch = (self.rt.empty(ctx.n_tokens * s.n_heads * plan[1] * (self.v_row + 2), dtype=torch.float32)
                            if plan[1] > 1 else None)
                 ops.attention_f32(q, cache.k_pages, cache.v_pages, cache.block_table, ctx.tok_seq, ctx.tok_pos, attn, scratch,
                                   s.n_heads, s.n_kv_heads, self.k_row, s.scale, plan, self.rt.sm_count, self.span, self.v_row,
-                                  s.slope_base, self.sinks, **extra)
+                                  s.slope_base, self.sinks, n_seqs=ctx.n_seqs, **extra)
                 return
             ops.attention(q, cache.k_pages, cache.v_pages, cache.block_table, ctx.tok_seq, ctx.tok_pos, attn,
                           s.n_heads, s.n_kv_heads, self.k_row, s.scale, self.span, self.v_row, s.slope_base, self.sinks,

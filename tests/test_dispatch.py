@@ -20,3 +20,12 @@ def test_short_portions_token_by_token(n_seqs, tokens, n_kv, window, longest, fe
     part = Attention.__new__(Attention)
     part.spec = SimpleNamespace(n_kv_heads=n_kv, window=window, keep_first=0, chunk=0)
     assert part._few_over_short(SimpleNamespace(n_seqs=n_seqs, n_tokens=tokens, max_kv_len=longest)) is few
+
+
+@pytest.mark.parametrize("tokens,decode,n_seqs,by_token", [
+    (1, True, 1, True), (500, True, 500, True), (2, False, 1, True), (64, False, 1, True), (65, False, 1, False),
+    (83, False, 64, True),                  # decode rows beside a portion
+    (192, False, 64, True), (256, False, 64, True), (257, False, 64, False), (331, False, 32, False)])
+def test_float32_attention_token_by_token(tokens, decode, n_seqs, by_token):
+    chunk, stretches = ops.attention_f32_plan(tokens, decode, 700, n_seqs)
+    assert (chunk > 0) is by_token and (stretches * chunk >= 700 or tokens > 64 or not by_token)

@@ -186,3 +186,19 @@ def test_attention_of_more_tokens_than_a_grid_is_high(ops):
     want = torch.empty(n, 32 * 4, device=DEV)
     ops.attention(q, kp, vp, table, seq, pos, want, 32, 1, 4, 0.5, 70)
     check(run_attention(ops, q, kp, vp, table, seq, pos, 32, 1, 4, 4, 4, (0, 0), window=70), want, 2e-5, "prompt")
+
+
+def test_sequences_of_a_tile_have_blocks_of_their_own(ops):
+    """However many blocks a tile of query rows has for the sequences in it (one, fewer than there are, one for each, more): the same
+    bits, padding between them included."""
+    nh, nkv, hd = 4, 2, 32
+    seqs = [700, 130, 64, 1, 65, 300, 90]
+    kp, vp, table, _, _ = scatter_pages(32, nkv, hd, seqs, torch.float32, seed=5)
+    tok = [(0, 699), (1, 128), (1, 129), (2, 63), (3, 0), (-1, 9), (4, 64), (5, 299), (6, 88), (6, 89)] + [(5, p) for p in range(40)]
+    seq, pos = (torch.tensor([t[i] for t in tok], dtype=torch.int32, device=DEV) for i in (0, 1))
+    q = torch.randn(len(tok), nh * hd, generator=torch.Generator().manual_seed(6)).to(DEV)
+    want = torch.empty(len(tok), nh * hd, device=DEV)
+    ops.attention(q, kp, vp, table, seq, pos, want, nh, nkv, hd, 1 / math.sqrt(hd))
+    outs = [run_attention(ops, q, kp, vp, table, seq, pos, nh, nkv, hd, hd, hd, (0, 0), n_seqs=n) for n in (0, 1, 2, 7, 40)]
+    check(outs[0], want, 2e-5, "tiles")
+    assert all(torch.equal(o, outs[0]) for o in outs[1:])
