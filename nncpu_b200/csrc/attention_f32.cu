@@ -4,8 +4,9 @@
 //
 //   * decode_f32_kernel: a block takes one token, the query heads of one key/value head, and one stretch of the keys;
 //     a warp reads whole rows (32 lanes x 16 bytes), eight of them in flight.  The stretches' parts meet in
-//     merge_f32_kernel.  Stretches have a length that the longest possible sequence decides, not the step, so a row's
-//     result does not depend on the batch.
+//     merge_f32_kernel.  How long a row's stretches are follows from its own position and from how many stretches the
+//     launch has room for, so a row's result does not depend on the rows beside it as long as that room is the same (the
+//     callers': 32, in steps of more than 64 tokens 8).
 //   * prompt_f32_kernel: a block takes 32 query rows (a few neighbouring tokens of one sequence times the query heads of one
 //     key/value head) and walks through the pages they see; scores and outputs are 32-bit products out of shared memory, four by four
 //     and four by eight numbers per thread.
@@ -41,9 +42,16 @@ struct AttnF32 {
     float cap;
     const float* head_gate;
     int gate_ld;
-    int chunk, n_chunks;       // keys of a stretch (a multiple of 128), stretches of the longest sequence
+    int chunk, n_chunks;       // least keys of a stretch (a multiple of 128), most stretches of a token
     int runs;                  // prompts: blocks a tile of tokens has for the sequences in it
 };
+
+// Keys of a stretch for the token at `pos`: the least, doubled until the token's keys fit the stretches there is room for.
+__device__ __forceinline__ int stretch_of(const AttnF32& p, int pos) {
+    int chunk = p.chunk;
+    while ((long)chunk * p.n_chunks <= pos) chunk *= 2;
+    return chunk;
+}
 
 __device__ __forceinline__ float slope_of(const AttnF32& p, int h) {
     return p.slope_base != 0.0f ? exp2f(-p.slope_base * (float)(h + 1) / (float)p.n_heads) : 0.0f;
@@ -93,6 +101,7 @@ decode_f32_kernel(const AttnF32 p) {
     }
     const int pos = p.tok_pos[t];
     const int first = first_visible_key(pos, p.window);
+    const int chunk = stretch_of(p, pos);
     const int d4 = lane * 4;
     const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     float4 q[GB];
@@ -104,7 +113,7 @@ decode_f32_kernel(const AttnF32 p) {
         slope[g] = slope_of(p, h);
     }
     for (int c = blockIdx.z; c < p.n_chunks; c += gridDim.z) {
-        const int begin = c * p.chunk, end = min(begin + p.chunk, pos + 1);
+        const int begin = c * chunk, end = min(begin + chunk, pos + 1);
         if (begin > pos) break;
         float m[GB], l[GB];
         float4 o[GB];
@@ -225,7 +234,7 @@ merge_f32_kernel(const AttnF32 p) {
         if (d < p.vo) p.out[out] = 0.0f;
         return;
     }
-    const int n = p.tok_pos[t] / p.chunk + 1;
+    const int n = p.tok_pos[t] / stretch_of(p, p.tok_pos[t]) + 1;
     const size_t slot0 = ((size_t)t * p.n_heads + h) * p.n_chunks;
     const float* ml = p.part + (size_t)p.n_tok * p.n_heads * p.n_chunks * p.vd + slot0 * 2;
     float m = -INFINITY;
@@ -458,8 +467,9 @@ extern "C" int nncpu_attention_f32_supported(int n_heads, int n_kv, int hd, int 
            vd > 0 && vd <= 128 && vd % 4 == 0 && vo > 0 && vo <= vd && vo % 4 == 0;
 }
 
-// chunk > 0: token by token, every token's keys in stretches of `chunk` (a multiple of 128), n_chunks for the longest sequence that
-// the step may hold (more than one: `part` holds n_tok * n_heads * n_chunks * (vd + 2) floats).  chunk 0: query rows in tiles; tokens of one sequence stand together, in ascending order of position;
+// chunk > 0: token by token, every token's keys in at most n_chunks stretches (more than one: `part` holds n_tok * n_heads *
+// n_chunks * (vd + 2) floats) of `chunk` keys, a multiple of 128, or of its double, its quadruple and so on where the token has
+// more keys than that.  chunk 0: query rows in tiles; tokens of one sequence stand together, in ascending order of position;
 // n_seqs: sequences of the step, each of which gets blocks of its own in a tile (0: not known).
 extern "C" int nncpu_attention_f32(const void* q, const void* k_pages, const void* v_pages, const int* block_table,
                                    int bt_stride, const int* tok_seq, const int* tok_pos, void* out, void* part, int n_tok,

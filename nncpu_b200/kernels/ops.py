@@ -666,16 +666,15 @@ ATTENTION_F32_FEW_PER_SEQUENCE = 4
 
 
 def attention_f32_plan(n_tokens: int, is_decode: bool, longest: int, n_seqs: int = 1):
-    """(keys of a stretch, stretches of the longest sequence) for the token-by-token kernel, or (0, 0) for the kernel of
-    whole prompts, one tile of whose query rows walks through its keys on a single SM.  A sequence of up to 4 096 keys (1 024 in
-    a step of more than 64 tokens, which has blocks enough) is cut every 128 keys whatever else the step holds; beyond, the
-    stretches grow, so that there are at most 32 (8) to keep room for and to add up."""
+    """(least keys of a stretch, most stretches of a token) for the token-by-token kernel, or (0, 0) for the kernel of whole
+    prompts, one tile of whose query rows walks through its keys on a single SM.  ``longest``: at least as many keys as any token
+    sees.  A token's keys are cut every 128, or where that makes more than 32 stretches (8 in a step of more than 64 tokens,
+    which has blocks enough) every 256, 512 and so on, by the token's own position: the cut of a row is the same whatever the
+    other rows are and however long ``longest`` says they may be."""
     if not (is_decode or n_tokens <= ATTENTION_F32_FEW_TOKENS or n_tokens <= ATTENTION_F32_FEW_PER_SEQUENCE * n_seqs):
         return 0, 0
-    chunk = ATTENTION_F32_STRETCH
-    while longest > chunk * (32 if n_tokens <= ATTENTION_F32_FEW_TOKENS else 8):
-        chunk *= 2
-    return chunk, max(1, (longest + chunk - 1) // chunk)
+    most = 32 if n_tokens <= ATTENTION_F32_FEW_TOKENS else 8
+    return ATTENTION_F32_STRETCH, max(1, min(most, (longest + ATTENTION_F32_STRETCH - 1) // ATTENTION_F32_STRETCH))
 
 
 def attention_f32(q, k_pages, v_pages, block_table, tok_seq, tok_pos, out, scratch, n_heads: int, n_kv: int, head_dim: int,

@@ -202,3 +202,25 @@ def test_sequences_of_a_tile_have_blocks_of_their_own(ops):
     outs = [run_attention(ops, q, kp, vp, table, seq, pos, nh, nkv, hd, hd, hd, (0, 0), n_seqs=n) for n in (0, 1, 2, 7, 40)]
     check(outs[0], want, 2e-5, "tiles")
     assert all(torch.equal(o, outs[0]) for o in outs[1:])
+
+
+def test_a_rows_stretches_follow_from_its_own_position(ops):
+    """The bits of a token are the same whatever the longest sequence of the step may be and whichever rows stand beside it, in
+    decode steps and short portions of up to 64 tokens: 128 keys a stretch up to 4 096, 256 up to 8 192."""
+    nh, nkv, hd = 4, 1, 64
+    seqs = [700, 4096, 4097, 5000, 90]
+    kp, vp, table, _, _ = scatter_pages(260, nkv, hd, seqs, torch.float32, seed=8)
+    seq = torch.arange(5, dtype=torch.int32, device=DEV)
+    pos = torch.tensor([n - 1 for n in seqs], dtype=torch.int32, device=DEV)
+    q = torch.randn(5, nh * hd, generator=torch.Generator().manual_seed(9)).to(DEV)
+    want = torch.empty(5, nh * hd, device=DEV)
+    ops.attention(q, kp, vp, table, seq, pos, want, nh, nkv, hd, 1 / math.sqrt(hd))
+    args = (nh, nkv, hd, hd, hd)
+    whole = run_attention(ops, q, kp, vp, table, seq, pos, *args, ops.attention_f32_plan(5, True, 5000, 5))
+    check(whole, want, 2e-5, "token by token")
+    assert torch.equal(whole, run_attention(ops, q, kp, vp, table, seq, pos, *args, ops.attention_f32_plan(5, True, 40960, 5)))
+    for t, n in enumerate(seqs):
+        for longest in (n, 5000, 40960):
+            plan = ops.attention_f32_plan(1, False, longest)
+            one = run_attention(ops, q[t:t + 1], kp, vp, table, seq[t:t + 1].clone(), pos[t:t + 1].clone(), *args, plan)
+            assert torch.equal(one[0], whole[t]), (n, longest)
