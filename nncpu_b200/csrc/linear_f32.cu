@@ -138,6 +138,8 @@ cudaError_t launch_few(const float* X, const float* W, const void* bias, int bia
 // K 6144 4.8e-7 / 1.4e-6.  Cutting with six warps and integer rounding instead of four and cvt.rna, and asking the
 // weights into L2 eight k-blocks ahead, took 12 % off.
 // ---------------------------------------------------------------------------
+// What the status word says when a wait ran out (each library has its own hundred).
+enum LinearF32Status : int { kTimeoutEmpty = 301, kTimeoutAccumEmpty = 302, kTimeoutCut = 303, kTimeoutFull = 304, kTimeoutAccumFull = 305 };
 constexpr int kManyThreads = 16 * 32;
 constexpr int kCutters = 6;            // warps 2 to 7
 constexpr int kManyRegsFew = 72, kManyRegsMany = 184;
@@ -247,7 +249,7 @@ f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 for (int kb = first_kb(slice); kb < first_kb(slice + 1); ++kb, ++run) {
                     const int s = run % kStages;
                     if (!mbar_wait(&empty[s], ((run / kStages) & 1) ^ 1)) {
-                        atomicExch(p.status, 201);
+                        atomicExch(p.status, kTimeoutEmpty);
                         ok = false;
                         break;
                     }
@@ -271,12 +273,12 @@ f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 for (int kb = kb0; kb < kb1; ++kb, ++run) {
                     const int s = run % kStages, nth = (kb - kb0) % kManyFlush;
                     if (nth == 0 && !mbar_wait(&acc_empty[sum & 1], ((sum >> 1) & 1) ^ 1)) {
-                        atomicExch(p.status, 202);
+                        atomicExch(p.status, kTimeoutAccumEmpty);
                         ok = false;
                         break;
                     }
                     if (!mbar_wait(&cut[s], (run / kStages) & 1)) {
-                        atomicExch(p.status, 203);
+                        atomicExch(p.status, kTimeoutCut);
                         ok = false;
                         break;
                     }
@@ -307,7 +309,7 @@ f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 for (int kb = 0; kb < n_kb; ++kb, ++run) {
                     const int s = run % kStages;
                     if (!mbar_wait(&full[s], (run / kStages) & 1)) {
-                        if (lane == 0) atomicExch(p.status, 204);
+                        if (lane == 0) atomicExch(p.status, kTimeoutFull);
                         ok = false;
                         break;
                     }
@@ -342,7 +344,7 @@ f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             for (int c = 0; c < kCols; ++c) acc[c] = 0.0f;
             for (int kb = kb0; kb < kb1; kb += kManyFlush, ++sum) {
                 if (!mbar_wait(&acc_full[sum & 1], (sum >> 1) & 1)) {
-                    if (lane == 0) atomicExch(p.status, 205);
+                    if (lane == 0) atomicExch(p.status, kTimeoutAccumFull);
                     ok = false;
                     break;
                 }
