@@ -11,11 +11,14 @@
 // An element is summed over k in an order that K alone decides (per lane ascending, then the lanes' tree, then the
 // four warps), so a row's result does not depend on how many tokens the step has, up to the 16.
 //
-// More tokens: the tensor cores, on numbers cut in two.  x = h + l with h the nearest tf32 number (11 bits); the rest l is at most
-// 2^11 of x's last places, so it is a tf32 number too and nothing is lost.  w . x = h h' + h l' + l h' (l l' is below 2^-24 of
-// the product), all three accumulated in 32-bit by tcgen05.mma kind::tf32.  The tensor core does not round its running
-// sum to nearest, so it only sums 64 columns at a time; these sums are added in registers, with float additions.  Against
-// 64-bit sums the result is as near as the CUDA cores' chain of fmaf or nearer (figures at f32_many_kernel).
+// More tokens: the tensor cores, on numbers cut in three.  x = a + b + c, a the nearest bfloat16 number (8 bits), b the nearest one
+// to the rest, c what is left: 24 bits are three times eight, so nothing of x is lost (down to 2^-110 in magnitude, from where on
+// c's last bits lie below bfloat16's smallest number; see kTiny).  Of the nine products of parts, exact each, the six that
+// matter are taken: b c', c b' and c c' are together at most 2^-24 of the product, half a last place of it.  They are accumulated in
+// 32-bit by tcgen05.mma kind::f16.  The tensor core does not round its running sum to nearest, so it only sums 64 columns at a time
+// (32 where K is short); these sums are added in registers, with float additions.  Against 64-bit sums the result is nearer than
+// the CUDA cores' chain of fmaf (figures at f32_many_kernel), and a row with a single one in it passes the weights through
+// unchanged.
 // Weights are the 128-row operand and tokens the other one (BN of them), K may be cut into slices that a second kernel adds.
 //
 // The reference computes these products with its float row kernels (crates/nncpu/src/kernels/mod.rs:337-360).
@@ -124,19 +127,23 @@ cudaError_t launch_few(const float* X, const float* W, const void* bias, int bia
 // ---------------------------------------------------------------------------
 // More tokens.
 //
-// A block's warps: 0 copies tiles of 32 columns to shared memory by TMA, 1 issues the matrix instructions, 2-7 cut what arrived into h (in its place) and l (behind it), 8-15 add the sums of 64 columns that
-// tensor memory holds in turn to their registers (two warps per quarter of the lanes, half of the tokens each) and store.
+// A block's warps: 0 copies tiles of 32 columns to shared memory by TMA, 1 issues the matrix instructions, 2-7 cut what arrived
+// into its parts (a and b in its place, c behind it), 8-15 add the sums of 64 columns that tensor memory holds in turn to their
+// registers (two warps per quarter of the lanes, half of the tokens each) and store.
 // The adders take registers over from the others: 2 x 72 + 2 x 184 a warpgroup's thread, the 4 x 128 of the launch.
 //
-// Bound by shared memory: per k-block a block moves its (128 + BN) x 128 bytes seven times through it (in by TMA, out and
-// twice in by the cutters, three times out to the tensor core), 128 bytes a cycle, which takes longer than the matrix
-// instructions themselves up to BN 256; so BN is as large as the tokens and the two accumulators of tensor memory allow.
-// Measured (weights from memory): N 12288, K 2048, 300 tokens 143 us, 2 048 tokens 644 us (160 TFLOP/s of true 32-bit results,
-// where the CUDA cores' peak is 72); N 2048, K 6144, 300 tokens 63 us.  A layer of 300 tokens (hidden
-// 2048): 279 us for its four products, 3 130 us in the general kernel.
-// Error against 64-bit sums (2-norm, N(0, 1) times N(0, 0.02)), here / the general kernel's chain of fmaf: K 2048 4.7e-7 / 8.1e-7,
-// K 6144 4.8e-7 / 1.4e-6.  Cutting with six warps and integer rounding instead of four and cvt.rna, and asking the
-// weights into L2 eight k-blocks ahead, took 12 % off.
+// Bound by shared memory and by the cutting: of every number of a k-block four bytes go in by TMA, four out to the cutters,
+// six in from them and twelve out to the tensor core, (128 + BN) x 6.5 cycles at 128 bytes; the kernel takes 1.3 times that.  (300
+// tokens of N 12288, K 2048 took 126 of 143 us without the cutters' arithmetic, 123 without their stores, 126 with one product of parts
+// instead of six.)  So BN is as large as the tokens and the two accumulators of tensor memory allow, and the cutters' work is what
+// counts: conversions in pairs (cvt.rn.bf16x2) and 16-byte stores; ten cutting warps, the next group's loads ahead, or 8-byte
+// stores without selects were no faster.
+// Measured (weights from memory): N 12288, K 2048, 17 tokens 42 us, 300 tokens 145, 2 048 tokens 644 (160 TFLOP/s of true 32-bit
+// results, where the CUDA cores' peak is 72); N 2048, K 6144, 300 tokens 75.  A layer of 300 tokens (hidden 2048): 297 us for its
+// four products, 3 130 us in the general kernel.  Cut into two tf32 numbers they took 251 us, but of a quarter of all numbers
+// the last bit was lost.
+// Error against 64-bit sums (2-norm, N(0, 1) times N(0, 0.02)), here / the general kernel's chain of fmaf: K 64 0.6e-7 / 1.5e-7,
+// 512 3.2e-7 / 4.1e-7, 2048 3.2e-7 / 8.1e-7, 6144 3.3e-7 / 1.4e-6; single products within 2.3 x 2^-24.
 // ---------------------------------------------------------------------------
 // What the status word says when a wait ran out (each library has its own hundred).
 enum LinearF32Status : int { kTimeoutEmpty = 301, kTimeoutAccumEmpty = 302, kTimeoutCut = 303, kTimeoutFull = 304, kTimeoutAccumFull = 305 };
@@ -145,7 +152,10 @@ constexpr int kCutters = 6;            // warps 2 to 7
 constexpr int kManyRegsFew = 72, kManyRegsMany = 184;
 static_assert(2 * kManyRegsFew + 2 * kManyRegsMany <= 4 * 128, "no more registers than the launch has");
 constexpr int kManyK = 32;             // columns of a k-block: 128 bytes, one swizzle row
-constexpr int kManyFlush = 2;          // k-blocks that the tensor core sums by itself
+// Columns that the tensor core sums by itself: its sums are cut, not rounded, at every step, which over 64 columns leaves 3.2e-7 of
+// a result's 2-norm whatever K is, and over 32 columns 0.6 to 1.7e-7.  A chain of fmaf has 1.5e-7 at K 64, 2.9e-7 at 256, 3.5e-7 at
+// 384, 4.1e-7 at 512; so below kShortK it is 32, which costs some 7 % there.
+constexpr int kShortK = 512;
 constexpr int kManyAhead = 8;          // k-blocks of weights that are asked into L2 ahead of their copies
 
 struct ManyParams {
@@ -158,22 +168,30 @@ struct ManyParams {
     float* part;          // slices > 1: [slices, M, N]
     int M, N, K, lda, ldc, accumulate;
     int tiles_a, tiles_b, slices, kb_total;
+    int flush;            // k-blocks that the tensor core sums by itself
     int* status;
 };
 
-__device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n"
-        "}\n" ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
+// The nearest bfloat16 numbers to two floats, the first in the lower half; and the floats they are.
+__device__ __forceinline__ uint32_t nearest_bf16(float x, float y) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(y), "f"(x));
+    return r;
 }
+__device__ __forceinline__ float lower(uint32_t two) { return __uint_as_float(two << 16); }
+__device__ __forceinline__ float upper(uint32_t two) { return __uint_as_float(two & 0xFFFF0000u); }
 
-// The nearest number of 11 bits (halves away from zero), in two integer instructions at full rate.  The sum may carry into the
-// exponent, as it should, up to infinity; of a NaN it may make a number, and x minus that is the NaN again.
-__device__ __forceinline__ float nearest_tf32(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u); }
+// Shared-memory matrix descriptor of a K-major tile whose rows are 64 bytes, swizzled in 64-byte mode: groups of 8 rows are
+// 512 bytes apart.
+__device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t addr) {
+    uint64_t d = 0;
+    d |= (uint64_t)((addr & 0x3FFFF) >> 4);
+    d |= (uint64_t)1 << 16;
+    d |= (uint64_t)(512 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)4 << 61;                  // 64-byte swizzle
+    return d;
+}
 
 // Asks for a tile to come to L2.
 __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
@@ -181,24 +199,37 @@ __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, i
 }
 
 // One result in plain float arithmetic over its slice of K: what a sum that is not finite is replaced by, because the cut
-// of an infinity, or of a number next to the largest, is not a number (inf - inf) where the product itself may be one.
+// of an infinity, or of a number next to the largest, is not a number (inf - inf) where the product itself may be one; and
+// what a sum below kTiny is replaced by, whose numbers may be so small that their third parts are not kept.  (A sum of zero
+// stays: it is that of a row of zeros, unless every number of it is below 2^-134.)
+constexpr float kTiny = 0x1p-60f;
+// (n is a multiple of 4 and both rows start at 16 bytes.)
 __device__ __noinline__ float plain_dot(const float* x, const float* w, int n) {
     float a = 0.0f;
-    for (int k = 0; k < n; ++k) a = fmaf(x[k], w[k], a);
+#pragma unroll 4
+    for (int k = 0; k < n; k += 4) {
+        const float4 u = *reinterpret_cast<const float4*>(x + k), v = *reinterpret_cast<const float4*>(w + k);
+        a = fmaf(u.x, v.x, a);
+        a = fmaf(u.y, v.y, a);
+        a = fmaf(u.z, v.z, a);
+        a = fmaf(u.w, v.w, a);
+    }
     return a;
 }
 
 template <int BN>
-constexpr int kManyStages = BN > 160 ? 2 : (BN > 96 ? 3 : 4);     // as many as shared memory holds
+constexpr int kManyStages = BN > 160 ? 3 : (BN > 96 ? 4 : 5);     // as many as shared memory holds
 template <int BN>
-constexpr size_t kManySmem = 1024 + (size_t)kManyStages<BN> * 2 * (128 + BN) * 128 + 256;
+constexpr size_t kManySmem = 1024 + (size_t)kManyStages<BN> * (128 + BN) * 192 + 256;
 
 template <int BN>
 __global__ void __launch_bounds__(kManyThreads, 1)
 f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const ManyParams p) {
     constexpr int kStages = kManyStages<BN>;
-    constexpr int kHalfBytes = (128 + BN) * 128;      // the h (or l) parts of a k-block: 128 rows of weights, BN of tokens
-    constexpr int kStageBytes = 2 * kHalfBytes;
+    // A k-block: 128 rows of weights, then BN of tokens.  128 bytes a row, as TMA brings them (128-byte swizzle) and, cut, 32 numbers
+    // a and 32 numbers b; behind them 64 bytes a row of numbers c (64-byte swizzle).
+    constexpr int kRawBytes = (128 + BN) * 128;
+    constexpr int kStageBytes = (128 + BN) * 192;
     constexpr int kTmemCols = BN <= 32 ? 64 : (BN <= 64 ? 128 : (BN <= 128 ? 256 : 512));     // two accumulators
     constexpr int kCols = BN / 2;                     // columns of an adding thread
     extern __shared__ uint8_t smem_raw[];
@@ -253,7 +284,7 @@ f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                         ok = false;
                         break;
                     }
-                    mbar_expect_tx(&full[s], kHalfBytes);     // (rows past the end are filled with zeros and counted)
+                    mbar_expect_tx(&full[s], kRawBytes);     // (rows past the end are filled with zeros and counted)
                     if (kb + kManyAhead < first_kb(slice + 1)) tma_prefetch_2d(&map_w, (kb + kManyAhead) * kManyK, m0);
                     tma_load_2d(smem + s * kStageBytes, &map_w, &full[s], kb * kManyK, m0);
                     tma_load_2d(smem + s * kStageBytes + 128 * 128, &map_x, &full[s], kb * kManyK, n0);
@@ -264,14 +295,14 @@ f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                 for (int r = max(0, run - kStages); r < run; ++r) mbar_wait(&full[r % kStages], (r / kStages) & 1);
         }
         if (warp == 1 && lane == 0) {
-            // 32-bit accumulator, tf32 operands, both K-major
-            constexpr uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+            constexpr uint32_t idesc = instr_desc_bf16(128, BN);
             int run = 0, sum = 0;
             bool ok = true;
             for (int i = blockIdx.x; i < n_items && ok; i += gridDim.x) {
-                const int slice = i / tiles, kb0 = first_kb(slice), kb1 = first_kb(slice + 1);
-                for (int kb = kb0; kb < kb1; ++kb, ++run) {
-                    const int s = run % kStages, nth = (kb - kb0) % kManyFlush;
+                const int slice = i / tiles, kb1 = first_kb(slice + 1);
+                int nth = 0;                                  // of the k-blocks in the sum
+                for (int kb = first_kb(slice); kb < kb1; ++kb, ++run) {
+                    const int s = run % kStages;
                     if (nth == 0 && !mbar_wait(&acc_empty[sum & 1], ((sum >> 1) & 1) ^ 1)) {
                         atomicExch(p.status, kTimeoutAccumEmpty);
                         ok = false;
@@ -284,24 +315,37 @@ f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t d = tmem_base + (uint32_t)((sum & 1) * BN);
-                    const uint32_t wh = smem_u32(smem + s * kStageBytes), xh = wh + 128 * 128;
-                    const uint32_t wl = wh + kHalfBytes, xl = xh + kHalfBytes;
+                    const uint32_t w_at = smem_u32(smem + s * kStageBytes), x_at = w_at + 128 * 128;
+                    const uint32_t w_rest = w_at + kRawBytes, x_rest = w_rest + 128 * 64;
+                    // the parts' products of 16 columns each, the smallest first
+                    constexpr uint8_t kOrder[6][2] = {{0, 2}, {2, 0}, {1, 1}, {0, 1}, {1, 0}, {0, 0}};
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {             // 8 columns an instruction
-                        umma_tf32(d, smem_desc_sw128(wl + k * 32), smem_desc_sw128(xh + k * 32), idesc, (nth > 0 || k > 0) ? 1u : 0u);
-                        umma_tf32(d, smem_desc_sw128(wh + k * 32), smem_desc_sw128(xl + k * 32), idesc, 1u);
-                        umma_tf32(d, smem_desc_sw128(wh + k * 32), smem_desc_sw128(xh + k * 32), idesc, 1u);
+                    for (int i = 0; i < 6; ++i) {
+                        const int pw = kOrder[i][0], px = kOrder[i][1];
+#pragma unroll
+                        for (int k = 0; k < 2; ++k)
+                            umma_bf16(d, pw == 2 ? smem_desc_sw64(w_rest + k * 32) : smem_desc_sw128(w_at + pw * 64 + k * 32),
+                                      px == 2 ? smem_desc_sw64(x_rest + k * 32) : smem_desc_sw128(x_at + px * 64 + k * 32), idesc,
+                                      (nth > 0 || i > 0 || k > 0) ? 1u : 0u);
                     }
                     umma_commit(&empty[s]);
-                    if (nth == kManyFlush - 1 || kb + 1 == kb1) {
+                    if (++nth == p.flush || kb + 1 == kb1) {
                         umma_commit(&acc_full[sum & 1]);
                         ++sum;
+                        nth = 0;
                     }
                 }
             }
         }
         if (warp >= 2) {
-            const int tid = threadIdx.x - 64;
+            // A lane cuts eight numbers of a row, four lanes a row, a warp eight rows at a time, two such groups at once.  They read
+            // all of a row before they write a and b in its place, and neighbouring rows write a and b in turn: no two lanes of
+            // a quarter of a warp meet in a bank, reading or writing.
+            const int r = lane >> 2, c = lane & 3, r7 = r & 7;
+            const int in0 = r * 128 + (((2 * c) ^ r7) << 4), in1 = r * 128 + (((2 * c + 1) ^ r7) << 4);
+            const int out_a = r * 128 + ((c ^ r7) << 4), out_b = r * 128 + (((4 + c) ^ r7) << 4);
+            const int out_c = r * 64 + ((c ^ ((r >> 1) & 3)) << 4);
+            const bool odd = r & 1;
             int run = 0;
             bool ok = true;
             for (int i = blockIdx.x; i < n_items && ok; i += gridDim.x) {
@@ -313,16 +357,41 @@ f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                         ok = false;
                         break;
                     }
-                    float4* h = reinterpret_cast<float4*>(smem + s * kStageBytes);
-                    float4* l = reinterpret_cast<float4*>(smem + s * kStageBytes + kHalfBytes);
-#pragma unroll 4
-                    for (int e = tid; e < kHalfBytes / 16; e += kCutters * 32) {
-                        const float4 v = h[e];
-                        float4 hi, lo;
-                        hi.x = nearest_tf32(v.x); hi.y = nearest_tf32(v.y); hi.z = nearest_tf32(v.z); hi.w = nearest_tf32(v.w);
-                        lo.x = v.x - hi.x; lo.y = v.y - hi.y; lo.z = v.z - hi.z; lo.w = v.w - hi.w;
-                        h[e] = hi;
-                        l[e] = lo;
+                    __syncwarp();
+                    uint8_t* const raw = smem + s * kStageBytes;
+                    uint8_t* const rest = raw + kRawBytes;
+                    constexpr int kGroups = (128 + BN) / 8;
+#pragma unroll 1
+                    for (int g0 = warp - 2; g0 < kGroups; g0 += 2 * kCutters) {
+                        const int g1 = g0 + kCutters;
+                        float x[2][8];
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            const int g = u == 0 ? g0 : g1;
+                            if (g < kGroups) {
+                                *reinterpret_cast<float4*>(&x[u][0]) = *reinterpret_cast<const float4*>(raw + g * 1024 + in0);
+                                *reinterpret_cast<float4*>(&x[u][4]) = *reinterpret_cast<const float4*>(raw + g * 1024 + in1);
+                            }
+                        }
+                        __syncwarp();
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            const int g = u == 0 ? g0 : g1;
+                            if (g >= kGroups) break;
+                            uint32_t a[4], b[4], rest_of[4];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                const float x0 = x[u][2 * j], x1 = x[u][2 * j + 1];
+                                a[j] = nearest_bf16(x0, x1);
+                                const float y0 = x0 - lower(a[j]), y1 = x1 - upper(a[j]);
+                                b[j] = nearest_bf16(y0, y1);
+                                rest_of[j] = nearest_bf16(y0 - lower(b[j]), y1 - upper(b[j]));      // 7 bits at most: exact
+                            }
+                            const uint4 va = make_uint4(a[0], a[1], a[2], a[3]), vb = make_uint4(b[0], b[1], b[2], b[3]);
+                            *reinterpret_cast<uint4*>(raw + g * 1024 + (odd ? out_b : out_a)) = odd ? vb : va;
+                            *reinterpret_cast<uint4*>(raw + g * 1024 + (odd ? out_a : out_b)) = odd ? va : vb;
+                            *reinterpret_cast<uint4*>(rest + g * 512 + out_c) = make_uint4(rest_of[0], rest_of[1], rest_of[2], rest_of[3]);
+                        }
                     }
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     __syncwarp();
@@ -342,7 +411,7 @@ f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
             float acc[kCols];
 #pragma unroll
             for (int c = 0; c < kCols; ++c) acc[c] = 0.0f;
-            for (int kb = kb0; kb < kb1; kb += kManyFlush, ++sum) {
+            for (int kb = kb0; kb < kb1; kb += p.flush, ++sum) {
                 if (!mbar_wait(&acc_full[sum & 1], (sum >> 1) & 1)) {
                     if (lane == 0) atomicExch(p.status, kTimeoutAccumFull);
                     ok = false;
@@ -379,7 +448,7 @@ f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     const int t = n0 + c0 + c;
                     if (t >= p.M) break;
                     float v = acc[c0 + c];
-                    if (!(fabsf(v) < INFINITY)) {
+                    if (!(fabsf(v) < INFINITY) || (fabsf(v) < kTiny && v != 0.0f)) {
                         const int k0 = kb0 * kManyK;
                         v = plain_dot(p.x + (size_t)t * p.lda + k0, p.w + (size_t)row * p.K + k0, min(kb1 * kManyK, p.K) - k0);
                     }
@@ -445,8 +514,8 @@ struct ManyPlan {
 };
 
 // The slices with the smallest sum of rounds of the SMs times k-blocks of a slice (six more for filling and draining a
-// block's pipeline), and the passes of the slices' sums through memory, in k-blocks too: one takes (128 + BN) x 7
-// cycles of shared memory; the sums pass at some 2 KB a cycle, and a launch costs 4 000 cycles.
+// block's pipeline), and the passes of the slices' sums through memory, in k-blocks too: one takes some (128 + BN) x 7
+// cycles; the sums pass at some 2 KB a cycle, and a launch costs 4 000 cycles.
 ManyPlan many_plan(int M, int N, int K) {
     ManyPlan plan;
     plan.tiles_b = (M + 255) / 256;
@@ -562,7 +631,7 @@ extern "C" int nncpu_linear_f32_many(const void* X, const void* W, const void* b
     const ManyPlan plan = many_plan(M, N, K);
     NN_CHECK(plan.slices == 1 || scratch != nullptr, "linear (32-bit): %d slices of K need scratch memory", plan.slices);
     ManyParams p{(const float*)X, (const float*)W, bias, bias_dt, C, c_dt, (float*)scratch, M, N, K, lda, ldc, accumulate,
-                 (N + 127) / 128, plan.tiles_b, plan.slices, (K + kManyK - 1) / kManyK, status};
+                 (N + 127) / 128, plan.tiles_b, plan.slices, (K + kManyK - 1) / kManyK, K < kShortK ? 1 : 2, status};
     NN_CHECK((long)p.tiles_a * p.tiles_b * p.slices < (1L << 31), "linear (32-bit): %d tokens of %d features", M, N);
     switch (plan.bn) {
         case 32: return launch_many<32>(p, st);

@@ -309,7 +309,7 @@ def linear_f32_many_scratch_floats(m: int, n: int, k: int) -> int:
 
 
 def linear_f32_many(x, w, bias, out, scratch, workspace: "GemmWorkspace", accumulate: bool = False) -> None:
-    """out (+)= x . w^T + bias for any number of rows: the tensor cores on numbers cut in two, with the error of a
+    """out (+)= x . w^T + bias for any number of rows: the tensor cores on numbers cut in three, with the error of a
     32-bit sum.  ``scratch`` holds ``linear_f32_many_scratch_floats`` floats (None where that is 0)."""
     m, k = x.shape
     n = w.shape[0]

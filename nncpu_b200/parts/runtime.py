@@ -152,8 +152,8 @@ class Runtime:
                activation=None) -> None:
         """out (+)= x . w^T + bias.  bfloat16 inputs whose sizes keep TMA's
         alignment rule go to the tensor cores; everything else runs in true 32-bit: float32 products of a million
-        weights or more by the kernels made for them (few rows: CUDA cores; more: tensor cores on numbers cut in two
-        without loss), the rest on CUDA cores by the general kernel.
+        weights or more by the kernels made for them (few rows: CUDA cores; more: tensor cores on numbers cut in
+        three, of which nothing is lost), the rest on CUDA cores by the general kernel.
 
         ``x`` may be a ``DeferredNorm`` (a norm's unfinished output): the few-token product and the product of
         whole prompts finish it, any other path makes the ordinary tensor first.  ``then_norm`` (a ``NormRequest``):

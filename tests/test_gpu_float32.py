@@ -50,7 +50,7 @@ def test_few_token_product(ops, m, n, k):
 @pytest.mark.parametrize("m", [1, 17, 32, 33, 64, 90, 128, 160, 190, 224, 256, 257, 300, 520])
 @pytest.mark.parametrize("n,k", [(5, 4), (128, 32), (129, 36), (200, 100), (201, 1000), (300, 1000), (1536, 2048), (256, 6144)])
 def test_many_token_product(ops, m, n, k):
-    """On the tensor cores with numbers cut in two: the bound of a 32-bit sum holds, and over longer sums the error is no
+    """On the tensor cores with numbers cut in three: the bound of a 32-bit sum holds, and over longer sums the error is no
     larger than that of the general kernel, which adds k products one after the other."""
     g = torch.Generator(device=DEV).manual_seed(m * n + k)
     x, w, b = (torch.randn(s, generator=g, device=DEV) for s in ((m, k), (n, k), (n,)))
@@ -164,6 +164,92 @@ def test_attention_keeps_to_what_a_query_sees(ops):
         for t in (0, 63, 64, 89):
             one = run_attention(ops, q[t:t + 1], kp, vp, table, seq[t:t + 1].clone(), pos[t:t + 1].clone(), *args, plan)
             assert torch.equal(one[0], want[t])
+
+
+@pytest.mark.parametrize("m", [17, 40, 200, 300])
+def test_many_token_product_keeps_every_bit_of_its_operands(ops, m):
+    """A row with a single power of two in it passes the weights through unchanged, whichever side it is on: nothing of a
+    number's 24 bits is lost on the way to the tensor cores.  A row with a single number in it gives that product to 2^-22: what is
+    left out is 2^-24 of it at most, and the sum of the six products is cut, not rounded, to 24 bits: 2^-23 once or twice."""
+    n, k = 1100, 1024
+    g = torch.Generator(device=DEV).manual_seed(m)
+    work = ops.GemmWorkspace(DEV)
+
+    def product(x, w):
+        floats = ops.linear_f32_many_scratch_floats(x.shape[0], w.shape[0], k)
+        out = torch.empty(x.shape[0], w.shape[0], device=DEV)
+        ops.linear_f32_many(x, w, None, out, torch.empty(floats, device=DEV) if floats else None, work)
+        return out
+
+    def single(rows):
+        x = torch.zeros(rows, k, device=DEV)
+        at = torch.randint(0, k, (rows,), generator=g, device=DEV)
+        sign = torch.randint(0, 2, (rows,), generator=g, device=DEV) * 2 - 1
+        x[torch.arange(rows, device=DEV), at] = torch.ldexp(sign.float(), torch.randint(-20, 21, (rows,), generator=g, device=DEV))
+        return x
+    w, x = torch.randn(n, k, generator=g, device=DEV), single(m)
+    assert torch.equal(product(x, w).double(), x.double() @ w.double().T)
+    w, x = single(n), torch.randn(m, k, generator=g, device=DEV)
+    assert torch.equal(product(x, w).double(), x.double() @ w.double().T)
+    w, x = torch.randn(n, k, generator=g, device=DEV), single(m) * torch.randn(m, 1, generator=g, device=DEV)
+    want = x.double() @ w.double().T
+    assert ((product(x, w) - want).abs() <= 2.0 ** -22 * want.abs()).all()
+    assert int(work.status.item()) == 0
+
+
+@pytest.mark.parametrize("m,n", [(40, 1024), (300, 2048)])
+@pytest.mark.parametrize("k", [32, 64, 100, 160, 256, 384, 508, 512, 768])
+def test_many_token_product_is_as_near_as_the_chain(ops, m, n, k):
+    """Over short sums too, where the tensor core's own sums are 32 columns long, the error is no larger than the general kernel's."""
+    g = torch.Generator(device=DEV).manual_seed(m + k)
+    x, w = torch.randn(m, k, generator=g, device=DEV), torch.randn(n, k, generator=g, device=DEV) * 0.02
+    floats = ops.linear_f32_many_scratch_floats(m, n, k)
+    out, general, work = torch.empty(m, n, device=DEV), torch.empty(m, n, device=DEV), ops.GemmWorkspace(DEV)
+    ops.linear_f32_many(x, w, None, out, torch.empty(floats, device=DEV) if floats else None, work)
+    ops.linear_simt(x, w, None, general)
+    want = x.double() @ w.double().T
+    assert (out - want).norm() <= (general - want).norm() and int(work.status.item()) == 0
+
+
+@pytest.mark.parametrize("scale_x,scale_w", [(2.0 ** -118, 2.0 ** 10), (2.0 ** -126, 2.0 ** 20), (2.0 ** 100, 2.0 ** -118),
+                                             (2.0 ** -80, 2.0 ** -60), (2.0 ** -105, 2.0 ** 60)])
+def test_many_token_product_of_tiny_numbers(ops, scale_x, scale_w):
+    """Numbers whose last bits lie below the smallest that their parts can be, and sums below float's normal range: as near to
+    64-bit sums as a 32-bit sum may be (2^-149 a term, a float's smallest step, on top)."""
+    m, n, k = 40, 1100, 1024
+    g = torch.Generator(device=DEV).manual_seed(7)
+    x, w = torch.randn(m, k, generator=g, device=DEV) * scale_x, torch.randn(n, k, generator=g, device=DEV) * scale_w
+    floats = ops.linear_f32_many_scratch_floats(m, n, k)
+    out = torch.empty(m, n, device=DEV)
+    ops.linear_f32_many(x, w, None, out, torch.empty(floats, device=DEV) if floats else None, ops.GemmWorkspace(DEV))
+    assert ((out - x.double() @ w.double().T).abs() <= bound(x, w) + (k + 4) * 2.0 ** -149).all()
+
+
+def test_a_model_whose_products_are_large(tmp_path):
+    """A float32 model whose matrices go to the kernels of this file (2^20 weights and more): a whole prompt, portions of up to 16
+    tokens, of more, and token by token, against a float64 statement of the model.  14 products, each as near as 2^-20 in the
+    2-norm (measured: 5e-7), and their sum is far above what attention, norms and activations add."""
+    from plain_torch import TorchQwen3
+    from nncpu_b200 import Engine, Model
+    from nncpu_b200.config import config_from_dict
+    from nncpu_b200.weights import write_model_folder
+    cfg = config_from_dict(dict(architectures=["Qwen3ForCausalLM"], num_hidden_layers=2, hidden_size=1024, num_attention_heads=8,
+                                num_key_value_heads=2, head_dim=128, intermediate_size=1536, vocab_size=1100, rope_theta=1e6,
+                                rms_norm_eps=1e-6, tie_word_embeddings=False, attention_bias=True, max_position_embeddings=4096))
+    folder = write_model_folder(tmp_path / "m", cfg, 3, torch.float32)
+    toks = torch.randint(0, 1100, (150,), generator=torch.Generator().manual_seed(1)).tolist()
+    want = torch.from_numpy(TorchQwen3(folder).logits(toks))
+    model = Model.load(folder, dtype="float32", device=DEV)
+
+    def through(cuts):
+        engine = Engine(model, max_tokens=256, n_slots=1, max_seq_len=256)
+        slot, rows = engine.alloc_slot(), []
+        for a, b in zip(cuts, cuts[1:]):
+            rows.append(engine.step([slot], [toks[a:b]], [list(range(b - a))]).double().cpu())
+        return torch.cat(rows)
+    for cuts in ([0, 150], [0, 16, 32, 35, 51, 60, 150], [0, 17, 57, 120, 150], [0, 100] + list(range(101, 151))):
+        got = through(cuts)
+        assert float((got - want).norm() / want.norm()) <= 14 * 2.0 ** -20, cuts
 
 
 def test_attention_of_more_tokens_than_a_grid_is_high(ops):
