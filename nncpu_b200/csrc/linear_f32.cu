@@ -6,8 +6,8 @@
 // of its four rows, four groups ahead, straight into registers.  The general kernel (64 x 16 tiles through shared
 // memory, scalar loads, no load in flight while it multiplies) leaves memory idle nine tenths of the time.  Measured (weights
 // from memory, us here / us there): N 12288, K 2048, two tokens 16.3 (6.2 TB/s) / 212; N 2048, K 6144 8.4 (6.0 TB/s) / 601;
-// sixteen tokens of N 12288 44 / 241.  From 2^20 weights on products come here (N 1024, K 1024, two tokens: 1.6 / 97;
-// N 512, K 512: 1.5 / 36); below, the general kernel's one order of sums for any number of rows is kept.
+// sixteen tokens of N 12288 44 / 241.  From 2^20 weights on products come here unless their rows are short (N 1024, K 1024, two
+// tokens: 1.6 / 97; N 512, K 512: 1.5 / 36); below, the general kernel's one order of sums for any number of rows is kept.
 // An element is summed over k in an order that K alone decides (per lane ascending, then the lanes' tree, then the
 // four warps), so a row's result does not depend on how many tokens the step has, up to the 16.
 //

@@ -286,6 +286,15 @@ LINEAR_F32_MAX_TOKENS = 16
 LINEAR_F32_MIN_WEIGHTS = 1 << 20
 
 
+def linear_f32_pays(m: int, n: int, k: int) -> bool:
+    """Whether a float32 product of ``m`` rows is faster by the kernels made for it than by ``linear_simt``: with enough weights, in
+    rows long enough.  The few-row kernel shares a row among four warps of 128 columns each, which in short rows have nothing to
+    do (us, here / there, N 150 000: one row K 192 71 / 71, K 256 70 / 93; four rows K 192 94 / 72, K 256 93 / 94; eight rows
+    K 512 208 / 188, K 640 214 / 232; N 65 536, K 16: 22 / 6.5), the tensor cores take 32 columns at a time (2 048 rows of N
+    32 768, K 32 273 / 241; of N 21 856, K 48 204 / 225)."""
+    return n * k >= LINEAR_F32_MIN_WEIGHTS and k >= (256 if m <= 4 else 640 if m <= LINEAR_F32_MAX_TOKENS else 48)
+
+
 def linear_f32_supported(x, w) -> bool:
     """Whether ``linear_f32`` and ``linear_f32_many`` take this product: float32 rows of whole 16-byte pieces on both sides."""
     return (x.dtype == torch.float32 and w.dtype == torch.float32 and x.shape[0] > 0 and x.shape[1] % 4 == 0

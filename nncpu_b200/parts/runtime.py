@@ -152,7 +152,7 @@ class Runtime:
                activation=None) -> None:
         """out (+)= x . w^T + bias.  bfloat16 inputs whose sizes keep TMA's
         alignment rule go to the tensor cores; everything else runs in true 32-bit: float32 products of a million
-        weights or more by the kernels made for them (few rows: CUDA cores; more: tensor cores on numbers cut in
+        weights or more, in rows that are not too short, by the kernels made for them (few rows: CUDA cores; more: tensor cores on numbers cut in
         three, of which nothing is lost), the rest on CUDA cores by the general kernel.
 
         ``x`` may be a ``DeferredNorm`` (a norm's unfinished output): the few-token product and the product of
@@ -198,7 +198,7 @@ class Runtime:
         else:
             assert epilogue == "plain" and activation is None, "fused epilogues exist on the tensor-core path only"
             # small layers stay with the kernel whose sums have one order for every number of rows: see the constant
-            if w.numel() < ops.LINEAR_F32_MIN_WEIGHTS or not ops.linear_f32_supported(x, w):
+            if not (ops.linear_f32_pays(x.shape[0], *w.shape) and ops.linear_f32_supported(x, w)):
                 ops.linear_simt(x, w, bias, out, accumulate)
             elif x.shape[0] <= ops.LINEAR_F32_MAX_TOKENS:
                 ops.linear_f32(x, w, bias, out, accumulate)

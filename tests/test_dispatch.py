@@ -29,3 +29,11 @@ def test_short_portions_token_by_token(n_seqs, tokens, n_kv, window, longest, fe
 def test_float32_attention_token_by_token(tokens, decode, n_seqs, by_token):
     chunk, stretches = ops.attention_f32_plan(tokens, decode, 700, n_seqs)
     assert (chunk > 0) is by_token and (stretches * chunk >= 700 or tokens > 64 or not by_token)
+
+
+@pytest.mark.parametrize("m,n,k,pays", [
+    (1, 1024, 1024, True), (1, 1023, 1024, False), (300, 1023, 1024, False), (300, 1024, 1024, True),
+    (1, 4096, 256, True), (4, 150000, 252, False), (5, 150000, 512, False), (16, 150000, 640, True),
+    (17, 65536, 32, False), (17, 21856, 48, True), (1, 65536, 16, False)])
+def test_float32_products(m, n, k, pays):
+    assert ops.linear_f32_pays(m, n, k) is pays
