@@ -39,9 +39,10 @@
 // first bytes' way from memory.  So the kernel is launched to overlap with the end of the kernel before it
 // (programmatic dependent launch): its blocks take the places that blocks of the earlier kernel leave, ask for
 // their first weights, which depend on nobody, and only then wait for the earlier kernel's results.  Only after
-// another product of this kind, though: a block that moves in beside blocks of a kernel with much shared memory
-// (decode attention) keeps the SM in that kernel's split of shared memory and L1 for as long as the chain of
-// overlapping products lasts, and with little L1 these products crawl (a decode layer took 135 us instead of 91).
+// kernels that use little shared memory, though (other products of this kind, norms, the sums of routed experts: the
+// caller says so): a block that moves in beside blocks of a kernel with much of it (decode attention) keeps the SM in
+// that kernel's split of shared memory and L1 for as long as the chain of overlapping products lasts, and with little
+// L1 these products crawl (a decode layer took 135 us instead of 91).
 
 #include <math.h>
 
@@ -355,12 +356,12 @@ extern "C" int nncpu_linear_skinny_norm_words() { return 16 * kBinWords; }
 //     bins_out, which must be zero, the sums of squares of C's rows; bins_clear (may be null) is set to zero;
 //   consumer: X holds such C * gamma rows of width K and bins_in their accumulators: the result is multiplied by
 //     1 / sqrt(sum / K + eps) per row before bias and activation.
-// after_skinny: the kernel before this one in the stream is a product of this function too; then this one may start
-// while that one ends (switched off for the whole library by nncpu_launch_overlap_linear_skinny(0)).
+// may_overlap: the kernel before this one in the stream uses little shared memory (see the head of this file); then this one may
+// start while that one ends (switched off for the whole library by nncpu_launch_overlap_linear_skinny(0)).
 extern "C" int nncpu_linear_skinny(const void* X, const void* W, const void* bias, int bias_dt, void* C, int c_dt,
                                    int M, int N, int K, int lda, int ldc, int accumulate, int epilogue, void* xg_out,
                                    const void* gamma, int gamma_dt, void* bins_out, void* bins_clear,
-                                   const void* bins_in, float eps, int act, float act_a, float act_b, int after_skinny,
+                                   const void* bins_in, float eps, int act, float act_a, float act_b, int may_overlap,
                                    void* stream_) {
     cudaStream_t stream = (cudaStream_t)stream_;
     NN_CHECK(nncpu_linear_skinny_supported(M, N, K, lda),
@@ -394,11 +395,11 @@ extern "C" int nncpu_linear_skinny(const void* X, const void* W, const void* bia
     if (epilogue == kSwiglu) {
         NN_CHECK(N % 16 == 0 && bias == nullptr && !accumulate,
                  "linear (few tokens): the gated epilogue needs N %% 16 == 0, no bias and no accumulation (N %d)", N);
-        return M <= 8 ? launch<1, kSwiglu>(X, W, bias, bias_dt, C, c_dt, M, N, K, lda, ldc, accumulate, nf, after_skinny != 0, stream)
-                      : launch<2, kSwiglu>(X, W, bias, bias_dt, C, c_dt, M, N, K, lda, ldc, accumulate, nf, after_skinny != 0, stream);
+        return M <= 8 ? launch<1, kSwiglu>(X, W, bias, bias_dt, C, c_dt, M, N, K, lda, ldc, accumulate, nf, may_overlap != 0, stream)
+                      : launch<2, kSwiglu>(X, W, bias, bias_dt, C, c_dt, M, N, K, lda, ldc, accumulate, nf, may_overlap != 0, stream);
     }
-    return M <= 8 ? launch<1, kPlain>(X, W, bias, bias_dt, C, c_dt, M, N, K, lda, ldc, accumulate, nf, after_skinny != 0, stream)
-                  : launch<2, kPlain>(X, W, bias, bias_dt, C, c_dt, M, N, K, lda, ldc, accumulate, nf, after_skinny != 0, stream);
+    return M <= 8 ? launch<1, kPlain>(X, W, bias, bias_dt, C, c_dt, M, N, K, lda, ldc, accumulate, nf, may_overlap != 0, stream)
+                  : launch<2, kPlain>(X, W, bias, bias_dt, C, c_dt, M, N, K, lda, ldc, accumulate, nf, may_overlap != 0, stream);
 }
 
 // C[r, :] = X[r, :] . W_e^T for the rows r of group e, in tiles of at most 8 or 16 rows (the routed experts of a step of up to

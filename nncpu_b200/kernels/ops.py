@@ -115,9 +115,10 @@ def _call(libname: str, fn: str, *args) -> None:
 
 def launch_overlap(on: bool) -> None:
     """Whether kernels that can do so are launched to start while the kernel before them ends: a few-token
-    product after another one (it asks for its first weights before it waits for that one's results), the
-    tensor-core products (their set-up; up to 64 tokens also their first weight tiles), prefill attention (its
-    set-up) and the norms between them.
+    product after a kernel of little shared memory and the float32 products of few rows (they ask for their first weights
+    before they wait for that one's results), the tensor-core products (their set-up; up to 64 bfloat16 tokens also their first
+    weight tiles), prefill attention (its set-up), float32 attention token by token, the norms and the small kernels of routers,
+    routed experts, gates and the stream between them.
     On by default; off, every kernel waits for the one before it to be over, and the results are the same bits."""
     for name in ("linear_skinny", "gemm_sm100", "generic", "attention_tc", "linear_f32", "attention_f32"):
         getattr(library.load(name), f"nncpu_launch_overlap_{name}")(ctypes.c_int(1 if on else 0))
@@ -490,12 +491,12 @@ def linear_skinny(x, w, bias, out, accumulate: bool = False, epilogue: str = "pl
         assert norm_out is None, "a product is a norm's producer or its consumer"
         bins_in, eps = norm_in
         assert bins_in.dtype == torch.int64 and bins_in.numel() == NORM_WORDS
-    # a product that follows another one may start while that one ends (see launch_overlap)
-    after_skinny = _last_fn in _BEFORE_SKINNY
+    # a product may start while a kernel that uses little shared memory ends (see launch_overlap)
+    may_overlap = _last_fn in _BEFORE_SKINNY
     _call("linear_skinny", "nncpu_linear_skinny", _ptr(x), _ptr(w), _ptr(bias), _i(_code(bias)), _ptr(out),
           _i(_code(out)), _i(m), _i(n), _i(k), _i(k), _i(out.shape[1]), _i(accumulate), _i(EPILOGUES[epilogue]),
           _ptr(xg), _ptr(gamma), _i(_code(gamma)), _ptr(bins_out), _ptr(bins_clear), _ptr(bins_in), _f(eps),
-          *_activation(activation), _i(after_skinny), _stream())
+          *_activation(activation), _i(may_overlap), _stream())
 
 
 def linear_skinny_force_warps(warps: int) -> None:
