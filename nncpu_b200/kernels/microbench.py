@@ -5,8 +5,11 @@ GFLOP/s for its row kernels and one attention block.
 
     python -m nncpu_b200.kernels.microbench linear M N K [--epilogue swiglu] [--accumulate] [--norm producer|consumer]
     python -m nncpu_b200.kernels.microbench linear-qkv TOKENS [--hidden K]
+    python -m nncpu_b200.kernels.microbench linear-f32 M N K
+    python -m nncpu_b200.kernels.microbench experts TOKENS [--experts 16] [--top 2] [--hidden 2048] [--inter 1536]
+    python -m nncpu_b200.kernels.microbench attention-f32 SEQUENCES TOKENS [--past KEYS]
     python -m nncpu_b200.kernels.microbench attention-decode BATCH CONTEXT [--splits S] [--cluster] [--from-projections]
-    python -m nncpu_b200.kernels.microbench attention-prefill BATCH TOKENS [--cap C]
+    python -m nncpu_b200.kernels.microbench attention-prefill BATCH TOKENS [--past KEYS] [--capacity KEYS] [--cap C]
     python -m nncpu_b200.kernels.microbench qk-conv BATCH TOKENS [--taps 4]
     python -m nncpu_b200.kernels.microbench rmsnorm ROWS DIM
     python -m nncpu_b200.kernels.microbench gla BATCH TOKENS [--columns 2|4]
@@ -125,9 +128,65 @@ def linear_qkv(args) -> None:
     print(f"linear-qkv M={m} N={n} K={k}: {ms * 1e3:.1f} us, {2 * m * n * k / ms / 1e9:.1f} TFLOP/s")
 
 
-def _cache(batch, ctx, nkv, hd, copies):
+def linear_f32(args) -> None:
+    """A float32 product: a stream over the weights up to 16 rows, beyond on the tensor cores, on numbers cut in three."""
+    m, n, k = args.m, args.n, args.k
+    ws = [torch.randn(n, k, device=DEV) * 0.02 for _ in range(max(2, 4 * L2_BYTES // (n * k * 4) + 1))]
+    x, out, work = torch.randn(m, k, device=DEV), torch.empty(m, n, device=DEV), ops.GemmWorkspace(DEV)
+    if m <= ops.LINEAR_F32_MAX_TOKENS:
+        run = lambda w: ops.linear_f32(x, w, None, out)
+    else:
+        floats = ops.linear_f32_many_scratch_floats(m, n, k)
+        scratch = torch.empty(floats, device=DEV) if floats else None
+        run = lambda w: ops.linear_f32_many(x, w, None, out, scratch, work)
+    ms = _time([lambda w=w: run(w) for w in ws], args.once)
+    if int(work.status.item()):
+        raise SystemExit(f"the kernel gave up waiting (status {int(work.status.item())})")
+    print(f"linear-f32 M={m} N={n} K={k}: {ms * 1e3:.1f} us, {n * k * 4 / ms / 1e6:.0f} GB/s of weights, "
+          f"{2 * m * n * k / ms / 1e9:.1f} TFLOP/s")
+
+
+def experts(args) -> None:
+    """The two products of routed experts in a step of few tokens: gate and up with the activation, and down."""
+    n, E, top, h, f = args.tokens, args.experts, args.top, args.hidden, args.inter
+    S, rows = n * top, ops.skinny_grouped_rows(n)
+    copies = max(2, 4 * L2_BYTES // (E * 3 * f * h * 2) + 1)
+    sets = [((torch.randn(E, 2 * f, h, device=DEV) * 0.02).bfloat16(), (torch.randn(E, h, f, device=DEV) * 0.02).bfloat16())
+            for _ in range(copies)]
+    ids = torch.stack([torch.randperm(E, device=DEV)[:top] for _ in range(n)]).to(torch.int32)
+    row_of_slot, slot_of_row = (torch.empty(S, dtype=torch.int32, device=DEV) for _ in range(2))
+    plan = torch.empty(1 + 3 * ops.moe_plan_tiles(S, E, rows), dtype=torch.int32, device=DEV)
+    ops.moe_plan(ids, E, row_of_slot, slot_of_row, plan, rows)
+    xs, mid = torch.randn(S, h, device=DEV).bfloat16(), torch.empty(S, f, dtype=torch.bfloat16, device=DEV)
+    y = torch.empty(S, h, device=DEV)
+    read = int(torch.unique(ids).numel())
+    for name, call, nbytes in (("gate/up", lambda u, d: ops.linear_skinny_grouped(xs, u, mid, plan, E, n, "swiglu"), read * 4 * f * h),
+                               ("down", lambda u, d: ops.linear_skinny_grouped(mid, d, y, plan, E, n), read * 2 * f * h)):
+        ms = _time([lambda u=u, d=d: call(u, d) for u, d in sets], args.once)
+        print(f"experts {name} tokens={n} top={top} of {E} ({read} read) {f} x {h}: {ms * 1e3:.1f} us, {nbytes / ms / 1e6:.0f} GB/s of weights")
+
+
+def attention_f32(args) -> None:
+    """Float32 attention of sequences that bring `tokens` tokens each behind `past` keys, by the kernel that a step takes."""
+    nh, nkv, hd, b, t, ctx = args.heads, args.kv_heads, args.head_dim, args.sequences, args.tokens, args.past + args.tokens
+    sets, table = _cache(b, ctx, nkv, hd, max(2, 4 * L2_BYTES // (b * ctx * nkv * hd * 8) + 1), torch.float32)
+    seq = torch.arange(b, dtype=torch.int32, device=DEV).repeat_interleave(t)
+    pos = torch.arange(args.past, ctx, dtype=torch.int32, device=DEV).repeat(b)
+    q = torch.randn(b * t, nh * hd, device=DEV)
+    out = torch.empty_like(q)
+    plan = ops.attention_f32_plan(b * t, t == 1, ctx, b)
+    scratch = torch.empty(b * t * nh * plan[1] * (hd + 2), device=DEV) if plan[1] > 1 else None
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    ms = _time([lambda kp=kp, vp=vp: ops.attention_f32(q, kp, vp, table, seq, pos, out, scratch, nh, nkv, hd, hd ** -0.5, plan, sms,
+                                                       n_seqs=b) for kp, vp in sets], args.once)
+    flops = 4.0 * nh * hd * b * t * (args.past + (t + 1) / 2)
+    print(f"attention-f32 sequences={b} tokens={t} past={args.past} {'token by token' if plan[0] else 'tiles'}: {ms * 1e3:.1f} us, "
+          f"{b * ctx * nkv * hd * 8 / ms / 1e6:.0f} GB/s of cache, {flops / ms / 1e9:.1f} TFLOP/s")
+
+
+def _cache(batch, ctx, nkv, hd, copies, dtype=torch.bfloat16):
     pages = batch * ((ctx + 63) // 64)
-    sets = [(torch.randn(pages, nkv, 64, hd, device=DEV).bfloat16(), torch.randn(pages, nkv, 64, hd, device=DEV).bfloat16())
+    sets = [(torch.randn(pages, nkv, 64, hd, device=DEV).to(dtype), torch.randn(pages, nkv, 64, hd, device=DEV).to(dtype))
             for _ in range(copies)]
     table = torch.randperm(pages, device=DEV).to(torch.int32).view(batch, -1)
     return sets, table
@@ -163,9 +222,9 @@ def attention_decode(args) -> None:
 
 def attention_prefill(args) -> None:
     nh, nkv, hd, b, t = args.heads, args.kv_heads, args.head_dim, args.batch, args.tokens
-    sets, table = _cache(b, t, nkv, hd, 1)
+    sets, table = _cache(b, args.past + t, nkv, hd, 1)
     kp, vp = sets[0]
-    pos = torch.arange(t, dtype=torch.int32, device=DEV).repeat(b)
+    pos = torch.arange(args.past, args.past + t, dtype=torch.int32, device=DEV).repeat(b)
     cu = torch.arange(b + 1, dtype=torch.int32, device=DEV) * t
     q = torch.randn(b * t, nh * hd, device=DEV).bfloat16()
     out = torch.empty_like(q)
@@ -174,12 +233,12 @@ def attention_prefill(args) -> None:
     else:
         status = torch.zeros(1, dtype=torch.int32, device=DEV)
         run = lambda: ops.attention_prefill_tc(q, kp, vp, table, cu, pos, out, status, b, nh, nkv, hd,
-                                               1 / math.sqrt(hd), 0, cap=args.cap)
+                                               1 / math.sqrt(hd), 0, cap=args.cap, longest=args.capacity or args.past + t)
     ms = _time([run] * 3, args.once)
     if not args.legacy and int(status.item()):
         raise SystemExit(f"the kernel gave up waiting (status {int(status.item())})")
-    flops = 4.0 * nh * hd * b * t * (t + 1) / 2
-    print(f"attention-prefill batch={b} tokens={t}{f' cap={args.cap:g}' if args.cap else ''}: {ms * 1e3:.1f} us, {flops / ms / 1e9:.0f} TFLOP/s (causal)")
+    flops = 4.0 * nh * hd * b * t * (args.past + (t + 1) / 2)
+    print(f"attention-prefill batch={b} tokens={t}{f' past={args.past}' if args.past else ''}{f' cap={args.cap:g}' if args.cap else ''}: {ms * 1e3:.1f} us, {flops / ms / 1e9:.0f} TFLOP/s (causal)")
 
 
 def qk_conv(args) -> None:
@@ -322,6 +381,8 @@ def main(argv=None) -> int:
         p.add_argument("--head-dim", type=int, default=128); p.add_argument("--splits", type=int, default=0)
         p.add_argument("--cluster", action="store_true", help="merge the splits inside a cluster (at most 8)")
         p.add_argument("--cap", type=float, default=0.0, help="prefill: scores are capped, C tanh(z / C)")
+        p.add_argument("--past", type=int, default=0, help="prefill: keys before the new tokens")
+        p.add_argument("--capacity", type=int, default=0, help="prefill: keys that the step may have (0: those it has)")
         p.add_argument("--legacy", action="store_true", help="prefill: the mma.sync kernel instead of tcgen05")
         p.add_argument("--from-projections", action="store_true",
                        help="decode: start from the float32 q/k/v projections (norm, rotation, append inside), as a step does")
@@ -336,6 +397,18 @@ def main(argv=None) -> int:
     p.add_argument("--heads", type=int, default=32); p.add_argument("--kv-heads", type=int, default=8)
     p.add_argument("--head-dim", type=int, default=128)
     p.set_defaults(fn=linear_qkv)
+    p = sub.add_parser("linear-f32")
+    p.add_argument("m", type=int); p.add_argument("n", type=int); p.add_argument("k", type=int)
+    p.set_defaults(fn=linear_f32)
+    p = sub.add_parser("experts")
+    p.add_argument("tokens", type=int); p.add_argument("--experts", type=int, default=16); p.add_argument("--top", type=int, default=2)
+    p.add_argument("--hidden", type=int, default=2048); p.add_argument("--inter", type=int, default=1536)
+    p.set_defaults(fn=experts)
+    p = sub.add_parser("attention-f32")
+    p.add_argument("sequences", type=int); p.add_argument("tokens", type=int); p.add_argument("--past", type=int, default=0)
+    p.add_argument("--heads", type=int, default=16); p.add_argument("--kv-heads", type=int, default=4)
+    p.add_argument("--head-dim", type=int, default=128)
+    p.set_defaults(fn=attention_f32)
     p = sub.add_parser("rmsnorm")
     p.add_argument("rows", type=int); p.add_argument("dim", type=int)
     p.set_defaults(fn=rmsnorm)
