@@ -43,13 +43,15 @@ struct AttnF32 {
     const float* head_gate;
     int gate_ld;
     int chunk, n_chunks;       // least keys of a stretch (a multiple of 128), most stretches of a token
+    unsigned room;             // chunk * n_chunks, at most 2^31
+    int t0;                    // token by token: the launch's first token
     int runs;                  // prompts: blocks a tile of tokens has for the sequences in it
 };
 
 // Keys of a stretch for the token at `pos`: the least, doubled until the token's keys fit the stretches there is room for.
 __device__ __forceinline__ int stretch_of(const AttnF32& p, int pos) {
     int chunk = p.chunk;
-    while ((long)chunk * p.n_chunks <= pos) chunk *= 2;
+    for (unsigned keys = p.room; keys <= (unsigned)pos; keys *= 2) chunk *= 2;      // (room is at least 128: ends below 2^32)
     return chunk;
 }
 
@@ -77,6 +79,7 @@ __device__ __forceinline__ void axpy4(float a, const float4& x, float4& y) {
 }
 
 constexpr int kDecodeKeys = 128;   // keys per round of a block: 32 per warp, half a page
+constexpr int kTokensPerLaunch = 65535;
 
 // GB: query heads a block takes (1, 2, 4 or 8), of the n_heads / n_kv that share a key/value head.
 template <int GB>
@@ -89,8 +92,8 @@ decode_f32_kernel(const AttnF32 p) {
     wait_for_previous_kernels();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int group = p.n_heads / p.n_kv, per_kv = (group + GB - 1) / GB;
-    const int kvh = blockIdx.y / per_kv, g0 = (blockIdx.y % per_kv) * GB;
-    const int t = blockIdx.x;                    // (the dimension of a grid that takes any number of tokens)
+    const int kvh = blockIdx.x / per_kv, g0 = (blockIdx.x % per_kv) * GB;
+    const int t = p.t0 + blockIdx.z;
     const int seq = p.tok_seq[t];
     if (seq < 0) {          // padding: zeros (from the block of the first stretch when nothing is merged)
         if (p.n_chunks == 1)
@@ -112,7 +115,7 @@ decode_f32_kernel(const AttnF32 p) {
         q[g] = d4 < p.hd ? *reinterpret_cast<const float4*>(p.q + ((size_t)t * p.n_heads + h) * p.hd + d4) : zero;
         slope[g] = slope_of(p, h);
     }
-    for (int c = blockIdx.z; c < p.n_chunks; c += gridDim.z) {
+    for (int c = blockIdx.y; c < p.n_chunks; c += gridDim.y) {
         const int begin = c * chunk, end = min(begin + chunk, pos + 1);
         if (begin > pos) break;
         float m[GB], l[GB];
@@ -228,7 +231,7 @@ __global__ void __launch_bounds__(128)
 merge_f32_kernel(const AttnF32 p) {
     let_next_kernel_start();
     wait_for_previous_kernels();
-    const int t = blockIdx.x, h = blockIdx.y, d = threadIdx.x;
+    const int h = blockIdx.x, t = p.t0 + blockIdx.y, d = threadIdx.x;
     const size_t out = ((size_t)t * p.n_heads + h) * p.vo + d;
     if (p.tok_seq[t] < 0) {
         if (d < p.vo) p.out[out] = 0.0f;
@@ -488,32 +491,36 @@ extern "C" int nncpu_attention_f32(const void* q, const void* k_pages, const voi
     cudaStream_t st = (cudaStream_t)stream;
     AttnF32 p{(const float*)q, (const float*)k_pages, (const float*)v_pages, block_table, bt_stride, tok_seq, tok_pos,
               (float*)out, (float*)part, n_tok, n_heads, n_kv, hd, vd, vo, scale, window, keep, slope_base, sinks, cap,
-              head_gate, gate_ld, chunk, n_chunks, 1};
+              head_gate, gate_ld, chunk, n_chunks, 0, 0, 1};
     const int group = n_heads / n_kv;
-    NN_CHECK(n_heads <= 65535, "attention (32-bit): %d heads", n_heads);
     if (chunk > 0) {
+        p.room = (unsigned)((long)chunk * n_chunks < (1L << 31) ? (long)chunk * n_chunks : 1L << 31);
         const int gb = group >= 8 ? 8 : (group > 2 ? 4 : group);
         const int blocks_x = n_kv * ((group + gb - 1) / gb);
         // as many blocks as eight per SM ask for; a block with several stretches takes them in turn
         const long pairs = (long)blocks_x * n_tok;
         long per = (8L * sm_count + pairs - 1) / pairs;
         if (per > n_chunks) per = n_chunks;
-        const dim3 grid((unsigned)n_tok, (unsigned)blocks_x, (unsigned)per);
         // both launched to start while the kernel before them ends: their launches are as long as their work
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = grid;
         cfg.blockDim = dim3(128);
         cfg.stream = st;
         cudaLaunchAttribute attr[1];
         cfg.attrs = attr;
         cfg.numAttrs = overlap_attribute(attr);
         const auto kernel = gb == 8 ? decode_f32_kernel<8> : gb == 4 ? decode_f32_kernel<4> : gb == 2 ? decode_f32_kernel<2> : decode_f32_kernel<1>;
-        cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
-        NN_CHECK(e == cudaSuccess, "attention (32-bit): launch failed: %s", cudaGetErrorString(e));
-        if (n_chunks > 1) {
-            cfg.gridDim = dim3((unsigned)n_tok, (unsigned)n_heads);
-            e = cudaLaunchKernelEx(&cfg, merge_f32_kernel, p);
-            NN_CHECK(e == cudaSuccess, "attention (32-bit, merge): launch failed: %s", cudaGetErrorString(e));
+        // Tokens are the last dimension of the grids, which ends at 65 535: a step of more is several launches.  (With tokens
+        // in the first dimension, or all in one, eight sequences of 1 000 keys took 16.5 and sixteen 24 us instead of 13.7 and 17.4.)
+        for (p.t0 = 0; p.t0 < n_tok; p.t0 += kTokensPerLaunch) {
+            const unsigned tokens = (unsigned)(n_tok - p.t0 < kTokensPerLaunch ? n_tok - p.t0 : kTokensPerLaunch);
+            cfg.gridDim = dim3((unsigned)blocks_x, (unsigned)per, tokens);
+            cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
+            NN_CHECK(e == cudaSuccess, "attention (32-bit): launch failed: %s", cudaGetErrorString(e));
+            if (n_chunks > 1) {
+                cfg.gridDim = dim3((unsigned)n_heads, tokens);
+                e = cudaLaunchKernelEx(&cfg, merge_f32_kernel, p);
+                NN_CHECK(e == cudaSuccess, "attention (32-bit, merge): launch failed: %s", cudaGetErrorString(e));
+            }
         }
         return 0;
     }
