@@ -1185,6 +1185,17 @@ def skinny_grouped_rows(most_rows: int) -> int:
     return 8 if most_rows <= 8 else 16
 
 
+# Up to so many token slots routed experts go through ``linear_skinny_grouped``; with more, the experts that are read make it a
+# stream that the tensor-core kernel's larger blocks carry better.  Measured (us, gate/up and down together, here / there): 8 tokens,
+# top 2 of 16, 2048 x 1536 45 / 70; 8, top 8 of 64, 4096 x 1024 171 / 211; 16, top 4 of 64, 7168 x 2048 595 / 593; 16, top 8 of 64,
+# 4096 x 1024 288 / 238; 12, top 8 of 128, 2048 x 1024 177 / 162; 16, top 8 of 256, 4096 x 512 269 / 231.
+SKINNY_GROUPED_MAX_SLOTS = 64
+
+
+def skinny_grouped_pays(n_tokens: int, n_slots: int) -> bool:
+    return n_tokens <= SKINNY_MAX_TOKENS and n_slots <= SKINNY_GROUPED_MAX_SLOTS
+
+
 def linear_skinny_grouped(xs, w, out, plan, n_experts: int, most_rows: int, epilogue: str = "plain", activation=None) -> None:
     """``linear_tc_grouped`` for steps of ``most_rows`` <= 16 tokens: a stream over the weights of the experts that have any row.
     ``plan`` is ``moe_plan``'s with tiles of ``skinny_grouped_rows(most_rows)`` rows: a token that is not a number may choose an

@@ -237,7 +237,7 @@ class RoutedExperts(FeedForward):
             # many tokens: sorted by expert, one grouped product each for gate/up (activation in its epilogue) and
             # down on the tensor cores, then the choices of a token added up in their order
             act = (s.activation, float(s.limit), 0.0) if s.activation != "silu" else None
-            few = n <= ops.SKINNY_MAX_TOKENS
+            few = ops.skinny_grouped_pays(n, S)
             tile_rows = ops.skinny_grouped_rows(n) if few else 128
             with rt.phase("moe_sort", nbytes=4.0 * S * h):
                 rows, slots = rt.empty(S, dtype=torch.int32), rt.empty(S, dtype=torch.int32)

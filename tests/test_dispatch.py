@@ -37,3 +37,8 @@ def test_float32_attention_token_by_token(tokens, decode, n_seqs, by_token):
     (17, 65536, 32, False), (17, 21856, 48, True), (1, 65536, 16, False)])
 def test_float32_products(m, n, k, pays):
     assert ops.linear_f32_pays(m, n, k) is pays
+
+
+@pytest.mark.parametrize("tokens,top,pays", [(8, 2, True), (16, 4, True), (8, 8, True), (16, 5, False), (9, 8, False), (17, 1, False)])
+def test_routed_experts_by_the_few_row_product(tokens, top, pays):
+    assert ops.skinny_grouped_pays(tokens, tokens * top) is pays
