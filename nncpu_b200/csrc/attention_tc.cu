@@ -30,8 +30,7 @@
 // each walking six steps one after the other while 140 SMs idle.  There a cluster of 2, 4 or 8 blocks shares a tile: each walks
 // its part of the steps, leaves reference maximum, sum and O (32-bit) in its shared memory, and adds up its share of the columns
 // over the cluster's blocks, in their order, through distributed shared memory.  The launch knows only how many keys there may
-// be (a captured step: the cache's capacity), the device how many there are: a tile of up to kAloneSteps steps is walked by its
-// cluster's first block alone, the others leave.
+// be (a captured step: the cache's capacity), the device how many there are: a tile of up to kAloneSteps steps is not shared.
 //
 // The reference computes the same attention row by
 // row (crates/nncpu/src/model/forward.rs:141-160,383-426); softmax runs in 32-bit here
@@ -234,14 +233,17 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     const PageWalk walk(key_lo, key_hi, p.keep);     // the pages that hold keys these rows see
     const int n_pages = walk.n;
     // two pages a step, of which the last may hold one; this block walks the steps s0 .. s0 + n_steps - 1 of them
-    const int all_steps = (n_pages + 1) / 2, split = (int)blockIdx.x % p.splits;
-    const int splits = all_steps <= kAloneSteps ? 1 : p.splits;      // the same for all blocks of a cluster
-    if (split >= splits) return;                                     // (nobody of its cluster will wait for it)
+    const int all_steps = (n_pages + 1) / 2;
+    const int splits = all_steps <= kAloneSteps ? 1 : p.splits;      // the same for all blocks of a tile
+    const int split = (int)blockIdx.x % splits;
     const int s0 = split * all_steps / splits, n_steps = (split + 1) * all_steps / splits - s0;
     // the heads of a key/value head are dealt out two to a block; an odd group's last block has one
     const int group = p.n_heads / p.n_kv;
     const int per_kv = (group + kStreams - 1) / kStreams;
-    const int head_block = (int)blockIdx.x / p.splits;
+    // A tile that is not shared takes the grid's first blocks, all of a cluster's, and the other clusters leave whole: the places
+    // of a cluster's blocks are free for the next kernel only when its last block ends.
+    const int head_block = (int)blockIdx.x / splits;
+    if (head_block >= p.n_kv * per_kv) return;
     const int kvh = head_block / per_kv;
     const int head0 = kvh * group + (head_block % per_kv) * kStreams;
     const int n_streams = min(kStreams, group - (head_block % per_kv) * kStreams);
