@@ -85,7 +85,7 @@ struct AttnParams {
     // two scores an instruction.  Elsewhere u = 1 - 2 / (1 + 2^(cap_in * unscaled score)): two more special-function
     // results a score, which is what the softmax has least of.
     float cap_in, cap_x, cap_small, score_mul;
-    int splits;               // blocks of the cluster that shares a tile's steps (1: none)
+    int split_shift;          // 2 to this many blocks are a cluster that shares a tile's steps (0: none)
     const float* head_gate;   // or null: row t (at t * gate_ld) holds a logit a head, whose sigmoid multiplies the head's output
     long gate_ld;
     int* status;
@@ -234,15 +234,15 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     const int n_pages = walk.n;
     // two pages a step, of which the last may hold one; this block walks the steps s0 .. s0 + n_steps - 1 of them
     const int all_steps = (n_pages + 1) / 2;
-    const int splits = all_steps <= kAloneSteps ? 1 : p.splits;      // the same for all blocks of a tile
-    const int split = (int)blockIdx.x % splits;
-    const int s0 = split * all_steps / splits, n_steps = (split + 1) * all_steps / splits - s0;
+    const int shift = all_steps <= kAloneSteps ? 0 : p.split_shift;  // the same for all blocks of a tile
+    const int splits = 1 << shift, split = (int)blockIdx.x & (splits - 1);
+    const int s0 = split * all_steps >> shift, n_steps = ((split + 1) * all_steps >> shift) - s0;
     // the heads of a key/value head are dealt out two to a block; an odd group's last block has one
     const int group = p.n_heads / p.n_kv;
     const int per_kv = (group + kStreams - 1) / kStreams;
     // A tile that is not shared takes the grid's first blocks, all of a cluster's, and the other clusters leave whole: the places
     // of a cluster's blocks are free for the next kernel only when its last block ends.
-    const int head_block = (int)blockIdx.x / splits;
+    const int head_block = (int)blockIdx.x >> shift;
     if (head_block >= p.n_kv * per_kv) return;
     const int kvh = head_block / per_kv;
     const int head0 = kvh * group + (head_block % per_kv) * kStreams;
@@ -634,7 +634,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             if (p.head_gate != nullptr && row < n_rows)
                 inv *= 1.0f / (1.0f + expf(-p.head_gate[(size_t)(q0 + row) * p.gate_ld + h]));
             __nv_bfloat16* dst = p.out + ((size_t)(q0 + row) * p.n_heads + h) * p.vo;
-            const int cols = VD / splits;        // 8 at least
+            const int cols = VD >> shift;        // 8 at least
 #pragma unroll 1
             for (int c0 = split * cols; c0 < (split + 1) * cols; c0 += 8) {
                 float acc[8];
@@ -762,7 +762,7 @@ int launch_one(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& 
     // which 14 fit, and 34 us as clusters of 4).  How many fit is the device's to say: clusters lie within a GPC.
     static int fit[64][4] = {};      // per device, for clusters of 2, 4 and 8 (0: not asked yet)
     int dev = 0;
-    p.splits = 1;
+    p.split_shift = 0;
     if (longest > kAloneSteps * kKeys && cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64) {
         for (int n = 2, i = 1; n <= kMaxSplits && (n - 1) * kKeys < longest; n *= 2, ++i) {
             if (fit[dev][i] == 0) {
@@ -774,14 +774,14 @@ int launch_one(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& 
                 }
                 fit[dev][i] = clusters > 0 ? clusters : -1;
             }
-            if ((long)head_blocks * tiles <= fit[dev][i]) p.splits = n;
+            if ((long)head_blocks * tiles <= fit[dev][i]) p.split_shift = i;
         }
     }
     if (splits_only != nullptr) {
-        *splits_only = p.splits;
+        *splits_only = 1 << p.split_shift;
         return 0;
     }
-    with_splits(p.splits);
+    with_splits(1 << p.split_shift);
     cfg.numAttrs += overlap_attribute(attr + 1);
     const cudaError_t e = cudaLaunchKernelEx(&cfg, prefill_tc_kernel<HD, VD, kStreams, kCap>, mq, mk, mv, p);
     NN_CHECK(e == cudaSuccess, "attention prefill (tensor cores): launch failed: %s", cudaGetErrorString(e));

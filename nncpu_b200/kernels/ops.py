@@ -733,12 +733,15 @@ DECODE_CLUSTER_MAX_SPLITS = 8      # up to here the splits merge inside a thread
 
 
 # A short portion of one sequence goes through the decode kernel, token by token, while its tokens times key/value heads times
-# the keys that the step may hold are at most the first (a captured step may hold as many as the cache's sequences can grow to,
-# whatever its sequence holds), and its tokens times key/value heads, which are blocks of their own, at most the second; beyond,
-# as tiles of 128 rows (``attention_prefill_tc``).  Measured (us, token by token / tiles): at the first line, 16 heads over
-# 4, 64 tokens behind 700 14.5 / 15.3, 32 over 8, 16 behind 1 500 16.4 / 16.1; below it (32 tokens of 16 heads over 4 behind
-# 100) 4.9 / 8.1; above (32 over 8, 64 behind 1 500) 49 / 19; above the second (32 over 8, 64 tokens, no past) 8.1 / 7.0.
+# the keys that the step may hold are at most the first (the second for portions of up to 16 tokens), and its tokens times
+# key/value heads, which are blocks of their own, at most the third; beyond, as tiles of 128 rows (``attention_prefill_tc``).  A
+# captured step may hold as many keys as the cache's sequences can grow to, whatever its sequence holds.
+# Measured, the kernel alone (us, token by token / tiles): at the first line, 16 heads over 4, 64 tokens behind 700 14.5 / 15.3;
+# below it (32 tokens of 16 heads over 4 behind 100) 4.9 / 8.1; above (32 over 8, 64 behind 1 500) 49 / 19; above the third (32
+# over 8, 64 tokens, no past) 8.1 / 7.0.  Eight layers of 32 heads over 8 whole, 16 rows: no past 865 / 908, behind 700 891 / 984, behind
+# 3 000 1 016 / 1 045, behind 4 000 1 062 / 1 076.
 FEW_TOKENS_MAX_KEYS = 200_000
+FEWER_TOKENS_MAX_KEYS = 600_000
 FEW_TOKENS_MAX_BLOCKS = 256
 
 

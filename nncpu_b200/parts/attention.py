@@ -304,8 +304,9 @@ class Attention(Mixer):
         as one tile of 128 rows: while its tokens are few, and the keys that they may read together.  (In a captured step
         these are as many as the cache's sequences can grow to: the step is captured once for all lengths.)"""
         blocks = ctx.n_tokens * self.spec.n_kv_heads
+        keys = ops.FEWER_TOKENS_MAX_KEYS if ctx.n_tokens <= ops.SKINNY_MAX_TOKENS else ops.FEW_TOKENS_MAX_KEYS
         return (ctx.n_seqs == 1 and ctx.n_tokens <= 64 and blocks <= ops.FEW_TOKENS_MAX_BLOCKS
-                and blocks * self._longest_span(ctx) <= ops.FEW_TOKENS_MAX_KEYS)
+                and blocks * self._longest_span(ctx) <= keys)
 
     def _longest_span(self, ctx) -> int:
         s = self.spec

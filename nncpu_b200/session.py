@@ -40,7 +40,9 @@ class SessionParams:
     (crates/nncpu/src/session/engine.rs:113-117); ``seed`` 0 = random
     (crates/nncpu/src/session/engine.rs:125); ``kv_f32`` keeps the cache in
     float32 whatever the run's element type (the reference's ``--kv-f32``);
-    ``max_batch``: sequences generated together; ``system_prompt`` opens the
+    ``max_batch``: sequences generated together (in either precision a
+    sequence's logits depend on the others by rounding alone: the kernels of
+    a step follow from its size); ``system_prompt`` opens the
     session's conversation (crates/nncpu/src/session/mod.rs:37-83);
     ``reply_open`` is text the chat template puts at the start of every reply
     (Qwen3 without reasoning: ``"<think>\\n\\n</think>\\n\\n"``,

@@ -11,7 +11,7 @@ from nncpu_b200.parts.attention import Attention
 
 @pytest.mark.parametrize("n_seqs,tokens,n_kv,window,longest,few", [
     (1, 24, 4, 0, 724, True), (1, 24, 4, 0, 4096, False),      # by the keys there may be
-    (1, 16, 8, 0, 1500, True), (1, 16, 8, 0, 1600, False),
+    (1, 16, 8, 0, 4096, True), (1, 16, 8, 0, 4700, False), (1, 17, 8, 0, 4096, False),
     (1, 64, 4, 0, 300, True), (1, 64, 8, 0, 65, False),        # by the blocks
     (1, 32, 8, 0, 100, True), (1, 33, 8, 0, 100, False),
     (1, 24, 4, 512, 40960, True),                              # a window bounds the keys
