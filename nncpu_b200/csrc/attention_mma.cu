@@ -505,6 +505,31 @@ __device__ __forceinline__ float row_squares(const float* __restrict__ src, int 
     return ss;
 }
 
+// Which of n <= kByLengthMax tokens has the nth most keys (ties in their order, padding last).  A grid of more blocks than run at
+// once begins with the long sequences, so that the blocks that start last are short ones: a block's share of the bandwidth is
+// what it can keep in flight, and a long sequence that starts when the others are done streams alone (two blocks an SM; 64
+// sequences of 125 to 1 875 keys, 8 key/value heads, 512 blocks for 296 places: 61.8 us in the tokens' order, 50.0 by length; of
+// 384 to 5 760 keys 159 and 123; 40 of 125 to 1 875 43.2 and 39.8).
+constexpr int kByLengthMax = 128;
+__device__ __forceinline__ int nth_longest(const int* __restrict__ tok_seq, const int* __restrict__ tok_pos, int n, int nth) {
+    __shared__ __align__(16) int len_s[kByLengthMax];
+    __shared__ int found_s;
+    const int i = threadIdx.x;
+    const int mine = i < n ? (tok_seq[i] < 0 ? -1 : tok_pos[i]) : -2;
+    len_s[i] = mine;
+    __syncthreads();
+    int before = 0;
+#pragma unroll 4
+    for (int j = 0; j < n; j += 4) {          // (places behind n hold -2: before nobody)
+        const int4 o = *reinterpret_cast<const int4*>(&len_s[j]);
+        before += (o.x > mine || (o.x == mine && j < i)) + (o.y > mine || (o.y == mine && j + 1 < i)) +
+                  (o.z > mine || (o.z == mine && j + 2 < i)) + (o.w > mine || (o.w == mine && j + 3 < i));
+    }
+    if (i < n && before == nth) found_s = i;
+    __syncthreads();
+    return found_s;
+}
+
 // kMore: with a cap on the scores or a short convolution before the heads; kernels without either do not carry them.
 template <int HD, int VD, int NT, bool kCluster, bool kFused, bool kMore>
 __global__ void __launch_bounds__(128, 2)
@@ -513,15 +538,16 @@ decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restri
                    const int* __restrict__ tok_seq, const int* __restrict__ tok_pos, __nv_bfloat16* __restrict__ out,
                    float* __restrict__ part_o, float* __restrict__ part_ml, int n_heads, int n_kv, float scale2,
                    int window, int keep, const FusedQK f, const float* __restrict__ sinks, int kv_rep, int vo,
-                   const ScoreCap cap, const OutGate gate) {
+                   const ScoreCap cap, const OutGate gate, int by_length) {
     constexpr int kTileBytes = kPage * HD * 2, kStageBytes = kPage * (HD + VD) * 2;
     constexpr int kChunks = HD / 8, kVChunks = VD / 8;
     constexpr int W = VD + 2;
     extern __shared__ __align__(128) uint8_t dsm[];  // stages of [K page | V page]; afterwards the merge buffers
-    const int split = blockIdx.x, n_splits = gridDim.x, kvh = blockIdx.y, t = blockIdx.z;
+    const int split = blockIdx.x, n_splits = gridDim.x, kvh = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int c = lane & 3, r = lane >> 2;
     const int G = n_heads / n_kv;
+    const int t = by_length ? nth_longest(tok_seq, tok_pos, (int)gridDim.z, (int)blockIdx.z) : (int)blockIdx.z;
     const int seq = tok_seq[t];
     const size_t out_row = ((size_t)t * n_heads + (size_t)kvh * G) * vo;
     if (seq < 0) {  // padding: zeros (every block of a cluster takes this way out together)
@@ -849,7 +875,7 @@ int launch_decode_one(const void* q, const void* k_pages, const void* v_pages, c
                   float slope_base, const float* sinks, float cap, const OutGate& gate) {
     using Kernel = void (*)(const __nv_bfloat16*, const __nv_bfloat16*, const __nv_bfloat16*, const int*, int, const int*,
                             const int*, __nv_bfloat16*, float*, float*, int, int, float, int, int, const FusedQK, const float*,
-                            int, int, const ScoreCap, const OutGate);
+                            int, int, const ScoreCap, const OutGate, int);
     // a block serves at most 16 heads of a key/value head: where more share one, kv_rep blocks take a part each
     int kv_rep = 1;
     while ((n_heads / n_kv) % kv_rep != 0 || n_heads / n_kv / kv_rep > 16) ++kv_rep;
@@ -875,6 +901,8 @@ int launch_decode_one(const void* q, const void* k_pages, const void* v_pages, c
                                                    (int)(stages > (size_t)5 * 16 * (VD + 2) * 4 ? stages : (size_t)5 * 16 * (VD + 2) * 4));
         NN_CHECK(e == cudaSuccess, "attention decode: cannot reserve shared memory: %s", cudaGetErrorString(e));
     }
+    // two blocks run on an SM; with more than that they start in the order of their lengths
+    const int by_length = n_tok <= kByLengthMax && (long)n_splits * n_kv * n_tok > 2l * sm_count() ? 1 : 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(n_splits, n_kv, n_tok);
     cfg.blockDim = dim3(128);
@@ -890,7 +918,7 @@ int launch_decode_one(const void* q, const void* k_pages, const void* v_pages, c
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pages,
                                              (const __nv_bfloat16*)v_pages, block_table, bt_stride, tok_seq, tok_pos,
                                              (__nv_bfloat16*)out, part_o, part_ml, n_heads, n_kv, scale * kLog2e, window, keep, f,
-                                             sinks, kv_rep, vo, score_cap(scale, cap), gate);
+                                             sinks, kv_rep, vo, score_cap(scale, cap), gate, by_length);
     NN_CHECK(e == cudaSuccess, "attention decode (%d splits%s): launch failed: %s", n_splits, cluster ? ", cluster" : "",
              cudaGetErrorString(e));
     if (n_splits > 1 && !cluster) {
