@@ -138,8 +138,8 @@ cudaError_t launch_few(const float* X, const float* W, const void* bias, int bia
 // instead of six.)  So BN is as large as the tokens and the two accumulators of tensor memory allow, and the cutters' work is what
 // counts: conversions in pairs (cvt.rn.bf16x2) and 16-byte stores; ten cutting warps, the next group's loads ahead, or 8-byte
 // stores without selects were no faster.
-// Measured (weights from memory): N 12288, K 2048, 17 tokens 42 us, 300 tokens 145, 2 048 tokens 644 (160 TFLOP/s of true 32-bit
-// results, where the CUDA cores' peak is 72); N 2048, K 6144, 300 tokens 75.  A layer of 300 tokens (hidden 2048): 297 us for its
+// Measured (weights from memory, tokens cut beforehand from 96 on): N 12288, K 2048, 17 tokens 42 us, 300 tokens 120, 600 tokens 168 (180
+// TFLOP/s of true 32-bit results, where the CUDA cores' peak is 72); N 2048, K 6144, 300 tokens 64.  A layer of 300 tokens (hidden 2048): 254 us for its
 // four products, 3 130 us in the general kernel.  Cut into two tf32 numbers they took 251 us, but of a quarter of all numbers
 // the last bit was lost.
 // Error against 64-bit sums (2-norm, N(0, 1) times N(0, 0.02)), here / the general kernel's chain of fmaf: K 64 0.6e-7 / 1.5e-7,
@@ -166,6 +166,7 @@ struct ManyParams {
     void* out;
     int out_dt;
     float* part;          // slices > 1: [slices, M, N]
+    uint16_t *cut_ab, *cut_c;   // the tokens cut beforehand: [M][kb_total][32 a, 32 b] and [M][kb_total][32 c] (see f32_cut_kernel)
     int M, N, K, lda, ldc, accumulate;
     int tiles_a, tiles_b, slices, kb_total;
     int flush;            // k-blocks that the tensor core sums by itself
@@ -222,9 +223,50 @@ constexpr int kManyStages = BN > 160 ? 3 : (BN > 96 ? 4 : 5);     // as many as 
 template <int BN>
 constexpr size_t kManySmem = 1024 + (size_t)kManyStages<BN> * (128 + BN) * 192 + 256;
 
-template <int BN>
+// Eight numbers in their three parts.
+__device__ __forceinline__ void cut_eight(const float (&x)[8], uint4& va, uint4& vb, uint4& vc) {
+    uint32_t a[4], b[4], c[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float x0 = x[2 * j], x1 = x[2 * j + 1];
+        a[j] = nearest_bf16(x0, x1);
+        const float y0 = x0 - lower(a[j]), y1 = x1 - upper(a[j]);
+        b[j] = nearest_bf16(y0, y1);
+        c[j] = nearest_bf16(y0 - lower(b[j]), y1 - upper(b[j]));      // 7 bits at most: exact
+    }
+    va = make_uint4(a[0], a[1], a[2], a[3]);
+    vb = make_uint4(b[0], b[1], b[2], b[3]);
+    vc = make_uint4(c[0], c[1], c[2], c[3]);
+}
+
+// The tokens' parts, made once (bound by its launch: 300 tokens of K 2048 are 2 MB).  Every tile of 128 weight rows multiplies
+// with all tokens, so cut where they arrive the tokens are cut N / 128 times: 160 rows of them for 128 of weights in the
+// products of a 300-token prompt.  Cut beforehand, 300 tokens of N 12288 x K 2048 take 145 -> 120 us.
+__global__ void __launch_bounds__(256) f32_cut_kernel(const ManyParams p) {
+    let_next_kernel_start();
+    wait_for_previous_kernels();
+    const long i = (long)blockIdx.x * 256 + threadIdx.x;        // eight numbers each
+    const int per_row = p.kb_total * (kManyK / 8);
+    const int row = (int)(i / per_row), g = (int)(i % per_row), k = g * 8;
+    if (row >= p.M) return;
+    float x[8];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)       // (K is a multiple of 4)
+        *reinterpret_cast<float4*>(&x[4 * h]) = k + 4 * h < p.K ? *reinterpret_cast<const float4*>(p.x + (size_t)row * p.lda + k + 4 * h)
+                                                              : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    uint4 va, vb, vc;
+    cut_eight(x, va, vb, vc);
+    uint16_t* ab = p.cut_ab + ((size_t)row * p.kb_total + k / kManyK) * 64 + k % kManyK;
+    *reinterpret_cast<uint4*>(ab) = va;
+    *reinterpret_cast<uint4*>(ab + 32) = vb;
+    *reinterpret_cast<uint4*>(p.cut_c + (size_t)row * p.kb_total * 32 + k) = vc;
+}
+
+// kCutX: the tokens' parts come ready-made by TMA (map_x their a and b, map_c their c) and only the weights are cut here.
+template <int BN, bool kCutX>
 __global__ void __launch_bounds__(kManyThreads, 1)
-f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const ManyParams p) {
+f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+                const __grid_constant__ CUtensorMap map_c, const ManyParams p) {
     constexpr int kStages = kManyStages<BN>;
     // A k-block: 128 rows of weights, then BN of tokens.  128 bytes a row, as TMA brings them (128-byte swizzle) and, cut, 32 numbers
     // a and 32 numbers b; behind them 64 bytes a row of numbers c (64-byte swizzle).
@@ -241,7 +283,13 @@ f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     uint64_t* acc_empty = acc_full + 2;     // [2]
     uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int kCopied = 128 * 128 + BN * (kCutX ? 192 : 128);      // bytes that arrive for a stage
     let_next_kernel_start();
+    const int tiles = p.tiles_a * p.tiles_b, n_items = tiles * p.slices;
+    // item i: the tiles of tokens of one tile of weights stand together, so that its weights are read from memory once
+    auto first_kb = [&](int slice) { return (int)((long)slice * p.kb_total / p.slices); };
+    const int slice0 = (int)blockIdx.x / tiles;                        // of this block's first item
+    const int n_first = kCutX ? min(kStages, first_kb(slice0 + 1) - first_kb(slice0)) : 0;
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
             mbar_init(&full[s], 1);
@@ -254,6 +302,11 @@ f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        // the first weights are asked for while the tokens are being cut
+        for (int r = 0; r < n_first; ++r) {
+            mbar_expect_tx(&full[r], kCopied);
+            tma_load_2d(smem + r * kStageBytes, &map_w, &full[r], (first_kb(slice0) + r) * kManyK, ((int)blockIdx.x / p.tiles_b % p.tiles_a) * 128);
+        }
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kTmemCols)
@@ -265,10 +318,6 @@ f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
     wait_for_previous_kernels();
-
-    const int tiles = p.tiles_a * p.tiles_b, n_items = tiles * p.slices;
-    // item i: the tiles of tokens of one tile of weights stand together, so that its weights are read from memory once
-    auto first_kb = [&](int slice) { return (int)((long)slice * p.kb_total / p.slices); };
 
     if (warp < 8) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kManyRegsFew));
@@ -284,10 +333,17 @@ f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                         ok = false;
                         break;
                     }
-                    mbar_expect_tx(&full[s], kRawBytes);     // (rows past the end are filled with zeros and counted)
-                    if (kb + kManyAhead < first_kb(slice + 1)) tma_prefetch_2d(&map_w, (kb + kManyAhead) * kManyK, m0);
-                    tma_load_2d(smem + s * kStageBytes, &map_w, &full[s], kb * kManyK, m0);
-                    tma_load_2d(smem + s * kStageBytes + 128 * 128, &map_x, &full[s], kb * kManyK, n0);
+                    if (run >= n_first) {                      // (the first weights have been asked for)
+                        mbar_expect_tx(&full[s], kCopied);     // (rows past the end are filled with zeros and counted)
+                        if (kb + kManyAhead < first_kb(slice + 1)) tma_prefetch_2d(&map_w, (kb + kManyAhead) * kManyK, m0);
+                        tma_load_2d(smem + s * kStageBytes, &map_w, &full[s], kb * kManyK, m0);
+                    }
+                    if constexpr (kCutX) {
+                        tma_load_2d(smem + s * kStageBytes + 128 * 128, &map_x, &full[s], kb * 64, n0);
+                        tma_load_2d(smem + s * kStageBytes + kRawBytes + 128 * 64, &map_c, &full[s], kb * 32, n0);
+                    } else {
+                        tma_load_2d(smem + s * kStageBytes + 128 * 128, &map_x, &full[s], kb * kManyK, n0);
+                    }
                 }
             }
             // let the copies in flight land before the block gives up its shared memory
@@ -308,7 +364,8 @@ f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                         ok = false;
                         break;
                     }
-                    if (!mbar_wait(&cut[s], (run / kStages) & 1)) {
+                    // (the tokens' parts that TMA brought belong to `full`, which the cutters have waited for, too)
+                    if (!mbar_wait(&cut[s], (run / kStages) & 1) || (kCutX && !mbar_wait(&full[s], (run / kStages) & 1))) {
                         atomicExch(p.status, kTimeoutCut);
                         ok = false;
                         break;
@@ -360,7 +417,7 @@ f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                     __syncwarp();
                     uint8_t* const raw = smem + s * kStageBytes;
                     uint8_t* const rest = raw + kRawBytes;
-                    constexpr int kGroups = (128 + BN) / 8;
+                    constexpr int kGroups = (kCutX ? 128 : 128 + BN) / 8;
 #pragma unroll 1
                     for (int g0 = warp - 2; g0 < kGroups; g0 += 2 * kCutters) {
                         const int g1 = g0 + kCutters;
@@ -378,19 +435,11 @@ f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                         for (int u = 0; u < 2; ++u) {
                             const int g = u == 0 ? g0 : g1;
                             if (g >= kGroups) break;
-                            uint32_t a[4], b[4], rest_of[4];
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                const float x0 = x[u][2 * j], x1 = x[u][2 * j + 1];
-                                a[j] = nearest_bf16(x0, x1);
-                                const float y0 = x0 - lower(a[j]), y1 = x1 - upper(a[j]);
-                                b[j] = nearest_bf16(y0, y1);
-                                rest_of[j] = nearest_bf16(y0 - lower(b[j]), y1 - upper(b[j]));      // 7 bits at most: exact
-                            }
-                            const uint4 va = make_uint4(a[0], a[1], a[2], a[3]), vb = make_uint4(b[0], b[1], b[2], b[3]);
+                            uint4 va, vb, vc;
+                            cut_eight(x[u], va, vb, vc);
                             *reinterpret_cast<uint4*>(raw + g * 1024 + (odd ? out_b : out_a)) = odd ? vb : va;
                             *reinterpret_cast<uint4*>(raw + g * 1024 + (odd ? out_a : out_b)) = odd ? va : vb;
-                            *reinterpret_cast<uint4*>(rest + g * 512 + out_c) = make_uint4(rest_of[0], rest_of[1], rest_of[2], rest_of[3]);
+                            *reinterpret_cast<uint4*>(rest + g * 512 + out_c) = vc;
                         }
                     }
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -553,16 +602,37 @@ int make_map_f32(CUtensorMap* map, const void* base, int rows, int K, long ld, i
     return 0;
 }
 
-template <int BN>
+// The cut tokens: [rows, cols] 16-bit parts, in boxes of box_rows x box_cols (64: a and b; 32: c).
+int make_map_cut(CUtensorMap* map, const void* base, int rows, long cols, int box_rows, int box_cols) {
+    EncodeTiledFn fn = encode_tiled();
+    NN_CHECK(fn != nullptr, "linear (32-bit): the driver does not offer cuTensorMapEncodeTiled");
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
+    const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
+    const cuuint32_t elem[2] = {1, 1};
+    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    NN_CHECK(r == CUDA_SUCCESS, "linear (32-bit): cuTensorMapEncodeTiled failed with code %d (parts of %d rows)", (int)r, rows);
+    return 0;
+}
+
+template <int BN, bool kCutX>
 int launch_many(const ManyParams& p, cudaStream_t stream) {
-    CUtensorMap mw, mx;
+    CUtensorMap mw, mx, mc;
     if (int e = make_map_f32(&mw, p.w, p.N, p.K, p.K, 128)) return e;
-    if (int e = make_map_f32(&mx, p.x, p.M, p.K, p.lda, BN)) return e;
+    if constexpr (kCutX) {
+        if (int e = make_map_cut(&mx, p.cut_ab, p.M, (long)p.kb_total * 64, BN, 64)) return e;
+        if (int e = make_map_cut(&mc, p.cut_c, p.M, (long)p.kb_total * 32, BN, 32)) return e;
+    } else {
+        if (int e = make_map_f32(&mx, p.x, p.M, p.K, p.lda, BN)) return e;
+        mc = mx;
+    }
     constexpr size_t smem = kManySmem<BN>;
     static_assert(smem <= 227 * 1024, "the stages fit shared memory");
     static bool configured[64] = {};
     if (first_use_on_this_device(configured)) {
-        const cudaError_t e = cudaFuncSetAttribute(f32_many_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = cudaFuncSetAttribute(f32_many_kernel<BN, kCutX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         NN_CHECK(e == cudaSuccess, "linear (32-bit): cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
     }
     const long items = (long)p.tiles_a * p.tiles_b * p.slices;
@@ -574,7 +644,16 @@ int launch_many(const ManyParams& p, cudaStream_t stream) {
     cudaLaunchAttribute attr[1];
     cfg.numAttrs = overlap_attribute(attr);
     cfg.attrs = attr;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, f32_many_kernel<BN>, mw, mx, p);
+    cudaError_t e = cudaSuccess;
+    if constexpr (kCutX) {
+        cudaLaunchConfig_t pre = cfg;
+        pre.gridDim = dim3((unsigned)(((long)p.M * p.kb_total * (kManyK / 8) + 255) / 256));
+        pre.blockDim = dim3(256);
+        pre.dynamicSmemBytes = 0;
+        e = cudaLaunchKernelEx(&pre, f32_cut_kernel, p);
+        NN_CHECK(e == cudaSuccess, "linear (32-bit, cutting): launch failed: %s", cudaGetErrorString(e));
+    }
+    e = cudaLaunchKernelEx(&cfg, f32_many_kernel<BN, kCutX>, mw, mx, mc, p);
     NN_CHECK(e == cudaSuccess, "linear (32-bit): launch failed: %s", cudaGetErrorString(e));
     if (p.slices > 1) {
         const bool vec = p.N % 4 == 0 && p.ldc % 4 == 0 && p.out_dt == DT_F32 && (uintptr_t)p.out % 16 == 0 && (uintptr_t)p.part % 16 == 0;
@@ -589,6 +668,15 @@ int launch_many(const ManyParams& p, cudaStream_t stream) {
 }
 
 }  // namespace
+
+// Floats that the parts of M tokens take where they are cut beforehand (0: cut where they arrive).  The cutting is a launch of its
+// own, and with few tokens there is little of them to cut beside 128 rows of weights (us, on arrival / beforehand, N x K 12288 x
+// 2048 and 2048 x 6144: 17 tokens 42.6 / 44.5 and 26.1 / 28.1, 64 tokens 46.8 / 47.5 and 29.6 / 32.3, 100 tokens 66.8 / 58.0 and
+// 41.7 / 36.3, 300 tokens 145 / 120 and 74.7 / 64.1, 600 tokens 210 / 168 and 119 / 107; 100 tokens of 2048 x 2048 22.3 / 21.5).
+constexpr int kCutFrom = 96;
+static long cut_floats(int M, int K) {
+    return M < kCutFrom ? 0 : (long)M * ((K + kManyK - 1) / kManyK) * (kManyK * 3 / 2);
+}
 
 // What the products here take: rows of whole 16-byte pieces.
 extern "C" int nncpu_linear_f32_supported(int M, int N, int K, int lda) {
@@ -617,7 +705,7 @@ extern "C" int nncpu_linear_f32(const void* X, const void* W, const void* bias, 
 extern "C" long nncpu_linear_f32_many_scratch(int M, int N, int K) {
     if (M <= 0 || N <= 0 || K <= 0) return 0;
     const ManyPlan plan = many_plan(M, N, K);
-    return plan.slices > 1 ? (long)plan.slices * M * N : 0;
+    return cut_floats(M, K) + (plan.slices > 1 ? (long)plan.slices * M * N : 0);
 }
 
 // The same product for any number of tokens, on the tensor cores.  `scratch`: see above.  `status` is set when a bounded wait
@@ -630,17 +718,20 @@ extern "C" int nncpu_linear_f32_many(const void* X, const void* W, const void* b
     NN_CHECK((uintptr_t)X % 16 == 0 && (uintptr_t)W % 16 == 0, "linear (32-bit): operands must be 16-byte aligned");
     const ManyPlan plan = many_plan(M, N, K);
     NN_CHECK(plan.slices == 1 || scratch != nullptr, "linear (32-bit): %d slices of K need scratch memory", plan.slices);
-    ManyParams p{(const float*)X, (const float*)W, bias, bias_dt, C, c_dt, (float*)scratch, M, N, K, lda, ldc, accumulate,
+    ManyParams p{(const float*)X, (const float*)W, bias, bias_dt, C, c_dt, (float*)scratch, nullptr, nullptr, M, N, K, lda, ldc, accumulate,
                  (N + 127) / 128, plan.tiles_b, plan.slices, (K + kManyK - 1) / kManyK, K < kShortK ? 1 : 2, status};
     NN_CHECK((long)p.tiles_a * p.tiles_b * p.slices < (1L << 31), "linear (32-bit): %d tokens of %d features", M, N);
-    switch (plan.bn) {
-        case 32: return launch_many<32>(p, st);
-        case 64: return launch_many<64>(p, st);
-        case 96: return launch_many<96>(p, st);
-        case 128: return launch_many<128>(p, st);
-        case 160: return launch_many<160>(p, st);
-        case 192: return launch_many<192>(p, st);
-        case 224: return launch_many<224>(p, st);
-        default: return launch_many<256>(p, st);
+    const long floats = scratch != nullptr ? cut_floats(M, K) : 0;
+    if (floats > 0) {
+        NN_CHECK((uintptr_t)scratch % 16 == 0, "linear (32-bit): scratch memory must be 16-byte aligned");
+        p.cut_ab = (uint16_t*)scratch;
+        p.cut_c = p.cut_ab + (size_t)M * p.kb_total * 64;
+        p.part = (float*)scratch + floats;
     }
+#define NN_MANY(BN_) case BN_: return floats > 0 ? launch_many<BN_, true>(p, st) : launch_many<BN_, false>(p, st);
+    switch (plan.bn) {
+        NN_MANY(32) NN_MANY(64) NN_MANY(96) NN_MANY(128) NN_MANY(160) NN_MANY(192) NN_MANY(224)
+        default: return floats > 0 ? launch_many<256, true>(p, st) : launch_many<256, false>(p, st);
+    }
+#undef NN_MANY
 }
