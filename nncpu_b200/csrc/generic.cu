@@ -103,21 +103,56 @@ __global__ void rmsnorm_kernel(const void* __restrict__ x, int x_dt, const void*
     }
 }
 
+// The sum over a block of 256 threads, in block_sum's order of additions (the same bits) with one barrier instead of
+// three: every thread adds the eight warps' sums for itself.  `part` must not have been read since the last barrier.
+__device__ __forceinline__ float sum_of_256(float v, float* part) {
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    return ((part[0] + part[4]) + (part[2] + part[6])) + ((part[1] + part[5]) + (part[3] + part[7]));
+}
+
+// Four weights of a norm from element 4 i on, with one load where the rows allow it.
+__device__ __forceinline__ float4 norm_weights(const void* g, int i, int dt, bool wide, float offset) {
+    float4 w = wide ? ld_f4(g, 4 * (size_t)i, dt)
+                    : make_float4(ld_f(g, 4 * i, dt), ld_f(g, 4 * i + 1, dt), ld_f(g, 4 * i + 2, dt), ld_f(g, 4 * i + 3, dt));
+    w.x += offset; w.y += offset; w.z += offset; w.w += offset;
+    return w;
+}
+
 // The common case, float32 rows of a width that is a multiple of 4 and at most 256 * 4 * kVec: every
 // thread keeps its part of the row in registers between the sum of squares and the scaling, so the
 // row is read once, 16 bytes at a time.
+// At a few rows a norm is a chain of round trips to memory, so all loads are asked for at its start (kAhead): the weights, which no
+// kernel of a step writes, before it waits for its predecessor, and what the result is added to with the row.
 template <int kVec>
 __global__ void __launch_bounds__(256)
 rmsnorm_f32_kernel(const float* __restrict__ x, const void* __restrict__ gamma, int g_dt, void* __restrict__ y,
                    int y_dt, const int* __restrict__ rows, int dim, float eps, float gamma_offset, int accumulate) {
-    __shared__ float scratch[33];
+    constexpr bool kAhead = kVec <= 4;       // (more weights than that would cost registers of many-row steps)
+    __shared__ float part[8];
     // launched to start while the kernel before it ends: the product that follows may set itself up meanwhile
     let_next_kernel_start();
-    wait_for_previous_kernels();
     const int r_out = blockIdx.x;
-    const int r_in = rows ? rows[r_out] : r_out;
     const int n4 = dim >> 2;
-    float4 v[kVec];
+    const bool wide = (reinterpret_cast<uintptr_t>(gamma) & 15) == 0;
+    float4 v[kVec], g[kAhead ? kVec : 1], was[kAhead ? kVec : 1];
+    if constexpr (kAhead) {
+#pragma unroll
+        for (int j = 0; j < kVec; ++j) {
+            const int i = threadIdx.x + j * 256;
+            if (gamma && i < n4) g[j] = norm_weights(gamma, i, g_dt, wide, gamma_offset);
+        }
+    }
+    wait_for_previous_kernels();
+    const int r_in = rows ? rows[r_out] : r_out;
+    if constexpr (kAhead) {
+#pragma unroll
+        for (int j = 0; j < kVec; ++j) {
+            const int i = threadIdx.x + j * 256;
+            if (accumulate && r_in >= 0 && i < n4) was[j] = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(y) + (size_t)r_out * dim)[i];
+        }
+    }
     float ss = 0.0f;
     if (r_in >= 0) {
         const float4* src = reinterpret_cast<const float4*>(x + (size_t)r_in * dim);
@@ -132,7 +167,7 @@ rmsnorm_f32_kernel(const float* __restrict__ x, const void* __restrict__ gamma, 
 #pragma unroll
         for (int j = 0; j < kVec; ++j) v[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
-    ss = block_sum(ss, scratch);
+    ss = sum_of_256(ss, part);
     const float scale = r_in >= 0 ? 1.0f / sqrtf(ss * (1.0f / (float)dim) + eps) : 0.0f;
 #pragma unroll
     for (int j = 0; j < kVec; ++j) {
@@ -140,14 +175,14 @@ rmsnorm_f32_kernel(const float* __restrict__ x, const void* __restrict__ gamma, 
         if (i >= n4) continue;
         float o[4] = {v[j].x * scale, v[j].y * scale, v[j].z * scale, v[j].w * scale};
         if (gamma) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) o[e] *= ld_f(gamma, 4 * i + e, g_dt) + gamma_offset;
+            const float4 w = kAhead ? g[kAhead ? j : 0] : norm_weights(gamma, i, g_dt, wide, gamma_offset);
+            o[0] *= w.x; o[1] *= w.y; o[2] *= w.z; o[3] *= w.w;
         }
         const size_t at = (size_t)r_out * dim + 4 * i;
         if (accumulate) {          // float32 y (checked by the launcher): the norm is added to what y holds
             if (r_in < 0) continue;
-            const float4 was = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(y) + at);
-            o[0] += was.x; o[1] += was.y; o[2] += was.z; o[3] += was.w;
+            const float4 old = kAhead ? was[kAhead ? j : 0] : *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(y) + at);
+            o[0] += old.x; o[1] += old.y; o[2] += old.z; o[3] += old.w;
         }
         if (y_dt == DT_BF16) {
             __nv_bfloat162 h[2] = {__floats2bfloat162_rn(o[0], o[1]), __floats2bfloat162_rn(o[2], o[3])};
@@ -199,45 +234,59 @@ __global__ void __launch_bounds__(256)
 rmsnorm_pair_kernel(const float* __restrict__ b, float* __restrict__ r, const void* __restrict__ g1, float off1,
                     const void* __restrict__ g2, float off2, int g_dt, void* __restrict__ y, int y_dt, int dim,
                     float eps1, float eps2) {
+    constexpr bool kAhead = kVec <= 4;       // as in rmsnorm_f32_kernel
+    __shared__ float part[2][8];
     let_next_kernel_start();
-    wait_for_previous_kernels();
-    __shared__ float scratch[33];
     const int row = blockIdx.x, n4 = dim >> 2;
-    float4 v[kVec];
+    const bool wide = ((reinterpret_cast<uintptr_t>(g1) | reinterpret_cast<uintptr_t>(g2)) & 15) == 0;
+    float4 v[kVec], w1[kAhead ? kVec : 1], w2[kAhead ? kVec : 1], was[kAhead ? kVec : 1];
+    if constexpr (kAhead) {
+#pragma unroll
+        for (int j = 0; j < kVec; ++j) {
+            const int i = threadIdx.x + j * 256;
+            if (i < n4) {
+                w1[j] = norm_weights(g1, i, g_dt, wide, off1);
+                w2[j] = norm_weights(g2, i, g_dt, wide, off2);
+            }
+        }
+    }
+    wait_for_previous_kernels();
+    float4* const stream_row = reinterpret_cast<float4*>(r + (size_t)row * dim);
     float ss = 0.0f;
 #pragma unroll
     for (int j = 0; j < kVec; ++j) {
         const int i = threadIdx.x + j * 256;
         v[j] = i < n4 ? reinterpret_cast<const float4*>(b + (size_t)row * dim)[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (kAhead && i < n4) was[kAhead ? j : 0] = stream_row[i];
+    }
+#pragma unroll
+    for (int j = 0; j < kVec; ++j) {
         ss = fmaf(v[j].x, v[j].x, ss); ss = fmaf(v[j].y, v[j].y, ss);
         ss = fmaf(v[j].z, v[j].z, ss); ss = fmaf(v[j].w, v[j].w, ss);
     }
-    ss = block_sum(ss, scratch);
+    ss = sum_of_256(ss, part[0]);
     const float s1 = 1.0f / sqrtf(ss * (1.0f / (float)dim) + eps1);
     float ss2 = 0.0f;
 #pragma unroll
     for (int j = 0; j < kVec; ++j) {
         const int i = threadIdx.x + j * 256;
         if (i >= n4) continue;
-        float4* at = reinterpret_cast<float4*>(r + (size_t)row * dim) + i;
-        const float4 was = *at;
-        float o[4] = {v[j].x * s1, v[j].y * s1, v[j].z * s1, v[j].w * s1};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) o[e] *= ld_f(g1, 4 * i + e, g_dt) + off1;
-        v[j] = make_float4(was.x + o[0], was.y + o[1], was.z + o[2], was.w + o[3]);
-        *at = v[j];
+        const float4 old = kAhead ? was[kAhead ? j : 0] : stream_row[i];
+        const float4 w = kAhead ? w1[kAhead ? j : 0] : norm_weights(g1, i, g_dt, wide, off1);
+        const float o[4] = {(v[j].x * s1) * w.x, (v[j].y * s1) * w.y, (v[j].z * s1) * w.z, (v[j].w * s1) * w.w};
+        v[j] = make_float4(old.x + o[0], old.y + o[1], old.z + o[2], old.w + o[3]);
+        stream_row[i] = v[j];
         ss2 = fmaf(v[j].x, v[j].x, ss2); ss2 = fmaf(v[j].y, v[j].y, ss2);
         ss2 = fmaf(v[j].z, v[j].z, ss2); ss2 = fmaf(v[j].w, v[j].w, ss2);
     }
-    ss2 = block_sum(ss2, scratch);
+    ss2 = sum_of_256(ss2, part[1]);
     const float s2 = 1.0f / sqrtf(ss2 * (1.0f / (float)dim) + eps2);
 #pragma unroll
     for (int j = 0; j < kVec; ++j) {
         const int i = threadIdx.x + j * 256;
         if (i >= n4) continue;
-        float o[4] = {v[j].x * s2, v[j].y * s2, v[j].z * s2, v[j].w * s2};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) o[e] *= ld_f(g2, 4 * i + e, g_dt) + off2;
+        const float4 w = kAhead ? w2[kAhead ? j : 0] : norm_weights(g2, i, g_dt, wide, off2);
+        const float o[4] = {(v[j].x * s2) * w.x, (v[j].y * s2) * w.y, (v[j].z * s2) * w.z, (v[j].w * s2) * w.w};
         const size_t at = (size_t)row * dim + 4 * i;
         if (y_dt == DT_BF16) {
             __nv_bfloat162 h[2] = {__floats2bfloat162_rn(o[0], o[1]), __floats2bfloat162_rn(o[2], o[3])};
@@ -2115,10 +2164,23 @@ template <int kVec>
 __global__ void __launch_bounds__(256)
 rmsnorm_dual_f32_kernel(const float* __restrict__ x, const void* __restrict__ g1, const void* __restrict__ g2, int g_dt,
                         float eps1, float eps2, void* __restrict__ y1, void* __restrict__ y2, int y_dt, int dim) {
+    constexpr bool kAhead = kVec <= 4;       // as in rmsnorm_f32_kernel
+    __shared__ float part[8];
     let_next_kernel_start();
-    wait_for_previous_kernels();
-    __shared__ float scratch[33];
     const int n4 = dim >> 2;
+    const bool wide = ((reinterpret_cast<uintptr_t>(g1) | reinterpret_cast<uintptr_t>(g2)) & 15) == 0;
+    float4 w[2][kAhead ? kVec : 1];
+    if constexpr (kAhead) {
+#pragma unroll
+        for (int j = 0; j < kVec; ++j) {
+            const int i = threadIdx.x + j * 256;
+            if (i < n4) {
+                w[0][j] = norm_weights(g1, i, g_dt, wide, 0.0f);
+                w[1][j] = norm_weights(g2, i, g_dt, wide, 0.0f);
+            }
+        }
+    }
+    wait_for_previous_kernels();
     const float4* src = reinterpret_cast<const float4*>(x + (size_t)blockIdx.x * dim);
     float4 v[kVec];
     float ss = 0.0f;
@@ -2129,7 +2191,7 @@ rmsnorm_dual_f32_kernel(const float* __restrict__ x, const void* __restrict__ g1
         ss = fmaf(v[j].x, v[j].x, ss); ss = fmaf(v[j].y, v[j].y, ss);
         ss = fmaf(v[j].z, v[j].z, ss); ss = fmaf(v[j].w, v[j].w, ss);
     }
-    ss = block_sum(ss, scratch);
+    ss = sum_of_256(ss, part);
     const float mean = ss * (1.0f / (float)dim);
     const float s1 = 1.0f / sqrtf(mean + eps1), s2 = 1.0f / sqrtf(mean + eps2);
 #pragma unroll
@@ -2143,9 +2205,8 @@ rmsnorm_dual_f32_kernel(const float* __restrict__ x, const void* __restrict__ g1
             const void* g = which ? g2 : g1;
             void* y = which ? y2 : y1;
             const float sc = which ? s2 : s1;
-            float o[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) o[e] = (in[e] * sc) * ld_f(g, 4 * i + e, g_dt);
+            const float4 f = kAhead ? w[which][kAhead ? j : 0] : norm_weights(g, i, g_dt, wide, 0.0f);
+            const float o[4] = {(in[0] * sc) * f.x, (in[1] * sc) * f.y, (in[2] * sc) * f.z, (in[3] * sc) * f.w};
             if (y_dt == DT_BF16) {
                 __nv_bfloat162 h[2] = {__floats2bfloat162_rn(o[0], o[1]), __floats2bfloat162_rn(o[2], o[3])};
                 *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(y) + at) = *reinterpret_cast<uint2*>(h);
