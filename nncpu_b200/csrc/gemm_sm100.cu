@@ -1543,14 +1543,35 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     }
 }
 
+}  // namespace
+
+#include "gemm_stripe.cuh"
+
+namespace {
+
 // ---------------------------------------------------------------------------
 // Host side: tensor maps (cached by what they describe) and the launcher.
 // ---------------------------------------------------------------------------
 
 // A [rows, K] bfloat16 matrix with row stride `ld` elements, cut in boxes of box_rows x 64.
-int make_map(CUtensorMap* map, const void* base, int rows, int K, long ld, int box_rows) {
+// box_chunks > 0: as three dimensions instead (64 columns, row, chunk of 64 columns; K a multiple of 64), in boxes of
+// 64 x box_rows x box_chunks.
+int make_map(CUtensorMap* map, const void* base, int rows, int K, long ld, int box_rows, int box_chunks) {
     EncodeTiledFn fn = encode_tiled();
     NN_CHECK(fn != nullptr, "gemm: the driver does not offer cuTensorMapEncodeTiled");
+    if (box_chunks > 0) {
+        NN_CHECK(K % kBlockK == 0, "gemm: K %d is no multiple of %d", K, kBlockK);
+        const cuuint64_t dims[3] = {(cuuint64_t)kBlockK, (cuuint64_t)rows, (cuuint64_t)(K / kBlockK)};
+        const cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)kBlockK * 2};
+        const cuuint32_t box[3] = {(cuuint32_t)kBlockK, (cuuint32_t)box_rows, (cuuint32_t)box_chunks};
+        const cuuint32_t elem[3] = {1, 1, 1};
+        const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, elem,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        NN_CHECK(r == CUDA_SUCCESS, "gemm: cuTensorMapEncodeTiled failed with code %d (rows %d, K %d, ld %ld, box %d x %d)",
+                 (int)r, rows, K, ld, box_rows, box_chunks);
+        return 0;
+    }
     const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
     const cuuint32_t box[2] = {(cuuint32_t)kBlockK, (cuuint32_t)box_rows};
@@ -1565,15 +1586,15 @@ int make_map(CUtensorMap* map, const void* base, int rows, int K, long ld, int b
 
 struct MapCache {
     std::mutex lock;
-    std::map<std::tuple<const void*, int, int, long, int>, CUtensorMap> maps;
+    std::map<std::tuple<const void*, int, int, long, int, int>, CUtensorMap> maps;
 
-    int get(CUtensorMap* out, const void* base, int rows, int K, long ld, int box_rows) {
+    int get(CUtensorMap* out, const void* base, int rows, int K, long ld, int box_rows, int box_chunks = 0) {
         std::lock_guard<std::mutex> g(lock);
-        const auto key = std::make_tuple(base, rows, K, ld, box_rows);
+        const auto key = std::make_tuple(base, rows, K, ld, box_rows, box_chunks);
         auto it = maps.find(key);
         if (it == maps.end()) {
             CUtensorMap m;
-            if (int e = make_map(&m, base, rows, K, ld, box_rows)) return e;
+            if (int e = make_map(&m, base, rows, K, ld, box_rows, box_chunks)) return e;
             if (maps.size() > 65536) maps.clear();
             it = maps.emplace(key, m).first;
         }
@@ -1729,6 +1750,90 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams& p, cud
     return 0;
 }
 
+
+constexpr int kStripeRing = 200 * 1024;
+
+// The stripes of a product of M tokens with N features of width K: see gemm_stripe.cuh.
+StripeShape stripe_shape(int mode, int M, int N, int K) {
+    StripeShape s{};
+    const int blocks = mode == kStripe64 ? 1 : 2, units = sm_count() / blocks;
+    const int row_cols = mode == kStripePair256 ? 2 : 1;     // accumulator columns for a weight row of a block
+    for (int rounds = 1;; ++rounds) {
+        const int share = (N + units * blocks * rounds - 1) / (units * blocks * rounds);
+        s.bn = (share + 15) / 16 * 16;
+        s.n_acc = rounds > 1 ? 2 : 1;
+        if (s.bn <= 256 && s.n_acc * row_cols * s.bn <= 512) break;
+    }
+    s.n_tiles = (N + blocks * s.bn - 1) / (blocks * s.bn);
+    const bool two = mode != kStripe64 && s.bn > 128;
+    s.h0 = two ? (s.bn / 2 + 15) / 16 * 16 : s.bn;
+    s.h1 = s.bn - s.h0;
+    s.acc_cols = row_cols * s.bn;
+    s.tmem_cols = 32;
+    while (s.tmem_cols < s.n_acc * s.acc_cols) s.tmem_cols *= 2;
+    s.trows = ((M + blocks - 1) / blocks + 7) / 8 * 8;
+    const int chunk = (s.trows + s.bn) * 128, chunks = K / kBlockK;
+    // Each stage costs some 0.14 us beside its chunks: larger stages where chunks are small (o product of 64 tokens, 4 096 x 4 096,
+    // one, two, four chunks a stage 17.5, 13.8, 11.1 us), but at least three of them (gate/up of 200 tokens, 24 576 x 4 096, one
+    // and two chunks 51.6, 59.2 us).
+    s.kc = chunk <= 16 * 1024 ? 4 : chunk <= 24 * 1024 ? 2 : 1;
+    s.k_stages = (chunks + s.kc - 1) / s.kc;
+    const int rounds = (s.n_tiles + units - 1) / units;
+    const int read = mode == kStripePair256 ? 128 : 64;
+    s.pad = (read - s.trows - s.kc * s.bn) * 128;
+    if (s.pad < 0) s.pad = 0;
+    s.stages = (kStripeRing - s.pad) / (s.kc * chunk);
+    if (s.stages > s.k_stages * rounds) s.stages = s.k_stages * rounds;
+    return s;
+}
+
+template <int kMode, int kEpi>
+int launch_stripe(const CUtensorMap& mx, const CUtensorMap& mw, const GemmParams& p, const StripeShape& s, cudaStream_t stream) {
+    const size_t smem = 1024 + (size_t)s.stages * s.kc * (s.trows + s.bn) * 128 + s.pad + (2 * s.stages + 4) * sizeof(uint64_t) + 16;
+    NN_CHECK(smem <= 227 * 1024 && s.stages >= 1, "gemm (stripes): %zu bytes of shared memory", smem);
+    static bool configured[64] = {};
+    if (first_use_on_this_device(configured)) {
+        const cudaError_t e = cudaFuncSetAttribute(gemm_stripe_kernel<kMode, kEpi>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        NN_CHECK(e == cudaSuccess, "gemm: cannot reserve shared memory: %s", cudaGetErrorString(e));
+    }
+    constexpr int blocks = kMode == kStripe64 ? 1 : 2;
+    const int units = s.n_tiles < sm_count() / blocks ? s.n_tiles : sm_count() / blocks;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(blocks * units));
+    cfg.blockDim = dim3(kStripeThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    cfg.attrs = attr;
+    cfg.numAttrs = overlap_attribute(attr);
+    if (blocks == 2) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = 2;
+        attr[cfg.numAttrs].val.clusterDim.y = 1;
+        attr[cfg.numAttrs].val.clusterDim.z = 1;
+        ++cfg.numAttrs;
+    }
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_stripe_kernel<kMode, kEpi>, mx, mw, p, s);
+    NN_CHECK(e == cudaSuccess, "gemm (stripes): launch failed: %s", cudaGetErrorString(e));
+    return 0;
+}
+
+template <int kEpi>
+int dispatch_stripe(const void* X, const void* W, int M, int N, int K, int lda, GemmParams& p, cudaStream_t stream) {
+    const int mode = M <= 64 ? kStripe64 : M <= 128 ? kStripePair128 : kStripePair256;
+    const StripeShape s = stripe_shape(mode, M, N, K);
+    p.swap = 0;
+    p.rows_a = M; p.rows_b = N;
+    CUtensorMap mx, mw;
+    if (int e = g_maps.get(&mx, X, M, K, lda, s.trows, s.kc)) return e;
+    if (int e = g_maps.get(&mw, W, N, K, K, s.bn, s.kc)) return e;
+    switch (mode) {
+        case kStripe64: return launch_stripe<kStripe64, kEpi>(mx, mw, p, s, stream);
+        case kStripePair128: return launch_stripe<kStripePair128, kEpi>(mx, mw, p, s, stream);
+        default: return launch_stripe<kStripePair256, kEpi>(mx, mw, p, s, stream);
+    }
+}
+
 template <int kEpi>
 int dispatch_cluster(int bn, const CUtensorMap& ma, const CUtensorMap& mb, GemmParams& p, cudaStream_t stream) {
     switch (bn) {
@@ -1843,8 +1948,9 @@ extern "C" int nncpu_linear_tc_wait_probe(const void* X, const void* W, float* o
 // floats) serves the products that deal their k-blocks out evenly; launches that share it must not
 // overlap on the GPU.  `status` is a device word that a kernel sets when one of its bounded waits ran out.
 // `plan` chooses among the kernels where a measurement or a test wants another one than the sizes would get:
-// 0 the default (products of 512 or more tokens on pairs of SMs with 256 x 256 tiles; 65 to 256 tokens with their
-// k-blocks dealt out evenly over the SMs; 17 to 64 tokens a cluster per output tile); kPlanEvenFrom17: dealt out
+// 0 the default (products of 512 or more tokens on pairs of SMs with 256 x 256 tiles; 17 to 256 tokens in stripes of the
+// weights where stripes_take says so, else 65 to 256 tokens with their k-blocks dealt out evenly over the SMs and 17 to 64
+// tokens a cluster per output tile); kPlanNoStripes: never stripes (nor with any other of these); kPlanEvenFrom17: dealt out
 // evenly from 17 tokens on; kPlanNeverEven: never dealt out evenly; kPlanNoPairs: one SM per 128 x 256 tile;
 // kPlanNarrowUnits: units of 128 weight rows where 256 would be taken.
 template <int BN, int kStages, int kEpi>
@@ -1945,7 +2051,7 @@ extern "C" int nncpu_linear_tc_heads(const void* X, const void* W, void* C, int 
                      : launch_grouped<128, 6, kPlain>(ma, mb, p, g, (cudaStream_t)stream);
 }
 
-enum Plan : int { kPlanEvenFrom17 = 1, kPlanNeverEven = 2, kPlanNoPairs = 4, kPlanNarrowUnits = 8 };
+enum Plan : int { kPlanEvenFrom17 = 1, kPlanNeverEven = 2, kPlanNoPairs = 4, kPlanNarrowUnits = 8, kPlanNoStripes = 16 };
 
 //
 // The norms around a product of whole prompts can ride on it as they do on the few-token products (linear_skinny.cu),
@@ -1960,6 +2066,21 @@ enum Plan : int { kPlanEvenFrom17 = 1, kPlanNeverEven = 2, kPlanNoPairs = 4, kPl
 extern "C" int nncpu_linear_tc_fuses_norms(int M, int N) { return M >= 512 && N >= 512; }
 
 namespace {
+// Whether a product of 17 to 256 tokens runs in stripes of the weights (gemm_stripe.cuh), for K of whole chunks.
+// Above 64 tokens: everywhere but with the longest rows, where every SM reads more tokens than weights (us, k-blocks dealt out
+// evenly and their parts added by a second kernel / stripes; 100 tokens: N x K 2048 x 2048 14.6 / 7.3, 4096 x 4096 19.3 / 11.3, 6144
+// x 4096 21.3 / 15.2, gated 24576 x 4096 53.5 / 42.3, 4096 x 12288 31.7 / 25.5, 5120 x 17408 44.9 / 46.0; 200 tokens 17.4 / 8.1,
+// 22.7 / 15.7, 25.3 / 18.3, 68.3 / 51.6, 37.1 / 35.8, 51.8 / 52.6; 512 x 1024 11.7 / 5.1).
+// Up to 64 tokens: not with long rows, since a stripe is narrow there, so its instructions are many and small, while a cluster of
+// eight blocks has an eighth of them each (clusters / stripes, 24 tokens 4096 x 4096 11.9 / 10.3, 4096 x 12288 22.5 / 26.0; 64 tokens
+// 13.6 / 10.2, 25.0 / 26.0); and gated ones, which have tiles for all SMs, from 33 tokens on (24 tokens of 24576 x 4096 38.6 / 39.3;
+// 64 tokens 43.4 / 40.6, of 12288 x 2048 17.4 / 13.5, of 34816 x 5120 63.5 / 64.5).
+bool stripes_take(int M, int N, int K, bool gated) {
+    if (M < 17 || M > 256 || K % kBlockK != 0) return false;
+    if (M > 64) return K <= 16384;
+    return gated ? M > 32 && K <= 4096 : K <= 5120;
+}
+
 // The cluster size that nncpu_linear_tc picks for a product of 17 to 64 tokens (1: whole tiles per block).
 int cluster_blocks(int bn, int n_tiles, int kb_total) {
     if (!(bn >= 32 && bn <= 128 && n_tiles < sm_count())) return 1;
@@ -1971,13 +2092,23 @@ int cluster_blocks(int bn, int n_tiles, int kb_total) {
 }
 }  // namespace
 
-extern "C" int nncpu_linear_tc_norm_roles(int M, int N, int K) {
+namespace {
+int norm_roles(int M, int N, int K, bool stripes) {
     if (nncpu_linear_tc_fuses_norms(M, N)) return 3;
-    if (M < 17 || M > 64) return 0;
+    if (M < 17 || M > 256) return 0;
+    if (stripes) {
+        // below 2^22 weights a norm's own kernel, a launch like the product, does as well as norms carried for 65 tokens and more
+        if (M > 64 && (long)N * K < (1l << 22)) return 0;
+        return 1 | (N % 16 == 0 && (N + kBlockM - 1) / kBlockM < sm_count() ? 2 : 0);
+    }
+    if (M > 64) return 0;
     const int bn = M <= 32 ? 32 : 64;
     const int s = cluster_blocks(bn, (N + kBlockM - 1) / kBlockM, (K + kBlockK - 1) / kBlockK);
     return 1 | ((s > 1 && (bn + s - 1) / s <= 16) ? 2 : 0);
 }
+}  // namespace
+
+extern "C" int nncpu_linear_tc_norm_roles(int M, int N, int K) { return norm_roles(M, N, K, stripes_take(M, N, K, false)); }
 
 extern "C" int nncpu_linear_tc(const void* X, const void* W, const void* bias, int bias_dt, void* C, int c_dt, int M,
                                int N, int K, int lda, int ldc, int accumulate, int epilogue, int plan, void* xg_out,
@@ -2002,8 +2133,10 @@ extern "C" int nncpu_linear_tc(const void* X, const void* W, const void* bias, i
     p.scratch = scratch; p.status = status;
     const int esize = c_dt == DT_F32 ? 4 : 2;
     p.vec = ((uintptr_t)C % 16 == 0) && ((size_t)ldc * esize % 16 == 0);
+    // (stripes leave a norm's input in whole 16-byte pieces only)
+    const bool stripes = plan == 0 && stripes_take(M, N, K, epilogue == kSwiglu) && (xg_out == nullptr || p.vec);
     if (xg_out != nullptr || bins_in != nullptr) {
-        const int roles = plan == 0 ? nncpu_linear_tc_norm_roles(M, N, K) : (nncpu_linear_tc_fuses_norms(M, N) && !(plan & kPlanNoPairs) ? 3 : 0);
+        const int roles = plan == 0 ? norm_roles(M, N, K, stripes) : (nncpu_linear_tc_fuses_norms(M, N) && !(plan & kPlanNoPairs) ? 3 : 0);
         NN_CHECK((bins_in == nullptr || (roles & 1)) && (xg_out == nullptr || (roles & 2)),
                  "gemm: this product cannot carry that norm (M %d, N %d, K %d: see nncpu_linear_tc_norm_roles)", M, N, K);
         NN_CHECK(xg_out == nullptr || bins_in == nullptr, "gemm: a product is a norm's producer or its consumer");
@@ -2029,6 +2162,9 @@ extern "C" int nncpu_linear_tc(const void* X, const void* W, const void* bias, i
                  ((act == kActGateGelu || act == kActGateSwishClamp) && epilogue == kSwiglu),
              "gemm: activation %d goes with the plain epilogue (without accumulation or a norm after it) or, as a gate, with the gated one", act);
     p.nf.act = act; p.nf.act_a = act_a; p.nf.act_b = act_b;
+    if (stripes)
+        return epilogue == kSwiglu ? dispatch_stripe<kSwiglu>(X, W, M, N, K, lda, p, stream)
+                                   : dispatch_stripe<kPlain>(X, W, M, N, K, lda, p, stream);
     CUtensorMap ma, mb;
     int bn;
     if (M <= 256) {

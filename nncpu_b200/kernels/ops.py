@@ -353,7 +353,7 @@ class GemmWorkspace:
 
 
 # Which kernel a tensor-core product runs with, where a measurement or a test wants another than its sizes would get.
-PLANS = {"auto": 0, "even_from_17": 1, "never_even": 2, "no_pairs": 4, "narrow_units": 8}
+PLANS = {"auto": 0, "even_from_17": 1, "never_even": 2, "no_pairs": 4, "narrow_units": 8, "no_stripes": 16}
 
 EPILOGUES = {"plain": 0, "swiglu": 1}
 
@@ -386,7 +386,8 @@ def linear_tc_fuses_norms(m: int, n: int) -> bool:
 def linear_tc_norm_roles(m: int, n: int, k: int) -> int:
     """Which norms the tensor-core product of ``m`` tokens, ``n`` output features and width ``k`` can carry: bit 0 the
     norm before it (``norm_in``), bit 1 the norm after it (``norm_out``).  Whole prompts both; 17 to 64 tokens the
-    norm before, and the norm after where a cluster shares every output tile."""
+    norm before, and the norm after where a cluster shares every output tile or the weights go in stripes; 65 to 256 tokens
+    both where the weights go in stripes and are many."""
     return int(library.load("gemm_sm100").nncpu_linear_tc_norm_roles(m, n, k))
 
 
@@ -395,8 +396,8 @@ def linear_tc(x, w, bias, out, workspace: GemmWorkspace, accumulate: bool = Fals
     """out (+)= x . w^T + bias on the tensor cores; x and w bfloat16.  With
     ``epilogue="swiglu"`` the rows of w hold gate and up rows interleaved in
     blocks of 8 and out [m, n/2] receives silu(gate) * up.  ``plan``: "auto",
-    or for measurements and tests "even_from_17" (17 to 64 tokens deal their
-    k-blocks out evenly like 65 to 256), "never_even", "no_pairs".
+    or for measurements and tests "no_stripes" (17 to 256 tokens never as stripes of the weights), "even_from_17" (17 to 64
+    tokens deal their k-blocks out evenly like 65 to 256 without stripes), "never_even", "no_pairs".
 
     Where ``linear_tc_norm_roles(m, n, k)`` says so, the product can carry the RMS norms around it as
     ``linear_skinny`` does: ``norm_out = (xg, gamma, bins, bins_clear)`` and ``norm_in = (bins, eps)`` with accumulators of
@@ -462,7 +463,7 @@ def linear_tc_qkv(x, w_qkv, q_gamma, k_gamma, eps, cos_sin, tok_seq, tok_pos, bl
 
 
 SKINNY_MAX_TOKENS = 16
-CLUSTER_MAX_TOKENS = 64    # up to here a tensor-core product's weights are the 128-row operand of one tile row
+STRIPE_MAX_TOKENS = 256    # up to here a tensor-core product may have all tokens in one tile and carry norms
 
 
 def linear_skinny(x, w, bias, out, accumulate: bool = False, epilogue: str = "plain", norm_out=None,

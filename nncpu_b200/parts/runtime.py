@@ -210,11 +210,11 @@ class Runtime:
 
     def fuses_norms(self, n_tokens: int, n_out: int) -> bool:
         """Whether the bfloat16 products of a step of ``n_tokens`` rows (``n_out`` output features) may carry the norms
-        around them: the few-token product always, the tensor-core product on pairs of SMs, and from 17 to 64
+        around them: the few-token product always, the tensor-core product on pairs of SMs, and from 17 to 256
         tokens the kernels that ``ops.linear_tc_norm_roles`` names (each product is asked when its turn comes; one
         that cannot leaves the norm to its own kernel)."""
         return (n_tokens <= ops.SKINNY_MAX_TOKENS or ops.linear_tc_fuses_norms(n_tokens, n_out)
-                or n_tokens <= ops.CLUSTER_MAX_TOKENS)
+                or n_tokens <= ops.STRIPE_MAX_TOKENS)
 
     def begin_norm_fusion(self, n_tokens: int) -> None:
         """Once per step whose products may carry norms: two sets of exact accumulators, one row each per token (16
