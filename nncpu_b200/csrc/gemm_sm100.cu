@@ -14,9 +14,11 @@
 // BN-row tile of "B":
 //   * many tokens:  A = activations, B = weights; from 512 tokens on two SMs
 //     share a 256 x 256 tile (gemm_pair_kernel);
-//   * few tokens (up to 256):  A = weights, B = activations, and the epilogue
-//     stores the tile transposed: every weight byte is read once and no
-//     tensor-core row is spent on padding.  There are few output tiles then, so
+//   * 17 to 256 tokens, mostly (stripes_take):  A = all activations, B = a
+//     stripe of the weights per SM (gemm_stripe.cuh);
+//   * the other products of up to 256 tokens:  A = weights, B = activations, and
+//     the epilogue stores the tile transposed: every weight byte is read once and
+//     no tensor-core row is spent on padding.  There are few output tiles then, so
 //     K is cut: either the k-blocks of all tiles are dealt out evenly to the
 //     blocks and a second kernel adds the parts of split tiles
 //     (gemm_streamk_kernel), or a thread-block cluster shares a tile and adds
@@ -1753,10 +1755,30 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams& p, cud
 
 constexpr int kStripeRing = 200 * 1024;
 
+// Whether a product of 17 to 256 tokens runs in stripes of the weights (gemm_stripe.cuh), for K of whole chunks.
+// Above 64 tokens: everywhere but with the longest rows, where every SM reads more tokens than weights (us, k-blocks dealt out
+// evenly and their parts added by a second kernel / stripes; 100 tokens: N x K 2048 x 2048 14.6 / 7.3, 4096 x 4096 19.3 / 11.3, 6144
+// x 4096 21.3 / 15.2, gated 24576 x 4096 53.5 / 42.3, 4096 x 12288 31.7 / 25.5, 5120 x 17408 44.9 / 46.0; 200 tokens 17.4 / 8.1,
+// 22.7 / 15.7, 25.3 / 18.3, 68.3 / 51.6, 37.1 / 35.8, 51.8 / 52.6; 512 x 1024 11.7 / 5.1).
+// Up to 64 tokens: a stripe is narrow there, so its instructions are many and small, and where rows are long two blocks share one
+// of twice the width, half of K each (stripe_halves; clusters of up to eight blocks a tile / stripes / halves: 24 tokens 2048 x 2048
+// 8.8 / 6.3 / 6.1, 4096 x 4096 11.9 / 10.3 / 9.6, 6144 x 4096 13.8 / 12.2 / 12.5, 2048 x 6144 11.8 / 12.9 / 9.9, 4096 x 12288
+// 21.8 / 23.7 / 20.0, 5120 x 17408 33.3 / 35.2 / 32.9; 64 tokens 9.9 / 6.2 / 6.2, 13.5 / 10.3 / 10.0, 15.4 / 13.2 / 13.3, 13.2
+// / 12.6 / 9.6, 23.6 / 24.3 / 21.3, 35.2 / 44.3 / 34.5).  Gated ones have tiles for all SMs: from 33 tokens on, with rows that are
+// not long (24 tokens of 24576 x 4096 38.6 / 39.3; 64 tokens 43.4 / 40.6, of 12288 x 2048 17.4 / 13.5, of 34816 x 5120 63.5 / 64.5).
+constexpr int kHalvesFrom = 5120;
+bool stripe_halves(int M, int N, int K) { return M <= 64 && K > kHalvesFrom && N <= sm_count() / 2 * 256; }
+bool stripes_take(int M, int N, int K, bool gated) {
+    if (M < 17 || M > 256 || K % kBlockK != 0) return false;
+    if (M > 64) return K <= 16384;
+    return gated ? M > 32 && K <= 4096 : K <= kHalvesFrom || stripe_halves(M, N, K);
+}
+
 // The stripes of a product of M tokens with N features of width K: see gemm_stripe.cuh.
 StripeShape stripe_shape(int mode, int M, int N, int K) {
     StripeShape s{};
-    const int blocks = mode == kStripe64 ? 1 : 2, units = sm_count() / blocks;
+    const int two_blocks = mode != kStripe64, units = sm_count() >> two_blocks;
+    const int blocks = mode == kStripePair128 || mode == kStripePair256 ? 2 : 1;     // stripes of a unit, parts of the tokens
     const int row_cols = mode == kStripePair256 ? 2 : 1;     // accumulator columns for a weight row of a block
     for (int rounds = 1;; ++rounds) {
         const int share = (N + units * blocks * rounds - 1) / (units * blocks * rounds);
@@ -1765,7 +1787,7 @@ StripeShape stripe_shape(int mode, int M, int N, int K) {
         if (s.bn <= 256 && s.n_acc * row_cols * s.bn <= 512) break;
     }
     s.n_tiles = (N + blocks * s.bn - 1) / (blocks * s.bn);
-    const bool two = mode != kStripe64 && s.bn > 128;
+    const bool two = blocks == 2 && s.bn > 128;
     s.h0 = two ? (s.bn / 2 + 15) / 16 * 16 : s.bn;
     s.h1 = s.bn - s.h0;
     s.acc_cols = row_cols * s.bn;
@@ -1776,20 +1798,22 @@ StripeShape stripe_shape(int mode, int M, int N, int K) {
     // Each stage costs some 0.14 us beside its chunks: larger stages where chunks are small (o product of 64 tokens, 4 096 x 4 096,
     // one, two, four chunks a stage 17.5, 13.8, 11.1 us), but at least three of them (gate/up of 200 tokens, 24 576 x 4 096, one
     // and two chunks 51.6, 59.2 us).
-    s.kc = chunk <= 16 * 1024 ? 4 : chunk <= 24 * 1024 ? 2 : 1;
+    s.kc = chunk < 16 * 1024 ? 4 : chunk <= 24 * 1024 ? 2 : 1;
     s.k_stages = (chunks + s.kc - 1) / s.kc;
     const int rounds = (s.n_tiles + units - 1) / units;
     const int read = mode == kStripePair256 ? 128 : 64;
     s.pad = (read - s.trows - s.kc * s.bn) * 128;
     if (s.pad < 0) s.pad = 0;
-    s.stages = (kStripeRing - s.pad) / (s.kc * chunk);
-    if (s.stages > s.k_stages * rounds) s.stages = s.k_stages * rounds;
+    const int k_most = mode == kStripeSplit64 ? s.k_stages - s.k_stages / 2 : s.k_stages;
+    s.recv = mode == kStripeSplit64 ? (s.bn / 16 + 1) / 2 * 16 * 64 * 4 : 0;
+    s.stages = (kStripeRing - s.pad - s.recv) / (s.kc * chunk);
+    if (s.stages > k_most * rounds) s.stages = k_most * rounds;
     return s;
 }
 
 template <int kMode, int kEpi>
 int launch_stripe(const CUtensorMap& mx, const CUtensorMap& mw, const GemmParams& p, const StripeShape& s, cudaStream_t stream) {
-    const size_t smem = 1024 + (size_t)s.stages * s.kc * (s.trows + s.bn) * 128 + s.pad + (2 * s.stages + 4) * sizeof(uint64_t) + 16;
+    const size_t smem = 1024 + (size_t)s.stages * s.kc * (s.trows + s.bn) * 128 + s.pad + (2 * s.stages + 5) * sizeof(uint64_t) + 32 + s.recv;
     NN_CHECK(smem <= 227 * 1024 && s.stages >= 1, "gemm (stripes): %zu bytes of shared memory", smem);
     static bool configured[64] = {};
     if (first_use_on_this_device(configured)) {
@@ -1820,7 +1844,7 @@ int launch_stripe(const CUtensorMap& mx, const CUtensorMap& mw, const GemmParams
 
 template <int kEpi>
 int dispatch_stripe(const void* X, const void* W, int M, int N, int K, int lda, GemmParams& p, cudaStream_t stream) {
-    const int mode = M <= 64 ? kStripe64 : M <= 128 ? kStripePair128 : kStripePair256;
+    const int mode = stripe_halves(M, N, K) ? kStripeSplit64 : M <= 64 ? kStripe64 : M <= 128 ? kStripePair128 : kStripePair256;
     const StripeShape s = stripe_shape(mode, M, N, K);
     p.swap = 0;
     p.rows_a = M; p.rows_b = N;
@@ -1830,6 +1854,7 @@ int dispatch_stripe(const void* X, const void* W, int M, int N, int K, int lda, 
     switch (mode) {
         case kStripe64: return launch_stripe<kStripe64, kEpi>(mx, mw, p, s, stream);
         case kStripePair128: return launch_stripe<kStripePair128, kEpi>(mx, mw, p, s, stream);
+        case kStripeSplit64: return launch_stripe<kStripeSplit64, kEpi>(mx, mw, p, s, stream);
         default: return launch_stripe<kStripePair256, kEpi>(mx, mw, p, s, stream);
     }
 }
@@ -2061,26 +2086,11 @@ enum Plan : int { kPlanEvenFrom17 = 1, kPlanNeverEven = 2, kPlanNoPairs = 4, kPl
 // Consumer: X holds such rows of width K and bins_in [M, 16] their accumulators: the result is multiplied by
 // 1 / sqrt(sum / K + eps) per row before bias and activation.
 // From 17 to 64 tokens the same holds where nncpu_linear_tc_norm_roles says so (bit 0: may be a consumer, bit 1: may
-// be a producer): the cluster kernel does both (a producer with at most 16 tokens a block), the kernel of whole
+// be a producer): stripes do both, up to 256 tokens, the cluster kernel too (a producer with at most 16 tokens a block), the kernel of whole
 // 128-row tiles per block consumes.
 extern "C" int nncpu_linear_tc_fuses_norms(int M, int N) { return M >= 512 && N >= 512; }
 
 namespace {
-// Whether a product of 17 to 256 tokens runs in stripes of the weights (gemm_stripe.cuh), for K of whole chunks.
-// Above 64 tokens: everywhere but with the longest rows, where every SM reads more tokens than weights (us, k-blocks dealt out
-// evenly and their parts added by a second kernel / stripes; 100 tokens: N x K 2048 x 2048 14.6 / 7.3, 4096 x 4096 19.3 / 11.3, 6144
-// x 4096 21.3 / 15.2, gated 24576 x 4096 53.5 / 42.3, 4096 x 12288 31.7 / 25.5, 5120 x 17408 44.9 / 46.0; 200 tokens 17.4 / 8.1,
-// 22.7 / 15.7, 25.3 / 18.3, 68.3 / 51.6, 37.1 / 35.8, 51.8 / 52.6; 512 x 1024 11.7 / 5.1).
-// Up to 64 tokens: not with long rows, since a stripe is narrow there, so its instructions are many and small, while a cluster of
-// eight blocks has an eighth of them each (clusters / stripes, 24 tokens 4096 x 4096 11.9 / 10.3, 4096 x 12288 22.5 / 26.0; 64 tokens
-// 13.6 / 10.2, 25.0 / 26.0); and gated ones, which have tiles for all SMs, from 33 tokens on (24 tokens of 24576 x 4096 38.6 / 39.3;
-// 64 tokens 43.4 / 40.6, of 12288 x 2048 17.4 / 13.5, of 34816 x 5120 63.5 / 64.5).
-bool stripes_take(int M, int N, int K, bool gated) {
-    if (M < 17 || M > 256 || K % kBlockK != 0) return false;
-    if (M > 64) return K <= 16384;
-    return gated ? M > 32 && K <= 4096 : K <= 5120;
-}
-
 // The cluster size that nncpu_linear_tc picks for a product of 17 to 64 tokens (1: whole tiles per block).
 int cluster_blocks(int bn, int n_tiles, int kb_total) {
     if (!(bn >= 32 && bn <= 128 && n_tiles < sm_count())) return 1;
@@ -2195,7 +2205,7 @@ extern "C" int nncpu_linear_tc(const void* X, const void* W, const void* bias, i
     const int n_tiles = p.tiles_a * p.tiles_b;
     p.splits = 1;
     // Up to 16 tokens (the few-token kernel of linear_skinny.cu is the product path for those; this serves direct
-    // calls) and 65 to 256 tokens: the work is cut evenly over the SMs; 17 to 64: a cluster per output tile (measured:
+    // calls) and 65 to 256 tokens that do not go in stripes: the work is cut evenly over the SMs; 17 to 64: a cluster per output tile (measured:
     // at 96 tokens 139 us against 220 us for the four products of a Qwen3-8B layer, at 64 tokens 123 against 117)
     // The same for 257 and more tokens that do not fill the SMs with 128 x 256 tiles at least twice.
     const bool even_swap = p.swap && (bn <= 16 || bn >= (streamk_mode == 2 ? 32 : 128));

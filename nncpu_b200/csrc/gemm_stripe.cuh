@@ -5,17 +5,23 @@
 // SMs, so the tiles' k-blocks had to be shared among SMs and their partial sums exchanged (through a cluster's shared
 // memory up to 64 tokens, through scratch memory and a second kernel above).  Here the N operand is as many weight rows as make
 // one round over the SMs (a multiple of 16), so that all SMs stream alike and nothing is exchanged.  The price is that every
-// SM reads all tokens (from L2).  Up to 64 tokens a block multiplies alone (M 64); above, two SMs pair up, each loads half of the
+// SM reads all tokens (from L2).  Up to 64 tokens a block multiplies alone (M 64), or, with long rows, two blocks share a stripe, each
+// multiplies half of K and sends the other the sums of its half of the columns through distributed shared memory; above, two SMs pair up, each loads half of the
 // tokens and its own weight rows, and tcgen05.mma with cta_group::2 multiplies the two halves with both stripes.
 //
 // A stage of the ring holds `kc` chunks of 64 columns of the tokens and of the stripe (one three-dimensional tensor copy
 // each: column, row, chunk).  Only as many token rows are copied as there are; the tensor core reads the M rows all the
 // same, and what it makes of the bytes behind them are rows nobody stores.
+//
+// What bounds it (times at the rule that sends a product here): the instructions, of which a block issues one for 16 columns of
+// K whatever the width of its stripe, some 45 clk each at N 16 to 64, and some 0.14 us a stage; the weights' stream at the
+// larger widths (gated 24 576 x 4 096 at 64 tokens 40.6 us, 5.0 TB/s).  Neither where a unit begins its walk through K (all SMs
+// read the same tokens at one time) nor copies by a warp for each operand made a difference.
 #pragma once
 
 namespace {
 
-enum StripeMode : int { kStripe64 = 0, kStripePair128 = 1, kStripePair256 = 2 };
+enum StripeMode : int { kStripe64 = 0, kStripePair128 = 1, kStripePair256 = 2, kStripeSplit64 = 3 };
 // warp 0: copies, 1: instructions, 2 to 9: epilogue, two a lane quarter
 constexpr int kStripeThreads = 2 * 32 + 256;
 
@@ -28,6 +34,7 @@ struct StripeShape {
     int n_tiles;    // stripes of all blocks (of a pair: 2 bn rows)
     int acc_cols, n_acc, tmem_cols;
     int pad;        // bytes behind the ring that the tensor core may read beyond the last stage
+    int recv;       // bytes for the partner's sums
 };
 
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z) {
@@ -87,8 +94,10 @@ template <int kMode, int kEpi>
 __global__ void __launch_bounds__(kStripeThreads)
 gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const GemmParams p,
                    const StripeShape s) {
-    constexpr bool kPair = kMode != kStripe64;
-    constexpr int kM = kMode == kStripe64 ? 64 : kMode == kStripePair128 ? 128 : 256;
+    constexpr bool kPair = kMode == kStripePair128 || kMode == kStripePair256;
+    constexpr bool kSplit = kMode == kStripeSplit64;      // two blocks share a stripe, each half of K
+    constexpr bool kAlone64 = kMode == kStripe64 || kSplit;
+    constexpr int kM = kAlone64 ? 64 : kMode == kStripePair128 ? 128 : 256;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const int bytes_x = s.kc * s.trows * 128, bytes_w = s.kc * s.bn * 128, bytes_stage = bytes_x + bytes_w;
@@ -96,14 +105,21 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     uint64_t* empty = full + s.stages;
     uint64_t* acc_full = empty + s.stages;  // [2]
     uint64_t* acc_empty = acc_full + 2;     // [2]
-    uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
+    uint64_t* got = acc_empty + 2;          // kSplit: the partner's sums for this block's columns are here
+    uint32_t* tmem_slot = (uint32_t*)(got + 1);
+    float* recv = (float*)(((uintptr_t)(tmem_slot + 1) + 15) & ~(uintptr_t)15);   // kSplit: [column][64 rows]
 
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-    const int rank = kPair ? (int)cluster_rank() : 0;
-    const int unit = kPair ? (int)blockIdx.x >> 1 : (int)blockIdx.x, units = kPair ? (int)gridDim.x >> 1 : (int)gridDim.x;
+    constexpr bool kTwo = kPair || kSplit;              // blocks of a unit
+    const int half = kTwo ? (int)cluster_rank() : 0;
+    const int rank = kPair ? half : 0;
+    const int unit = kTwo ? (int)blockIdx.x >> 1 : (int)blockIdx.x, units = kTwo ? (int)gridDim.x >> 1 : (int)gridDim.x;
     const int tile_n = kPair ? 2 * s.bn : s.bn;
     const int my_tiles = unit < s.n_tiles ? (s.n_tiles - unit + units - 1) / units : 0;
-    const int my_runs = my_tiles * s.k_stages;          // stages this block works through
+    // this block's part of K, in stages (kSplit: the first half or the rest)
+    const int k_begin = kSplit && half ? s.k_stages / 2 : 0;
+    const int k_mine = kSplit ? (half ? s.k_stages - k_begin : s.k_stages / 2) : s.k_stages;
+    const int my_runs = my_tiles * k_mine;              // stages this block works through
     const int n_first = min(s.stages, my_runs);         // copies that need no free stage (they may reach into the next tile)
     const int first_row = unit * tile_n + rank * s.bn, next_row = units * tile_n;
     // One stage's copies: `st` its place in the ring, `ks` its place in K, `n0` the stripe's first row.  In a pair the first
@@ -111,19 +127,19 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     // beforehand costs a lone thread as long as a copy.)
     auto load_w = [&](int st, int ks, int n0) {
         uint8_t* const dst = smem + st * bytes_stage + bytes_x;
-        if constexpr (kPair) tma_load_3d_pair(dst, &map_w, map_to_rank(smem_u32(&full[st]), 0), 0, n0, ks * s.kc);
-        else tma_load_3d(dst, &map_w, &full[st], 0, n0, ks * s.kc);
+        if constexpr (kPair) tma_load_3d_pair(dst, &map_w, map_to_rank(smem_u32(&full[st]), 0), 0, n0, (k_begin + ks) * s.kc);
+        else tma_load_3d(dst, &map_w, &full[st], 0, n0, (k_begin + ks) * s.kc);
     };
     auto load_x = [&](int st, int ks) {
         uint8_t* const dst = smem + st * bytes_stage;
-        if constexpr (kPair) tma_load_3d_pair(dst, &map_x, map_to_rank(smem_u32(&full[st]), 0), 0, rank * s.trows, ks * s.kc);
-        else tma_load_3d(dst, &map_x, &full[st], 0, 0, ks * s.kc);
+        if constexpr (kPair) tma_load_3d_pair(dst, &map_x, map_to_rank(smem_u32(&full[st]), 0), 0, rank * s.trows, (k_begin + ks) * s.kc);
+        else tma_load_3d(dst, &map_x, &full[st], 0, 0, (k_begin + ks) * s.kc);
     };
     auto first_weights = [&]() {
         for (int r = 0, ks = 0, n0 = first_row; r < n_first; ++r) {
             if (rank == 0) mbar_expect_tx(&full[r], (kPair ? 2u : 1u) * (uint32_t)bytes_stage);
             load_w(r, ks, n0);
-            if (++ks == s.k_stages) { ks = 0; n0 += next_row; }
+            if (++ks == k_mine) { ks = 0; n0 += next_row; }
         }
     };
 
@@ -139,6 +155,7 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             mbar_init(&acc_full[b], 1);
             mbar_init(&acc_empty[b], kPair ? 16 : 8);
         }
+        mbar_init(got, 8);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         // the first weights are asked for before anything that the kernel before this one may still be writing is touched
@@ -155,7 +172,7 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncwarp();
-    if constexpr (kPair) cluster_barrier();      // both blocks' barriers exist before anyone signals across the pair
+    if constexpr (kTwo) cluster_barrier();       // both blocks' barriers exist before anyone signals across the cluster
     else __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
@@ -168,7 +185,7 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             int ks = 0, n0 = first_row, left = my_runs - n_first;
             for (int r = 0; r < n_first; ++r) {
                 load_x(r, ks);
-                if (++ks == s.k_stages) { ks = 0; n0 += next_row; }
+                if (++ks == k_mine) { ks = 0; n0 += next_row; }
             }
             int st = 0, phase = 0;
             for (; left > 0; --left) {
@@ -181,7 +198,7 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                 if (rank == 0) mbar_expect_tx(&full[st], (kPair ? 2u : 1u) * (uint32_t)bytes_stage);
                 load_w(st, ks, n0);
                 load_x(st, ks);
-                if (++ks == s.k_stages) { ks = 0; n0 += next_row; }
+                if (++ks == k_mine) { ks = 0; n0 += next_row; }
                 if (++st == s.stages) { st = 0; phase ^= 1; }
             }
             if (!ok) {
@@ -206,7 +223,7 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t tmem_d = tmem_base + (uint32_t)(buf * s.acc_cols);
-                for (int ks = 0; ks < s.k_stages; ++ks) {
+                for (int ks = 0; ks < k_mine; ++ks) {
                     if (!__all_sync(0xffffffffu, mbar_wait(&full[st], phase))) {
                         if (lane == 0) atomicExch(p.status, kTimeoutFull);
                         ok = false;
@@ -233,7 +250,7 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                         }
                         if constexpr (kPair) umma_commit_pair(&empty[st]);
                         else umma_commit(&empty[st]);
-                        if (ks + 1 == s.k_stages) {
+                        if (ks + 1 == k_mine) {
                             if constexpr (kPair) umma_commit_pair(&acc_full[buf]);
                             else umma_commit(&acc_full[buf]);
                         }
@@ -249,13 +266,13 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         // pair: rows 0 to 63 of this block in the first two quarters for the first block's stripe, in the last two for the
         // second's; M 256: 128 rows, the columns of both stripes.
         const int quarter = warp & 3, turn = (warp - 2) >> 2;
-        const int local = kMode == kStripe64 ? (lane < 16 ? quarter * 16 + lane : 1 << 20)
+        const int local = kAlone64 ? (lane < 16 ? quarter * 16 + lane : 1 << 20)
                           : kMode == kStripePair128 ? (quarter & 1) * 32 + lane : quarter * 32 + lane;
         const int token = rank * s.trows + local;
         const bool t_ok = local < s.trows && token < p.rows_a;
         const int n_groups = (kMode == kStripePair256 ? 2 * s.bn : s.bn) / 16;
         auto feature_of = [&](int g) {       // the first feature of a group, within the unit's stripes
-            if (kMode == kStripe64) return 16 * g;
+            if (kAlone64) return 16 * g;
             if (kMode == kStripePair128) return (quarter >> 1) * s.bn + 16 * g;
             int c = 16 * g, base = 0, h = s.h0;
             if (c >= 2 * s.h0) { c -= 2 * s.h0; base = s.h0; h = s.h1; }
@@ -279,7 +296,9 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         for (int it = 0; it < my_tiles; ++it) {
             const int n0 = (unit + it * units) * tile_n;
             const int buf = s.n_acc > 1 ? it & 1 : 0;
-            old_of(n0 + feature_of(turn), y);          // asked for under the stream
+            // kSplit: groups of columns belong to the two blocks in turn, and a block's groups to its two warps of a quarter
+            const int g_step = kSplit ? 4 : 2, g_first = kSplit ? 2 * turn + half : turn;
+            if (g_first < n_groups) old_of(n0 + feature_of(g_first), y);          // asked for under the stream
             const bool done = mbar_wait(&acc_full[buf], (s.n_acc > 1 ? it >> 1 : it) & 1);
             if (!__all_sync(0xffffffffu, done)) {
                 if (lane == 0) atomicExch(p.status, kTimeoutAccumFull);
@@ -287,12 +306,38 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * s.acc_cols);
+            if constexpr (kSplit) {
+                // the partner's columns go to its shared memory, a column of this warp's 16 rows at a time; its barrier counts
+                // the eight warps that have sent theirs
+                const uint32_t there = map_to_rank(smem_u32(recv + quarter * 16 + (lane & 15)), (uint32_t)(half ^ 1));
 #pragma unroll 1
-            for (int g = turn; g < n_groups; g += 2) {
+                for (int g = 2 * turn + (half ^ 1); g < n_groups; g += 4) {
+                    float v[16];
+                    tmem_ld16(taddr + (uint32_t)(16 * g), v);
+                    if (lane < 16) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j)
+                            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(there + (uint32_t)(((g >> 1) * 16 + j) * 64 * 4)), "f"(v[j]) : "memory");
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(got), (uint32_t)(half ^ 1)));
+                if (!__all_sync(0xffffffffu, mbar_wait(got, 0))) {
+                    if (lane == 0) atomicExch(p.status, kTimeoutAccumEmpty);
+                    break;
+                }
+                asm volatile("fence.acq_rel.cluster;" ::: "memory");
+            }
+#pragma unroll 1
+            for (int g = g_first; g < n_groups; g += g_step) {
                 const int f = n0 + feature_of(g);
-                if (g != turn) old_of(f, y);
+                if (g != g_first) old_of(f, y);
                 float v[16];
                 tmem_ld16(taddr + (uint32_t)(16 * g), v);     // every lane takes part, whatever its row
+                if constexpr (kSplit) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] += recv[((g >> 1) * 16 + j) * 64 + quarter * 16 + (lane & 15)];
+                }
 #pragma unroll
                 for (int j = 0; j < 16; ++j) v[j] *= row_scale;
                 if (!t_ok || f >= p.rows_b) continue;
@@ -310,7 +355,7 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncwarp();
-    if constexpr (kPair) cluster_barrier();      // the partner may still be reading this block's shared memory
+    if constexpr (kTwo) cluster_barrier();       // the partner may still be reading this block's shared memory, or writing to it
     else __syncthreads();
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

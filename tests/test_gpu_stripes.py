@@ -32,8 +32,9 @@ def f32(k, factor=1.0):
 # tokens: both ends of the three layouts, odd counts, rows that fill a block or leave one to the second block of a pair
 @pytest.mark.parametrize("m", [17, 24, 63, 64, 65, 71, 128, 129, 200, 255, 256])
 # features: fewer than a stripe each, ragged, one instruction and two, one round over the SMs and more; columns: one chunk, fewer than a
-# stage holds, no multiple of a stage
-@pytest.mark.parametrize("n,k", [(2050, 64), (2368, 192), (4097, 1088), (9480, 2048), (25008, 320), (76000, 128)])
+# stage holds, no multiple of a stage; rows so long that two blocks share them up to 64 tokens, in parts that are not equal
+@pytest.mark.parametrize("n,k", [(2050, 64), (2368, 192), (4097, 1088), (9480, 2048), (25008, 320), (76000, 128),
+                                 (2050, 5184), (1210, 6208), (80, 5248)])
 def test_stripes(ops, m, n, k):
     g = torch.Generator().manual_seed(m * 7 + n + k)
     x = torch.randn(m, k, generator=g).bfloat16().to(DEV)
@@ -63,7 +64,7 @@ def test_stripes(ops, m, n, k):
 
 
 @pytest.mark.parametrize("m", [17, 64, 65, 128, 129, 250, 256])
-@pytest.mark.parametrize("hidden,inter", [(2048, 2432), (4160, 1088)])
+@pytest.mark.parametrize("hidden,inter", [(2048, 2432), (4160, 1088), (1024, 5184)])
 def test_stripes_carry_the_norm_between_two_products(ops, m, hidden, inter):
     """The product that adds into the residual stream leaves residual * gamma and the exact sums of squares of its rows; the next one
     applies the rows' scales; the accumulators of the norm before are cleared.  Rows of C that are not 16-byte aligned: not
@@ -90,14 +91,15 @@ def test_stripes_carry_the_norm_between_two_products(ops, m, hidden, inter):
     want_ss = (residual.double() ** 2).sum(-1).cpu().numpy()
     assert np.abs(total - want_ss).max() <= 1e-6 * want_ss.max() and int(bins[:, 8].sum()) == 0
     normed = torch.from_numpy(P.rmsnorm(residual.cpu().numpy(), gamma.float().cpu().numpy(), eps)).double().to(DEV)
-    w_next = (torch.randn(2 * hidden, hidden, generator=g) * 0.1).bfloat16().to(DEV)
+    wide = max(2 * hidden, 4224)                   # with 2^22 weights a product of 65 tokens and more carries the norm before it
+    w_next = (torch.randn(wide, hidden, generator=g) * 0.1).bfloat16().to(DEV)
     want = normed @ w_next.double().T
-    out = torch.full((m, 2 * hidden), 9.0, device=DEV)
+    out = torch.full((m, wide), 9.0, device=DEV)
     ops.linear_tc(xg, w_next, None, out, ws, norm_in=(bins, eps))
     near(out, want, 0.02)                          # x * gamma is rounded to bfloat16 before the product
-    gated = torch.full((m, hidden), 9.0, device=DEV)
+    gated = torch.full((m, wide // 2), 9.0, device=DEV)
     ops.linear_tc(xg, w_next, None, gated, ws, epilogue="swiglu", norm_in=(bins, eps))
-    y = want.view(m, hidden // 8, 2, 8)
+    y = want.view(m, wide // 16, 2, 8)
     near(gated, (torch.nn.functional.silu(y[:, :, 0]) * y[:, :, 1]).reshape(m, -1), 0.1)   # a product of two such numbers, values up to 25 times the rms
     odd = torch.empty(m * hidden + 1, device=DEV)[1:].view(m, hidden)
     odd.copy_(residual0)
