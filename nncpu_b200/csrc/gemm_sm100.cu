@@ -33,6 +33,7 @@
 // *status and the block leaves through the common exit, which frees its
 // tensor memory.
 
+#include <algorithm>
 #include <cstdlib>
 #include <map>
 #include <mutex>
@@ -1791,8 +1792,6 @@ StripeShape stripe_shape(int mode, int M, int N, int K) {
     s.h0 = two ? (s.bn / 2 + 15) / 16 * 16 : s.bn;
     s.h1 = s.bn - s.h0;
     s.acc_cols = row_cols * s.bn;
-    s.tmem_cols = 32;
-    while (s.tmem_cols < s.n_acc * s.acc_cols) s.tmem_cols *= 2;
     s.trows = ((M + blocks - 1) / blocks + 7) / 8 * 8;
     const int chunk = (s.trows + s.bn) * 128, chunks = K / kBlockK;
     // Each stage costs some 0.14 us beside its chunks: larger stages where chunks are small (o product of 64 tokens, 4 096 x 4 096,
@@ -1805,6 +1804,10 @@ StripeShape stripe_shape(int mode, int M, int N, int K) {
     s.pad = (read - s.trows - s.kc * s.bn) * 128;
     if (s.pad < 0) s.pad = 0;
     const int k_most = mode == kStripeSplit64 ? s.k_stages - s.k_stages / 2 : s.k_stages;
+    const int segments = s.n_acc > 1 ? 1 : std::min(std::min(16, 512 / s.acc_cols), k_most);
+    s.seg_len = (k_most + segments - 1) / segments;
+    s.tmem_cols = 32;
+    while (s.tmem_cols < (s.n_acc > 1 ? s.n_acc : (k_most + s.seg_len - 1) / s.seg_len) * s.acc_cols) s.tmem_cols *= 2;
     s.recv = mode == kStripeSplit64 ? (s.bn / 16 + 1) / 2 * 16 * 64 * 4 : 0;
     s.stages = (kStripeRing - s.pad - s.recv) / (s.kc * chunk);
     if (s.stages > k_most * rounds) s.stages = k_most * rounds;

@@ -13,6 +13,11 @@
 // each: column, row, chunk).  Only as many token rows are copied as there are; the tensor core reads the M rows all the
 // same, and what it makes of the bytes behind them are rows nobody stores.
 //
+// The tensor core cuts its running sum at every instruction instead of rounding it, so a sum over all of K in one accumulator
+// would be further from 64 bits than the slices of K that clusters and dealt-out k-blocks add (K 12288: 1.4e-5 of the 2-norm
+// against 2.6e-6).  A block with one tile has tensor memory to spare: K is summed in up to 16 accumulators one after the other, which
+// the epilogue adds.
+//
 // What bounds it (times at the rule that sends a product here): the instructions, of which a block issues one for 16 columns of
 // K whatever the width of its stripe, some 45 clk each at N 16 to 64, and some 0.14 us a stage; the weights' stream at the
 // larger widths (gated 24 576 x 4 096 at 64 tokens 40.6 us, 5.0 TB/s).  Neither where a unit begins its walk through K (all SMs
@@ -33,6 +38,7 @@ struct StripeShape {
     int stages, k_stages;
     int n_tiles;    // stripes of all blocks (of a pair: 2 bn rows)
     int acc_cols, n_acc, tmem_cols;
+    int seg_len;    // stages that are summed into one accumulator (one tile a block: as many accumulators as there is room for)
     int pad;        // bytes behind the ring that the tensor core may read beyond the last stage
     int recv;       // bytes for the partner's sums
 };
@@ -49,6 +55,19 @@ __device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* m
         "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], "
         "[%2];" ::"r"(smem_u32(dst)),
         "l"((uint64_t)map), "r"(bar_cluster_addr), "r"(x), "r"(y), "r"(z)
+        : "memory");
+}
+
+// 16 columns from each of four places of tensor memory, in one round trip.
+__device__ __forceinline__ void tmem_ld16_four(const uint32_t (&at)[4], uint32_t (&u)[64]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%64];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%65];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47}, [%66];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%67];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=&r"(u[0]), "=&r"(u[1]), "=&r"(u[2]), "=&r"(u[3]), "=&r"(u[4]), "=&r"(u[5]), "=&r"(u[6]), "=&r"(u[7]), "=&r"(u[8]), "=&r"(u[9]), "=&r"(u[10]), "=&r"(u[11]), "=&r"(u[12]), "=&r"(u[13]), "=&r"(u[14]), "=&r"(u[15]), "=&r"(u[16]), "=&r"(u[17]), "=&r"(u[18]), "=&r"(u[19]), "=&r"(u[20]), "=&r"(u[21]), "=&r"(u[22]), "=&r"(u[23]), "=&r"(u[24]), "=&r"(u[25]), "=&r"(u[26]), "=&r"(u[27]), "=&r"(u[28]), "=&r"(u[29]), "=&r"(u[30]), "=&r"(u[31]), "=&r"(u[32]), "=&r"(u[33]), "=&r"(u[34]), "=&r"(u[35]), "=&r"(u[36]), "=&r"(u[37]), "=&r"(u[38]), "=&r"(u[39]), "=&r"(u[40]), "=&r"(u[41]), "=&r"(u[42]), "=&r"(u[43]), "=&r"(u[44]), "=&r"(u[45]), "=&r"(u[46]), "=&r"(u[47]), "=&r"(u[48]), "=&r"(u[49]), "=&r"(u[50]), "=&r"(u[51]), "=&r"(u[52]), "=&r"(u[53]), "=&r"(u[54]), "=&r"(u[55]), "=&r"(u[56]), "=&r"(u[57]), "=&r"(u[58]), "=&r"(u[59]), "=&r"(u[60]), "=&r"(u[61]), "=&r"(u[62]), "=&r"(u[63])
+        : "r"(at[0]), "r"(at[1]), "r"(at[2]), "r"(at[3])
         : "memory");
 }
 
@@ -222,8 +241,13 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t tmem_d = tmem_base + (uint32_t)(buf * s.acc_cols);
+                uint32_t tmem_d = tmem_base + (uint32_t)(buf * s.acc_cols);
+                int in_seg = 0;                       // stages of the accumulator at tmem_d
                 for (int ks = 0; ks < k_mine; ++ks) {
+                    if (in_seg == s.seg_len) {
+                        in_seg = 0;
+                        tmem_d += (uint32_t)s.acc_cols;
+                    }
                     if (!__all_sync(0xffffffffu, mbar_wait(&full[st], phase))) {
                         if (lane == 0) atomicExch(p.status, kTimeoutFull);
                         ok = false;
@@ -237,7 +261,7 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                             const uint64_t w_desc = smem_desc_sw128(stage + bytes_x + c * s.bn * 128);
 #pragma unroll
                             for (int k = 0; k < kBlockK / kUmmaK; ++k) {     // 32 bytes a step: 2 in a descriptor's units
-                                const uint32_t more = (ks > 0 || c > 0 || k > 0) ? 1u : 0u;
+                                const uint32_t more = (in_seg > 0 || c > 0 || k > 0) ? 1u : 0u;
                                 if constexpr (kPair) umma_bf16_pair(tmem_d, x_desc + 2 * k, w_desc + 2 * k, idesc0, more);
                                 else umma_bf16(tmem_d, x_desc + 2 * k, w_desc + 2 * k, idesc0, more);
                             }
@@ -245,7 +269,7 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                                 const uint64_t w1_desc = smem_desc_sw128(stage + bytes_x + c * s.bn * 128 + s.h0 * 128);
 #pragma unroll
                                 for (int k = 0; k < kBlockK / kUmmaK; ++k)
-                                    umma_bf16_pair(tmem_d + cols1, x_desc + 2 * k, w1_desc + 2 * k, idesc1, (ks > 0 || c > 0 || k > 0) ? 1u : 0u);
+                                    umma_bf16_pair(tmem_d + cols1, x_desc + 2 * k, w1_desc + 2 * k, idesc1, (in_seg > 0 || c > 0 || k > 0) ? 1u : 0u);
                             }
                         }
                         if constexpr (kPair) umma_commit_pair(&empty[st]);
@@ -256,6 +280,7 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                         }
                     }
                     __syncwarp();
+                    ++in_seg;
                     if (++st == s.stages) { st = 0; phase ^= 1; }
                 }
             }
@@ -306,6 +331,24 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * s.acc_cols);
+            // a group's sums: the tensor core cuts its running sums, so K is summed in segments, which are added here in their order
+            auto sums_of = [&](int g, float (&v)[16]) {
+                tmem_ld16(taddr + (uint32_t)(16 * g), v);     // every lane takes part, whatever its row
+                const int segments = (k_mine + s.seg_len - 1) / s.seg_len;
+#pragma unroll 1
+                for (int seg = 1; seg < segments; seg += 4) {
+                    uint32_t at[4], u[64];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) at[q] = taddr + (uint32_t)(min(seg + q, segments - 1) * s.acc_cols + 16 * g);
+                    tmem_ld16_four(at, u);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        if (seg + q < segments) {
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(u[16 * q + j]);
+                        }
+                }
+            };
             if constexpr (kSplit) {
                 // the partner's columns go to its shared memory, a column of this warp's 16 rows at a time; its barrier counts
                 // the eight warps that have sent theirs
@@ -313,7 +356,7 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
 #pragma unroll 1
                 for (int g = 2 * turn + (half ^ 1); g < n_groups; g += 4) {
                     float v[16];
-                    tmem_ld16(taddr + (uint32_t)(16 * g), v);
+                    sums_of(g, v);
                     if (lane < 16) {
 #pragma unroll
                         for (int j = 0; j < 16; ++j)
@@ -333,7 +376,7 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                 const int f = n0 + feature_of(g);
                 if (g != g_first) old_of(f, y);
                 float v[16];
-                tmem_ld16(taddr + (uint32_t)(16 * g), v);     // every lane takes part, whatever its row
+                sums_of(g, v);
                 if constexpr (kSplit) {
 #pragma unroll
                     for (int j = 0; j < 16; ++j) v[j] += recv[((g >> 1) * 16 + j) * 64 + quarter * 16 + (lane & 15)];
