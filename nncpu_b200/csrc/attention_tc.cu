@@ -209,6 +209,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // Launched to start while the kernel before it ends (its set-up needs nothing of that kernel; the step's
     // metadata was copied before the step's first kernel).  It waits before its first copy of q or of a page.
+    let_next_kernel_start();
 
     // the block's 128 query rows: tiles are numbered within each sequence from its end (long spans first)
     int tile = blockIdx.y;
@@ -268,7 +269,6 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
                      "r"(kTmemCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-        let_next_kernel_start();     // no sooner: see its declaration
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

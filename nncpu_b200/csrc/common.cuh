@@ -93,9 +93,7 @@ inline int sm_count() {
 // the stream still runs, once every block of that kernel has called let_next_kernel_start() (or has ended).  It
 // may do only what does not depend on earlier kernels (fetch weights) until wait_for_previous_kernels() returns:
 // from then on everything that earlier kernels wrote is visible and nothing of them still runs.  Every kernel that is
-// launched with the attribute calls both; without the attribute both do nothing.  A kernel that allocates tensor memory calls
-// the first only then (one warp is enough): a block of the next kernel that took an SM's tensor memory before this kernel's
-// block there would wait for this kernel to end, and this kernel for that block.  A library that uses this defines
+// launched with the attribute calls both; without the attribute both do nothing.  A library that uses this defines
 // NN_LAUNCH_OVERLAP before it includes this file and exports nncpu_launch_overlap_<library>(on) (default: on).
 __device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_previous_kernels() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

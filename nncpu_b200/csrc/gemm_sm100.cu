@@ -246,6 +246,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const int my_runs = my_tiles * p.kb_total;
     const int n_first = min(kStages, my_runs);   // copies that need no free stage
 
+    let_next_kernel_start();
     if (threadIdx.x == 0) {
         prefetch_tensormap(&map_a);
         prefetch_tensormap(&map_b);
@@ -273,7 +274,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                      "r"(kTmemCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-        let_next_kernel_start();     // no sooner: see its declaration
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -648,6 +648,7 @@ gemm_streamk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const int n_tiles = p.tiles_a * p.tiles_b;
     const long units = (long)n_tiles * p.kb_total;
     const int blocks = (int)gridDim.x;
+    let_next_kernel_start();   // the set-up below runs while the kernel before this one ends
     const long u_begin = streamk_start((int)blockIdx.x, units, blocks);
     const long u_end = streamk_start((int)blockIdx.x + 1, units, blocks);
     // this block's next segment from unit u on
@@ -677,7 +678,6 @@ gemm_streamk_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                      "r"(kTmemCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-        let_next_kernel_start();     // no sooner: see its declaration
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -944,6 +944,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const int cols = c_end - c_begin;
     const int n_first = min(kStages, kb1 - kb0);   // copies that need no free stage: issued before anything else
 
+    let_next_kernel_start();
     if (threadIdx.x == 0) {
         prefetch_tensormap(&map_a);
         prefetch_tensormap(&map_b);
@@ -975,7 +976,6 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                      "r"(kTmemCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-        let_next_kernel_start();     // no sooner: see its declaration
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -1325,6 +1325,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
 
     __shared__ float s_gamma[kEpi == kQkv ? 2 : 1][128];   // the q and k norm weights of the fused q/k/v epilogue
+    let_next_kernel_start();   // the set-up below runs while the kernel before this one ends
     if constexpr (kEpi == kQkv) {
         for (int i = threadIdx.x; i < 256; i += kPairThreads) {
             const void* gamma = i < 128 ? p.qkv.q_gamma : p.qkv.k_gamma;
@@ -1354,7 +1355,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                      "r"(kTmemCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-        let_next_kernel_start();     // no sooner: see its declaration
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncwarp();

@@ -162,6 +162,7 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         }
     };
 
+    let_next_kernel_start();
     if (threadIdx.x == 0) {
         prefetch_tensormap(&map_w);
         prefetch_tensormap(&map_x);
@@ -187,7 +188,6 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(s.tmem_cols) : "memory");
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         }
-        let_next_kernel_start();     // no sooner: see its declaration
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncwarp();
