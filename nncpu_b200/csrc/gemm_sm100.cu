@@ -1803,9 +1803,16 @@ StripeShape stripe_shape(int mode, int M, int N, int K) {
     const int read = mode == kStripePair256 ? 128 : 64;
     s.pad = (read - s.trows - s.kc * s.bn) * 128;
     if (s.pad < 0) s.pad = 0;
-    const int k_most = mode == kStripeSplit64 ? s.k_stages - s.k_stages / 2 : s.k_stages;
-    const int segments = s.n_acc > 1 ? 1 : std::min(std::min(16, 512 / s.acc_cols), k_most);
-    s.seg_len = (k_most + segments - 1) / segments;
+    // Where K is halved and which parts of it are summed by themselves goes by whole fours of chunks, so that it does not depend on how
+    // many chunks a stage holds, which the number of tokens decides.
+    const int half = mode == kStripeSplit64 ? chunks / 8 * 4 : 0, most = chunks - half;     // (half of 80 chunks at least: K > kHalvesFrom)
+    s.k_half = half / s.kc;
+    const int k_most = s.k_stages - s.k_half;
+    // A block with little shared memory may stand beside a block of the kernel before or after it on an SM, and then leaves it half of
+    // the tensor memory: one that found none would wait for the other's kernel to end, which may wait for it.
+    const bool beside = (long)k_most * rounds * s.kc * chunk < 112 * 1024;
+    const int room = s.n_acc > 1 ? 1 : std::max(1, std::min(16, (beside ? 256 : 512) / s.acc_cols));
+    s.seg_len = room == 1 ? k_most : ((most + room - 1) / room + 3) / 4 * 4 / s.kc;
     s.tmem_cols = 32;
     while (s.tmem_cols < (s.n_acc > 1 ? s.n_acc : (k_most + s.seg_len - 1) / s.seg_len) * s.acc_cols) s.tmem_cols *= 2;
     s.recv = mode == kStripeSplit64 ? (s.bn / 16 + 1) / 2 * 16 * 64 * 4 : 0;

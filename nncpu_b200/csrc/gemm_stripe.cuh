@@ -38,6 +38,7 @@ struct StripeShape {
     int stages, k_stages;
     int n_tiles;    // stripes of all blocks (of a pair: 2 bn rows)
     int acc_cols, n_acc, tmem_cols;
+    int k_half;     // kSplit: the first block's stages
     int seg_len;    // stages that are summed into one accumulator (one tile a block: as many accumulators as there is room for)
     int pad;        // bytes behind the ring that the tensor core may read beyond the last stage
     int recv;       // bytes for the partner's sums
@@ -136,8 +137,8 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     const int tile_n = kPair ? 2 * s.bn : s.bn;
     const int my_tiles = unit < s.n_tiles ? (s.n_tiles - unit + units - 1) / units : 0;
     // this block's part of K, in stages (kSplit: the first half or the rest)
-    const int k_begin = kSplit && half ? s.k_stages / 2 : 0;
-    const int k_mine = kSplit ? (half ? s.k_stages - k_begin : s.k_stages / 2) : s.k_stages;
+    const int k_begin = kSplit && half ? s.k_half : 0;
+    const int k_mine = kSplit ? (half ? s.k_stages - s.k_half : s.k_half) : s.k_stages;
     const int my_runs = my_tiles * k_mine;              // stages this block works through
     const int n_first = min(s.stages, my_runs);         // copies that need no free stage (they may reach into the next tile)
     const int first_row = unit * tile_n + rank * s.bn, next_row = units * tile_n;

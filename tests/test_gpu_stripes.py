@@ -111,3 +111,20 @@ def test_stripes_carry_the_norm_between_two_products(ops, m, hidden, inter):
     except ExtensionError:
         assert m > 64
     assert int(ws.status.item()) == 0
+
+
+@pytest.mark.parametrize("m,n,k", [(64, 2048, 2048), (64, 2048, 6336), (128, 6144, 1344), (256, 6144, 2112)])
+def test_a_token_has_the_same_bits_beside_any_others(ops, m, n, k):
+    """A stage holds one, two or four chunks of K by the number of tokens; halves of K and its parts that are summed by themselves do
+    not depend on that (within 17 to 64, 65 to 128 and 129 to 256 tokens)."""
+    g = torch.Generator().manual_seed(n)
+    x = torch.randn(m, k, generator=g).bfloat16().to(DEV)
+    w = (torch.randn(n, k, generator=g) * 0.1).bfloat16().to(DEV)
+    ws = ops.GemmWorkspace(DEV)
+    want = torch.empty(m, n, device=DEV)
+    ops.linear_tc(x, w, None, want, ws)
+    for rows in ((17, 31, 40, 57) if m == 64 else (m // 2 + 1, m // 2 + 20, m - 9)):
+        out = torch.empty(rows, n, device=DEV)
+        ops.linear_tc(x[:rows].contiguous(), w, None, out, ws)
+        assert torch.equal(out, want[:rows]), rows
+    assert int(ws.status.item()) == 0
