@@ -1811,7 +1811,7 @@ StripeShape stripe_shape(int mode, int M, int N, int K) {
     // A block with little shared memory may stand beside a block of the kernel before or after it on an SM, and then leaves it half of
     // the tensor memory: one that found none would wait for the other's kernel to end, which may wait for it.
     const bool beside = (long)k_most * rounds * s.kc * chunk < 112 * 1024;
-    const int room = s.n_acc > 1 ? 1 : std::max(1, std::min(16, (beside ? 256 : 512) / s.acc_cols));
+    const int room = s.n_acc > 1 ? 1 : std::max(1, std::min(8, (beside ? 256 : 512) / s.acc_cols));
     s.seg_len = room == 1 ? k_most : ((most + room - 1) / room + 3) / 4 * 4 / s.kc;
     s.tmem_cols = 32;
     while (s.tmem_cols < (s.n_acc > 1 ? s.n_acc : (k_most + s.seg_len - 1) / s.seg_len) * s.acc_cols) s.tmem_cols *= 2;

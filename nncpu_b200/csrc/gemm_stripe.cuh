@@ -15,7 +15,7 @@
 //
 // The tensor core cuts its running sum at every instruction instead of rounding it, so a sum over all of K in one accumulator
 // would be further from 64 bits than the slices of K that clusters and dealt-out k-blocks add (K 12288: 1.4e-5 of the 2-norm
-// against 2.6e-6).  A block with one tile has tensor memory to spare: K is summed in up to 16 accumulators one after the other, which
+// against 2.6e-6).  A block with one tile has tensor memory to spare: K is summed in up to 8 accumulators one after the other, which
 // the epilogue adds.
 //
 // What bounds it (times at the rule that sends a product here): the instructions, of which a block issues one for 16 columns of
@@ -56,19 +56,6 @@ __device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* m
         "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], "
         "[%2];" ::"r"(smem_u32(dst)),
         "l"((uint64_t)map), "r"(bar_cluster_addr), "r"(x), "r"(y), "r"(z)
-        : "memory");
-}
-
-// 16 columns from each of four places of tensor memory, in one round trip.
-__device__ __forceinline__ void tmem_ld16_four(const uint32_t (&at)[4], uint32_t (&u)[64]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%64];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%65];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47}, [%66];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%67];\n\t"
-        "tcgen05.wait::ld.sync.aligned;"
-        : "=&r"(u[0]), "=&r"(u[1]), "=&r"(u[2]), "=&r"(u[3]), "=&r"(u[4]), "=&r"(u[5]), "=&r"(u[6]), "=&r"(u[7]), "=&r"(u[8]), "=&r"(u[9]), "=&r"(u[10]), "=&r"(u[11]), "=&r"(u[12]), "=&r"(u[13]), "=&r"(u[14]), "=&r"(u[15]), "=&r"(u[16]), "=&r"(u[17]), "=&r"(u[18]), "=&r"(u[19]), "=&r"(u[20]), "=&r"(u[21]), "=&r"(u[22]), "=&r"(u[23]), "=&r"(u[24]), "=&r"(u[25]), "=&r"(u[26]), "=&r"(u[27]), "=&r"(u[28]), "=&r"(u[29]), "=&r"(u[30]), "=&r"(u[31]), "=&r"(u[32]), "=&r"(u[33]), "=&r"(u[34]), "=&r"(u[35]), "=&r"(u[36]), "=&r"(u[37]), "=&r"(u[38]), "=&r"(u[39]), "=&r"(u[40]), "=&r"(u[41]), "=&r"(u[42]), "=&r"(u[43]), "=&r"(u[44]), "=&r"(u[45]), "=&r"(u[46]), "=&r"(u[47]), "=&r"(u[48]), "=&r"(u[49]), "=&r"(u[50]), "=&r"(u[51]), "=&r"(u[52]), "=&r"(u[53]), "=&r"(u[54]), "=&r"(u[55]), "=&r"(u[56]), "=&r"(u[57]), "=&r"(u[58]), "=&r"(u[59]), "=&r"(u[60]), "=&r"(u[61]), "=&r"(u[62]), "=&r"(u[63])
-        : "r"(at[0]), "r"(at[1]), "r"(at[2]), "r"(at[3])
         : "memory");
 }
 
@@ -335,19 +322,11 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             // a group's sums: the tensor core cuts its running sums, so K is summed in segments, which are added here in their order
             auto sums_of = [&](int g, float (&v)[16]) {
                 tmem_ld16(taddr + (uint32_t)(16 * g), v);     // every lane takes part, whatever its row
-                const int segments = (k_mine + s.seg_len - 1) / s.seg_len;
-#pragma unroll 1
-                for (int seg = 1; seg < segments; seg += 4) {
-                    uint32_t at[4], u[64];
+                for (int seg = 1; seg * s.seg_len < k_mine; ++seg) {      // (four loads at once were slower: registers)
+                    float w[16];
+                    tmem_ld16(taddr + (uint32_t)(seg * s.acc_cols + 16 * g), w);
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) at[q] = taddr + (uint32_t)(min(seg + q, segments - 1) * s.acc_cols + 16 * g);
-                    tmem_ld16_four(at, u);
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        if (seg + q < segments) {
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(u[16 * q + j]);
-                        }
+                    for (int j = 0; j < 16; ++j) v[j] += w[j];
                 }
             };
             if constexpr (kSplit) {
