@@ -730,7 +730,7 @@ int launch_one(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& 
     static_assert((kStreams * VD + 2 * kStreams) * kQRows * 4 <= kStreams * kQRows * HD * 2 + kStages * kKeys * (HD + VD) * 2,
                   "a split tile's part fits the memory of its operands");
     static_assert(VD / kMaxSplits >= 8, "a block of a cluster adds up eight columns at least");
-    constexpr int smem = kStreams * kQRows * HD * 2 + kStages * kKeys * (HD + VD) * 2 + 256 + 1024;
+    constexpr int smem = (int)tmem_block_bytes(kStreams * kQRows * HD * 2 + kStages * kKeys * (HD + VD) * 2 + 256 + 1024, kStreams * kStreamCols);
     static bool configured[64] = {};
     if (first_use_on_this_device(configured)) {
         const cudaError_t e = cudaFuncSetAttribute(prefill_tc_kernel<HD, VD, kStreams, kCap>,

@@ -1615,7 +1615,7 @@ constexpr size_t smem_bytes() {
 
 template <int BN, int kStages, int kEpi>
 int launch(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams& p, int blocks_per_sm, cudaStream_t stream) {
-    constexpr size_t smem = smem_bytes<BN, kStages>();
+    constexpr size_t smem = tmem_block_bytes(smem_bytes<BN, kStages>(), 2 * (BN < 32 ? 32 : BN));
     static bool configured[64] = {};
     if (first_use_on_this_device(configured)) {
         const cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, kStages, kEpi>,
@@ -1639,7 +1639,8 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams& p, int bloc
 
 template <int BN, int kStages, int kEpi, int kTM = 1>
 int launch_streamk(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams& p, cudaStream_t stream) {
-    constexpr size_t smem = smem_bytes<BN, kStages>() + (size_t)kStages * (kTM - 1) * (kBlockM * kBlockK * 2);
+    constexpr int cols = kTM * (BN < 32 ? 32 : BN);
+    constexpr size_t smem = tmem_block_bytes(smem_bytes<BN, kStages>() + (size_t)kStages * (kTM - 1) * (kBlockM * kBlockK * 2), 2 * cols <= 512 ? 2 * cols : cols);
     static_assert(smem <= 227 * 1024, "the stages fit shared memory");
     static bool configured[64] = {};
     if (first_use_on_this_device(configured)) {
@@ -1697,7 +1698,7 @@ int dispatch_streamk_wide(int bn, const CUtensorMap& ma, const CUtensorMap& mb, 
 
 template <int BN, int kStages, int kEpi>
 int launch_cluster(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams& p, cudaStream_t stream) {
-    constexpr size_t smem = cluster_smem_bytes<BN, kStages>();
+    constexpr size_t smem = tmem_block_bytes(cluster_smem_bytes<BN, kStages>(), BN < 32 ? 32 : BN);
     static bool configured[64] = {};
     if (first_use_on_this_device(configured)) {
         const cudaError_t e = cudaFuncSetAttribute(gemm_cluster_kernel<BN, kStages, kEpi>,
@@ -1723,8 +1724,8 @@ int launch_cluster(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams& p, 
 
 template <int kStages, int kEpi>
 int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams& p, cudaStream_t stream) {
-    constexpr size_t smem = 1024 + (size_t)kStages * (kBlockM * kBlockK * 2 + 128 * kBlockK * 2) +
-                            (2 * kStages + 4) * sizeof(uint64_t) + 16;
+    constexpr size_t smem = tmem_block_bytes(1024 + (size_t)kStages * (kBlockM * kBlockK * 2 + 128 * kBlockK * 2) +
+                                             (2 * kStages + 4) * sizeof(uint64_t) + 16, 512);
     static bool configured[64] = {};
     if (first_use_on_this_device(configured)) {
         const cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<kStages, kEpi>,
@@ -1808,8 +1809,8 @@ StripeShape stripe_shape(int mode, int M, int N, int K) {
     const int half = mode == kStripeSplit64 ? chunks / 8 * 4 : 0, most = chunks - half;     // (half of 80 chunks at least: K > kHalvesFrom)
     s.k_half = half / s.kc;
     const int k_most = s.k_stages - s.k_half;
-    // A block with little shared memory may stand beside a block of the kernel before or after it on an SM, and then leaves it half of
-    // the tensor memory: one that found none would wait for the other's kernel to end, which may wait for it.
+    // A block with little shared memory takes half of the tensor memory at most: with more it would ask for so much shared memory
+    // (tmem_block_bytes) that no block of the kernel before or after it can stand beside it.
     const bool beside = (long)k_most * rounds * s.kc * chunk < 112 * 1024;
     const int room = s.n_acc > 1 ? 1 : std::max(1, std::min(8, (beside ? 256 : 512) / s.acc_cols));
     s.seg_len = room == 1 ? k_most : ((most + room - 1) / room + 3) / 4 * 4 / s.kc;
@@ -1818,13 +1819,17 @@ StripeShape stripe_shape(int mode, int M, int N, int K) {
     s.recv = mode == kStripeSplit64 ? (s.bn / 16 + 1) / 2 * 16 * 64 * 4 : 0;
     s.stages = (kStripeRing - s.pad - s.recv) / (s.kc * chunk);
     if (s.stages > k_most * rounds) s.stages = k_most * rounds;
+    s.smem = (int)tmem_block_bytes(1024 + (size_t)s.stages * s.kc * chunk + s.pad + (2 * s.stages + 5) * sizeof(uint64_t) + 32 + s.recv, s.tmem_cols);
     return s;
+}
+
+int stripe_mode(int M, int N, int K) {
+    return stripe_halves(M, N, K) ? kStripeSplit64 : M <= 64 ? kStripe64 : M <= 128 ? kStripePair128 : kStripePair256;
 }
 
 template <int kMode, int kEpi>
 int launch_stripe(const CUtensorMap& mx, const CUtensorMap& mw, const GemmParams& p, const StripeShape& s, cudaStream_t stream) {
-    const size_t smem = 1024 + (size_t)s.stages * s.kc * (s.trows + s.bn) * 128 + s.pad + (2 * s.stages + 5) * sizeof(uint64_t) + 32 + s.recv;
-    NN_CHECK(smem <= 227 * 1024 && s.stages >= 1, "gemm (stripes): %zu bytes of shared memory", smem);
+    NN_CHECK(s.smem <= 227 * 1024 && s.stages >= 1, "gemm (stripes): %d bytes of shared memory", s.smem);
     static bool configured[64] = {};
     if (first_use_on_this_device(configured)) {
         const cudaError_t e = cudaFuncSetAttribute(gemm_stripe_kernel<kMode, kEpi>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
@@ -1835,7 +1840,7 @@ int launch_stripe(const CUtensorMap& mx, const CUtensorMap& mw, const GemmParams
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(blocks * units));
     cfg.blockDim = dim3(kStripeThreads);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = (size_t)s.smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     cfg.attrs = attr;
@@ -1854,7 +1859,7 @@ int launch_stripe(const CUtensorMap& mx, const CUtensorMap& mw, const GemmParams
 
 template <int kEpi>
 int dispatch_stripe(const void* X, const void* W, int M, int N, int K, int lda, GemmParams& p, cudaStream_t stream) {
-    const int mode = stripe_halves(M, N, K) ? kStripeSplit64 : M <= 64 ? kStripe64 : M <= 128 ? kStripePair128 : kStripePair256;
+    const int mode = stripe_mode(M, N, K);
     const StripeShape s = stripe_shape(mode, M, N, K);
     p.swap = 0;
     p.rows_a = M; p.rows_b = N;
@@ -1990,7 +1995,7 @@ extern "C" int nncpu_linear_tc_wait_probe(const void* X, const void* W, float* o
 // kPlanNarrowUnits: units of 128 weight rows where 256 would be taken.
 template <int BN, int kStages, int kEpi>
 int launch_grouped(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams& p, const GroupPlan& g, cudaStream_t stream) {
-    constexpr size_t smem = smem_bytes<BN, kStages>();
+    constexpr size_t smem = tmem_block_bytes(smem_bytes<BN, kStages>(), 2 * BN);
     static_assert(smem <= 227 * 1024, "the stages fit shared memory");
     static bool configured[64] = {};
     if (first_use_on_this_device(configured)) {
@@ -2129,6 +2134,15 @@ int norm_roles(int M, int N, int K, bool stripes) {
 }  // namespace
 
 extern "C" int nncpu_linear_tc_norm_roles(int M, int N, int K) { return norm_roles(M, N, K, stripes_take(M, N, K, false)); }
+
+// Whether a product runs in stripes, and what a block of them holds: columns of tensor memory, bytes of shared memory.
+extern "C" int nncpu_linear_tc_stripes(int M, int N, int K, int epilogue, int* columns, int* bytes) {
+    if (M <= 0 || N <= 0 || K <= 0 || !stripes_take(M, N, K, epilogue == kSwiglu)) return 0;
+    const StripeShape s = stripe_shape(stripe_mode(M, N, K), M, N, K);
+    *columns = s.tmem_cols;
+    *bytes = s.smem;
+    return 1;
+}
 
 extern "C" int nncpu_linear_tc(const void* X, const void* W, const void* bias, int bias_dt, void* C, int c_dt, int M,
                                int N, int K, int lda, int ldc, int accumulate, int epilogue, int plan, void* xg_out,

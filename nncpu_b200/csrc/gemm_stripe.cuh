@@ -42,6 +42,7 @@ struct StripeShape {
     int seg_len;    // stages that are summed into one accumulator (one tile a block: as many accumulators as there is room for)
     int pad;        // bytes behind the ring that the tensor core may read beyond the last stage
     int recv;       // bytes for the partner's sums
+    int smem;       // bytes of dynamic shared memory (tmem_block_bytes)
 };
 
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z) {

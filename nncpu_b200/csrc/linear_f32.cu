@@ -221,7 +221,9 @@ __device__ __noinline__ float plain_dot(const float* x, const float* w, int n) {
 template <int BN>
 constexpr int kManyStages = BN > 160 ? 3 : (BN > 96 ? 4 : 5);     // as many as shared memory holds
 template <int BN>
-constexpr size_t kManySmem = 1024 + (size_t)kManyStages<BN> * (128 + BN) * 192 + 256;
+constexpr int kManyTmemCols = BN <= 32 ? 64 : (BN <= 64 ? 128 : (BN <= 128 ? 256 : 512));     // two accumulators
+template <int BN>
+constexpr size_t kManySmem = tmem_block_bytes(1024 + (size_t)kManyStages<BN> * (128 + BN) * 192 + 256, kManyTmemCols<BN>);
 
 // Eight numbers in their three parts.
 __device__ __forceinline__ void cut_eight(const float (&x)[8], uint4& va, uint4& vb, uint4& vc) {
@@ -272,7 +274,7 @@ f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     // a and 32 numbers b; behind them 64 bytes a row of numbers c (64-byte swizzle).
     constexpr int kRawBytes = (128 + BN) * 128;
     constexpr int kStageBytes = (128 + BN) * 192;
-    constexpr int kTmemCols = BN <= 32 ? 64 : (BN <= 64 ? 128 : (BN <= 128 ? 256 : 512));     // two accumulators
+    constexpr int kTmemCols = kManyTmemCols<BN>;
     constexpr int kCols = BN / 2;                     // columns of an adding thread
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);

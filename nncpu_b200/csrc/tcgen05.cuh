@@ -11,6 +11,18 @@ namespace {
 
 constexpr unsigned long long kWaitLimitNs = 2000000000ull;  // 2 s
 
+// The dynamic shared memory that a block asks for which needs `bytes` and allocates `cols` columns of tensor memory.
+// An allocation that finds too few of an SM's 512 columns free waits, without limit, for a block of another kernel to end; and
+// that one may be waiting for this block: to start early under this kernel's end, or for a partner in its cluster that stands
+// beside a block of this kernel.  So blocks whose columns do not fit an SM together shall not fit its 228 KB of shared memory
+// together either, a block's own 1 KB included: allocations (32 columns and twice as many, up to 512) that do not fit have 544 columns in two
+// blocks at least, and 2 x 32 KB + 544 x 312 bytes are 229.75 KB.  Every kernel that allocates tensor memory is launched by this rule.
+constexpr size_t tmem_block_bytes(size_t bytes, int cols) {
+    const size_t floor = (size_t)31 * 1024 + (size_t)cols * 312;
+    return bytes > floor ? bytes : floor;
+}
+static_assert(2 * (tmem_block_bytes(0, 0) + 1024) + 544 * 312 > 228 * 1024 && tmem_block_bytes(0, 512) <= 227 * 1024, "see above");
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, int count) {

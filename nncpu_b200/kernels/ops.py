@@ -391,6 +391,15 @@ def linear_tc_norm_roles(m: int, n: int, k: int) -> int:
     return int(library.load("gemm_sm100").nncpu_linear_tc_norm_roles(m, n, k))
 
 
+def linear_tc_stripes(m: int, n: int, k: int, epilogue: str = "plain"):
+    """None where ``linear_tc`` does not run this product in stripes of the weights, else what a block of them holds:
+    (columns of tensor memory, bytes of shared memory)."""
+    columns, nbytes = ctypes.c_int(), ctypes.c_int()
+    took = library.load("gemm_sm100").nncpu_linear_tc_stripes(_i(m), _i(n), _i(k), _i(EPILOGUES[epilogue]), ctypes.byref(columns),
+                                                              ctypes.byref(nbytes))
+    return (columns.value, nbytes.value) if took else None
+
+
 def linear_tc(x, w, bias, out, workspace: GemmWorkspace, accumulate: bool = False, epilogue: str = "plain",
               plan: str = "auto", norm_out=None, norm_in=None, activation=None) -> None:
     """out (+)= x . w^T + bias on the tensor cores; x and w bfloat16.  With
