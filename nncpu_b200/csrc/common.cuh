@@ -55,12 +55,15 @@ __device__ __forceinline__ float ld_f(const void* p, size_t i, int dt) {
                         : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[i]);
 }
 
+// The two bfloat16 numbers of a 32-bit word.  By its bits: read through a pointer to another type (__nv_bfloat162), which the language does
+// not allow, the upper one came out as garbage in a kernel that multiplied by four norm weights at a time.
+__device__ __forceinline__ float2 two_bf16(uint32_t u) { return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)); }
+
 // Four neighbouring elements from i on (a multiple of 4; 16-byte aligned rows).
 __device__ __forceinline__ float4 ld_f4(const void* p, size_t i, int dt) {
     if (dt == DT_F32) return *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p) + i);
     const uint2 u = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(p) + i);
-    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
-    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+    const float2 a = two_bf16(u.x), b = two_bf16(u.y);
     return make_float4(a.x, a.y, b.x, b.y);
 }
 

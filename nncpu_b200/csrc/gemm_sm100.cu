@@ -169,10 +169,10 @@ __device__ __forceinline__ void store16(const GemmParams& p, int a_row, int b0, 
                     __nv_bfloat162 h[4];
                     if (p.accumulate) {
                         const uint4 y = *reinterpret_cast<const uint4*>(dst + 8 * half);
-                        const __nv_bfloat162* yh = reinterpret_cast<const __nv_bfloat162*>(&y);
+                        const uint32_t yh[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
-                            const float2 f = __bfloat1622float2(yh[j]);
+                            const float2 f = two_bf16(yh[j]);
                             h[j] = __floats2bfloat162_rn(v[8 * half + 2 * j] + f.x, v[8 * half + 2 * j + 1] + f.y);
                         }
                     } else {
@@ -1476,10 +1476,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 #pragma unroll
                         for (int h = 0; h < 2; ++h) {
                             const uint4 w = gp[h];
-                            const __nv_bfloat162* wh = reinterpret_cast<const __nv_bfloat162*>(&w);
+                            const uint32_t wh[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
                             for (int j = 0; j < 4; ++j) {
-                                const float2 f = __bfloat1622float2(wh[j]);
+                                const float2 f = two_bf16(wh[j]);
                                 g[8 * h + 2 * j] = f.x;
                                 g[8 * h + 2 * j + 1] = f.y;
                             }

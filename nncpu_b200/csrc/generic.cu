@@ -2736,11 +2736,11 @@ __device__ __forceinline__ float warp_dot(const void* __restrict__ w, size_t row
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 if (i0 + 32 * u >= n8) break;
-                const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v[u]);
+                const uint32_t h[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
                 const float* xs = x + 8 * (i0 + 32 * u);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const float2 f = __bfloat1622float2(h[j]);
+                    const float2 f = two_bf16(h[j]);
                     acc = fmaf(f.x, xs[2 * j], acc);
                     acc = fmaf(f.y, xs[2 * j + 1], acc);
                 }
@@ -2996,14 +2996,15 @@ moe_gather_kernel(const void* __restrict__ x, int x_dt, const int* __restrict__ 
             const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(x) + (size_t)t * width);
             uint4* dst = reinterpret_cast<uint4*>(xs + (size_t)row * width);
             for (int i = threadIdx.x; i < (width >> 3); i += blockDim.x) {
-                uint4 v = src[i];
-                __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v);
+                const uint4 v = src[i];
+                const uint32_t in[4] = {v.x, v.y, v.z, v.w};
+                __nv_bfloat162 h[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const float2 f = __bfloat1622float2(h[j]);
+                    const float2 f = two_bf16(in[j]);
                     h[j] = __floats2bfloat162_rn(f.x * w, f.y * w);
                 }
-                dst[i] = v;
+                dst[i] = *reinterpret_cast<uint4*>(h);
             }
         } else {
             for (int i = threadIdx.x; i < width; i += blockDim.x)
@@ -3644,9 +3645,7 @@ token_gate_rows_kernel(const float* __restrict__ x, const void* __restrict__ w, 
             }
 #pragma unroll
             for (int k = 0; k < kGateRowsChunk; ++k) {
-                const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&wv[k]);
-                const float2 f0 = __bfloat1622float2(h2[0]), f1 = __bfloat1622float2(h2[1]);
-                const float2 f2 = __bfloat1622float2(h2[2]), f3 = __bfloat1622float2(h2[3]);
+                const float2 f0 = two_bf16(wv[k].x), f1 = two_bf16(wv[k].y), f2 = two_bf16(wv[k].z), f3 = two_bf16(wv[k].w);
                 s = fmaf(f0.x, xa[k].x, s); s = fmaf(f0.y, xa[k].y, s); s = fmaf(f1.x, xa[k].z, s); s = fmaf(f1.y, xa[k].w, s);
                 s = fmaf(f2.x, xb[k].x, s); s = fmaf(f2.y, xb[k].y, s); s = fmaf(f3.x, xb[k].z, s); s = fmaf(f3.y, xb[k].w, s);
             }

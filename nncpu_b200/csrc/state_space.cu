@@ -472,7 +472,7 @@ chunk_kernel(const float* __restrict__ proj, const Sizes z, const __nv_bfloat16*
                              : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(x_tile + buf * kNarrow + at));
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v[q]));
+                    const float2 f = two_bf16(v[q]);
                     split_pair(f.x * scale, f.y * scale, hi[q], lo[q]);
                 }
                 asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(xh_tile + at), "r"(hi[0]), "r"(hi[1]), "r"(hi[2]), "r"(hi[3]) : "memory");
@@ -557,7 +557,7 @@ chunk_kernel(const float* __restrict__ proj, const Sizes z, const __nv_bfloat16*
                 const int col = 8 * t + 2 * c;
                 uint32_t v;
                 asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(xt + narrow_off(i, t) + 4 * c));
-                const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v));
+                const float2 f = two_bf16(v);
                 const float o0 = fmaf(skip, f.x, acc[t][2 * half]), o1 = fmaf(skip, f.y, acc[t][2 * half + 1]);
                 if (col + 1 < cols && (z.P & 1) == 0) *reinterpret_cast<float2*>(dst + col) = make_float2(o0, o1);
                 else {
