@@ -337,6 +337,7 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
 #pragma unroll 1
                 for (int g = 2 * turn + (half ^ 1); g < n_groups; g += 4) {
                     float v[16];
+                    __syncwarp();                            // the load is the whole warp's
                     sums_of(g, v);
                     if (lane < 16) {
 #pragma unroll
@@ -357,6 +358,7 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                 const int f = n0 + feature_of(g);
                 if (g != g_first) old_of(f, y);
                 float v[16];
+                __syncwarp();                                // the load is the whole warp's
                 sums_of(g, v);
                 if constexpr (kSplit) {
 #pragma unroll
@@ -364,9 +366,10 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                 }
 #pragma unroll
                 for (int j = 0; j < 16; ++j) v[j] *= row_scale;
-                if (!t_ok || f >= p.rows_b) continue;
-                if (rows16 && f + 16 <= p.rows_b) ss += stripe_store16(p, token, f, v, y);
-                else store16<kEpi>(p, token, f, v);
+                if (t_ok && f < p.rows_b) {
+                    if (rows16 && f + 16 <= p.rows_b) ss += stripe_store16(p, token, f, v, y);
+                    else store16<kEpi>(p, token, f, v);
+                }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
