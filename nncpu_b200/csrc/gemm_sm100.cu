@@ -1757,23 +1757,51 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams& p, cud
 
 constexpr int kStripeRing = 200 * 1024;
 
-// Whether a product of 17 to 256 tokens runs in stripes of the weights (gemm_stripe.cuh), for K of whole chunks.
-// Above 64 tokens: everywhere but with the longest rows, where every SM reads more tokens than weights (us, k-blocks dealt out
-// evenly and their parts added by a second kernel / stripes; 100 tokens: N x K 2048 x 2048 14.6 / 7.3, 4096 x 4096 19.3 / 11.3, 6144
-// x 4096 21.3 / 15.2, gated 24576 x 4096 53.5 / 42.3, 4096 x 12288 31.7 / 25.5, 5120 x 17408 44.9 / 46.0; 200 tokens 17.4 / 8.1,
-// 22.7 / 15.7, 25.3 / 18.3, 68.3 / 51.6, 37.1 / 35.8, 51.8 / 52.6; 512 x 1024 11.7 / 5.1).
-// Up to 64 tokens: a stripe is narrow there, so its instructions are many and small, and where rows are long two blocks share one
-// of twice the width, half of K each (stripe_halves; clusters of up to eight blocks a tile / stripes / halves: 24 tokens 2048 x 2048
-// 8.8 / 6.3 / 6.1, 4096 x 4096 11.9 / 10.3 / 9.6, 6144 x 4096 13.8 / 12.2 / 12.5, 2048 x 6144 11.8 / 12.9 / 9.9, 4096 x 12288
-// 21.8 / 23.7 / 20.0, 5120 x 17408 33.3 / 35.2 / 32.9; 64 tokens 9.9 / 6.2 / 6.2, 13.5 / 10.3 / 10.0, 15.4 / 13.2 / 13.3, 13.2
-// / 12.6 / 9.6, 23.6 / 24.3 / 21.3, 35.2 / 44.3 / 34.5).  Gated ones have tiles for all SMs: from 33 tokens on, with rows that are
-// not long (24 tokens of 24576 x 4096 38.6 / 39.3; 64 tokens 43.4 / 40.6, of 12288 x 2048 17.4 / 13.5, of 34816 x 5120 63.5 / 64.5).
+// Rows from this many lanes on are shared by two blocks up to 64 tokens (see stripes_take).
 constexpr int kHalvesFrom = 5120;
 bool stripe_halves(int M, int N, int K) { return M <= 64 && K > kHalvesFrom && N <= sm_count() / 2 * 256; }
-bool stripes_take(int M, int N, int K, bool gated) {
-    if (M < 17 || M > 256 || K % kBlockK != 0) return false;
-    if (M > 64) return K <= 16384;
-    return gated ? M > 32 && K <= 4096 : K <= kHalvesFrom || stripe_halves(M, N, K);
+// More than 128 tokens of few features: the tokens in two parts, each with pairs of its own, where there are pairs for both.  The
+// accumulators of a pair are half as wide then, and K is cut into twice as many stretches.
+int stripe_parts(int M, int N) { return M > 128 && (N + 31) / 32 * 2 <= sm_count() / 2 ? 2 : 1; }
+int stripe_mode(int M, int N, int K) {
+    return stripe_halves(M, N, K) ? kStripeSplit64 : M <= 64 ? kStripe64 : M <= 128 || stripe_parts(M, N) > 1 ? kStripePair128 : kStripePair256;
+}
+
+// The cluster size that nncpu_linear_tc picks for a product of 17 to 64 tokens (1: whole tiles per block).
+int cluster_blocks(int bn, int n_tiles, int kb_total) {
+    if (!(bn >= 32 && bn <= 128 && n_tiles < sm_count())) return 1;
+    const int places = (bn <= 64 ? 2 : 1) * sm_count() * 87 / 100;
+    int best = 1;
+    for (int s = 2; s <= 8 && s <= bn && kb_total / s >= 4; ++s)
+        if (n_tiles * s <= places) best = s;
+    return best;
+}
+
+// The tensor core cuts its running sum at every instruction, so a stretch of K that is summed in one accumulator is off by its length
+// times its sum: by length^3 when squared.  Over all stretches of a result, in chunks (2-norm of the error against 64 bits, K 4096,
+// stretches of 4, 8, 16, 32, 64 chunks: 2.4e-7, 4.7e-7, 1.0e-6, 2.1e-6, 4.4e-6).  Here: what the kernels leave whose place
+// stripes take.  Up to 64 tokens a cluster's slices; above, a block's share of all tiles' chunks, which may begin anywhere in a tile.
+double error_without_stripes(int M, int N, int K) {
+    const long chunks = (K + kBlockK - 1) / kBlockK, tiles = (N + kBlockM - 1) / kBlockM;
+    const double all = (double)chunks;
+    if (M <= 64) {
+        const double slices = cluster_blocks(64, (int)tiles, (int)chunks);
+        return all * all * all / (slices * slices);
+    }
+    const long units = (tiles >= sm_count() ? (tiles + 1) / 2 : tiles) * chunks;
+    const double share = (double)units / (double)std::max(1l, std::min((long)sm_count(), units / 4));
+    return share < all ? share * share * (all - share / 2) : all * all * all * (1.0 - all / (2 * share));
+}
+
+// Into how many stretches of whole fours of chunks K is cut, at least, for sums that are as near (four chunks: as near as
+// it gets).
+int least_stretches(int M, int N, int K) {
+    const int chunks = K / kBlockK;
+    const double before = error_without_stripes(M, N, K);
+    for (int n = 1;; ++n) {
+        const int len = ((chunks + n - 1) / n + 3) / 4 * 4, rest = chunks % len;
+        if (len <= 4 || (double)(chunks / len) * len * len * len + (double)rest * rest * rest <= before) return n;
+    }
 }
 
 // The stripes of a product of M tokens with N features of width K: see gemm_stripe.cuh.
@@ -1782,19 +1810,23 @@ StripeShape stripe_shape(int mode, int M, int N, int K) {
     const int two_blocks = mode != kStripe64, units = sm_count() >> two_blocks;
     const int blocks = mode == kStripePair128 || mode == kStripePair256 ? 2 : 1;     // stripes of a unit, parts of the tokens
     const int row_cols = mode == kStripePair256 ? 2 : 1;     // accumulator columns for a weight row of a block
-    for (int rounds = 1;; ++rounds) {
+    const int chunks = K / kBlockK, of_all = least_stretches(M, N, K), need = mode == kStripeSplit64 ? (of_all + 1) / 2 : of_all;
+    for (int rounds = 1; s.n_buf == 0; ++rounds) {
         const int share = (N + units * blocks * rounds - 1) / (units * blocks * rounds);
         s.bn = (share + 15) / 16 * 16;
-        s.n_acc = rounds > 1 ? 2 : 1;
-        if (s.bn <= 256 && s.n_acc * row_cols * s.bn <= 512) break;
+        if (s.bn > 256) continue;
+        for (int sets = rounds > 1 ? 2 : 1; sets >= 1 && s.n_buf == 0; --sets)
+            if (sets * need * row_cols * s.bn <= 512) s.n_buf = sets;
+        if (s.bn == 16 && s.n_buf == 0) return s;
     }
     s.n_tiles = (N + blocks * s.bn - 1) / (blocks * s.bn);
     const bool two = blocks == 2 && s.bn > 128;
     s.h0 = two ? (s.bn / 2 + 15) / 16 * 16 : s.bn;
     s.h1 = s.bn - s.h0;
     s.acc_cols = row_cols * s.bn;
-    s.trows = ((M + blocks - 1) / blocks + 7) / 8 * 8;
-    const int chunk = (s.trows + s.bn) * 128, chunks = K / kBlockK;
+    s.parts = stripe_parts(M, N);
+    s.trows = ((M + blocks * s.parts - 1) / (blocks * s.parts) + 7) / 8 * 8;
+    const int chunk = (s.trows + s.bn) * 128;
     // Each stage costs some 0.14 us beside its chunks: larger stages where chunks are small (o product of 64 tokens, 4 096 x 4 096,
     // one, two, four chunks a stage 17.5, 13.8, 11.1 us), but at least three of them (gate/up of 200 tokens, 24 576 x 4 096, one
     // and two chunks 51.6, 59.2 us).
@@ -1811,11 +1843,14 @@ StripeShape stripe_shape(int mode, int M, int N, int K) {
     const int k_most = s.k_stages - s.k_half;
     // A block with little shared memory takes half of the tensor memory at most: with more it would ask for so much shared memory
     // (tmem_block_bytes) that no block of the kernel before or after it can stand beside it.
-    const bool beside = (long)k_most * rounds * s.kc * chunk < 112 * 1024;
-    const int room = s.n_acc > 1 ? 1 : std::max(1, std::min(8, (beside ? 256 : 512) / s.acc_cols));
+    const int most_rows = mode == kStripePair256 ? 128 : 64;
+    const bool beside = (long)most * rounds * (most_rows + s.bn) * 128 < 112 * 1024;
+    const int all = 512 / (s.n_buf * s.acc_cols);
+    const int room = std::max(1, std::min(all, std::max(need, std::min(8, beside ? all / 2 : all))));
     s.seg_len = room == 1 ? k_most : ((most + room - 1) / room + 3) / 4 * 4 / s.kc;
+    s.buf_cols = (k_most + s.seg_len - 1) / s.seg_len * s.acc_cols;
     s.tmem_cols = 32;
-    while (s.tmem_cols < (s.n_acc > 1 ? s.n_acc : (k_most + s.seg_len - 1) / s.seg_len) * s.acc_cols) s.tmem_cols *= 2;
+    while (s.tmem_cols < s.n_buf * s.buf_cols) s.tmem_cols *= 2;
     s.recv = mode == kStripeSplit64 ? (s.bn / 16 + 1) / 2 * 16 * 64 * 4 : 0;
     s.stages = (kStripeRing - s.pad - s.recv) / (s.kc * chunk);
     if (s.stages > k_most * rounds) s.stages = k_most * rounds;
@@ -1823,8 +1858,23 @@ StripeShape stripe_shape(int mode, int M, int N, int K) {
     return s;
 }
 
-int stripe_mode(int M, int N, int K) {
-    return stripe_halves(M, N, K) ? kStripeSplit64 : M <= 64 ? kStripe64 : M <= 128 ? kStripePair128 : kStripePair256;
+// Whether a product of 17 to 256 tokens runs in stripes of the weights (gemm_stripe.cuh), for K of whole chunks, in all of which there are
+// accumulators for as good sums.
+// Above 64 tokens: everywhere but with the longest rows, where every SM reads more tokens than weights (us, k-blocks dealt out
+// evenly and their parts added by a second kernel / stripes; 100 tokens: N x K 512 x 1024 10.0 / 4.6, 2048 x 2048 13.8 / 7.2, 4096 x
+// 4096 18.0 / 11.4, 6144 x 4096 19.5 / 14.7, gated 24576 x 4096 53.4 / 45.2, 4096 x 12288 30.3 / 25.3; 200 tokens 10.7 / 5.0, 16.2 /
+// 8.1, 21.6 / 15.2, 24.0 / 17.2, 68.5 / 62.5, 35.7 / 34.6; 5120 x 17408 would be 44.9 / 46.0 and 51.8 / 52.6; the least gain, 112 to 128 tokens of
+// gated 12288 x 2048 18.4 / 19.1).
+// Up to 64 tokens: a stripe is narrow there, so its instructions are many and small, and where rows are long two blocks share one
+// of twice the width, half of K each (stripe_halves; clusters of up to eight blocks a tile / stripes, from 2048 x 6144 on halves:
+// 24 tokens 2048 x 2048 8.8 / 6.2, 4096 x 4096 12.1 / 10.6, 6144 x 4096 13.8 / 12.2, 2048 x 6144 11.8 / 10.5, 4096 x 12288 22.0 / 21.1,
+// 5120 x 17408 33.7 / 33.2; 64 tokens 9.7 / 6.2, 13.8 / 10.4, 15.4 / 13.0, 13.2 / 10.4, 23.8 / 22.3, 35.5 / 34.2).
+// Gated ones have tiles for all SMs: from 33 tokens on, with rows that are not long (24 tokens of 24576 x 4096 38.6 / 39.3; 64 tokens
+// 43.6 / 40.4, of 12288 x 2048 17.8 / 14.9, of 34816 x 5120 63.5 / 64.5).
+bool stripes_take(int M, int N, int K, bool gated) {
+    if (M < 17 || M > 256 || K % kBlockK != 0) return false;
+    const bool pays = M > 64 ? K <= 16384 : gated ? M > 32 && K <= 4096 : K <= kHalvesFrom || stripe_halves(M, N, K);
+    return pays && stripe_shape(stripe_mode(M, N, K), M, N, K).n_buf > 0;
 }
 
 template <int kMode, int kEpi>
@@ -1836,7 +1886,7 @@ int launch_stripe(const CUtensorMap& mx, const CUtensorMap& mw, const GemmParams
         NN_CHECK(e == cudaSuccess, "gemm: cannot reserve shared memory: %s", cudaGetErrorString(e));
     }
     constexpr int blocks = kMode == kStripe64 ? 1 : 2;
-    const int units = s.n_tiles < sm_count() / blocks ? s.n_tiles : sm_count() / blocks;
+    const int units = s.n_tiles * s.parts < sm_count() / blocks ? s.n_tiles * s.parts : sm_count() / blocks;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(blocks * units));
     cfg.blockDim = dim3(kStripeThreads);
@@ -2106,18 +2156,6 @@ enum Plan : int { kPlanEvenFrom17 = 1, kPlanNeverEven = 2, kPlanNoPairs = 4, kPl
 extern "C" int nncpu_linear_tc_fuses_norms(int M, int N) { return M >= 512 && N >= 512; }
 
 namespace {
-// The cluster size that nncpu_linear_tc picks for a product of 17 to 64 tokens (1: whole tiles per block).
-int cluster_blocks(int bn, int n_tiles, int kb_total) {
-    if (!(bn >= 32 && bn <= 128 && n_tiles < sm_count())) return 1;
-    const int places = (bn <= 64 ? 2 : 1) * sm_count() * 87 / 100;
-    int best = 1;
-    for (int s = 2; s <= 8 && s <= bn && kb_total / s >= 4; ++s)
-        if (n_tiles * s <= places) best = s;
-    return best;
-}
-}  // namespace
-
-namespace {
 int norm_roles(int M, int N, int K, bool stripes) {
     if (nncpu_linear_tc_fuses_norms(M, N)) return 3;
     if (M < 17 || M > 256) return 0;
@@ -2135,12 +2173,14 @@ int norm_roles(int M, int N, int K, bool stripes) {
 
 extern "C" int nncpu_linear_tc_norm_roles(int M, int N, int K) { return norm_roles(M, N, K, stripes_take(M, N, K, false)); }
 
-// Whether a product runs in stripes, and what a block of them holds: columns of tensor memory, bytes of shared memory.
-extern "C" int nncpu_linear_tc_stripes(int M, int N, int K, int epilogue, int* columns, int* bytes) {
+// Whether a product runs in stripes, and what a block of them holds: columns of tensor memory, bytes of shared memory; and how many
+// chunks of K (64 columns) are summed in one accumulator.
+extern "C" int nncpu_linear_tc_stripes(int M, int N, int K, int epilogue, int* columns, int* bytes, int* stretch) {
     if (M <= 0 || N <= 0 || K <= 0 || !stripes_take(M, N, K, epilogue == kSwiglu)) return 0;
     const StripeShape s = stripe_shape(stripe_mode(M, N, K), M, N, K);
     *columns = s.tmem_cols;
     *bytes = s.smem;
+    *stretch = s.seg_len * s.kc;
     return 1;
 }
 

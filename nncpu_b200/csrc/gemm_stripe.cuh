@@ -15,8 +15,10 @@
 //
 // The tensor core cuts its running sum at every instruction instead of rounding it, so a sum over all of K in one accumulator
 // would be further from 64 bits than the slices of K that clusters and dealt-out k-blocks add (K 12288: 1.4e-5 of the 2-norm
-// against 2.6e-6).  A block with one tile has tensor memory to spare: K is summed in up to 8 accumulators one after the other, which
-// the epilogue adds.
+// against 2.6e-6).  So K is summed in several accumulators one after the other, which the epilogue adds: as many as those kernels' sums
+// ask for (least_stretches), eight where tensor memory has room.  Where all of a block's rows would not leave room for two, the
+// stripes are narrower and a block walks through K for several of them, with two sets of accumulators in turn (us and error, one accumulator / two;
+// 200 tokens: gated 24576 x 4096 57 / 62, 8.9e-6 / 4.3e-6, 65536 x 4096 111 / 121, 4.4e-6 / 2.1e-6; dealt-out k-blocks 69 and 4.5e-6, 173 and 3.7e-6).
 //
 // What bounds it (times at the rule that sends a product here): the instructions, of which a block issues one for 16 columns of
 // K whatever the width of its stripe, some 45 clk each at N 16 to 64, and some 0.14 us a stage; the weights' stream at the
@@ -34,12 +36,14 @@ struct StripeShape {
     int bn;         // weight rows of a block's stripe (a multiple of 16)
     int h0, h1;     // and how they are dealt to the (one or two) instructions of a k step
     int trows;      // rows of tokens that a block copies (a multiple of 8)
+    int parts;      // of the tokens, each with units of its own (2: more tokens than a unit multiplies, and few weight rows)
     int kc;         // chunks of 64 columns a stage
     int stages, k_stages;
     int n_tiles;    // stripes of all blocks (of a pair: 2 bn rows)
-    int acc_cols, n_acc, tmem_cols;
+    int acc_cols;   // columns of an accumulator
+    int n_buf, buf_cols, tmem_cols;   // sets of accumulators (one a tile), columns of a set, columns of all
     int k_half;     // kSplit: the first block's stages
-    int seg_len;    // stages that are summed into one accumulator (one tile a block: as many accumulators as there is room for)
+    int seg_len;    // stages that are summed into one accumulator
     int pad;        // bytes behind the ring that the tensor core may read beyond the last stage
     int recv;       // bytes for the partner's sums
     int smem;       // bytes of dynamic shared memory (tmem_block_bytes)
@@ -121,7 +125,9 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     constexpr bool kTwo = kPair || kSplit;              // blocks of a unit
     const int half = kTwo ? (int)cluster_rank() : 0;
     const int rank = kPair ? half : 0;
-    const int unit = kTwo ? (int)blockIdx.x >> 1 : (int)blockIdx.x, units = kTwo ? (int)gridDim.x >> 1 : (int)gridDim.x;
+    const int unit_of_all = kTwo ? (int)blockIdx.x >> 1 : (int)blockIdx.x, all_units = kTwo ? (int)gridDim.x >> 1 : (int)gridDim.x;
+    const int unit = unit_of_all >> (s.parts - 1), units = all_units >> (s.parts - 1);
+    const int first_token = (unit_of_all & (s.parts - 1)) * 2 * s.trows + rank * s.trows;
     const int tile_n = kPair ? 2 * s.bn : s.bn;
     const int my_tiles = unit < s.n_tiles ? (s.n_tiles - unit + units - 1) / units : 0;
     // this block's part of K, in stages (kSplit: the first half or the rest)
@@ -140,7 +146,7 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     };
     auto load_x = [&](int st, int ks) {
         uint8_t* const dst = smem + st * bytes_stage;
-        if constexpr (kPair) tma_load_3d_pair(dst, &map_x, map_to_rank(smem_u32(&full[st]), 0), 0, rank * s.trows, (k_begin + ks) * s.kc);
+        if constexpr (kPair) tma_load_3d_pair(dst, &map_x, map_to_rank(smem_u32(&full[st]), 0), 0, first_token, (k_begin + ks) * s.kc);
         else tma_load_3d(dst, &map_x, &full[st], 0, 0, (k_begin + ks) * s.kc);
     };
     auto first_weights = [&]() {
@@ -224,13 +230,13 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             int st = 0, phase = 0;
             bool ok = true;
             for (int it = 0; it < my_tiles && ok; ++it) {
-                const int buf = s.n_acc > 1 ? it & 1 : 0;
-                if (!__all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], ((s.n_acc > 1 ? it >> 1 : it) & 1) ^ 1))) {
+                const int buf = s.n_buf > 1 ? it & 1 : 0;
+                if (!__all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], ((s.n_buf > 1 ? it >> 1 : it) & 1) ^ 1))) {
                     if (lane == 0) atomicExch(p.status, kTimeoutAccumEmpty);
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                uint32_t tmem_d = tmem_base + (uint32_t)(buf * s.acc_cols);
+                uint32_t tmem_d = tmem_base + (uint32_t)(buf * s.buf_cols);
                 int in_seg = 0;                       // stages of the accumulator at tmem_d
                 for (int ks = 0; ks < k_mine; ++ks) {
                     if (in_seg == s.seg_len) {
@@ -282,7 +288,7 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         const int quarter = warp & 3, turn = (warp - 2) >> 2;
         const int local = kAlone64 ? (lane < 16 ? quarter * 16 + lane : 1 << 20)
                           : kMode == kStripePair128 ? (quarter & 1) * 32 + lane : quarter * 32 + lane;
-        const int token = rank * s.trows + local;
+        const int token = first_token + local;
         const bool t_ok = local < s.trows && token < p.rows_a;
         const int n_groups = (kMode == kStripePair256 ? 2 * s.bn : s.bn) / 16;
         auto feature_of = [&](int g) {       // the first feature of a group, within the unit's stripes
@@ -309,18 +315,18 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         float ss = 0.0f;
         for (int it = 0; it < my_tiles; ++it) {
             const int n0 = (unit + it * units) * tile_n;
-            const int buf = s.n_acc > 1 ? it & 1 : 0;
+            const int buf = s.n_buf > 1 ? it & 1 : 0;
             // kSplit: groups of columns belong to the two blocks in turn, and a block's groups to its two warps of a quarter
             const int g_step = kSplit ? 4 : 2, g_first = kSplit ? 2 * turn + half : turn;
             if (g_first < n_groups) old_of(n0 + feature_of(g_first), y);          // asked for under the stream
-            const bool done = mbar_wait(&acc_full[buf], (s.n_acc > 1 ? it >> 1 : it) & 1);
+            const bool done = mbar_wait(&acc_full[buf], (s.n_buf > 1 ? it >> 1 : it) & 1);
             if (!__all_sync(0xffffffffu, done)) {
                 if (lane == 0) atomicExch(p.status, kTimeoutAccumFull);
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * s.acc_cols);
-            // a group's sums: the tensor core cuts its running sums, so K is summed in segments, which are added here in their order
+            const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * s.buf_cols);
+            // a group's sums: K is summed in segments, which are added here in their order
             auto sums_of = [&](int g, float (&v)[16]) {
                 tmem_ld16(taddr + (uint32_t)(16 * g), v);     // every lane takes part, whatever its row
                 for (int seg = 1; seg * s.seg_len < k_mine; ++seg) {      // (four loads at once were slower: registers)

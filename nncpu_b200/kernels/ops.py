@@ -393,11 +393,11 @@ def linear_tc_norm_roles(m: int, n: int, k: int) -> int:
 
 def linear_tc_stripes(m: int, n: int, k: int, epilogue: str = "plain"):
     """None where ``linear_tc`` does not run this product in stripes of the weights, else what a block of them holds:
-    (columns of tensor memory, bytes of shared memory)."""
-    columns, nbytes = ctypes.c_int(), ctypes.c_int()
+    columns of tensor memory, bytes of shared memory; and how many chunks of 64 columns of K one accumulator sums."""
+    columns, nbytes, stretch = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
     took = library.load("gemm_sm100").nncpu_linear_tc_stripes(_i(m), _i(n), _i(k), _i(EPILOGUES[epilogue]), ctypes.byref(columns),
-                                                              ctypes.byref(nbytes))
-    return (columns.value, nbytes.value) if took else None
+                                                              ctypes.byref(nbytes), ctypes.byref(stretch))
+    return (columns.value, nbytes.value, stretch.value) if took else None
 
 
 def linear_tc(x, w, bias, out, workspace: GemmWorkspace, accumulate: bool = False, epilogue: str = "plain",
