@@ -62,9 +62,10 @@ def test_these_run_in_stripes(m, n, k, epilogue):
     assert ops.linear_tc_stripes(m, n, k, epilogue) is not None
 
 
-# few features of long rows above 64 tokens: no room for so many accumulators
+# few features of long rows above 64 tokens: no room for so many accumulators; gated ones whose clusters fill the SMs better
 @pytest.mark.parametrize("m,n,k,epilogue", [(100, 256, 16384, "plain"), (200, 512, 12288, "plain"), (200, 4096, 17408, "plain"),
-                                            (64, 24576, 4160, "swiglu"),
+                                            (64, 512, 4096, "swiglu"), (48, 2048, 4096, "swiglu"), (40, 5120, 4096, "swiglu"),
+                                            (64, 8192, 4096, "swiglu"), (33, 128, 3072, "swiglu"), (64, 24576, 4160, "swiglu"),
                                             (24, 4096, 2048, "swiglu"), (100, 2048, 2072, "plain"), (16, 4096, 4096, "plain"),
                                             (257, 4096, 4096, "plain")])
 def test_these_do_not(m, n, k, epilogue):
