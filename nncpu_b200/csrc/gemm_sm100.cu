@@ -2218,8 +2218,7 @@ extern "C" int nncpu_linear_tc(const void* X, const void* W, const void* bias, i
     p.scratch = scratch; p.status = status;
     const int esize = c_dt == DT_F32 ? 4 : 2;
     p.vec = ((uintptr_t)C % 16 == 0) && ((size_t)ldc * esize % 16 == 0);
-    // (stripes leave a norm's input in whole 16-byte pieces only)
-    const bool stripes = plan == 0 && stripes_take(M, N, K, epilogue == kSwiglu) && (xg_out == nullptr || p.vec);
+    const bool stripes = plan == 0 && stripes_take(M, N, K, epilogue == kSwiglu);
     if (xg_out != nullptr || bins_in != nullptr) {
         const int roles = plan == 0 ? norm_roles(M, N, K, stripes) : (nncpu_linear_tc_fuses_norms(M, N) && !(plan & kPlanNoPairs) ? 3 : 0);
         NN_CHECK((bins_in == nullptr || (roles & 1)) && (xg_out == nullptr || (roles & 2)),
@@ -2227,10 +2226,10 @@ extern "C" int nncpu_linear_tc(const void* X, const void* W, const void* bias, i
         NN_CHECK(xg_out == nullptr || bins_in == nullptr, "gemm: a product is a norm's producer or its consumer");
     }
     if (xg_out != nullptr) {
-        NN_CHECK(epilogue == kPlain && c_dt == DT_F32 && (p.vec || M <= 64) && N % 16 == 0 && gamma != nullptr && bins_out != nullptr &&
+        NN_CHECK(epilogue == kPlain && c_dt == DT_F32 && (p.vec || M <= 256) && N % 16 == 0 && gamma != nullptr && bins_out != nullptr &&
                      ((uintptr_t)xg_out % 16) == 0 && ((uintptr_t)gamma % 16) == 0 && ((uintptr_t)bins_out % 16) == 0 &&
                      ((uintptr_t)bins_clear % 16) == 0,
-                 "gemm: leaving a norm's input needs the plain epilogue, float32 output in 16-byte rows, N %% 16 == 0, "
+                 "gemm: leaving a norm's input needs the plain epilogue, float32 output (in 16-byte rows above 256 tokens), N %% 16 == 0, "
                  "the norm's weights and its accumulators (all 16-byte aligned)");
         p.nf.xg_out = (__nv_bfloat16*)xg_out;
         p.nf.gamma = gamma;

@@ -64,7 +64,7 @@ __device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* m
         : "memory");
 }
 
-// 16 results of one token, features f .. f + 15, through the plain epilogue into rows of whole 16-byte pieces of floats;
+// 16 results of one token, features f .. f + 15, through the plain epilogue into rows of floats (p.vec: of whole 16-byte pieces);
 // y: what they are added to (already loaded).  Returns the sum of squares when a norm after this product rides on it.
 __device__ __forceinline__ float stripe_store16(const GemmParams& p, int token, int f, float (&v)[16], const float4 (&y)[4]) {
     if (p.bias) {
@@ -81,9 +81,14 @@ __device__ __forceinline__ float stripe_store16(const GemmParams& p, int token, 
             v[4 * j] += y[j].x; v[4 * j + 1] += y[j].y; v[4 * j + 2] += y[j].z; v[4 * j + 3] += y[j].w;
         }
     }
-    float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + (size_t)token * p.ldc + f);
+    float* const row = reinterpret_cast<float*>(p.out) + (size_t)token * p.ldc + f;
+    if (p.vec) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) dst[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+        for (int j = 0; j < 4; ++j) reinterpret_cast<float4*>(row)[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) row[j] = v[j];
+    }
     float ss = 0.0f;
     if (p.nf.xg_out != nullptr) {
         __nv_bfloat162 o[8];
@@ -298,7 +303,8 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             if (c >= 2 * s.h0) { c -= 2 * s.h0; base = s.h0; h = s.h1; }
             return c >= h ? s.bn + base + c - h : base + c;
         };
-        const bool rows16 = kEpi == kPlain && p.out_dt == DT_F32 && p.vec;
+        // (a norm's producer goes through stripe_store16 whatever C's alignment)
+        const bool rows16 = kEpi == kPlain && p.out_dt == DT_F32 && (p.vec || p.nf.xg_out != nullptr);
         float row_scale = 1.0f;
         if (p.nf.bins_in != nullptr && t_ok)
             row_scale = 1.0f / sqrtf(bins_total(p.nf.bins_in + (size_t)token * kBinWords) * (1.0f / (float)p.K) + p.nf.eps);
@@ -306,9 +312,10 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             for (int i = threadIdx.x - 64; i < p.rows_a * kBinWords; i += 256) p.nf.bins_clear[i] = 0ull;
         auto old_of = [&](int f, float4 (&y)[4]) {
             if (rows16 && p.accumulate && t_ok && f + 16 <= p.rows_b) {
-                const float4* src = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.out) + (size_t)token * p.ldc + f);
+                const float* const src = reinterpret_cast<const float*>(p.out) + (size_t)token * p.ldc + f;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) y[j] = src[j];
+                for (int j = 0; j < 4; ++j)
+                    y[j] = p.vec ? reinterpret_cast<const float4*>(src)[j] : make_float4(src[4 * j], src[4 * j + 1], src[4 * j + 2], src[4 * j + 3]);
             }
         };
         float4 y[4] = {};
