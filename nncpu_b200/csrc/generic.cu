@@ -112,6 +112,13 @@ __device__ __forceinline__ float sum_of_256(float v, float* part) {
     return ((part[0] + part[4]) + (part[2] + part[6])) + ((part[1] + part[5]) + (part[3] + part[7]));
 }
 
+// Asks for the weights of a norm into L2 (at most 256 lines of 128 bytes, one a thread).
+__device__ __forceinline__ void weights_into_l2(const void* g, int dim, int dt) {
+    const int at = threadIdx.x * 128;
+    if (g != nullptr && at < dim * (dt == DT_F32 ? 4 : 2))
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(g) + at));
+}
+
 // Four weights of a norm from element 4 i on, with one load where the rows allow it.
 __device__ __forceinline__ float4 norm_weights(const void* g, int i, int dt, bool wide, float offset) {
     float4 w = wide ? ld_f4(g, 4 * (size_t)i, dt)
@@ -123,8 +130,9 @@ __device__ __forceinline__ float4 norm_weights(const void* g, int i, int dt, boo
 // The common case, float32 rows of a width that is a multiple of 4 and at most 256 * 4 * kVec: every
 // thread keeps its part of the row in registers between the sum of squares and the scaling, so the
 // row is read once, 16 bytes at a time.
-// At a few rows a norm is a chain of round trips to memory, so all loads are asked for at its start (kAhead): the weights, which no
-// kernel of a step writes, before it waits for its predecessor, and what the result is added to with the row.
+// At a few rows a norm is a chain of round trips to memory, so all loads are asked for at its start (kAhead), the weights and what the
+// result is added to with the row.  Before it waits for its predecessor, which may have written the weights, too, a norm only asks for
+// them into L2.
 template <int kVec>
 __global__ void __launch_bounds__(256)
 rmsnorm_f32_kernel(const float* __restrict__ x, const void* __restrict__ gamma, int g_dt, void* __restrict__ y,
@@ -137,19 +145,14 @@ rmsnorm_f32_kernel(const float* __restrict__ x, const void* __restrict__ gamma, 
     const int n4 = dim >> 2;
     const bool wide = (reinterpret_cast<uintptr_t>(gamma) & 15) == 0;
     float4 v[kVec], g[kAhead ? kVec : 1], was[kAhead ? kVec : 1];
-    if constexpr (kAhead) {
-#pragma unroll
-        for (int j = 0; j < kVec; ++j) {
-            const int i = threadIdx.x + j * 256;
-            if (gamma && i < n4) g[j] = norm_weights(gamma, i, g_dt, wide, gamma_offset);
-        }
-    }
+    weights_into_l2(gamma, dim, g_dt);
     wait_for_previous_kernels();
     const int r_in = rows ? rows[r_out] : r_out;
     if constexpr (kAhead) {
 #pragma unroll
         for (int j = 0; j < kVec; ++j) {
             const int i = threadIdx.x + j * 256;
+            if (gamma && i < n4) g[j] = norm_weights(gamma, i, g_dt, wide, gamma_offset);
             if (accumulate && r_in >= 0 && i < n4) was[j] = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(y) + (size_t)r_out * dim)[i];
         }
     }
@@ -240,16 +243,8 @@ rmsnorm_pair_kernel(const float* __restrict__ b, float* __restrict__ r, const vo
     const int row = blockIdx.x, n4 = dim >> 2;
     const bool wide = ((reinterpret_cast<uintptr_t>(g1) | reinterpret_cast<uintptr_t>(g2)) & 15) == 0;
     float4 v[kVec], w1[kAhead ? kVec : 1], w2[kAhead ? kVec : 1], was[kAhead ? kVec : 1];
-    if constexpr (kAhead) {
-#pragma unroll
-        for (int j = 0; j < kVec; ++j) {
-            const int i = threadIdx.x + j * 256;
-            if (i < n4) {
-                w1[j] = norm_weights(g1, i, g_dt, wide, off1);
-                w2[j] = norm_weights(g2, i, g_dt, wide, off2);
-            }
-        }
-    }
+    weights_into_l2(g1, dim, g_dt);
+    weights_into_l2(g2, dim, g_dt);
     wait_for_previous_kernels();
     float4* const stream_row = reinterpret_cast<float4*>(r + (size_t)row * dim);
     float ss = 0.0f;
@@ -257,7 +252,11 @@ rmsnorm_pair_kernel(const float* __restrict__ b, float* __restrict__ r, const vo
     for (int j = 0; j < kVec; ++j) {
         const int i = threadIdx.x + j * 256;
         v[j] = i < n4 ? reinterpret_cast<const float4*>(b + (size_t)row * dim)[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (kAhead && i < n4) was[kAhead ? j : 0] = stream_row[i];
+        if (kAhead && i < n4) {
+            was[kAhead ? j : 0] = stream_row[i];
+            w1[kAhead ? j : 0] = norm_weights(g1, i, g_dt, wide, off1);
+            w2[kAhead ? j : 0] = norm_weights(g2, i, g_dt, wide, off2);
+        }
     }
 #pragma unroll
     for (int j = 0; j < kVec; ++j) {
@@ -2170,6 +2169,9 @@ rmsnorm_dual_f32_kernel(const float* __restrict__ x, const void* __restrict__ g1
     const int n4 = dim >> 2;
     const bool wide = ((reinterpret_cast<uintptr_t>(g1) | reinterpret_cast<uintptr_t>(g2)) & 15) == 0;
     float4 w[2][kAhead ? kVec : 1];
+    weights_into_l2(g1, dim, g_dt);
+    weights_into_l2(g2, dim, g_dt);
+    wait_for_previous_kernels();
     if constexpr (kAhead) {
 #pragma unroll
         for (int j = 0; j < kVec; ++j) {
@@ -2180,7 +2182,6 @@ rmsnorm_dual_f32_kernel(const float* __restrict__ x, const void* __restrict__ g1
             }
         }
     }
-    wait_for_previous_kernels();
     const float4* src = reinterpret_cast<const float4*>(x + (size_t)blockIdx.x * dim);
     float4 v[kVec];
     float ss = 0.0f;
