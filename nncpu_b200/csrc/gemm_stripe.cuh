@@ -64,6 +64,10 @@ __device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* m
         : "memory");
 }
 
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* map, int x, int y, int z) {
+    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global [%0, {%1, %2, %3}];" ::"l"((uint64_t)map), "r"(x), "r"(y), "r"(z) : "memory");
+}
+
 // 16 results of one token, features f .. f + 15, through the plain epilogue into rows of floats (p.vec: of whole 16-byte pieces);
 // y: what they are added to (already loaded).  Returns the sum of squares when a norm after this product rides on it.
 __device__ __forceinline__ float stripe_store16(const GemmParams& p, int token, int f, float (&v)[16], const float4 (&y)[4]) {
@@ -154,10 +158,16 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         if constexpr (kPair) tma_load_3d_pair(dst, &map_x, map_to_rank(smem_u32(&full[st]), 0), 0, first_token, (k_begin + ks) * s.kc);
         else tma_load_3d(dst, &map_x, &full[st], 0, 0, (k_begin + ks) * s.kc);
     };
+    // What may be asked for before the kernel before this one is over: up to 64 tokens the weights themselves, which that kernel must
+    // not have written (as without stripes); above, it may have, and they are asked for into L2 only.
     auto first_weights = [&]() {
         for (int r = 0, ks = 0, n0 = first_row; r < n_first; ++r) {
-            if (rank == 0) mbar_expect_tx(&full[r], (kPair ? 2u : 1u) * (uint32_t)bytes_stage);
-            load_w(r, ks, n0);
+            if constexpr (kPair) {
+                tma_prefetch_3d(&map_w, 0, n0, (k_begin + ks) * s.kc);
+            } else {
+                mbar_expect_tx(&full[r], (uint32_t)bytes_stage);
+                load_w(r, ks, n0);
+            }
             if (++ks == k_mine) { ks = 0; n0 += next_row; }
         }
     };
@@ -177,8 +187,7 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         mbar_init(got, 8);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        // the first weights are asked for before anything that the kernel before this one may still be writing is touched
-        if constexpr (!kPair) first_weights();
+        first_weights();
     }
     if (warp == 1) {
         if constexpr (kPair) {
@@ -195,7 +204,6 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     else __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
-    if (kPair && threadIdx.x == 0) first_weights();
     wait_for_previous_kernels();
 
     if (warp == 0) {
@@ -203,6 +211,11 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             bool ok = true;
             int ks = 0, n0 = first_row, left = my_runs - n_first;
             for (int r = 0; r < n_first; ++r) {
+                if constexpr (kPair) {
+                    // (the partner's copies cannot complete a phase early: see gemm_pair_kernel)
+                    if (rank == 0) mbar_expect_tx(&full[r], 2u * (uint32_t)bytes_stage);
+                    load_w(r, ks, n0);
+                }
                 load_x(r, ks);
                 if (++ks == k_mine) { ks = 0; n0 += next_row; }
             }
@@ -213,7 +226,6 @@ gemm_stripe_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                     ok = false;
                     break;
                 }
-                // (the partner's copies cannot complete a phase early: see gemm_pair_kernel)
                 if (rank == 0) mbar_expect_tx(&full[st], (kPair ? 2u : 1u) * (uint32_t)bytes_stage);
                 load_w(st, ks, n0);
                 load_x(st, ks);

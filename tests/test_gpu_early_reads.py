@@ -39,6 +39,22 @@ def both(write, read, target):
     return got, want
 
 
+@pytest.mark.parametrize("m", [65, 100, 128, 129, 200, 256])
+def test_stripes_of_weights_just_written(ops, slow, m):
+    x, w = slow
+    weights = torch.empty(16, WIDTH, dtype=torch.bfloat16, device=DEV)
+    act = torch.randn(m, WIDTH, device=DEV).bfloat16()
+    ws, outs = ops.GemmWorkspace(DEV), [torch.empty(m, 16, device=DEV) for _ in range(3)]
+
+    def read():
+        out = outs.pop()
+        ops.linear_tc(act, weights, None, out, ws)
+        return out
+
+    got, want = both(lambda: ops.linear_skinny(x, w[:WIDTH], None, weights), read, weights)
+    assert ops.linear_tc_stripes(m, 16, WIDTH) is not None and torch.equal(got, want) and int(ws.status.item()) == 0
+
+
 @pytest.mark.parametrize("dim", [1024, 2048, 4096])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("kind", ["one", "pair", "dual"])
