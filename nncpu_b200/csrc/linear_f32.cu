@@ -304,11 +304,9 @@ f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        // the first weights are asked for while the tokens are being cut
-        for (int r = 0; r < n_first; ++r) {
-            mbar_expect_tx(&full[r], kCopied);
-            tma_load_2d(smem + r * kStageBytes, &map_w, &full[r], (first_kb(slice0) + r) * kManyK, ((int)blockIdx.x / p.tiles_b % p.tiles_a) * 128);
-        }
+        // the first weights are asked for, into L2, while the tokens are being cut: what ran before that may have written them
+        for (int r = 0; r < n_first; ++r)
+            tma_prefetch_2d(&map_w, (first_kb(slice0) + r) * kManyK, ((int)blockIdx.x / p.tiles_b % p.tiles_a) * 128);
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kTmemCols)
@@ -335,11 +333,9 @@ f32_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
                         ok = false;
                         break;
                     }
-                    if (run >= n_first) {                      // (the first weights have been asked for)
-                        mbar_expect_tx(&full[s], kCopied);     // (rows past the end are filled with zeros and counted)
-                        if (kb + kManyAhead < first_kb(slice + 1)) tma_prefetch_2d(&map_w, (kb + kManyAhead) * kManyK, m0);
-                        tma_load_2d(smem + s * kStageBytes, &map_w, &full[s], kb * kManyK, m0);
-                    }
+                    mbar_expect_tx(&full[s], kCopied);         // (rows past the end are filled with zeros and counted)
+                    if (kb + kManyAhead < first_kb(slice + 1)) tma_prefetch_2d(&map_w, (kb + kManyAhead) * kManyK, m0);
+                    tma_load_2d(smem + s * kStageBytes, &map_w, &full[s], kb * kManyK, m0);
                     if constexpr (kCutX) {
                         tma_load_2d(smem + s * kStageBytes + 128 * 128, &map_x, &full[s], kb * 64, n0);
                         tma_load_2d(smem + s * kStageBytes + kRawBytes + 128 * 64, &map_c, &full[s], kb * 32, n0);

@@ -55,6 +55,24 @@ def test_stripes_of_weights_just_written(ops, slow, m):
     assert ops.linear_tc_stripes(m, 16, WIDTH) is not None and torch.equal(got, want) and int(ws.status.item()) == 0
 
 
+@pytest.mark.parametrize("m", [96, 300])
+def test_float32_product_of_weights_just_written(ops, slow, m):
+    x, w = slow
+    weights = torch.empty(16, WIDTH, device=DEV)
+    act = torch.randn(m, WIDTH, device=DEV)
+    floats = ops.linear_f32_many_scratch_floats(m, 16, WIDTH)
+    scratch, ws = torch.empty(floats, device=DEV), ops.GemmWorkspace(DEV)
+    outs = [torch.empty(m, 16, device=DEV) for _ in range(3)]
+
+    def read():
+        out = outs.pop()
+        ops.linear_f32_many(act, weights, None, out, scratch, ws)
+        return out
+
+    got, want = both(lambda: ops.linear_skinny(x, w[:WIDTH], None, weights), read, weights)
+    assert torch.equal(got, want) and int(ws.status.item()) == 0
+
+
 @pytest.mark.parametrize("dim", [1024, 2048, 4096])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("kind", ["one", "pair", "dual"])
