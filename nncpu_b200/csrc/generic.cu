@@ -119,12 +119,30 @@ __device__ __forceinline__ void weights_into_l2(const void* g, int dim, int dt) 
         asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(g) + at));
 }
 
-// Four weights of a norm from element 4 i on, with one load where the rows allow it.
+// Four weights of a norm from element 4 i on, with one load where the rows allow it (wide).  As loaded: what is asked for ahead is
+// not looked at, so that the loads after it do not wait for it.
+__device__ __forceinline__ uint4 norm_weights_ahead(const void* g, int i, int dt, bool wide) {
+    uint4 u = make_uint4(0, 0, 0, 0);
+    if (!wide) {
+        u = make_uint4(__float_as_uint(ld_f(g, 4 * i, dt)), __float_as_uint(ld_f(g, 4 * i + 1, dt)), __float_as_uint(ld_f(g, 4 * i + 2, dt)),
+                       __float_as_uint(ld_f(g, 4 * i + 3, dt)));
+    } else if (dt == DT_F32) {
+        u = reinterpret_cast<const uint4*>(g)[i];
+    } else {
+        const uint2 h = reinterpret_cast<const uint2*>(g)[i];
+        u.x = h.x;
+        u.y = h.y;
+    }
+    return u;
+}
+__device__ __forceinline__ float4 norm_weights_of(uint4 u, int dt, bool wide, float offset) {
+    const bool pairs = wide && dt != DT_F32;
+    const float2 a = two_bf16(u.x), b = two_bf16(u.y);
+    return make_float4((pairs ? a.x : __uint_as_float(u.x)) + offset, (pairs ? a.y : __uint_as_float(u.y)) + offset,
+                       (pairs ? b.x : __uint_as_float(u.z)) + offset, (pairs ? b.y : __uint_as_float(u.w)) + offset);
+}
 __device__ __forceinline__ float4 norm_weights(const void* g, int i, int dt, bool wide, float offset) {
-    float4 w = wide ? ld_f4(g, 4 * (size_t)i, dt)
-                    : make_float4(ld_f(g, 4 * i, dt), ld_f(g, 4 * i + 1, dt), ld_f(g, 4 * i + 2, dt), ld_f(g, 4 * i + 3, dt));
-    w.x += offset; w.y += offset; w.z += offset; w.w += offset;
-    return w;
+    return norm_weights_of(norm_weights_ahead(g, i, dt, wide), dt, wide, offset);
 }
 
 // The common case, float32 rows of a width that is a multiple of 4 and at most 256 * 4 * kVec: every
@@ -144,31 +162,35 @@ rmsnorm_f32_kernel(const float* __restrict__ x, const void* __restrict__ gamma, 
     const int r_out = blockIdx.x;
     const int n4 = dim >> 2;
     const bool wide = (reinterpret_cast<uintptr_t>(gamma) & 15) == 0;
-    float4 v[kVec], g[kAhead ? kVec : 1], was[kAhead ? kVec : 1];
+    float4 v[kVec], was[kAhead ? kVec : 1];
+    uint4 g[kAhead ? kVec : 1];
     weights_into_l2(gamma, dim, g_dt);
     wait_for_previous_kernels();
     const int r_in = rows ? rows[r_out] : r_out;
-    if constexpr (kAhead) {
-#pragma unroll
-        for (int j = 0; j < kVec; ++j) {
-            const int i = threadIdx.x + j * 256;
-            if (gamma && i < n4) g[j] = norm_weights(gamma, i, g_dt, wide, gamma_offset);
-            if (accumulate && r_in >= 0 && i < n4) was[j] = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(y) + (size_t)r_out * dim)[i];
-        }
-    }
-    float ss = 0.0f;
     if (r_in >= 0) {
         const float4* src = reinterpret_cast<const float4*>(x + (size_t)r_in * dim);
 #pragma unroll
         for (int j = 0; j < kVec; ++j) {
             const int i = threadIdx.x + j * 256;
             v[j] = i < n4 ? src[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            ss = fmaf(v[j].x, v[j].x, ss); ss = fmaf(v[j].y, v[j].y, ss);
-            ss = fmaf(v[j].z, v[j].z, ss); ss = fmaf(v[j].w, v[j].w, ss);
         }
     } else {
 #pragma unroll
         for (int j = 0; j < kVec; ++j) v[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    if constexpr (kAhead) {
+#pragma unroll
+        for (int j = 0; j < kVec; ++j) {
+            const int i = threadIdx.x + j * 256;
+            if (gamma && i < n4) g[j] = norm_weights_ahead(gamma, i, g_dt, wide);
+            if (accumulate && r_in >= 0 && i < n4) was[j] = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(y) + (size_t)r_out * dim)[i];
+        }
+    }
+    float ss = 0.0f;
+#pragma unroll
+    for (int j = 0; j < kVec; ++j) {
+        ss = fmaf(v[j].x, v[j].x, ss); ss = fmaf(v[j].y, v[j].y, ss);
+        ss = fmaf(v[j].z, v[j].z, ss); ss = fmaf(v[j].w, v[j].w, ss);
     }
     ss = sum_of_256(ss, part);
     const float scale = r_in >= 0 ? 1.0f / sqrtf(ss * (1.0f / (float)dim) + eps) : 0.0f;
@@ -178,7 +200,7 @@ rmsnorm_f32_kernel(const float* __restrict__ x, const void* __restrict__ gamma, 
         if (i >= n4) continue;
         float o[4] = {v[j].x * scale, v[j].y * scale, v[j].z * scale, v[j].w * scale};
         if (gamma) {
-            const float4 w = kAhead ? g[kAhead ? j : 0] : norm_weights(gamma, i, g_dt, wide, gamma_offset);
+            const float4 w = kAhead ? norm_weights_of(g[kAhead ? j : 0], g_dt, wide, gamma_offset) : norm_weights(gamma, i, g_dt, wide, gamma_offset);
             o[0] *= w.x; o[1] *= w.y; o[2] *= w.z; o[3] *= w.w;
         }
         const size_t at = (size_t)r_out * dim + 4 * i;
@@ -242,7 +264,8 @@ rmsnorm_pair_kernel(const float* __restrict__ b, float* __restrict__ r, const vo
     let_next_kernel_start();
     const int row = blockIdx.x, n4 = dim >> 2;
     const bool wide = ((reinterpret_cast<uintptr_t>(g1) | reinterpret_cast<uintptr_t>(g2)) & 15) == 0;
-    float4 v[kVec], w1[kAhead ? kVec : 1], w2[kAhead ? kVec : 1], was[kAhead ? kVec : 1];
+    float4 v[kVec], was[kAhead ? kVec : 1];
+    uint4 w1[kAhead ? kVec : 1], w2[kAhead ? kVec : 1];
     weights_into_l2(g1, dim, g_dt);
     weights_into_l2(g2, dim, g_dt);
     wait_for_previous_kernels();
@@ -254,8 +277,8 @@ rmsnorm_pair_kernel(const float* __restrict__ b, float* __restrict__ r, const vo
         v[j] = i < n4 ? reinterpret_cast<const float4*>(b + (size_t)row * dim)[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (kAhead && i < n4) {
             was[kAhead ? j : 0] = stream_row[i];
-            w1[kAhead ? j : 0] = norm_weights(g1, i, g_dt, wide, off1);
-            w2[kAhead ? j : 0] = norm_weights(g2, i, g_dt, wide, off2);
+            w1[kAhead ? j : 0] = norm_weights_ahead(g1, i, g_dt, wide);
+            w2[kAhead ? j : 0] = norm_weights_ahead(g2, i, g_dt, wide);
         }
     }
 #pragma unroll
@@ -271,7 +294,7 @@ rmsnorm_pair_kernel(const float* __restrict__ b, float* __restrict__ r, const vo
         const int i = threadIdx.x + j * 256;
         if (i >= n4) continue;
         const float4 old = kAhead ? was[kAhead ? j : 0] : stream_row[i];
-        const float4 w = kAhead ? w1[kAhead ? j : 0] : norm_weights(g1, i, g_dt, wide, off1);
+        const float4 w = kAhead ? norm_weights_of(w1[kAhead ? j : 0], g_dt, wide, off1) : norm_weights(g1, i, g_dt, wide, off1);
         const float o[4] = {(v[j].x * s1) * w.x, (v[j].y * s1) * w.y, (v[j].z * s1) * w.z, (v[j].w * s1) * w.w};
         v[j] = make_float4(old.x + o[0], old.y + o[1], old.z + o[2], old.w + o[3]);
         stream_row[i] = v[j];
@@ -284,7 +307,7 @@ rmsnorm_pair_kernel(const float* __restrict__ b, float* __restrict__ r, const vo
     for (int j = 0; j < kVec; ++j) {
         const int i = threadIdx.x + j * 256;
         if (i >= n4) continue;
-        const float4 w = kAhead ? w2[kAhead ? j : 0] : norm_weights(g2, i, g_dt, wide, off2);
+        const float4 w = kAhead ? norm_weights_of(w2[kAhead ? j : 0], g_dt, wide, off2) : norm_weights(g2, i, g_dt, wide, off2);
         const float o[4] = {(v[j].x * s2) * w.x, (v[j].y * s2) * w.y, (v[j].z * s2) * w.z, (v[j].w * s2) * w.w};
         const size_t at = (size_t)row * dim + 4 * i;
         if (y_dt == DT_BF16) {
@@ -2168,20 +2191,10 @@ rmsnorm_dual_f32_kernel(const float* __restrict__ x, const void* __restrict__ g1
     let_next_kernel_start();
     const int n4 = dim >> 2;
     const bool wide = ((reinterpret_cast<uintptr_t>(g1) | reinterpret_cast<uintptr_t>(g2)) & 15) == 0;
-    float4 w[2][kAhead ? kVec : 1];
+    uint4 w[2][kAhead ? kVec : 1];
     weights_into_l2(g1, dim, g_dt);
     weights_into_l2(g2, dim, g_dt);
     wait_for_previous_kernels();
-    if constexpr (kAhead) {
-#pragma unroll
-        for (int j = 0; j < kVec; ++j) {
-            const int i = threadIdx.x + j * 256;
-            if (i < n4) {
-                w[0][j] = norm_weights(g1, i, g_dt, wide, 0.0f);
-                w[1][j] = norm_weights(g2, i, g_dt, wide, 0.0f);
-            }
-        }
-    }
     const float4* src = reinterpret_cast<const float4*>(x + (size_t)blockIdx.x * dim);
     float4 v[kVec];
     float ss = 0.0f;
@@ -2189,6 +2202,13 @@ rmsnorm_dual_f32_kernel(const float* __restrict__ x, const void* __restrict__ g1
     for (int j = 0; j < kVec; ++j) {
         const int i = threadIdx.x + j * 256;
         v[j] = i < n4 ? src[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (kAhead && i < n4) {
+            w[0][kAhead ? j : 0] = norm_weights_ahead(g1, i, g_dt, wide);
+            w[1][kAhead ? j : 0] = norm_weights_ahead(g2, i, g_dt, wide);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < kVec; ++j) {
         ss = fmaf(v[j].x, v[j].x, ss); ss = fmaf(v[j].y, v[j].y, ss);
         ss = fmaf(v[j].z, v[j].z, ss); ss = fmaf(v[j].w, v[j].w, ss);
     }
@@ -2206,7 +2226,7 @@ rmsnorm_dual_f32_kernel(const float* __restrict__ x, const void* __restrict__ g1
             const void* g = which ? g2 : g1;
             void* y = which ? y2 : y1;
             const float sc = which ? s2 : s1;
-            const float4 f = kAhead ? w[which][kAhead ? j : 0] : norm_weights(g, i, g_dt, wide, 0.0f);
+            const float4 f = kAhead ? norm_weights_of(w[which][kAhead ? j : 0], g_dt, wide, 0.0f) : norm_weights(g, i, g_dt, wide, 0.0f);
             const float o[4] = {(in[0] * sc) * f.x, (in[1] * sc) * f.y, (in[2] * sc) * f.z, (in[3] * sc) * f.w};
             if (y_dt == DT_BF16) {
                 __nv_bfloat162 h[2] = {__floats2bfloat162_rn(o[0], o[1]), __floats2bfloat162_rn(o[2], o[3])};
