@@ -25,6 +25,8 @@
 
 #include <math.h>
 
+#include <algorithm>
+
 #define NN_LIB linear_f32
 #define NN_LAUNCH_OVERLAP
 #include "common.cuh"
@@ -671,9 +673,17 @@ int launch_many(const ManyParams& p, cudaStream_t stream) {
 // own, and with few tokens there is little of them to cut beside 128 rows of weights (us, on arrival / beforehand, N x K 12288 x
 // 2048 and 2048 x 6144: 17 tokens 42.6 / 44.5 and 26.1 / 28.1, 64 tokens 46.8 / 47.5 and 29.6 / 32.3, 100 tokens 66.8 / 58.0 and
 // 41.7 / 36.3, 300 tokens 145 / 120 and 74.7 / 64.1, 600 tokens 210 / 168 and 119 / 107; 100 tokens of 2048 x 2048 22.3 / 21.5).
+// The parts are half as large again as the tokens, so that many tokens go through the product in bands, each a product of its own, whose
+// parts take kCutMost floats at most (256 MB).  8192 tokens of K 6144 would take 302 MB beside 201 MB of tokens (N 2048: 1 240 us; in two
+// bands of 151 MB, sums of slices included, 1 180 us).
 constexpr int kCutFrom = 96;
+constexpr long kCutMost = 1l << 26;
 static long cut_floats(int M, int K) {
     return M < kCutFrom ? 0 : (long)M * ((K + kManyK - 1) / kManyK) * (kManyK * 3 / 2);
+}
+static int cut_band(int M, int K) {
+    const long bands = (cut_floats(M, K) + kCutMost - 1) / kCutMost;
+    return bands <= 1 ? M : (int)((M + 256 * bands - 1) / (256 * bands)) * 256;
 }
 
 // What the products here take: rows of whole 16-byte pieces.
@@ -702,8 +712,14 @@ extern "C" int nncpu_linear_f32(const void* X, const void* W, const void* bias, 
 // Floats of scratch that nncpu_linear_f32_many needs at these sizes (0: none).
 extern "C" long nncpu_linear_f32_many_scratch(int M, int N, int K) {
     if (M <= 0 || N <= 0 || K <= 0) return 0;
-    const ManyPlan plan = many_plan(M, N, K);
-    return cut_floats(M, K) + (plan.slices > 1 ? (long)plan.slices * M * N : 0);
+    const int band = cut_band(M, K);
+    long most = 0;
+    for (const int m : {band, M % band}) {
+        if (m == 0) continue;
+        const ManyPlan plan = many_plan(m, N, K);
+        most = std::max(most, cut_floats(m, K) + (plan.slices > 1 ? (long)plan.slices * m * N : 0));
+    }
+    return most;
 }
 
 // The same product for any number of tokens, on the tensor cores.  `scratch`: see above.  `status` is set when a bounded wait
@@ -714,22 +730,30 @@ extern "C" int nncpu_linear_f32_many(const void* X, const void* W, const void* b
     NN_CHECK(M > 0 && N > 0 && K > 0 && K % 4 == 0 && lda % 4 == 0 && lda >= K && ldc >= N,
              "linear (32-bit): M %d, N %d, K %d, lda %d, ldc %d", M, N, K, lda, ldc);
     NN_CHECK((uintptr_t)X % 16 == 0 && (uintptr_t)W % 16 == 0, "linear (32-bit): operands must be 16-byte aligned");
-    const ManyPlan plan = many_plan(M, N, K);
-    NN_CHECK(plan.slices == 1 || scratch != nullptr, "linear (32-bit): %d slices of K need scratch memory", plan.slices);
-    ManyParams p{(const float*)X, (const float*)W, bias, bias_dt, C, c_dt, (float*)scratch, nullptr, nullptr, M, N, K, lda, ldc, accumulate,
-                 (N + 127) / 128, plan.tiles_b, plan.slices, (K + kManyK - 1) / kManyK, K < kShortK ? 1 : 2, status};
-    NN_CHECK((long)p.tiles_a * p.tiles_b * p.slices < (1L << 31), "linear (32-bit): %d tokens of %d features", M, N);
-    const long floats = scratch != nullptr ? cut_floats(M, K) : 0;
-    if (floats > 0) {
-        NN_CHECK((uintptr_t)scratch % 16 == 0, "linear (32-bit): scratch memory must be 16-byte aligned");
-        p.cut_ab = (uint16_t*)scratch;
-        p.cut_c = p.cut_ab + (size_t)M * p.kb_total * 64;
-        p.part = (float*)scratch + floats;
-    }
-#define NN_MANY(BN_) case BN_: return floats > 0 ? launch_many<BN_, true>(p, st) : launch_many<BN_, false>(p, st);
-    switch (plan.bn) {
-        NN_MANY(32) NN_MANY(64) NN_MANY(96) NN_MANY(128) NN_MANY(160) NN_MANY(192) NN_MANY(224)
-        default: return floats > 0 ? launch_many<256, true>(p, st) : launch_many<256, false>(p, st);
-    }
+    NN_CHECK(scratch != nullptr || many_plan(M, N, K).slices == 1, "linear (32-bit): slices of K need scratch memory (%d tokens)", M);
+    const int band = scratch != nullptr ? cut_band(M, K) : M;
+    for (int m0 = 0; m0 < M; m0 += band) {
+        const int m = std::min(band, M - m0);
+        const ManyPlan plan = many_plan(m, N, K);
+        ManyParams p{(const float*)X + (size_t)m0 * lda, (const float*)W, bias, bias_dt,
+                     (char*)C + (size_t)m0 * ldc * (c_dt == DT_F32 ? 4 : 2), c_dt, (float*)scratch, nullptr, nullptr, m, N, K, lda, ldc, accumulate,
+                     (N + 127) / 128, plan.tiles_b, plan.slices, (K + kManyK - 1) / kManyK, K < kShortK ? 1 : 2, status};
+        NN_CHECK((long)p.tiles_a * p.tiles_b * p.slices < (1L << 31), "linear (32-bit): %d tokens of %d features", M, N);
+        const long floats = scratch != nullptr ? cut_floats(m, K) : 0;
+        if (floats > 0) {
+            NN_CHECK((uintptr_t)scratch % 16 == 0, "linear (32-bit): scratch memory must be 16-byte aligned");
+            p.cut_ab = (uint16_t*)scratch;
+            p.cut_c = p.cut_ab + (size_t)m * p.kb_total * 64;
+            p.part = (float*)scratch + floats;
+        }
+        int e;
+#define NN_MANY(BN_) case BN_: e = floats > 0 ? launch_many<BN_, true>(p, st) : launch_many<BN_, false>(p, st); break;
+        switch (plan.bn) {
+            NN_MANY(32) NN_MANY(64) NN_MANY(96) NN_MANY(128) NN_MANY(160) NN_MANY(192) NN_MANY(224)
+            default: e = floats > 0 ? launch_many<256, true>(p, st) : launch_many<256, false>(p, st);
+        }
 #undef NN_MANY
+        if (e != 0) return e;
+    }
+    return 0;
 }

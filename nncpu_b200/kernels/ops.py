@@ -312,7 +312,8 @@ def linear_f32(x, w, bias, out, accumulate: bool = False) -> None:
 
 
 def linear_f32_many_scratch_floats(m: int, n: int, k: int) -> int:
-    """Floats of scratch that ``linear_f32_many`` needs at these sizes."""
+    """Floats of scratch that ``linear_f32_many`` needs at these sizes: from 96 tokens on the tokens' parts (1.5 floats a number, of
+    at most 256 MB of them at a time), and the sums of K's slices where there are few tiles."""
     lib = library.load("linear_f32")
     lib.nncpu_linear_f32_many_scratch.restype = ctypes.c_long
     return lib.nncpu_linear_f32_many_scratch(_i(m), _i(n), _i(k))

@@ -42,3 +42,13 @@ def test_float32_products(m, n, k, pays):
 @pytest.mark.parametrize("tokens,top,pays", [(8, 2, True), (16, 4, True), (8, 8, True), (16, 5, False), (9, 8, False), (17, 1, False)])
 def test_routed_experts_by_the_few_row_product(tokens, top, pays):
     assert ops.skinny_grouped_pays(tokens, tokens * top) is pays
+
+
+@pytest.mark.parametrize("m", [95, 96, 3000, 7281, 7282, 8192, 20000, 100000])
+@pytest.mark.parametrize("n,k", [(2048, 6144), (12288, 2048), (256, 17408), (128, 100000)])
+def test_float32_parts_are_bounded(m, n, k):
+    """The scratch of float32 products of many tokens: the tokens' parts, in bands of 2^26 floats (and less than 256 tokens more), and
+    the sums of K's slices where there are few tiles."""
+    blocks = (k + 31) // 32 * 48
+    most = min(m, (1 << 26) // blocks + 256)
+    assert ops.linear_f32_many_scratch_floats(m, n, k) <= (most * blocks if m >= 96 else 0) + 8 * most * n

@@ -35,3 +35,24 @@ def test_tokens_cut_beforehand(m, k):
     ops.linear_f32_many(x, w, bias, other, None, work, accumulate=True)
     assert torch.equal(out, other) and bool(torch.isinf(out[m // 2]).all())
     assert int(work.status.item()) == 0
+
+
+def test_many_tokens_go_in_bands():
+    """The tokens' parts take 256 MB at most; a band has the bits of a product of its own."""
+    from nncpu_b200.kernels import ops
+    m, n, k, band = 7300, 264, 6144, 3840
+    floats = ops.linear_f32_many_scratch_floats(m, n, k)
+    assert floats == max(ops.linear_f32_many_scratch_floats(rows, n, k) for rows in (band, m - band)) < m * k * 3 // 2
+    g = torch.Generator(device=DEV).manual_seed(5)
+    x, w = torch.randn(m, k, generator=g, device=DEV), torch.randn(n, k, generator=g, device=DEV) * 0.02
+    bias, work = torch.randn(n, generator=g, device=DEV), ops.GemmWorkspace(DEV)
+    scratch = torch.full((floats + 1,), 7.0, device=DEV)
+    for dtype in (torch.float32, torch.bfloat16):
+        out, parts = [torch.full((m, n), 9.0, dtype=dtype, device=DEV) for _ in range(2)]
+        ops.linear_f32_many(x, w, bias, out, scratch[:floats], work)
+        for rows in (slice(0, band), slice(band, m)):
+            ops.linear_f32_many(x[rows], w, bias, parts[rows], scratch[:floats], work)
+        assert torch.equal(out, parts) and float(scratch[-1]) == 7.0
+        want = x.double() @ w.double().T + bias.double()
+        assert ((out.double() - want).norm() / want.norm()).item() < (4.3e-7 if dtype == torch.float32 else 2.0 ** -8)
+    assert int(work.status.item()) == 0
