@@ -505,29 +505,24 @@ __device__ __forceinline__ float row_squares(const float* __restrict__ src, int 
     return ss;
 }
 
-// Which of n <= kByLengthMax tokens has the nth most keys (ties in their order, padding last).  A grid of more blocks than run at
-// once begins with the long sequences, so that the blocks that start last are short ones: a block's share of the bandwidth is
-// what it can keep in flight, and a long sequence that starts when the others are done streams alone (two blocks an SM; 64
-// sequences of 125 to 1 875 keys, 8 key/value heads, 512 blocks for 296 places: 61.8 us in the tokens' order, 50.0 by length; of
-// 384 to 5 760 keys 159 and 123; 40 of 125 to 1 875 43.2 and 39.8).
-constexpr int kByLengthMax = 128;
-__device__ __forceinline__ int nth_longest(const int* __restrict__ tok_seq, const int* __restrict__ tok_pos, int n, int nth) {
-    __shared__ __align__(16) int len_s[kByLengthMax];
-    __shared__ int found_s;
-    const int i = threadIdx.x;
-    const int mine = i < n ? (tok_seq[i] < 0 ? -1 : tok_pos[i]) : -2;
-    len_s[i] = mine;
+// The tokens of a decode step in the order in which their blocks start, those with the most keys first (ties in their order, padding
+// last): order[i] = (token, its sequence, its position, 0).  A grid of more blocks than run at once then ends with short
+// sequences: a block's share of the bandwidth is what it can keep in flight, and a long sequence that starts when the others
+// are done streams alone (two blocks an SM; 64 sequences of 125 to 1 875 keys, 8 key/value heads, 512 blocks for 296 places:
+// 50.7 us in the tokens' order, 43.2 by length; 40 sequences 40.3 and 36.1, 128 92.5 and 84.3; 64 of 1 000 keys each 45.5 and 45.9).
+// Made once for all layers of a step: a block that works it out for itself starts 1 us later, which 128 sequences
+// of 100 keys pay three times (10.0 us, 13.9).
+constexpr int kOrderMax = 1024;
+__global__ void __launch_bounds__(256) decode_order_kernel(const int* __restrict__ tok_seq, const int* __restrict__ tok_pos, int4* __restrict__ order, int n) {
+    __shared__ int keys[kOrderMax];
+    for (int i = threadIdx.x; i < n; i += 256) keys[i] = tok_seq[i] < 0 ? -1 : tok_pos[i];
     __syncthreads();
-    int before = 0;
-#pragma unroll 4
-    for (int j = 0; j < n; j += 4) {          // (places behind n hold -2: before nobody)
-        const int4 o = *reinterpret_cast<const int4*>(&len_s[j]);
-        before += (o.x > mine || (o.x == mine && j < i)) + (o.y > mine || (o.y == mine && j + 1 < i)) +
-                  (o.z > mine || (o.z == mine && j + 2 < i)) + (o.w > mine || (o.w == mine && j + 3 < i));
+    for (int i = threadIdx.x; i < n; i += 256) {
+        const int mine = keys[i];
+        int before = 0;
+        for (int j = 0; j < n; ++j) before += keys[j] > mine || (keys[j] == mine && j < i);
+        order[before] = make_int4(i, mine < 0 ? -1 : tok_seq[i], mine, 0);
     }
-    if (i < n && before == nth) found_s = i;
-    __syncthreads();
-    return found_s;
 }
 
 // kMore: with a cap on the scores or a short convolution before the heads; kernels without either do not carry them.
@@ -538,7 +533,7 @@ decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restri
                    const int* __restrict__ tok_seq, const int* __restrict__ tok_pos, __nv_bfloat16* __restrict__ out,
                    float* __restrict__ part_o, float* __restrict__ part_ml, int n_heads, int n_kv, float scale2,
                    int window, int keep, const FusedQK f, const float* __restrict__ sinks, int kv_rep, int vo,
-                   const ScoreCap cap, const OutGate gate, int by_length) {
+                   const ScoreCap cap, const OutGate gate, const int4* __restrict__ order) {
     constexpr int kTileBytes = kPage * HD * 2, kStageBytes = kPage * (HD + VD) * 2;
     constexpr int kChunks = HD / 8, kVChunks = VD / 8;
     constexpr int W = VD + 2;
@@ -547,8 +542,14 @@ decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restri
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int c = lane & 3, r = lane >> 2;
     const int G = n_heads / n_kv;
-    const int t = by_length ? nth_longest(tok_seq, tok_pos, (int)gridDim.z, (int)blockIdx.z) : (int)blockIdx.z;
-    const int seq = tok_seq[t];
+    int t = blockIdx.z, seq, pos;
+    if (order != nullptr) {
+        const int4 o = order[t];
+        t = o.x; seq = o.y; pos = o.z;
+    } else {
+        seq = tok_seq[t];
+        pos = tok_pos[t];
+    }
     const size_t out_row = ((size_t)t * n_heads + (size_t)kvh * G) * vo;
     if (seq < 0) {  // padding: zeros (every block of a cluster takes this way out together)
         if (n_splits == 1 || split == 0)
@@ -560,7 +561,6 @@ decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restri
         }
         return;
     }
-    const int pos = tok_pos[t];
     const int first = first_visible_key(pos, window);
     const PageWalk walk(first, pos, keep);
     const int p_last = pos / kPage;
@@ -872,10 +872,10 @@ template <int HD, int VD, bool kMore>
 int launch_decode_one(const void* q, const void* k_pages, const void* v_pages, const int* block_table, int bt_stride,
                   const int* tok_seq, const int* tok_pos, void* out, float* scratch, int n_tok, int n_heads, int n_kv,
                   float scale, int window, int keep, int vo, int n_splits, cudaStream_t stream, const FusedQK* fused,
-                  float slope_base, const float* sinks, float cap, const OutGate& gate) {
+                  float slope_base, const float* sinks, float cap, const OutGate& gate, const int4* order) {
     using Kernel = void (*)(const __nv_bfloat16*, const __nv_bfloat16*, const __nv_bfloat16*, const int*, int, const int*,
                             const int*, __nv_bfloat16*, float*, float*, int, int, float, int, int, const FusedQK, const float*,
-                            int, int, const ScoreCap, const OutGate, int);
+                            int, int, const ScoreCap, const OutGate, const int4*);
     // a block serves at most 16 heads of a key/value head: where more share one, kv_rep blocks take a part each
     int kv_rep = 1;
     while ((n_heads / n_kv) % kv_rep != 0 || n_heads / n_kv / kv_rep > 16) ++kv_rep;
@@ -901,8 +901,6 @@ int launch_decode_one(const void* q, const void* k_pages, const void* v_pages, c
                                                    (int)(stages > (size_t)5 * 16 * (VD + 2) * 4 ? stages : (size_t)5 * 16 * (VD + 2) * 4));
         NN_CHECK(e == cudaSuccess, "attention decode: cannot reserve shared memory: %s", cudaGetErrorString(e));
     }
-    // two blocks run on an SM; with more than that they start in the order of their lengths
-    const int by_length = n_tok <= kByLengthMax && (long)n_splits * n_kv * n_tok > 2l * sm_count() ? 1 : 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(n_splits, n_kv, n_tok);
     cfg.blockDim = dim3(128);
@@ -918,7 +916,7 @@ int launch_decode_one(const void* q, const void* k_pages, const void* v_pages, c
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_pages,
                                              (const __nv_bfloat16*)v_pages, block_table, bt_stride, tok_seq, tok_pos,
                                              (__nv_bfloat16*)out, part_o, part_ml, n_heads, n_kv, scale * kLog2e, window, keep, f,
-                                             sinks, kv_rep, vo, score_cap(scale, cap), gate, by_length);
+                                             sinks, kv_rep, vo, score_cap(scale, cap), gate, order);
     NN_CHECK(e == cudaSuccess, "attention decode (%d splits%s): launch failed: %s", n_splits, cluster ? ", cluster" : "",
              cudaGetErrorString(e));
     if (n_splits > 1 && !cluster) {
@@ -933,11 +931,11 @@ template <int HD, int VD>
 int launch_decode(const void* q, const void* k_pages, const void* v_pages, const int* block_table, int bt_stride,
                   const int* tok_seq, const int* tok_pos, void* out, float* scratch, int n_tok, int n_heads, int n_kv,
                   float scale, int window, int keep, int vo, int n_splits, cudaStream_t stream, const FusedQK* fused,
-                  float slope_base, const float* sinks, float cap, const OutGate& gate) {
+                  float slope_base, const float* sinks, float cap, const OutGate& gate, const int4* order) {
     const bool more = cap > 0.0f || (fused != nullptr && fused->conv.w != nullptr);
     return (more ? launch_decode_one<HD, VD, true> : launch_decode_one<HD, VD, false>)(
         q, k_pages, v_pages, block_table, bt_stride, tok_seq, tok_pos, out, scratch, n_tok, n_heads, n_kv, scale, window, keep, vo,
-        n_splits, stream, fused, slope_base, sinks, cap, gate);
+        n_splits, stream, fused, slope_base, sinks, cap, gate, order);
 }
 
 template <int HD, int VD>
@@ -979,6 +977,16 @@ extern "C" long nncpu_attention_decode_scratch_floats(int n_tok, int n_heads, in
     return (long)n_tok * n_kv * n_splits * G * (vp + 2);
 }
 
+// The order in which the blocks of a decode step of at most 1 024 tokens start (decode_order_kernel); order: [n_tok, 4] ints.
+extern "C" int nncpu_attention_decode_order(const int* tok_seq, const int* tok_pos, int* order, int n_tok, void* stream) {
+    NN_CHECK(n_tok >= 0 && n_tok <= kOrderMax && (uintptr_t)order % 16 == 0, "attention decode: an order of %d tokens (at most %d, 16-byte aligned)",
+             n_tok, kOrderMax);
+    if (n_tok == 0) return 0;
+    decode_order_kernel<<<1, 256, 0, (cudaStream_t)stream>>>(tok_seq, tok_pos, (int4*)order, n_tok);
+    NN_LAUNCH_OK("attention decode (order)");
+    return 0;
+}
+
 // One token per sequence: token t belongs to sequence tok_seq[t] (negative: padding) and sits at
 // position tok_pos[t]; its keys 0..tok_pos[t] (or the last `window` of them) are in the cache.
 extern "C" int nncpu_attention_decode_mma(const void* q, const void* k_pages, const void* v_pages,
@@ -986,10 +994,11 @@ extern "C" int nncpu_attention_decode_mma(const void* q, const void* k_pages, co
                                           const int* tok_pos, void* out, float* scratch, long scratch_floats,
                                           int n_tok, int n_heads, int n_kv, int hd, int vp, int vo, float scale, int window,
                                           int keep, int n_splits, float slope_base, const float* sinks, float cap,
-                                          const float* head_gate, int gate_ld, void* stream) {
+                                          const float* head_gate, int gate_ld, const int* order, void* stream) {
     // pages of keys have rows of hd lanes, pages of values rows of vp; a head's output has vo lanes.  keep: with a
     // window, the sequence's first keys that stay visible.  cap > 0: a scaled score z becomes cap tanh(z / cap).
     // head_gate (or null): token t's n_heads logits at t * gate_ld, whose sigmoids multiply the heads' outputs.
+    // order (or null: the tokens' own): nncpu_attention_decode_order of these tokens; the results are the same.
     NN_CHECK(cap >= 0.0f && (head_gate == nullptr || gate_ld >= n_heads), "attention decode: cap %f, gate rows of %d", cap, gate_ld);
     const OutGate gate{head_gate, gate_ld, 1};
     NN_CHECK(nncpu_attention_mma_supported(n_heads, n_kv, hd),
@@ -1008,7 +1017,7 @@ extern "C" int nncpu_attention_decode_mma(const void* q, const void* k_pages, co
 #define NN_DECODE(HD_, VD_)                                                                                                 \
     return launch_decode<HD_, VD_>(q, k_pages, v_pages, block_table, bt_stride, tok_seq, tok_pos, out, scratch, n_tok,      \
                                    n_heads, n_kv, scale, window, keep, vo, n_splits, (cudaStream_t)stream, nullptr, slope_base, sinks, \
-                                   cap, gate)
+                                   cap, gate, (const int4*)order)
     if (hd == 64) NN_DECODE(64, 64);
     if (vp == 64) NN_DECODE(128, 64);
     NN_DECODE(128, 128);
@@ -1032,7 +1041,7 @@ extern "C" int nncpu_attention_decode_mma_from_qkv(const float* qkv, const void*
                                                    int rot_pairs, float scale, int window, int keep, int n_splits, float slope_base,
                                                    float temp_coef, int temp_every, const float* sinks,
                                                    int values_are_keys, int gated, float cap, const float* conv_w, int taps,
-                                                   float* conv_state, long conv_stride, const int* seq_slots, void* stream) {
+                                                   float* conv_state, long conv_stride, const int* seq_slots, const int* order, void* stream) {
     // gated: 1 a logit a lane of the output ends a token's row, 2 a logit a head, 0 none.  cap: as above.  conv_w (or null)
     // [taps, C]: the short convolution over the C lanes of q and k, its state rows conv_stride floats apart.
     NN_CHECK(nncpu_attention_mma_supported(n_heads, n_kv, hd),
@@ -1089,7 +1098,7 @@ extern "C" int nncpu_attention_decode_mma_from_qkv(const float* qkv, const void*
 #define NN_DECODE(HD_, VD_)                                                                                                 \
     return launch_decode<HD_, VD_>(nullptr, k_pages, v_pages, block_table, bt_stride, tok_seq, tok_pos, out, scratch, n_tok, \
                                    n_heads, n_kv, scale, window, keep, v_head_dim, n_splits, (cudaStream_t)stream, &f, 0.0f, sinks, \
-                                   cap, gate)
+                                   cap, gate, (const int4*)order)
     if (hd == 64) NN_DECODE(64, 64);
     if (vp == 64) NN_DECODE(128, 64);
     NN_DECODE(128, 128);
@@ -1199,5 +1208,5 @@ extern "C" int nncpu_attention_decode_mma_static(const void* q, const void* k_pa
     if (int e = static_scratch(&scratch)) return e;
     return nncpu_attention_decode_mma(q, k_pages, v_pages, block_table, bt_stride, tok_seq, tok_pos, out, scratch,
                                       kStaticScratchFloats, n_tok, n_heads, n_kv, hd, hd, hd, scale, window, 0, n_splits, 0.0f, nullptr,
-                                      0.0f, nullptr, 0, stream);
+                                      0.0f, nullptr, 0, nullptr, stream);
 }

@@ -770,16 +770,35 @@ def attention_decode_scratch_floats(n_tok: int, n_heads: int, n_kv: int, head_di
     return 0 if n_splits <= 1 else n_tok * n_kv * n_splits * (n_heads // n_kv) * (head_dim + 2)
 
 
+DECODE_ORDER_MAX = 1024
+
+
+def attention_decode_order_pays(n: int, n_heads: int, n_kv: int, k_row: int, v_row: int, n_splits: int, sm_count: int) -> bool:
+    """Whether a decode step of ``n`` tokens has more blocks than run at once (a block serves at most 16 heads; an SM holds two with rows
+    of 128 lanes and three or four with shorter ones): then those of the longest sequences should start first."""
+    group = n_heads // n_kv
+    parts = next(r for r in range(1, group + 1) if group % r == 0 and group // r <= 16)
+    return n <= DECODE_ORDER_MAX and n * n_kv * parts * n_splits > -(-512 // (k_row + v_row)) * sm_count
+
+
+def attention_decode_order(tok_seq, tok_pos, out) -> None:
+    """The order in which the blocks of a decode step start, the longest sequences first, for the ``order`` of
+    ``attention_decode_mma`` and ``attention_decode_mma_from_qkv``: out int32 [n, 4], n at most 1 024."""
+    n = tok_pos.shape[0]
+    assert out.shape == (n, 4) and out.dtype == tok_seq.dtype == tok_pos.dtype == torch.int32
+    _call("attention_mma", "nncpu_attention_decode_order", _ptr(tok_seq), _ptr(tok_pos), _ptr(out), _i(n), _stream())
+
+
 def attention_decode_mma(q, k_pages, v_pages, block_table, tok_seq, tok_pos, out, scratch, n_heads: int, n_kv: int,
                          head_dim: int, scale: float, window: int, n_splits: int, slope_base: float = 0.0,
-                         sinks=None, keep: int = 0, v_lanes: int = 0, cap: float = 0.0, head_gate=None) -> None:
+                         sinks=None, keep: int = 0, v_lanes: int = 0, cap: float = 0.0, head_gate=None, order=None) -> None:
     """One token per sequence; each token's keys are cut into ``n_splits``
     splits that run in parallel.  ``head_dim`` is the size of q's heads and of the pages' key rows, ``v_lanes`` that of
     the output's heads (0: ``head_dim``; at most the value rows').  With ``scratch`` (float32,
     ``attention_decode_scratch_floats`` elements) a second kernel merges them;
     with ``scratch`` None and at most 8 splits they form a thread-block
     cluster and merge through distributed shared memory.  ``sinks`` as in ``attention``: the term joins where the
-    splits merge, once."""
+    splits merge, once.  ``order``: ``attention_decode_order`` of these tokens (the results are the same bits)."""
     n = q.shape[0]
     v_lanes = v_lanes or head_dim
     assert q.shape == (n, n_heads * head_dim) and out.shape == (n, n_heads * v_lanes)
@@ -789,7 +808,7 @@ def attention_decode_mma(q, k_pages, v_pages, block_table, tok_seq, tok_pos, out
           _i(block_table.shape[1]), _ptr(tok_seq), _ptr(tok_pos), _ptr(out), _ptr(scratch),
           ctypes.c_long(0 if scratch is None else scratch.numel()), _i(n), _i(n_heads), _i(n_kv), _i(head_dim),
           _i(v_pages.shape[-1]), _i(v_lanes), _f(scale), _i(window), _i(keep), _i(n_splits), _f(slope_base), _ptr(sinks),
-          _f(cap), *_head_gate(head_gate, n, n_heads), _stream())
+          _f(cap), *_head_gate(head_gate, n, n_heads), _ptr(order), _stream())
 
 
 def attention_decode_mma_from_qkv(qkv, q_gamma, k_gamma, eps, cos_sin, k_pages, v_pages, append: bool, block_table,
@@ -797,7 +816,7 @@ def attention_decode_mma_from_qkv(qkv, q_gamma, k_gamma, eps, cos_sin, k_pages, 
                                   window: int, n_splits: int, slope_base: float = 0.0, q_temp=None, sinks=None,
                                   values_are_keys: bool = False, gated: bool = False, keep: int = 0, v_head_dim: int = 0,
                                   whole_norm: bool = False, rot_pairs: bool = False, cap: float = 0.0,
-                                  head_gated: bool = False, conv=None) -> None:
+                                  head_gated: bool = False, conv=None, order=None) -> None:
     """Decode attention that starts from the float32 projections ``qkv`` [n, per_tok * head_dim] (q heads, then with
     ``append`` the k and v heads): every block makes its queries itself (per-head norm, rotation by ``cos_sin``
     [n, head_dim / 2, 2]), and with ``append`` the token's key and value are made, written to the cache and used.
@@ -809,7 +828,7 @@ def attention_decode_mma_from_qkv(qkv, q_gamma, k_gamma, eps, cos_sin, k_pages, 
     all of a token's query (key) lanes at once, as in ``qk_whole_norm_append``.  ``rot_pairs``: ``cos_sin`` [n, pairs, 2]
     turns a head's first neighbouring pairs of lanes.  ``cap``: as in ``attention``.  ``head_gated``: n_heads logits end the
     rows, one a head.  ``conv = (w [taps, C], state, seq_slots)``: the short convolution of ``qk_conv_norm_append`` (every token
-    is its sequence's only one); a value that is the key is taken after it."""
+    is its sequence's only one); a value that is the key is taken after it.  ``order`` as in ``attention_decode_mma``."""
     n = out.shape[0]
     v_head_dim = v_head_dim or head_dim
     row = n_heads * head_dim + ((n_kv * head_dim + (0 if values_are_keys else n_kv * v_head_dim)) if append else 0)
@@ -838,7 +857,7 @@ def attention_decode_mma_from_qkv(qkv, q_gamma, k_gamma, eps, cos_sin, k_pages, 
           _i(whole_norm), _i(rot_half), _i(rot_pairs), _f(scale), _i(window), _i(keep), _i(n_splits), _f(slope_base),
           _f(q_temp[0] if q_temp else 0.0), _i(q_temp[1] if q_temp else 1), _ptr(sinks), _i(values_are_keys),
           _i(2 if head_gated else 1 if gated else 0), _f(cap), _ptr(conv_w), _i(0 if conv is None else conv_w.shape[0]),
-          _ptr(conv_state), _l(0 if conv is None else conv_state.shape[1]), _ptr(slots), _stream())
+          _ptr(conv_state), _l(0 if conv is None else conv_state.shape[1]), _ptr(slots), _ptr(order), _stream())
 
 
 def attention_prefill_mma(q, k_pages, v_pages, block_table, cu_seqlens, tok_pos, out, n_seqs: int, n_heads: int,

@@ -234,7 +234,8 @@ class Attention(Mixer):
                                                       gated=s.out_gate, keep=s.keep_first, v_head_dim=self.v_dim,
                                                       whole_norm=s.qk_norm_whole, rot_pairs=self.pairs, cap=s.score_cap,
                                                       head_gated=s.head_gate,
-                                                      conv=(self.w_conv, cache.state, ctx.seq_slots) if self.convolved else None)
+                                                      conv=(self.w_conv, cache.state, ctx.seq_slots) if self.convolved else None,
+                                                      order=self._decode_order(ctx, n_splits))
             else:
                 q = rt.empty(n, s.n_heads * self.k_row)
                 n_kv = 0 if self.shared_kv else s.n_kv_heads
@@ -288,6 +289,11 @@ class Attention(Mixer):
             return False
         return (not self.plain_core and ops.attention_mma_supported(s.n_heads, s.n_kv_heads, self.k_row)
                 and self.v_row in (64, self.k_row))
+
+    def _decode_order(self, ctx, n_splits):
+        """The order in which a decode step's blocks start (a window makes long sequences short: none)."""
+        s = self.spec
+        return None if self.span else self.rt.decode_order(ctx, s.n_heads, s.n_kv_heads, self.k_row, self.v_row, n_splits)
 
     def _decode_splits(self, ctx):
         """Splits of every token's keys in a decode step, and the scratch their merge needs (None: they merge
@@ -345,7 +351,7 @@ class Attention(Mixer):
             n_splits, scratch = self._decode_splits(ctx)
             ops.attention_decode_mma(q, cache.k_pages, cache.v_pages, cache.block_table, ctx.tok_seq, ctx.tok_pos,
                                      attn, scratch, s.n_heads, s.n_kv_heads, self.k_row, s.scale, self.span, n_splits,
-                                     s.slope_base, self.sinks, **extra)
+                                     s.slope_base, self.sinks, order=self._decode_order(ctx, n_splits), **extra)
         elif (ctx.n_tokens >= 32 * ctx.n_seqs or ctx.n_seqs == 1) and ops.attention_prefill_tc_supported(
                 s.n_heads, s.n_kv_heads, self.k_row, q, cache.k_pages, attn):
             # prompts: 128-row tiles on the tcgen05 tensor cores, the keys of few tiles shared by several blocks

@@ -208,7 +208,7 @@ class LatentAttention(Mixer):
                 ctx.n_tokens, H, 1, r, n_splits)
             scratch = rt.empty(floats, dtype=torch.float32) if floats else None
             ops.attention_decode_mma(q, pages, pages, cache.block_table, ctx.tok_seq, ctx.tok_pos, out, scratch, H, 1, r,
-                                     s.scale, 0, n_splits, 0.0, self.sinks)
+                                     s.scale, 0, n_splits, 0.0, self.sinks, order=rt.decode_order(ctx, H, 1, r, r, n_splits))
         elif ctx.n_tokens >= 32 * ctx.n_seqs and ops.attention_prefill_tc_supported(H, 1, r, q, pages, out):
             ops.attention_prefill_tc(q, pages, pages, cache.block_table, ctx.cu_seqlens, ctx.tok_pos, out,
                                      rt.workspace.status, ctx.n_seqs, H, 1, r, s.scale, 0, 0.0, self.sinks, longest=ctx.max_kv_len)

@@ -208,6 +208,17 @@ class Runtime:
                     scratch = self.empty(floats, dtype=torch.float32) if floats else None
                     ops.linear_f32_many(x, w, bias, out, scratch, self.workspace, accumulate)
 
+    def decode_order(self, ctx, n_heads: int, n_kv: int, k_row: int, v_row: int, n_splits: int):
+        """The order in which the blocks of a decode step's attention start, the longest sequences first (made once for all its
+        layers), or None where all blocks run at once."""
+        if not (ctx.is_decode and ops.attention_decode_order_pays(ctx.n_tokens, n_heads, n_kv, k_row, v_row, n_splits, self.sm_count)):
+            return None
+        order = ctx.memo.get("decode_order")
+        if order is None:
+            order = ctx.memo["decode_order"] = self.empty(ctx.n_tokens, 4, dtype=torch.int32, keep=True)
+            ops.attention_decode_order(ctx.tok_seq, ctx.tok_pos, order)
+        return order
+
     def fuses_norms(self, n_tokens: int, n_out: int) -> bool:
         """Whether the bfloat16 products of a step of ``n_tokens`` rows (``n_out`` output features) may carry the norms
         around them: the few-token product always, the tensor-core product on pairs of SMs, and from 17 to 256

@@ -52,3 +52,12 @@ def test_float32_parts_are_bounded(m, n, k):
     blocks = (k + 31) // 32 * 48
     most = min(m, (1 << 26) // blocks + 256)
     assert ops.linear_f32_many_scratch_floats(m, n, k) <= (most * blocks if m >= 96 else 0) + 8 * most * n
+
+
+@pytest.mark.parametrize("n,heads,n_kv,k_row,v_row,splits,pays", [
+    (37, 32, 8, 128, 128, 1, False), (38, 32, 8, 128, 128, 1, True), (19, 32, 8, 128, 128, 2, True),        # two blocks an SM
+    (55, 16, 8, 128, 64, 1, False), (56, 16, 8, 128, 64, 1, True), (74, 16, 8, 64, 64, 1, False), (75, 16, 8, 64, 64, 1, True),
+    (74, 64, 1, 128, 128, 1, False), (75, 64, 1, 128, 128, 1, True),                                        # four blocks share a key/value head
+    (1024, 32, 8, 128, 128, 1, True), (1025, 32, 8, 128, 128, 1, False)])
+def test_decode_blocks_start_by_length(n, heads, n_kv, k_row, v_row, splits, pays):
+    assert ops.attention_decode_order_pays(n, heads, n_kv, k_row, v_row, splits, 148) is pays
