@@ -141,22 +141,28 @@ __device__ __forceinline__ float4 norm_weights_of(uint4 u, int dt, bool wide, fl
     return make_float4((pairs ? a.x : __uint_as_float(u.x)) + offset, (pairs ? a.y : __uint_as_float(u.y)) + offset,
                        (pairs ? b.x : __uint_as_float(u.z)) + offset, (pairs ? b.y : __uint_as_float(u.w)) + offset);
 }
-__device__ __forceinline__ float4 norm_weights(const void* g, int i, int dt, bool wide, float offset) {
-    return norm_weights_of(norm_weights_ahead(g, i, dt, wide), dt, wide, offset);
+// The same where they are needed.
+__device__ __forceinline__ float4 norm_weights(const void* g, int i, int dt, float offset) {
+    return make_float4(ld_f(g, 4 * i, dt) + offset, ld_f(g, 4 * i + 1, dt) + offset, ld_f(g, 4 * i + 2, dt) + offset, ld_f(g, 4 * i + 3, dt) + offset);
 }
+
+// Up to two rows an SM a norm is a chain of round trips to memory, and its kernels have few barriers and, up to 4096 lanes, ask for
+// everything at their start.  With more rows others hide the trips, and the registers cost blocks an SM (us, one barrier a sum and loads
+// ahead / neither, bfloat16 weights, 4096 lanes: a pair of norms of 8 rows 2.3 / 4.1, 200 rows 3.1 / 5.3, two norms of 8192 rows 78.9 / 42.4;
+// 8192 lanes, added to what is there, 290 rows 6.7 / 7.6, 600 rows 11.7 / 8.1).
+inline bool few_norm_rows(int n_rows) { return n_rows <= 2 * sm_count(); }
 
 // The common case, float32 rows of a width that is a multiple of 4 and at most 256 * 4 * kVec: every
 // thread keeps its part of the row in registers between the sum of squares and the scaling, so the
 // row is read once, 16 bytes at a time.
-// At a few rows a norm is a chain of round trips to memory, so all loads are asked for at its start (kAhead), the weights and what the
-// result is added to with the row.  Before it waits for its predecessor, which may have written the weights, too, a norm only asks for
-// them into L2.
-template <int kVec>
+// kFew: few_norm_rows.  kAhead: all loads are asked for at the start, the weights and what the result is added to with the row.  Before it
+// waits for its predecessor, which may have written the weights, too, a norm only asks for them into L2.
+template <int kVec, bool kFew>
 __global__ void __launch_bounds__(256)
 rmsnorm_f32_kernel(const float* __restrict__ x, const void* __restrict__ gamma, int g_dt, void* __restrict__ y,
                    int y_dt, const int* __restrict__ rows, int dim, float eps, float gamma_offset, int accumulate) {
-    constexpr bool kAhead = kVec <= 4;       // (more weights than that would cost registers of many-row steps)
-    __shared__ float part[8];
+    constexpr bool kAhead = kFew && kVec <= 4;
+    __shared__ float part[kFew ? 8 : 33];
     // launched to start while the kernel before it ends: the product that follows may set itself up meanwhile
     let_next_kernel_start();
     const int r_out = blockIdx.x;
@@ -164,15 +170,20 @@ rmsnorm_f32_kernel(const float* __restrict__ x, const void* __restrict__ gamma, 
     const bool wide = (reinterpret_cast<uintptr_t>(gamma) & 15) == 0;
     float4 v[kVec], was[kAhead ? kVec : 1];
     uint4 g[kAhead ? kVec : 1];
-    weights_into_l2(gamma, dim, g_dt);
+    if constexpr (kAhead) weights_into_l2(gamma, dim, g_dt);
     wait_for_previous_kernels();
     const int r_in = rows ? rows[r_out] : r_out;
+    float ss = 0.0f;
     if (r_in >= 0) {
         const float4* src = reinterpret_cast<const float4*>(x + (size_t)r_in * dim);
 #pragma unroll
         for (int j = 0; j < kVec; ++j) {
             const int i = threadIdx.x + j * 256;
             v[j] = i < n4 ? src[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (!kFew) {
+                ss = fmaf(v[j].x, v[j].x, ss); ss = fmaf(v[j].y, v[j].y, ss);
+                ss = fmaf(v[j].z, v[j].z, ss); ss = fmaf(v[j].w, v[j].w, ss);
+            }
         }
     } else {
 #pragma unroll
@@ -186,13 +197,16 @@ rmsnorm_f32_kernel(const float* __restrict__ x, const void* __restrict__ gamma, 
             if (accumulate && r_in >= 0 && i < n4) was[j] = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(y) + (size_t)r_out * dim)[i];
         }
     }
-    float ss = 0.0f;
+    if constexpr (kFew) {
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) {
-        ss = fmaf(v[j].x, v[j].x, ss); ss = fmaf(v[j].y, v[j].y, ss);
-        ss = fmaf(v[j].z, v[j].z, ss); ss = fmaf(v[j].w, v[j].w, ss);
+        for (int j = 0; j < kVec; ++j) {
+            ss = fmaf(v[j].x, v[j].x, ss); ss = fmaf(v[j].y, v[j].y, ss);
+            ss = fmaf(v[j].z, v[j].z, ss); ss = fmaf(v[j].w, v[j].w, ss);
+        }
+        ss = sum_of_256(ss, part);
+    } else {
+        ss = block_sum(ss, part);
     }
-    ss = sum_of_256(ss, part);
     const float scale = r_in >= 0 ? 1.0f / sqrtf(ss * (1.0f / (float)dim) + eps) : 0.0f;
 #pragma unroll
     for (int j = 0; j < kVec; ++j) {
@@ -200,8 +214,13 @@ rmsnorm_f32_kernel(const float* __restrict__ x, const void* __restrict__ gamma, 
         if (i >= n4) continue;
         float o[4] = {v[j].x * scale, v[j].y * scale, v[j].z * scale, v[j].w * scale};
         if (gamma) {
-            const float4 w = kAhead ? norm_weights_of(g[kAhead ? j : 0], g_dt, wide, gamma_offset) : norm_weights(gamma, i, g_dt, wide, gamma_offset);
-            o[0] *= w.x; o[1] *= w.y; o[2] *= w.z; o[3] *= w.w;
+            if constexpr (kFew) {
+                const float4 w = kAhead ? norm_weights_of(g[kAhead ? j : 0], g_dt, wide, gamma_offset) : norm_weights(gamma, i, g_dt, gamma_offset);
+                o[0] *= w.x; o[1] *= w.y; o[2] *= w.z; o[3] *= w.w;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) o[e] *= ld_f(gamma, 4 * i + e, g_dt) + gamma_offset;
+            }
         }
         const size_t at = (size_t)r_out * dim + 4 * i;
         if (accumulate) {          // float32 y (checked by the launcher): the norm is added to what y holds
@@ -234,7 +253,10 @@ extern "C" int nncpu_rmsnorm(const void* x, int x_dt, const void* gamma, int g_d
         cudaLaunchAttribute attr[1];
         cfg.attrs = attr;
         cfg.numAttrs = overlap_attribute(attr);
-        const auto kernel = dim <= 256 * 4 * 2 ? rmsnorm_f32_kernel<2> : dim <= 256 * 4 * 4 ? rmsnorm_f32_kernel<4> : rmsnorm_f32_kernel<8>;
+        const bool few = few_norm_rows(n_rows);
+        const auto kernel = dim <= 256 * 4 * 2   ? (few ? rmsnorm_f32_kernel<2, true> : rmsnorm_f32_kernel<2, false>)
+                            : dim <= 256 * 4 * 4 ? (few ? rmsnorm_f32_kernel<4, true> : rmsnorm_f32_kernel<4, false>)
+                                                 : (few ? rmsnorm_f32_kernel<8, true> : rmsnorm_f32_kernel<8, false>);
         const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, xf, gamma, g_dt, y, y_dt, rows, dim, eps, gamma_offset,
                                                  accumulate);
         NN_CHECK(e == cudaSuccess, "rmsnorm: launch failed: %s", cudaGetErrorString(e));
@@ -254,20 +276,22 @@ extern "C" int nncpu_rmsnorm(const void* x, int x_dt, const void* gamma, int g_d
 // b and r are float32 rows of `dim`; a thread keeps its part of the row in registers between the two sums, so
 // b and r are read once and r and y written once.  dim <= 256 * 4 * kVec, a multiple of 4.
 // ---------------------------------------------------------------------------
-template <int kVec>
+template <int kVec, bool kFew>            // as in rmsnorm_f32_kernel
 __global__ void __launch_bounds__(256)
 rmsnorm_pair_kernel(const float* __restrict__ b, float* __restrict__ r, const void* __restrict__ g1, float off1,
                     const void* __restrict__ g2, float off2, int g_dt, void* __restrict__ y, int y_dt, int dim,
                     float eps1, float eps2) {
-    constexpr bool kAhead = kVec <= 4;       // as in rmsnorm_f32_kernel
-    __shared__ float part[2][8];
+    constexpr bool kAhead = kFew && kVec <= 4;
+    __shared__ float part[kFew ? 16 : 33];
     let_next_kernel_start();
     const int row = blockIdx.x, n4 = dim >> 2;
     const bool wide = ((reinterpret_cast<uintptr_t>(g1) | reinterpret_cast<uintptr_t>(g2)) & 15) == 0;
     float4 v[kVec], was[kAhead ? kVec : 1];
     uint4 w1[kAhead ? kVec : 1], w2[kAhead ? kVec : 1];
-    weights_into_l2(g1, dim, g_dt);
-    weights_into_l2(g2, dim, g_dt);
+    if constexpr (kAhead) {
+        weights_into_l2(g1, dim, g_dt);
+        weights_into_l2(g2, dim, g_dt);
+    }
     wait_for_previous_kernels();
     float4* const stream_row = reinterpret_cast<float4*>(r + (size_t)row * dim);
     float ss = 0.0f;
@@ -280,13 +304,19 @@ rmsnorm_pair_kernel(const float* __restrict__ b, float* __restrict__ r, const vo
             w1[kAhead ? j : 0] = norm_weights_ahead(g1, i, g_dt, wide);
             w2[kAhead ? j : 0] = norm_weights_ahead(g2, i, g_dt, wide);
         }
+        if (!kFew) {
+            ss = fmaf(v[j].x, v[j].x, ss); ss = fmaf(v[j].y, v[j].y, ss);
+            ss = fmaf(v[j].z, v[j].z, ss); ss = fmaf(v[j].w, v[j].w, ss);
+        }
     }
+    if (kFew) {
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) {
-        ss = fmaf(v[j].x, v[j].x, ss); ss = fmaf(v[j].y, v[j].y, ss);
-        ss = fmaf(v[j].z, v[j].z, ss); ss = fmaf(v[j].w, v[j].w, ss);
+        for (int j = 0; j < kVec; ++j) {
+            ss = fmaf(v[j].x, v[j].x, ss); ss = fmaf(v[j].y, v[j].y, ss);
+            ss = fmaf(v[j].z, v[j].z, ss); ss = fmaf(v[j].w, v[j].w, ss);
+        }
     }
-    ss = sum_of_256(ss, part[0]);
+    ss = kFew ? sum_of_256(ss, part) : block_sum(ss, part);
     const float s1 = 1.0f / sqrtf(ss * (1.0f / (float)dim) + eps1);
     float ss2 = 0.0f;
 #pragma unroll
@@ -294,21 +324,33 @@ rmsnorm_pair_kernel(const float* __restrict__ b, float* __restrict__ r, const vo
         const int i = threadIdx.x + j * 256;
         if (i >= n4) continue;
         const float4 old = kAhead ? was[kAhead ? j : 0] : stream_row[i];
-        const float4 w = kAhead ? norm_weights_of(w1[kAhead ? j : 0], g_dt, wide, off1) : norm_weights(g1, i, g_dt, wide, off1);
-        const float o[4] = {(v[j].x * s1) * w.x, (v[j].y * s1) * w.y, (v[j].z * s1) * w.z, (v[j].w * s1) * w.w};
+        float o[4] = {v[j].x * s1, v[j].y * s1, v[j].z * s1, v[j].w * s1};
+        if constexpr (kAhead) {
+            const float4 w = norm_weights_of(w1[kAhead ? j : 0], g_dt, wide, off1);
+            o[0] *= w.x; o[1] *= w.y; o[2] *= w.z; o[3] *= w.w;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[e] *= ld_f(g1, 4 * i + e, g_dt) + off1;
+        }
         v[j] = make_float4(old.x + o[0], old.y + o[1], old.z + o[2], old.w + o[3]);
         stream_row[i] = v[j];
         ss2 = fmaf(v[j].x, v[j].x, ss2); ss2 = fmaf(v[j].y, v[j].y, ss2);
         ss2 = fmaf(v[j].z, v[j].z, ss2); ss2 = fmaf(v[j].w, v[j].w, ss2);
     }
-    ss2 = sum_of_256(ss2, part[1]);
+    ss2 = kFew ? sum_of_256(ss2, part + (kFew ? 8 : 0)) : block_sum(ss2, part);
     const float s2 = 1.0f / sqrtf(ss2 * (1.0f / (float)dim) + eps2);
 #pragma unroll
     for (int j = 0; j < kVec; ++j) {
         const int i = threadIdx.x + j * 256;
         if (i >= n4) continue;
-        const float4 w = kAhead ? norm_weights_of(w2[kAhead ? j : 0], g_dt, wide, off2) : norm_weights(g2, i, g_dt, wide, off2);
-        const float o[4] = {(v[j].x * s2) * w.x, (v[j].y * s2) * w.y, (v[j].z * s2) * w.z, (v[j].w * s2) * w.w};
+        float o[4] = {v[j].x * s2, v[j].y * s2, v[j].z * s2, v[j].w * s2};
+        if constexpr (kAhead) {
+            const float4 w = norm_weights_of(w2[kAhead ? j : 0], g_dt, wide, off2);
+            o[0] *= w.x; o[1] *= w.y; o[2] *= w.z; o[3] *= w.w;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[e] *= ld_f(g2, 4 * i + e, g_dt) + off2;
+        }
         const size_t at = (size_t)row * dim + 4 * i;
         if (y_dt == DT_BF16) {
             __nv_bfloat162 h[2] = {__floats2bfloat162_rn(o[0], o[1]), __floats2bfloat162_rn(o[2], o[3])};
@@ -328,10 +370,12 @@ extern "C" int nncpu_rmsnorm_pair(const float* b, float* r, const void* g1, floa
              "rmsnorm_pair: rows must be 16-byte aligned and the branch must not be the stream");
     if (n_rows == 0) return 0;
     cudaStream_t st = (cudaStream_t)stream;
-    if (dim <= 256 * 4) launch_overlapped(rmsnorm_pair_kernel<1>, dim3(n_rows), 256, 0, st, b, r, g1, off1, g2, off2, g_dt, y, y_dt, dim, eps1, eps2);
-    else if (dim <= 256 * 4 * 2) launch_overlapped(rmsnorm_pair_kernel<2>, dim3(n_rows), 256, 0, st, b, r, g1, off1, g2, off2, g_dt, y, y_dt, dim, eps1, eps2);
-    else if (dim <= 256 * 4 * 4) launch_overlapped(rmsnorm_pair_kernel<4>, dim3(n_rows), 256, 0, st, b, r, g1, off1, g2, off2, g_dt, y, y_dt, dim, eps1, eps2);
-    else launch_overlapped(rmsnorm_pair_kernel<8>, dim3(n_rows), 256, 0, st, b, r, g1, off1, g2, off2, g_dt, y, y_dt, dim, eps1, eps2);
+    const bool few = few_norm_rows(n_rows);      // (of more than 4096 lanes no row gains)
+    const auto kernel = dim <= 256 * 4       ? (few ? rmsnorm_pair_kernel<1, true> : rmsnorm_pair_kernel<1, false>)
+                        : dim <= 256 * 4 * 2 ? (few ? rmsnorm_pair_kernel<2, true> : rmsnorm_pair_kernel<2, false>)
+                        : dim <= 256 * 4 * 4 ? (few ? rmsnorm_pair_kernel<4, true> : rmsnorm_pair_kernel<4, false>)
+                                             : rmsnorm_pair_kernel<8, false>;
+    launch_overlapped(kernel, dim3(n_rows), 256, 0, st, b, r, g1, off1, g2, off2, g_dt, y, y_dt, dim, eps1, eps2);
     NN_LAUNCH_OK("rmsnorm_pair");
     return 0;
 }
@@ -2182,18 +2226,20 @@ rmsnorm_dual_kernel(const float* __restrict__ x, const void* __restrict__ g1, co
 
 // The common case: a width that is a multiple of 4 and at most 256 * 4 * kVec; every thread keeps its part of the row
 // in registers between the sum of squares and the two scalings, so the row is read once, 16 bytes at a time.
-template <int kVec>
+template <int kVec, bool kFew>            // as in rmsnorm_f32_kernel
 __global__ void __launch_bounds__(256)
 rmsnorm_dual_f32_kernel(const float* __restrict__ x, const void* __restrict__ g1, const void* __restrict__ g2, int g_dt,
                         float eps1, float eps2, void* __restrict__ y1, void* __restrict__ y2, int y_dt, int dim) {
-    constexpr bool kAhead = kVec <= 4;       // as in rmsnorm_f32_kernel
-    __shared__ float part[8];
+    constexpr bool kAhead = kFew && kVec <= 4;
+    __shared__ float part[kFew ? 8 : 33];
     let_next_kernel_start();
     const int n4 = dim >> 2;
     const bool wide = ((reinterpret_cast<uintptr_t>(g1) | reinterpret_cast<uintptr_t>(g2)) & 15) == 0;
     uint4 w[2][kAhead ? kVec : 1];
-    weights_into_l2(g1, dim, g_dt);
-    weights_into_l2(g2, dim, g_dt);
+    if constexpr (kAhead) {
+        weights_into_l2(g1, dim, g_dt);
+        weights_into_l2(g2, dim, g_dt);
+    }
     wait_for_previous_kernels();
     const float4* src = reinterpret_cast<const float4*>(x + (size_t)blockIdx.x * dim);
     float4 v[kVec];
@@ -2206,13 +2252,21 @@ rmsnorm_dual_f32_kernel(const float* __restrict__ x, const void* __restrict__ g1
             w[0][kAhead ? j : 0] = norm_weights_ahead(g1, i, g_dt, wide);
             w[1][kAhead ? j : 0] = norm_weights_ahead(g2, i, g_dt, wide);
         }
+        if (!kFew) {
+            ss = fmaf(v[j].x, v[j].x, ss); ss = fmaf(v[j].y, v[j].y, ss);
+            ss = fmaf(v[j].z, v[j].z, ss); ss = fmaf(v[j].w, v[j].w, ss);
+        }
     }
+    if constexpr (kFew) {
 #pragma unroll
-    for (int j = 0; j < kVec; ++j) {
-        ss = fmaf(v[j].x, v[j].x, ss); ss = fmaf(v[j].y, v[j].y, ss);
-        ss = fmaf(v[j].z, v[j].z, ss); ss = fmaf(v[j].w, v[j].w, ss);
+        for (int j = 0; j < kVec; ++j) {
+            ss = fmaf(v[j].x, v[j].x, ss); ss = fmaf(v[j].y, v[j].y, ss);
+            ss = fmaf(v[j].z, v[j].z, ss); ss = fmaf(v[j].w, v[j].w, ss);
+        }
+        ss = sum_of_256(ss, part);
+    } else {
+        ss = block_sum(ss, part);
     }
-    ss = sum_of_256(ss, part);
     const float mean = ss * (1.0f / (float)dim);
     const float s1 = 1.0f / sqrtf(mean + eps1), s2 = 1.0f / sqrtf(mean + eps2);
 #pragma unroll
@@ -2226,8 +2280,14 @@ rmsnorm_dual_f32_kernel(const float* __restrict__ x, const void* __restrict__ g1
             const void* g = which ? g2 : g1;
             void* y = which ? y2 : y1;
             const float sc = which ? s2 : s1;
-            const float4 f = kAhead ? norm_weights_of(w[which][kAhead ? j : 0], g_dt, wide, 0.0f) : norm_weights(g, i, g_dt, wide, 0.0f);
-            const float o[4] = {(in[0] * sc) * f.x, (in[1] * sc) * f.y, (in[2] * sc) * f.z, (in[3] * sc) * f.w};
+            float o[4] = {in[0] * sc, in[1] * sc, in[2] * sc, in[3] * sc};
+            if constexpr (kAhead) {
+                const float4 f = norm_weights_of(w[which][kAhead ? j : 0], g_dt, wide, 0.0f);
+                o[0] *= f.x; o[1] *= f.y; o[2] *= f.z; o[3] *= f.w;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) o[e] *= ld_f(g, 4 * i + e, g_dt);
+            }
             if (y_dt == DT_BF16) {
                 __nv_bfloat162 h[2] = {__floats2bfloat162_rn(o[0], o[1]), __floats2bfloat162_rn(o[2], o[3])};
                 *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(y) + at) = *reinterpret_cast<uint2*>(h);
@@ -2244,8 +2304,10 @@ extern "C" int nncpu_rmsnorm_dual(const float* x, const void* g1, const void* g2
     if (n_rows == 0) return 0;
     if (dim % 4 == 0 && dim >= 512 && dim <= 256 * 4 * 8 && (uintptr_t)x % 16 == 0 && (uintptr_t)y1 % 16 == 0 &&
         (uintptr_t)y2 % 16 == 0) {
-        const auto kernel = dim <= 256 * 4 * 2 ? rmsnorm_dual_f32_kernel<2> : dim <= 256 * 4 * 4 ? rmsnorm_dual_f32_kernel<4>
-                                                                                                    : rmsnorm_dual_f32_kernel<8>;
+        const bool few = few_norm_rows(n_rows);
+        const auto kernel = dim <= 256 * 4 * 2   ? (few ? rmsnorm_dual_f32_kernel<2, true> : rmsnorm_dual_f32_kernel<2, false>)
+                            : dim <= 256 * 4 * 4 ? (few ? rmsnorm_dual_f32_kernel<4, true> : rmsnorm_dual_f32_kernel<4, false>)
+                                                 : (few ? rmsnorm_dual_f32_kernel<8, true> : rmsnorm_dual_f32_kernel<8, false>);
         launch_overlapped(kernel, dim3(n_rows), 256, 0, (cudaStream_t)stream, x, g1, g2, g_dt, eps1, eps2, y1, y2, y_dt, dim);
         NN_LAUNCH_OK("rmsnorm (two outputs)");
         return 0;
