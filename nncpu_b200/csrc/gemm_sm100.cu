@@ -1869,15 +1869,16 @@ StripeShape stripe_shape(int mode, int M, int N, int K) {
 // of twice the width, half of K each (stripe_halves; clusters of up to eight blocks a tile / stripes, from 2048 x 6144 on halves:
 // 24 tokens 2048 x 2048 8.8 / 6.2, 4096 x 4096 12.1 / 10.6, 6144 x 4096 13.8 / 12.2, 2048 x 6144 11.8 / 10.5, 4096 x 12288 22.0 / 21.1,
 // 5120 x 17408 33.7 / 33.2; 64 tokens 9.7 / 6.2, 13.8 / 10.4, 15.4 / 13.0, 13.2 / 10.4, 23.8 / 22.3, 35.5 / 34.2).
-// Gated products of 33 to 64 tokens (clusters / stripes): all of short rows (64 tokens: 12288 x 2048 17.8 / 14.9, 4096 x 2560 10.7 / 9.5); of
+// Gated products of 33 to 64 tokens (clusters, or above 18 944 features whole tiles / stripes): all of short rows (64 tokens: 12288 x 2048
+// 17.8 / 14.9, 4096 x 2560 10.7 / 9.5), up to the number of features whose stripes of whole sixteens leave the SMs uneven (33 tokens of 20480 x
+// 2048 21.8 / 21.4, 24576 x 2048 23.8 / 24.6, 32768 x 2048 28.0 / 30.2, 65536 x 512 17.5 / 22.7); of
 // 3072 and 4096 lanes not those of few features, whose clusters of eight are done before a stripe has gone through K (512 x 4096 8.7
 // / 9.8, 2048 x 4096 10.1 / 10.6, 4096 x 4096 12.3 / 11.7, 512 x 3072 7.8 / 7.9, 1024 x 3072 8.4 / 8.2), nor those whose clusters fill
-// the SMs where stripes of whole sixteens do not (5120 x 4096 12.8 / 14.1, 8192 x 4096 16.8 / 17.2, 16384 x 4096 28.5 / 28.8; but 12288 x
+// the SMs where stripes do not (5120 x 4096 12.8 / 14.1, 8192 x 4096 16.8 / 17.2, 16384 x 4096 28.5 / 28.8; but 12288 x
 // 4096 25.2 / 23.5, 20480 x 4096 38.4 / 34.7, 24576 x 4096 43.6 / 40.4); nor longer rows (64 tokens of 34816 x 5120 63.5 / 64.5).  Up to 32
 // tokens clusters are as fast (24 tokens of 24576 x 4096 38.6 / 39.3).
 bool gated_stripes_pay(int N, int K) {
-    if (K <= 2560) return true;
-    if (K <= 3072) return N >= 1024;
+    if (K <= 3072) return N <= (K <= 512 ? 16384 : 20480) && (K <= 2560 || N >= 1024);
     const int tiles = (N + kBlockM - 1) / kBlockM;
     const bool fill = tiles * cluster_blocks(64, tiles, K / kBlockK) > 2 * sm_count() * 7 / 10 && tiles < sm_count();
     return K <= 4096 && N >= 2560 && (N <= 4096 || !fill);

@@ -55,7 +55,7 @@ def test_stretches(m):
     assert taken > 200
 
 
-@pytest.mark.parametrize("m,n,k,epilogue", [(24, 2048, 2048, "plain"), (64, 4096, 12288, "plain"), (64, 24576, 4096, "swiglu"),
+@pytest.mark.parametrize("m,n,k,epilogue", [(24, 2048, 2048, "plain"), (64, 4096, 12288, "plain"), (64, 24576, 4096, "swiglu"), (33, 20480, 2048, "swiglu"), (64, 12288, 512, "swiglu"),
                                             (100, 65536, 4096, "plain"), (128, 34816, 5120, "swiglu"), (200, 24576, 4096, "swiglu"),
                                             (200, 1024, 5184, "plain"), (256, 151936, 4096, "plain"), (256, 76000, 128, "plain")])
 def test_these_run_in_stripes(m, n, k, epilogue):
@@ -66,6 +66,7 @@ def test_these_run_in_stripes(m, n, k, epilogue):
 @pytest.mark.parametrize("m,n,k,epilogue", [(100, 256, 16384, "plain"), (200, 512, 12288, "plain"), (200, 4096, 17408, "plain"),
                                             (64, 512, 4096, "swiglu"), (48, 2048, 4096, "swiglu"), (40, 5120, 4096, "swiglu"),
                                             (64, 8192, 4096, "swiglu"), (33, 128, 3072, "swiglu"), (64, 24576, 4160, "swiglu"),
+                                            (64, 24576, 2048, "swiglu"), (33, 65536, 512, "swiglu"), (48, 18944, 512, "swiglu"),
                                             (24, 4096, 2048, "swiglu"), (100, 2048, 2072, "plain"), (16, 4096, 4096, "plain"),
                                             (257, 4096, 4096, "plain")])
 def test_these_do_not(m, n, k, epilogue):
