@@ -2162,9 +2162,9 @@ enum Plan : int { kPlanEvenFrom17 = 1, kPlanNeverEven = 2, kPlanNoPairs = 4, kPl
 // words, zero before the call) the exact sums of squares of C's rows; bins_clear [M, 16] (or null) is set to zero.
 // Consumer: X holds such rows of width K and bins_in [M, 16] their accumulators: the result is multiplied by
 // 1 / sqrt(sum / K + eps) per row before bias and activation.
-// From 17 to 64 tokens the same holds where nncpu_linear_tc_norm_roles says so (bit 0: may be a consumer, bit 1: may
-// be a producer): stripes do both, up to 256 tokens, the cluster kernel too (a producer with at most 16 tokens a block), the kernel of whole
-// 128-row tiles per block consumes.
+// From 17 to 256 tokens the same holds where nncpu_linear_tc_norm_roles says so (bit 0: may be a consumer, bit 1: may
+// be a producer): stripes do both; where those do not run, up to 64 tokens, the cluster kernel does both (a producer with at most 16
+// tokens a block) and the kernel of whole 128-row tiles per block consumes.  C's rows need no alignment up to 256 tokens.
 extern "C" int nncpu_linear_tc_fuses_norms(int M, int N) { return M >= 512 && N >= 512; }
 
 namespace {
@@ -2172,7 +2172,7 @@ int norm_roles(int M, int N, int K, bool stripes) {
     if (nncpu_linear_tc_fuses_norms(M, N)) return 3;
     if (M < 17 || M > 256) return 0;
     if (stripes) {
-        // below 2^22 weights a norm's own kernel, a launch like the product, does as well as norms carried for 65 tokens and more
+        // (below 2^22 weights a product of 65 tokens and more takes little longer than a norm's own kernel, and carries none)
         if (M > 64 && (long)N * K < (1l << 22)) return 0;
         return 1 | (N % 16 == 0 && (N + kBlockM - 1) / kBlockM < sm_count() ? 2 : 0);
     }
@@ -2221,7 +2221,7 @@ extern "C" int nncpu_linear_tc(const void* X, const void* W, const void* bias, i
     p.vec = ((uintptr_t)C % 16 == 0) && ((size_t)ldc * esize % 16 == 0);
     const bool stripes = plan == 0 && stripes_take(M, N, K, epilogue == kSwiglu);
     if (xg_out != nullptr || bins_in != nullptr) {
-        const int roles = plan == 0 ? norm_roles(M, N, K, stripes) : (nncpu_linear_tc_fuses_norms(M, N) && !(plan & kPlanNoPairs) ? 3 : 0);
+        const int roles = plan == 0 || plan == kPlanNoStripes ? norm_roles(M, N, K, stripes) : (nncpu_linear_tc_fuses_norms(M, N) && !(plan & kPlanNoPairs) ? 3 : 0);
         NN_CHECK((bins_in == nullptr || (roles & 1)) && (xg_out == nullptr || (roles & 2)),
                  "gemm: this product cannot carry that norm (M %d, N %d, K %d: see nncpu_linear_tc_norm_roles)", M, N, K);
         NN_CHECK(xg_out == nullptr || bins_in == nullptr, "gemm: a product is a norm's producer or its consumer");

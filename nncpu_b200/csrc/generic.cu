@@ -146,21 +146,22 @@ __device__ __forceinline__ float4 norm_weights(const void* g, int i, int dt, flo
     return make_float4(ld_f(g, 4 * i, dt) + offset, ld_f(g, 4 * i + 1, dt) + offset, ld_f(g, 4 * i + 2, dt) + offset, ld_f(g, 4 * i + 3, dt) + offset);
 }
 
-// Up to two rows an SM a norm is a chain of round trips to memory, and its kernels have few barriers and, up to 4096 lanes, ask for
+// Up to two rows an SM, four of one norm or a pair of up to 4096 lanes, a norm is a chain of round trips to memory, and its kernels have few barriers and, up to 4096 lanes, ask for
 // everything at their start.  With more rows others hide the trips, and the registers cost blocks an SM (us, one barrier a sum and loads
 // ahead / neither, bfloat16 weights, 4096 lanes: a pair of norms of 8 rows 2.3 / 4.1, 200 rows 3.1 / 5.3, two norms of 8192 rows 78.9 / 42.4;
 // 8192 lanes, added to what is there, 290 rows 6.7 / 7.6, 600 rows 11.7 / 8.1).
-inline bool few_norm_rows(int n_rows) { return n_rows <= 2 * sm_count(); }
+inline bool few_norm_rows(int n_rows, bool narrow = false) { return n_rows <= (narrow ? 4 : 2) * sm_count(); }
 
 // The common case, float32 rows of a width that is a multiple of 4 and at most 256 * 4 * kVec: every
 // thread keeps its part of the row in registers between the sum of squares and the scaling, so the
 // row is read once, 16 bytes at a time.
+// (No pointer is __restrict__ in the norms that start early: what is known to be read only may be loaded before the wait.)
 // kFew: few_norm_rows.  kAhead: all loads are asked for at the start, the weights and what the result is added to with the row.  Before it
 // waits for its predecessor, which may have written the weights, too, a norm only asks for them into L2.
 template <int kVec, bool kFew>
 __global__ void __launch_bounds__(256)
-rmsnorm_f32_kernel(const float* __restrict__ x, const void* __restrict__ gamma, int g_dt, void* __restrict__ y,
-                   int y_dt, const int* __restrict__ rows, int dim, float eps, float gamma_offset, int accumulate) {
+rmsnorm_f32_kernel(const float* x, const void* gamma, int g_dt, void* y,
+                   int y_dt, const int* rows, int dim, float eps, float gamma_offset, int accumulate) {
     constexpr bool kAhead = kFew && kVec <= 4;
     __shared__ float part[kFew ? 8 : 33];
     // launched to start while the kernel before it ends: the product that follows may set itself up meanwhile
@@ -253,7 +254,7 @@ extern "C" int nncpu_rmsnorm(const void* x, int x_dt, const void* gamma, int g_d
         cudaLaunchAttribute attr[1];
         cfg.attrs = attr;
         cfg.numAttrs = overlap_attribute(attr);
-        const bool few = few_norm_rows(n_rows);
+        const bool few = few_norm_rows(n_rows, dim <= 4096);
         const auto kernel = dim <= 256 * 4 * 2   ? (few ? rmsnorm_f32_kernel<2, true> : rmsnorm_f32_kernel<2, false>)
                             : dim <= 256 * 4 * 4 ? (few ? rmsnorm_f32_kernel<4, true> : rmsnorm_f32_kernel<4, false>)
                                                  : (few ? rmsnorm_f32_kernel<8, true> : rmsnorm_f32_kernel<8, false>);
@@ -278,8 +279,8 @@ extern "C" int nncpu_rmsnorm(const void* x, int x_dt, const void* gamma, int g_d
 // ---------------------------------------------------------------------------
 template <int kVec, bool kFew>            // as in rmsnorm_f32_kernel
 __global__ void __launch_bounds__(256)
-rmsnorm_pair_kernel(const float* __restrict__ b, float* __restrict__ r, const void* __restrict__ g1, float off1,
-                    const void* __restrict__ g2, float off2, int g_dt, void* __restrict__ y, int y_dt, int dim,
+rmsnorm_pair_kernel(const float* b, float* r, const void* g1, float off1,
+                    const void* g2, float off2, int g_dt, void* y, int y_dt, int dim,
                     float eps1, float eps2) {
     constexpr bool kAhead = kFew && kVec <= 4;
     __shared__ float part[kFew ? 16 : 33];
@@ -370,7 +371,7 @@ extern "C" int nncpu_rmsnorm_pair(const float* b, float* r, const void* g1, floa
              "rmsnorm_pair: rows must be 16-byte aligned and the branch must not be the stream");
     if (n_rows == 0) return 0;
     cudaStream_t st = (cudaStream_t)stream;
-    const bool few = few_norm_rows(n_rows);      // (of more than 4096 lanes no row gains)
+    const bool few = few_norm_rows(n_rows, true);      // (of more than 4096 lanes no row gains)
     const auto kernel = dim <= 256 * 4       ? (few ? rmsnorm_pair_kernel<1, true> : rmsnorm_pair_kernel<1, false>)
                         : dim <= 256 * 4 * 2 ? (few ? rmsnorm_pair_kernel<2, true> : rmsnorm_pair_kernel<2, false>)
                         : dim <= 256 * 4 * 4 ? (few ? rmsnorm_pair_kernel<4, true> : rmsnorm_pair_kernel<4, false>)
@@ -2228,8 +2229,8 @@ rmsnorm_dual_kernel(const float* __restrict__ x, const void* __restrict__ g1, co
 // in registers between the sum of squares and the two scalings, so the row is read once, 16 bytes at a time.
 template <int kVec, bool kFew>            // as in rmsnorm_f32_kernel
 __global__ void __launch_bounds__(256)
-rmsnorm_dual_f32_kernel(const float* __restrict__ x, const void* __restrict__ g1, const void* __restrict__ g2, int g_dt,
-                        float eps1, float eps2, void* __restrict__ y1, void* __restrict__ y2, int y_dt, int dim) {
+rmsnorm_dual_f32_kernel(const float* x, const void* g1, const void* g2, int g_dt,
+                        float eps1, float eps2, void* y1, void* y2, int y_dt, int dim) {
     constexpr bool kAhead = kFew && kVec <= 4;
     __shared__ float part[kFew ? 8 : 33];
     let_next_kernel_start();

@@ -141,13 +141,14 @@ def test_xielu_both_branches_and_soft_cap():
 
 
 @pytest.mark.parametrize("m", [1, 8, 16, 17, 40, 64, 100, 256, 300, 600, 1100])
-def test_xielu_in_the_epilogue_of_the_tensor_core_products(m):
-    """Every product kernel (few tokens, cluster, stream-K, persistent, pairs of SMs) with the activation on its
-    accumulators, against the product in float32 followed by the activation's own kernel."""
+@pytest.mark.parametrize("k", [192, 264])
+def test_xielu_in_the_epilogue_of_the_tensor_core_products(m, k):
+    """Every product kernel (few tokens, stripes, persistent, pairs of SMs; with K no multiple of 64 cluster and stream-K in place of
+    stripes) with the activation on its accumulators, against the product in float32 followed by the activation's own kernel."""
     from nncpu_b200.parts import Runtime
     rt = Runtime(DEV, torch.bfloat16)
     g = torch.Generator().manual_seed(m)
-    k, n = 192, 328
+    n = 328
     x = (torch.randn(m, k, generator=g) * 2).bfloat16().to(DEV)
     w = (torch.randn(n, k, generator=g) * 0.2).bfloat16().to(DEV)
     bias = torch.randn(n, generator=g).bfloat16().to(DEV)
