@@ -599,9 +599,9 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 // their partial tiles: each block writes its own to scratch memory, and a
 // second, wide kernel adds a tile's parts in block order (the order of k) and
 // runs the epilogue.  No block waits for another, and the sum does
-// not depend on timing.  Used for 65 to 256 tokens (from 17 on where the plan
-// asks for it; weights are the 128-row operand), where tiles are few and K is
-// long.
+// not depend on timing.  Used for the products of 65 to 256 tokens that do not
+// run in stripes (from 17 on where the plan asks for it; weights are the
+// 128-row operand), where tiles are few and K is long.
 // ---------------------------------------------------------------------------
 struct Segment {
     int tile, kb0, len;

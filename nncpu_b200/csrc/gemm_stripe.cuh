@@ -20,9 +20,10 @@
 // stripes are narrower and a block walks through K for several of them, with two sets of accumulators in turn (us and error, one accumulator / two;
 // 200 tokens: gated 24576 x 4096 57 / 62, 8.9e-6 / 4.3e-6, 65536 x 4096 111 / 121, 4.4e-6 / 2.1e-6; dealt-out k-blocks 69 and 4.5e-6, 173 and 3.7e-6).
 //
-// What bounds it (times at the rule that sends a product here): the instructions, of which a block issues one for 16 columns of
-// K whatever the width of its stripe, some 45 clk each at N 16 to 64, and some 0.14 us a stage; the weights' stream at the
-// larger widths (gated 24 576 x 4 096 at 64 tokens 40.6 us, 5.0 TB/s).  Neither where a unit begins its walk through K (all SMs
+// What bounds it (times at the rule that sends a product here): up to 64 tokens the instructions, of which a block issues one for 16
+// columns of K whatever the width of its stripe (some 45 clk each at N 16 to 64, from the times of different widths; issued back to back
+// and without a stage's wait they take 24), and some 0.14 us a stage; the weights' stream at the
+// larger widths (gated 24 576 x 4 096 at 64 tokens 40.4 us, 5.0 TB/s); above 64 tokens the tokens that every SM copies beside its weights.  Neither where a unit begins its walk through K (all SMs
 // read the same tokens at one time) nor copies by a warp for each operand made a difference.
 #pragma once
 

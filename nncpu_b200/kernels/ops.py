@@ -117,9 +117,11 @@ def launch_overlap(on: bool) -> None:
     """Whether kernels that can do so are launched to start while the kernel before them ends: a few-token
     product after a kernel of little shared memory and the float32 products of few rows (they ask for their first weights
     before they wait for that one's results), the tensor-core products (their set-up; up to 64 bfloat16 tokens also their first
-    weight tiles), prefill attention (its set-up), float32 attention token by token, the norms and the small kernels of routers,
+    weight tiles; above, and for float32 products of 96 tokens and more and the norms, the first weights go into L2 only), prefill attention (its set-up), float32 attention token by token, the norms and the small kernels of routers,
     routed experts, gates and the stream between them.
-    On by default; off, every kernel waits for the one before it to be over, and the results are the same bits."""
+    On by default; off, every kernel waits for the one before it to be over, and the results are the same bits.  Where a product
+    asks for its first weights themselves, the kernel of this library right before it in the stream must not be the one that
+    writes them."""
     for name in ("linear_skinny", "gemm_sm100", "generic", "attention_tc", "linear_f32", "attention_f32"):
         getattr(library.load(name), f"nncpu_launch_overlap_{name}")(ctypes.c_int(1 if on else 0))
 
@@ -388,7 +390,7 @@ def linear_tc_norm_roles(m: int, n: int, k: int) -> int:
     """Which norms the tensor-core product of ``m`` tokens, ``n`` output features and width ``k`` can carry: bit 0 the
     norm before it (``norm_in``), bit 1 the norm after it (``norm_out``).  Whole prompts both; 17 to 64 tokens the
     norm before, and the norm after where a cluster shares every output tile or the weights go in stripes; 65 to 256 tokens
-    both where the weights go in stripes and are many."""
+    both where the weights go in stripes and are 2^22 or more (the norm after only below 18 817 features)."""
     return int(library.load("gemm_sm100").nncpu_linear_tc_norm_roles(m, n, k))
 
 
@@ -406,7 +408,7 @@ def linear_tc(x, w, bias, out, workspace: GemmWorkspace, accumulate: bool = Fals
     """out (+)= x . w^T + bias on the tensor cores; x and w bfloat16.  With
     ``epilogue="swiglu"`` the rows of w hold gate and up rows interleaved in
     blocks of 8 and out [m, n/2] receives silu(gate) * up.  ``plan``: "auto",
-    or for measurements and tests "no_stripes" (17 to 256 tokens never as stripes of the weights), "even_from_17" (17 to 64
+    or for measurements and tests "no_stripes" (17 to 256 tokens never as stripes of the weights; norms as the kernels that run then can), "even_from_17" (17 to 64
     tokens deal their k-blocks out evenly like 65 to 256 without stripes), "never_even", "no_pairs".
 
     Where ``linear_tc_norm_roles(m, n, k)`` says so, the product can carry the RMS norms around it as

@@ -155,9 +155,9 @@ class Runtime:
         weights or more, in rows that are not too short, by the kernels made for them (few rows: CUDA cores; more: tensor cores on numbers cut in
         three, of which nothing is lost), the rest on CUDA cores by the general kernel.
 
-        ``x`` may be a ``DeferredNorm`` (a norm's unfinished output): the few-token product and the product of
-        whole prompts finish it, any other path makes the ordinary tensor first.  ``then_norm`` (a ``NormRequest``):
-        this product is the last write into ``out`` before that norm reads it; the same two products fulfil it.
+        ``x`` may be a ``DeferredNorm`` (a norm's unfinished output): the few-token product and the tensor-core products that
+        ``ops.linear_tc_norm_roles`` names finish it, any other path makes the ordinary tensor first.  ``then_norm`` (a
+        ``NormRequest``): this product is the last write into ``out`` before that norm reads it; such products fulfil it.
         ``activation`` (("xielu", a, b), see ``ops.linear_tc``): applied in the product's epilogue on its 32-bit
         accumulators; only where ``tensor_cores_take`` says the product runs on the tensor cores."""
         deferred = x if isinstance(x, DeferredNorm) else None
